@@ -858,6 +858,8 @@ class Accumulator {
     terms_.enabled = shared_destination(all.data(), all.size(), d) ? 1 : 0;
     terms_.propagation = propagation_;
     terms_.destination = d;
+    terms_.limits = widest_limits();
+    narrow_limits(all.data(), all.size(), terms_.limits);
   }
 
   void allocate_traces() {

@@ -134,11 +134,13 @@ void upload(UploadBlock const& block, void* out, std::size_t bytes, cudaStream_t
 }
 
 // Whether every observer seen shares one destination row (the ingest then
-// writes each track's source terms).
+// writes each track's source terms), and the track limits of all of them.
 struct SharedDestination {
   bool any = false, shared = true;
   c8r::Destination row{};
+  c8r::TrackLimits limits = c8r::widest_limits();
   void see(ObserverCache const& o) {
+    c8r::narrow_limits(&o, 1, limits);
     c8r::Destination d{};
     if (!c8r::shared_destination(&o, 1, d)) return;
     if (!any) {
@@ -301,6 +303,7 @@ void accumulate_no_alloc(c8r_config const& config, c8r_lepton_transport_record c
   terms.enabled = destination.any && destination.shared ? 1 : 0;
   terms.propagation = prop;
   terms.destination = destination.row;
+  terms.limits = destination.limits;
   ev.precomputed = static_cast<uint32_t>(terms.enabled);
 
   // records in chunks of at most kTrackCapacity: ingest into the scratch

@@ -454,9 +454,8 @@ __device__ __forceinline__ Track study_track(const double* base, uint64_t i) {
   t.bx = track_field(base, i, kBx);
   t.by = track_field(base, i, kBy);
   t.bz = track_field(base, i, kBz);
-  t.length = track_field(base, i, kLen);
-  t.beta_module = track_field(base, i, kBmod);
   t.constant = track_field(base, i, kConst);
+  derive_track(t);
   return t;
 }
 

@@ -71,20 +71,30 @@ struct Track {
   double length, beta_module, constant;
 };
 
-// Track workspace: a record of 24 doubles (192 bytes) per track.  The first
-// 16: start xyz, end xyz, t_start, t_end, beta xyz, length, |beta|, charge
-// constant, n_dst at the start point, one spare.  When every observer of the
-// event shares one destination row (SourceTerms below), the last 8 hold the
-// propagation terms of four source points, precomputed at ingest -- start,
-// end, the ZHS segment midpoint (start + (start + (end - start))) / 2 and the
-// CoREAS near-cone midpoint (start + end) / 2, each as (factor, n_src).
-// Records are stored in tiles (track_column below).
+// Track workspace: a record of 24 doubles (192 bytes) per track: start xyz,
+// end xyz, t_start, t_end, beta xyz, a packed word (below), the propagation
+// terms (factor, n_src; SourceTerms below) of the start, the end and the ZHS
+// segment midpoint when every observer of the event shares one destination
+// row, that midpoint (start + (start + (end - start))) / 2, the time in the
+// middle of the segment, half its duration, and the charge constant.  The
+// length and |beta| are recomputed from the fields where an exact evaluation
+// needs them (load_track: the same IEEE operations as at ingest).  Records are
+// stored in tiles (track_column below).
 enum TrackField : int {
-  kSx = 0, kSy, kSz, kEx, kEy, kEz, kTs, kTe, kBx, kBy, kBz, kLen, kBmod, kConst, kNdstStart, kSpare,
-  kFactorStart, kNsrcStart, kFactorEnd, kNsrcEnd, kFactorMidZhs, kNsrcMidZhs, kFactorMidCoreas,
-  kNsrcMidCoreas, kTrackDoubles
+  kSx = 0, kSy, kSz, kEx, kEy, kEz, kTs, kTe, kBx, kBy, kBz, kPack,
+  kFactorStart, kNsrcStart, kFactorEnd, kNsrcEnd, kFactorMid, kNsrcMid,
+  kMx, kMy, kMz, kTm, kHalf, kConst, kTrackDoubles
 };
 static_assert(kTrackDoubles == 24, "192-byte track records");
+
+// The packed word: the charge constant rounded to FP32 in its low half, and
+// in its high half what ingest found out about the track:
+//   kTrackRegular  the magnitudes for which the error bounds of the filtered
+//                  decisions below are written out hold (regular_track)
+//   kTrackDense    n_dst > 1 at the start point (shared destination row only)
+//   kTrackOneMid   the CoREAS near-cone midpoint (start + end) / 2 has the
+//                  source terms of the ZHS segment midpoint
+constexpr unsigned kTrackRegular = 1u, kTrackDense = 2u, kTrackOneMid = 4u;
 
 // The workspace holds tiles of kTrackTile consecutive tracks (6144 bytes): in
 // a tile, column k of the records (doubles 2k and 2k + 1, one 16-byte double2)
@@ -115,6 +125,14 @@ __host__ __device__ __forceinline__ double track_field(double const* base, uint6
 // Tracks a workspace for n tracks holds: n rounded up to whole tiles.
 __host__ __device__ constexpr uint64_t track_capacity(uint64_t n) {
   return (n + kTrackTile - 1) / kTrackTile * kTrackTile;
+}
+
+// Length and |beta| as make_radio_track_kinematics evaluates them
+// (RadioProjection.inl:145-168), from the track's other fields.
+__device__ __forceinline__ void derive_track(Track& t) {
+  double const dx = t.ex - t.sx, dy = t.ey - t.sy, dz = t.ez - t.sz;
+  t.length = sqrt(dx * dx + dy * dy + dz * dz);
+  t.beta_module = t.length / (kSpeedOfLight * (t.te - t.ts));
 }
 
 struct Path {
@@ -260,54 +278,104 @@ __device__ __forceinline__ Path propagate(Propagation const& p, ObserverCache co
   return propagate_with<kTime, kApproxDirection>(st, o, sx, sy, sz);
 }
 
-// propagate (RadioProjection.inl:170-238) for the filtered decisions of the
-// mixed-precision path.  The refractive indices and the integral ratio
-// (i_src - i_dst) / height are the reference's (same table reads, same IEEE
-// division); 1/|d| is an FP32 reciprocal square root refined by two Newton
-// steps in FP64, |d| = RN(|d|^2 (1/|d|)), k = d (1/|d|), and the travel time
-// multiplies by RN(1/c) instead of dividing by c.  With the final Newton
-// residual r = 1 - |d|^2 y^2, y lies within |r|/2 + u of 1/|d| (u = 2^-53);
-// `ok` requires |r| <= 2^-50, so y is within 5u, each direction component
-// within 8u |k| of the reference's, and the time within 12u |time|
-// (|d| within 7u, two products and RN(1/c) against one division):
-// `time_err` = 2^-48 |time| (32u).  `ok` is false (the caller evaluates
-// exactly) when |d|^2 lies outside [2^-100, 2^100], the residual is larger or
-// the time is not finite.
-struct FastPath {
-  double time, n_src, n_dst, dist, kx, ky, kz, time_err;
-  bool ok;
+// ---------------------------------------------------------------- filtered paths
+// The mixed-precision kernels evaluate distances, detection times and Doppler
+// factors with a few FP64 operations each, in units of the observer's bins,
+// and take a decision (a bin, a branch, an order) only where a fixed guard
+// shows that the reference's own arithmetic takes the same one; any other pair
+// or segment is evaluated exactly, operation by operation.  The guards hold
+// for "regular" tracks, whose magnitudes ingest has checked (regular_track):
+//
+//   |beta|_1 <= 4, 0 < n <= 4 at the source points; every time t of the track
+//   has (|t| + |t0|) fs <= 2^26 bins at every observer of the event, and the
+//   track lasts at most 2^21 bins (TrackLimits).
+//
+// With u = 2^-53, for a source point at displacement d from the observer
+// (the reference's own subtractions):
+//   s2 = d.d (one product, two fused adds) is within 2u of |d|^2 where the
+//   reference's is within 3u; y from lean_rsqrt is within 4u of 1/sqrt(s2);
+//   so |d| = RN(s2 y) is within 7u of the reference's and k = d y within 8u.
+//   w = beta.k and n w lie within 16 u n |beta|_1 <= 2^-45 of the reference's,
+//   hence 1 - n w within kDopplerGuard = 2^-43.
+//   A detection time in bins, x = (t - t0) fs + |d| factor fs / c, lies within
+//   32u (|t| + |t0| + time) fs of the reference's (t + time - t0) fs; where x
+//   falls on the trace (fewer than 2^26 bins) that is below 32u 2^28 = 2^-20,
+//   and the ZHS term n w (t - t_mid) adds at most 2^-43 2^20; kBinGuard =
+//   2^-19 covers both.  Where |x| is larger the error grows like 2^-46 |x|, so
+//   such an x is off the trace in the reference as well.
+constexpr double kDopplerGuard = 0x1p-43;
+constexpr double kBinGuard = 0x1p-19;
+constexpr double kMaxLeanBins = 67108864.0;  // 2^26
+
+// Limits on a track's times (s), from every observer of the event.
+struct TrackLimits {
+  double time = 0.;      // |t_start|, |t_end| at most this
+  double duration = 0.;  // t_end - t_start at most this
 };
 
-__device__ __forceinline__ FastPath propagate_fast_with(SourceTerms const& st, double ox, double oy, double oz,
-                                                        double sx, double sy, double sz) {
-  FastPath r;
-  double const dx = ox - sx, dy = oy - sy, dz = oz - sz;
-  double const s2 = dx * dx + dy * dy + dz * dz;
-  r.ok = s2 >= 0x1p-100 && s2 <= 0x1p100;
-  double y = static_cast<double>(rsqrtf(static_cast<float>(r.ok ? s2 : 1.)));
-#pragma unroll
-  for (int step = 0; step < 2; ++step) {
-    double const h = s2 * y;
-    y = fma(0.5 * y, fma(-h, y, 1.), y);
-  }
-  double const dist = s2 * y;
-  r.ok = r.ok && fabs(fma(-dist, y, 1.)) <= 0x1p-50;
-  r.kx = dx * y;
-  r.ky = dy * y;
-  r.kz = dz * y;
-  r.dist = dist;
-  constexpr double kInverseC = 1. / kSpeedOfLight;
-  r.time = st.factor * dist * kInverseC;
-  r.n_src = st.n_src;
-  r.n_dst = st.n_dst;
-  r.time_err = 0x1p-48 * fabs(r.time);
-  r.ok = r.ok && r.time_err < 1.e300;  // false for infinite or NaN times
-  return r;
+__device__ __forceinline__ bool lean_index(double n) { return (n > 0.) & (n <= 4.); }
+
+// 1/sqrt(s2) from the hardware's approximate reciprocal square root (about 20
+// bits) and one third-order step: with r = 1 - s2 y0^2 and |r| <= 2^-17
+// (checked, so the seed's accuracy is not relied on), y0 (1 + r/2 + 3 r^2/8)
+// is within (5/16) 2^-51 + 3u < 4u of it.  False when s2 lies outside
+// [2^-100, 2^100] or is not a number.
+__device__ __forceinline__ bool lean_rsqrt(double s2, double& y) {
+  double seed;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(seed) : "d"(s2));
+  double const r = fma(-(s2 * seed), seed, 1.);
+  y = fma(seed * r, fma(r, 0.375, 0.5), seed);
+  unsigned const high = static_cast<unsigned>(__double2hiint(s2)) - 0x39b00000u;  // 2^-100
+  return (fabs(r) <= 0x1p-17) & (high <= 0x46300000u - 0x39b00000u);               // 2^100
 }
 
-__device__ __forceinline__ FastPath propagate_fast(Propagation const& p, ObserverCache const& o,
-                                                   double sx, double sy, double sz) {
-  return propagate_fast_with(source_terms(p, destination_of(o), sz), o.px, o.py, o.pz, sx, sy, sz);
+// The nearest integer of x (|x| < 2^31 where the result is used) as `bin`, and
+// x minus it, in [-1/2, 1/2]: x + 1.5 2^52 rounds to an integer whose low word
+// is the integer's.
+__device__ __forceinline__ double lean_nearest(double x, int& bin) {
+  constexpr double kRound = 6755399441055744.0;  // 1.5 2^52
+  double const shifted = x + kRound;
+  bin = __double2loint(shifted);
+  return x - (shifted - kRound);
+}
+
+// The FP32 charge constants carry 2^60 and the observers' scales 2^-60, so
+// that neither leaves the FP32 range for any field limit whose fixed-point
+// scale is an FP32 number itself.
+constexpr double kConstantShift = 0x1p60;
+
+// Constants of the item's observer for the filtered paths, derived once per
+// work item from its ObserverCache.
+struct LeanObserver {
+  double rate;         // fs
+  double rate_over_c;  // fs / c
+  double half_rate;    // fs / 2
+  double gate_in;      // a CoREAS sample at kBinGuard < x < gate_in is recorded,
+  double gate_out;     // one at x < -kBinGuard or x > gate_out is not
+  double start_bins;   // t0 fs
+  double fraunhofer;   // 8 pi c^2 / (wavelength fs^2)
+  float scale;         // 2^-60 x fixed-point scale (x fs, CoREAS); 0 when counting samples
+  float bias;          // 1 when counting samples, else 0
+  uint32_t usable;     // the filtered paths may be used for this observer
+};
+
+template <int kAlgorithm>
+__device__ __forceinline__ void make_lean_observer(ObserverCache const& o, LeanObserver& l) {
+  double const fs = o.sample_rate;
+  l.rate = fs;
+  l.rate_over_c = fs / kSpeedOfLight;
+  l.half_rate = 0.5 * fs;
+  double const end = (o.end_time - o.start_time) * fs;
+  double const last = o.bins_d - 0.5;
+  double const gate = end < last ? end : last;
+  l.gate_in = gate - kBinGuard;
+  l.gate_out = gate + kBinGuard;
+  l.start_bins = o.start_time * fs;
+  l.fraunhofer = 8. * kPi * (kSpeedOfLight / fs) * (kSpeedOfLight / fs) / o.wavelength;
+  double const scale = (kAlgorithm == 0 ? fs * o.fixed_scale : o.fixed_scale) / kConstantShift;
+  l.scale = o.count_samples ? 0.f : static_cast<float>(scale);
+  l.bias = o.count_samples ? 1.f : 0.f;
+  l.usable = o.bins_d < kMaxLeanBins && fs < 0x1p200 ? 1u : 0u;
 }
 
 // separate_same_bin_endpoints, RadioProjection.inl:303-336.

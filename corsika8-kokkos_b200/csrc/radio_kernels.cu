@@ -351,60 +351,23 @@ __device__ __forceinline__ void coreas_pair(Track const& t, Propagation const& p
   add_sample<false, kFixed>(o, sink, er, fend, c.coreas, c.overflows, c.mag);
 }
 
-// The propagation of the filtered paths: propagate_fast when kFast, else the
-// exact propagate (time_err 0).  kPre: the point's source terms are `pre`
-// (precomputed at ingest), else they are looked up in the table.
-template <bool kFast, bool kPre = false>
-__device__ __forceinline__ FastPath filtered_path(Propagation const& p, ObserverCache const& o,
-                                                  double x, double y, double z,
-                                                  SourceTerms const& pre = SourceTerms{}) {
-  SourceTerms const st = kPre ? pre : source_terms(p, destination_of(o), z);
-  if (kFast) return propagate_fast_with(st, o.px, o.py, o.pz, x, y, z);
-  Path const e = propagate_with<true>(st, o, x, y, z);
-  return FastPath{e.time, e.n_src, e.n_dst, e.dist, e.kx, e.ky, e.kz, 0., true};
-}
-
-// The common CoREAS pair of the windowed kernel (RadioProjection.inl:339-409
-// without its near-Cherenkov branch).  Returns false, having deposited
-// nothing, when the pair needs the near-Cherenkov branch or (kFilter) an exact
-// evaluation; the kernel then defers it to coreas_drain_pair.
-//
-// kFilter (mixed precision): travel times, refractive indices and distances
-// are exact; emission directions are d * RN(1/|d|) (propagate's
-// kApproxDirection), so each Doppler factor 1 - n beta.k lies within
-// 14 u n |beta|_1 + 2 u of the reference's (u = 2^-53; used below with a 4.5x
-// margin).  The branches (near-Cherenkov |doppler| < 1e-3, the sign test
-// doppler < 1e-9) are taken here only when that bound cannot move them, and
-// pairs with |doppler| < 1e-6 are left to the exact evaluation.  Sample times
-// are exact, so bins are the reference's.  Returns kCoreasDeposited, or the
-// deferral: kCoreasExact, or kCoreasNearCone with bit 0 the branch's
-// start-before-end order (sr < er, exact times), both decided exactly, so the
+// What became of a pair in the windowed CoREAS track loop: deposited, or
+// deferred to coreas_drain_pair -- kCoreasExact, or kCoreasNearCone with bit 0
+// the branch's start-before-end order (sr < er), both decided exactly, so the
 // drain evaluates only the near-Cherenkov branch itself.
 constexpr int kCoreasDeposited = 0, kCoreasExact = 1, kCoreasNearCone = 2;
-template <bool kFixed, bool kFilter, bool kPre, class Amp, class Sink>
+
+// The common CoREAS pair of the windowed kernel (RadioProjection.inl:339-409
+// without its near-Cherenkov branch), evaluated exactly.  Deposits nothing
+// when it defers.
+template <bool kFixed, bool kPre, class Amp, class Sink>
 __device__ __forceinline__ int coreas_common(Track const& t, Propagation const& p,
                                               ObserverCache const& o, Sink& sink, Counts& c,
                                               SourceTerms const& pre_start, SourceTerms const& pre_end) {
-  Path const ps = kPre ? propagate_with<true, kFilter>(pre_start, o, t.sx, t.sy, t.sz)
-                       : propagate<true, kFilter>(p, o, t.sx, t.sy, t.sz);
-  Path const pe = kPre ? propagate_with<true, kFilter>(pre_end, o, t.ex, t.ey, t.ez)
-                       : propagate<true, kFilter>(p, o, t.ex, t.ey, t.ez);
-  double pre, post;
-  if (kFilter) {
-    pre = 1. - ps.n_src * (t.bx * ps.kx + t.by * ps.ky + t.bz * ps.kz);
-    post = 1. - pe.n_src * (t.bx * pe.kx + t.by * pe.ky + t.bz * pe.kz);
-    double const beta1 = fabs(t.bx) + fabs(t.by) + fabs(t.bz) + 1.;
-    double const err_pre = ps.n_src * beta1 * 0x1p-47 + 0x1p-50;
-    double const err_post = pe.n_src * beta1 * 0x1p-47 + 0x1p-50;
-    bool const ambiguous =
-        fabs(pre) < 1.e-6 || fabs(post) < 1.e-6 ||
-        (ps.n_dst > 1. && (fabs(fabs(pre) - kCoreasThreshold) <= err_pre ||
-                           fabs(fabs(post) - kCoreasThreshold) <= err_post));
-    if (ambiguous) return kCoreasExact;
-  } else {
-    pre = doppler(ps.n_src, t.bx, t.by, t.bz, ps.kx, ps.ky, ps.kz);
-    post = doppler(pe.n_src, t.bx, t.by, t.bz, pe.kx, pe.ky, pe.kz);
-  }
+  Path const ps = kPre ? propagate_with<true>(pre_start, o, t.sx, t.sy, t.sz) : propagate<true>(p, o, t.sx, t.sy, t.sz);
+  Path const pe = kPre ? propagate_with<true>(pre_end, o, t.ex, t.ey, t.ez) : propagate<true>(p, o, t.ex, t.ey, t.ez);
+  double const pre = doppler(ps.n_src, t.bx, t.by, t.bz, ps.kx, ps.ky, ps.kz);
+  double const post = doppler(pe.n_src, t.bx, t.by, t.bz, pe.kx, pe.ky, pe.kz);
   double sr = t.ts + ps.time;
   double er = t.te + pe.time;
   if (ps.n_dst > 1. && (fabs(pre) < kCoreasThreshold || fabs(post) < kCoreasThreshold))
@@ -417,7 +380,6 @@ __device__ __forceinline__ int coreas_common(Track const& t, Propagation const& 
       scaled(cross(ks, cross(ks, beta)), amp_div(static_cast<Amp>(cf), static_cast<Amp>(pre * ps.dist)));
   Vec3<Amp> fend =
       scaled(cross(ke, cross(ke, beta)), amp_div(static_cast<Amp>(-cf), static_cast<Amp>(post * pe.dist)));
-  // with the filter |pre|, |post| >= 1e-6, so "< 1e-9" is the sign of the factor
   if (pre < 1.e-9 || post < 1.e-9) {
     double const res = o.resolution;
     double const dt = er - sr;
@@ -431,6 +393,219 @@ __device__ __forceinline__ int coreas_common(Track const& t, Propagation const& 
   add_sample<false, kFixed>(o, sink, sr, fstart, c.coreas, c.overflows, c.mag);
   add_sample<false, kFixed>(o, sink, er, fend, c.coreas, c.overflows, c.mag);
   return kCoreasDeposited;
+}
+
+// The packed word's flags (kTrackRegular, ...) and FP32 constant.
+__device__ __forceinline__ unsigned pack_flags(double pack) {
+  return static_cast<unsigned>(__double2hiint(pack));
+}
+// n_dst as the projection looks at it: above 1 or not.
+__device__ __forceinline__ double dense_index(unsigned flags) { return (flags & kTrackDense) ? 2. : 1.; }
+__device__ __forceinline__ float pack_constant(double pack) { return __int_as_float(__double2loint(pack)); }
+
+// One endpoint (or midpoint) of a track seen from an observer, for the
+// filtered paths: distance, detection time in bins, Doppler factor 1 - n w and
+// w / |d|, from which k (k.beta) - beta = d (w / |d|) - beta.
+struct LeanPoint {
+  double dx, dy, dz, dist, inverse, x, w, factor, along;
+  bool ok;
+};
+__device__ __forceinline__ LeanPoint lean_point(ObserverCache const& o, LeanObserver const& l, double sx, double sy,
+                                                double sz, double t, double bx, double by, double bz,
+                                                double factor, double index) {
+  LeanPoint r;
+  r.dx = o.px - sx;
+  r.dy = o.py - sy;
+  r.dz = o.pz - sz;
+  double const s2 = fma(r.dz, r.dz, fma(r.dy, r.dy, r.dx * r.dx));
+  r.ok = lean_rsqrt(s2, r.inverse);
+  r.dist = s2 * r.inverse;
+  r.x = fma(r.dist, factor * l.rate_over_c, (t - o.start_time) * l.rate);
+  r.w = fma(bz, r.dz, fma(by, r.dy, bx * r.dx)) * r.inverse;
+  r.factor = fma(-index, r.w, 1.);
+  r.along = r.w * r.inverse;
+  return r;
+}
+
+// separate_same_bin_endpoints (RadioProjection.inl:303-336) in bins.  `u` =
+// x + t0 fs is the absolute time start / res; with the fraction of `u` at or
+// above one half exactly when its nearest-integer remainder r is negative, the
+// reference's cases reduce to the sign of the two remainders' sum: `high`
+// (the end in forward order) moves on where it is not negative, else `low`
+// moves back.  False when a guard cannot decide.
+__device__ __forceinline__ bool lean_separate(double& low, double& high, LeanObserver const& l) {
+  double const ul = low + l.start_bins, uh = high + l.start_bins;
+  int bl, bh;
+  double const rl = lean_nearest(ul, bl), rh = lean_nearest(uh, bh);
+  if (!(fabs(ul) < 0x1p30 && fabs(uh) < 0x1p30 && fabs(rl) < 0.5 - kBinGuard && fabs(rh) < 0.5 - kBinGuard))
+    return false;
+  if (bl != bh) return true;
+  double const sum = rl + rh;
+  if (fabs(sum) < 2. * kBinGuard) return false;
+  if (sum > 0.)
+    high += 1.;
+  else
+    low -= 1.;
+  return true;
+}
+
+// Where a CoREAS sample at x bins goes: its bin, no bin (`in` false), or
+// undecided (returns false).
+__device__ __forceinline__ bool lean_gate(double x, LeanObserver const& l, int& bin, bool& in) {
+  double const r = lean_nearest(x, bin);
+  in = (x > kBinGuard) & (x < l.gate_in) & (fabs(r) < 0.5 - kBinGuard);
+  return in | (x < -kBinGuard) | (x > l.gate_out);
+}
+
+// Adds one filtered sample, (vx, vy, vz) a in fixed-point units (1 per
+// component when counting samples).  Every component is below 2^61.
+template <bool kUnchecked>
+__device__ __forceinline__ void lean_add(WindowSink& sink, LeanObserver const& l, int bin, float vx, float vy,
+                                         float vz, float a, Counts& c) {
+  long long const x = __float2ll_rn(fmaf(vx, a, l.bias)), y = __float2ll_rn(fmaf(vy, a, l.bias)),
+                  z = __float2ll_rn(fmaf(vz, a, l.bias));
+  if (kUnchecked) {
+    // through a generic pointer (see deposit_unchecked)
+    unsigned long long* w = sink.win + bin;
+    asm volatile("" : "+l"(w));
+    atomicAdd(w, static_cast<unsigned long long>(x));
+    atomicAdd(w + sink.width, static_cast<unsigned long long>(y));
+    atomicAdd(w + 2 * sink.width, static_cast<unsigned long long>(z));
+    ++c.coreas;
+  } else {
+    float const mag = (fabsf(vx) + fabsf(vy) + fabsf(vz)) * fabsf(a) + 3.f * l.bias;
+    if (sink.add3(static_cast<uint64_t>(bin), x, y, z, true, true, true, mag, c.mag))
+      ++c.coreas;
+    else
+      ++c.overflows;
+  }
+}
+
+// The two samples of a CoREAS pair, fields (s) as and (e) ae, at xs and xe
+// bins.  False, having added nothing, when a bin is undecided or a component
+// might not convert.  kUnchecked: the window bound gains an upper bound of the
+// |components| (each factor's roundings inside 2^-20).
+template <bool kUnchecked>
+__device__ __forceinline__ bool lean_samples(WindowSink& sink, LeanObserver const& l, double xs, double xe,
+                                             Vec3<float> s, float as, Vec3<float> e, float ae, Counts& c) {
+  int bs, be;
+  bool ins, ine;
+  bool decided = lean_gate(xs, l, bs, ins);
+  decided = lean_gate(xe, l, be, ine) & decided;
+  float const ms = (fabsf(s.x) + fabsf(s.y) + fabsf(s.z)) * fabsf(as);
+  float const me = (fabsf(e.x) + fabsf(e.y) + fabsf(e.z)) * fabsf(ae);
+  if (!(decided & (ms + me < 0x1p60f))) return false;  // also NaN and infinities
+  if (ins) lean_add<kUnchecked>(sink, l, bs, s.x, s.y, s.z, as, c);
+  if (ine) lean_add<kUnchecked>(sink, l, be, e.x, e.y, e.z, ae, c);
+  if (kUnchecked) c.mag = fmaf(ms + me, 1.f + 0x1p-20f, c.mag) + 6.f * l.bias;
+  return true;
+}
+
+// The common CoREAS pair of the windowed kernel in mixed precision and fixed
+// point (RadioProjection.inl:339-409 without its near-Cherenkov branch), from
+// the track's columns `r`: detection times and Doppler factors in FP64 by the
+// filtered arithmetic above, transverse vectors k (k.beta) - beta in FP64
+// (k x (k x beta) of FP32 vectors cancels when they are nearly parallel),
+// amplitudes in FP32.  Returns one of the codes above; a deferred pair has
+// deposited nothing.  kPre: the points' source terms are the track's columns.
+//
+// Against exact times (a square root and four divisions an endpoint) and an
+// FP32 cross product the pair takes 358 instead of 621 warp instructions:
+// 1e7 x 160 x 8192 CoREAS 41.6 -> 27.4 ms, 5e6 x 64 in ice 9.0 -> 5.2 ms, and the
+// traces' relative error falls from 6e-7 to 1.1e-7.  What bounds it now is the
+// latency of the FP64 chain and of the track loads at 20 warps an SM (46% of
+// issue slots), with the atomics at 60% of the shared-memory pipe; blocks of
+// 512 / 768 / 1024 threads ran 30.6 / 33.1 (spills) / 30.2 ms.
+template <bool kPre, bool kUnchecked>
+__device__ __forceinline__ int coreas_lean(double2 const* __restrict__ r, Propagation const& p,
+                                           ObserverCache const& o, LeanObserver const& l, WindowSink& sink,
+                                           Counts& c) {
+  constexpr unsigned T = kTrackTile;
+  double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T),
+                cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
+  unsigned const flags = pack_flags(ce.y);
+  SourceTerms ts, te;
+  bool ok = (flags & kTrackRegular & l.usable) != 0u;
+  if (kPre) {
+    double2 const s = __ldg(r + kFactorStart / 2 * T), e = __ldg(r + kFactorEnd / 2 * T);
+    ts = SourceTerms{s.x, s.y, dense_index(flags)};
+    te = SourceTerms{e.x, e.y, 0.};
+  } else {
+    Destination const d = destination_of(o);
+    ts = source_terms(p, d, cb.x);
+    te = source_terms(p, d, cc.y);
+    ok = ok & lean_index(ts.n_src) & lean_index(te.n_src);
+  }
+  LeanPoint const s = lean_point(o, l, ca.x, ca.y, cb.x, ct.x, cd.x, cd.y, ce.x, ts.factor, ts.n_src);
+  LeanPoint const e = lean_point(o, l, cb.y, cc.x, cc.y, ct.y, cd.x, cd.y, ce.x, te.factor, te.n_src);
+  bool const dense = ts.n_dst > 1.;
+  ok = ok & s.ok & e.ok;
+  double const least = fmin(fabs(s.factor), fabs(e.factor));
+  // below 1e-3 the near-Cherenkov branch (n_dst > 1); below 1e-6 the factor's
+  // own error counts
+  if (!(ok & (least >= (dense ? kCoreasThreshold + kDopplerGuard : 1.e-6)))) {
+    if (ok && dense && least < kCoreasThreshold - kDopplerGuard && fabs(s.x - e.x) > 2. * kBinGuard &&
+        fabs(s.x) < 0x1p27 && fabs(e.x) < 0x1p27)
+      return kCoreasNearCone | (s.x < e.x ? 1 : 0);
+    return kCoreasExact;
+  }
+  float const constant = pack_constant(ce.y) * l.scale;
+  float as = __fdividef(constant, static_cast<float>(s.factor * s.dist));
+  float ae = __fdividef(-constant, static_cast<float>(e.factor * e.dist));
+  double xs = s.x, xe = e.x;
+  if ((s.factor < 0.) | (e.factor < 0.)) {  // |factor| >= 1e-6: the reference's "< 1e-9"
+    double const dt = fabs(xe - xs);
+    if (dt < 1. + kBinGuard) {
+      if (!(dt < 1. - kBinGuard && lean_separate(xs, xe, l))) return kCoreasExact;
+      as *= static_cast<float>(dt);
+      ae *= static_cast<float>(dt);
+    }
+  }
+  Vec3<float> const vs{static_cast<float>(fma(s.dx, s.along, -cd.x)), static_cast<float>(fma(s.dy, s.along, -cd.y)),
+                       static_cast<float>(fma(s.dz, s.along, -ce.x))};
+  Vec3<float> const ve{static_cast<float>(fma(e.dx, e.along, -cd.x)), static_cast<float>(fma(e.dy, e.along, -cd.y)),
+                       static_cast<float>(fma(e.dz, e.along, -ce.x))};
+  return lean_samples<kUnchecked>(sink, l, xs, xe, vs, as, ve, ae, c) ? kCoreasDeposited : kCoreasExact;
+}
+
+// The near-Cherenkov branch of a deferred pair (RadioProjection.inl:352-387)
+// by the filtered arithmetic: the midpoint field over the Doppler-compressed
+// duration |1 - n w| (t_end - t_start).  False, having added nothing, when a
+// guard cannot decide.
+template <bool kPre>
+__device__ __forceinline__ bool near_cone_lean(double2 const* __restrict__ r, bool start_before_end,
+                                               Propagation const& p, ObserverCache const& o,
+                                               LeanObserver const& l, WindowSink& sink, Counts& c) {
+  constexpr unsigned T = kTrackTile;
+  double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T),
+                cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
+  unsigned const flags = pack_flags(ce.y);
+  double const mz = (cb.x + cc.y) * 0.5;
+  SourceTerms m;
+  if (kPre && (flags & kTrackOneMid)) {
+    double2 const mid = __ldg(r + kFactorMid / 2 * T);
+    m = SourceTerms{mid.x, mid.y, 0.};
+  } else {
+    m = source_terms(p, destination_of(o), mz);
+  }
+  LeanPoint const s = lean_point(o, l, (ca.x + cb.y) * 0.5, (ca.y + cc.x) * 0.5, mz, (ct.x + ct.y) * 0.5, cd.x,
+                                 cd.y, ce.x, m.factor, m.n_src);
+  double const dt = (ct.y - ct.x) * l.rate * fabs(s.factor);
+  // |factor| > 8 guards: its sign and the field's are the reference's.  Where
+  // the samples share a bin the field is scaled by dt, which carries the
+  // same factor, so a small one costs no precision.
+  if (!((flags & kTrackRegular) && l.usable && s.ok && lean_index(m.n_src) && fabs(s.factor) > 8. * kDopplerGuard &&
+        fabs(dt - 1.) > 2. * kBinGuard && dt > 2. * kBinGuard))
+    return false;
+  double low = fma(-0.5, dt, s.x), high = fma(0.5, dt, s.x);
+  float a = __fdividef(pack_constant(ce.y) * l.scale, static_cast<float>(s.factor * s.dist));
+  if (dt < 1.) {
+    if (!lean_separate(low, high, l)) return false;
+    a *= static_cast<float>(dt);
+  }
+  Vec3<float> const v{static_cast<float>(fma(s.dx, s.along, -cd.x)), static_cast<float>(fma(s.dy, s.along, -cd.y)),
+                      static_cast<float>(fma(s.dz, s.along, -ce.x))};
+  return lean_samples<false>(sink, l, start_before_end ? low : high, start_before_end ? high : low, v, a, v, -a, c);
 }
 
 // Intermediate ZHS bins binned index by index with the reference's own
@@ -496,7 +671,7 @@ __device__ __noinline__ Counts zhs_multi_tail(ObserverCache const& o, Sink sink,
   return c;
 }
 
-// accumulate_zhs_segment, RadioProjection.inl:412-480.
+// accumulate_zhs_segment, RadioProjection.inl:412-480, every decision exact.
 //
 // kRuns = true (windowed kernel): the intermediate bins of a segment are the
 // consecutive bins nearest(x1) + i whenever x1 lies farther than a rounding
@@ -505,35 +680,19 @@ __device__ __noinline__ Counts zhs_multi_tail(ObserverCache const& o, Sink sink,
 // (the reference-shaped direct kernel), each index is binned by the
 // reference's own expression.
 //
-// kFilter = true (mixed precision): the emission direction is d * RN(1/|d|),
-// so n beta.k lies within e_nbk of the reference's value and each detection
-// time within e_d; every decision the segment takes (which detection time is
-// first, the nearest bin and floor(x + 0.5) of both, |1 - n beta.k| > 1e-15,
-// the consecutive-run test) is taken only when those bounds cannot change it,
-// else the segment returns false having deposited nothing (the caller then
-// evaluates it exactly).  Bins and counts are the reference's.
-template <bool kFixed, bool kRuns, bool kFilter, class Amp, class Sink>
-__device__ __forceinline__ bool zhs_segment(double p1x, double p1y, double p1z, double p2x,
+template <bool kFixed, bool kRuns, class Amp, class Sink>
+__device__ __forceinline__ void zhs_segment(double p1x, double p1y, double p1z, double p2x,
                                             double p2y, double p2z, double t1, double t2,
                                             Track const& t, Propagation const& p,
                                             ObserverCache const& o, Sink& sink, Counts& c,
                                             bool subdivided) {
   double const mx = (p1x + p2x) * 0.5, my = (p1y + p2y) * 0.5, mz = (p1z + p2z) * 0.5;
-  Path const path = propagate<true, kFilter>(p, o, mx, my, mz);
+  Path const path = propagate<true>(p, o, mx, my, mz);
   double const bk = t.bx * path.kx + t.by * path.ky + t.bz * path.kz;
   double const nbk = path.n_src * bk;
   double const mt = (t1 + t2) * 0.5;
   double d1 = t1 + path.time - nbk * (t1 - mt);
   double d2 = t2 + path.time - nbk * (t2 - mt);
-  double e_d = 0.;
-  if (kFilter) {
-    // |nbk - reference| <= 11.1 u n |beta|_1; each d within that times
-    // |t - mt| plus two ulps of its terms (bounds used with margins >= 4x)
-    double const beta1 = fabs(t.bx) + fabs(t.by) + fabs(t.bz) + 1.;
-    double const e_nbk = path.n_src * beta1 * 0x1p-47 + 0x1p-50;
-    double const h = fabs(t1 - mt) + fabs(t2 - mt);
-    e_d = e_nbk * h + 0x1p-50 * (fabs(t1 + path.time) + fabs(t2 + path.time) + fabs(nbk) * h);
-  }
   double sign = 1.;
   if (d1 > d2) {
     double const swap = d1;
@@ -557,17 +716,7 @@ __device__ __forceinline__ bool zhs_segment(double p1x, double p1y, double p1z, 
   // nearest(x1) + i for every i < nb.
   double const f1 = fabs(x1 - floor(x1) - 0.5);
   double const mag = fabs(x1) + static_cast<double>(nb) + fabs(d1 * fs) + fabs(o.start_time * fs) + 2.;
-  bool run_ok = mag < 0x1p50 && f1 > mag * 0x1p-48;
-  if (kFilter) {
-    double const e_x = (e_d + 0x1p-50 * (fabs(d1) + fabs(d2) + 2. * fabs(o.start_time))) * fs +
-                       0x1p-50 * (fabs(x1) + fabs(x2));
-    double const f2 = fabs(x2 - floor(x2) - 0.5);
-    run_ok = run_ok && f1 > mag * 0x1p-48 + e_x;
-    bool const ambiguous = fabs(d1 - d2) <= 2. * e_d || fabs(den) < 1.e-6 ||
-                           f1 <= e_x + 0x1p-50 * (fabs(x1) + 1.) ||
-                           f2 <= e_x + 0x1p-50 * (fabs(x2) + 1.) || (nb > 1 && !run_ok);
-    if (ambiguous) return false;
-  }
+  bool const run_ok = mag < 0x1p50 && f1 > mag * 0x1p-48;
   Vec3<Amp> const k{static_cast<Amp>(path.kx), static_cast<Amp>(path.ky), static_cast<Amp>(path.kz)};
   Vec3<Amp> const beta{static_cast<Amp>(t.bx), static_cast<Amp>(t.by), static_cast<Amp>(t.bz)};
   Vec3<Amp> const perp = cross(k, cross(beta, k));
@@ -585,13 +734,12 @@ __device__ __forceinline__ bool zhs_segment(double p1x, double p1y, double p1z, 
                            scaled(perp, amp_div(static_cast<Amp>(sc * frac_last),
                                                 static_cast<Amp>(den_last))),
                            c.zhs, c.overflows, c.mag);
-  if (single) return true;
+  if (single) return;
   Counts const d = zhs_multi_tail<kFixed, kRuns, Amp>(
       o, sink, d1, x1, sb, nb, perp, sc, dd, (subdivided ? 1. : sign) * t.constant, run_ok);
   c.zhs += d.zhs;
   c.overflows += d.overflows;
   c.mag += d.mag;
-  return true;
 }
 
 // The samples of one ZHS segment, staged for the warp (windowed kernel): the
@@ -617,43 +765,25 @@ struct StagedSegment<double> {
   uint32_t pad_[2];
 };
 
-// accumulate_zhs_segment (RadioProjection.inl:412-480) with every decision of
-// zhs_segment<kRuns = true, kFilter>, its samples staged instead of
-// deposited.  With kFilter the midpoint propagation is propagate_fast: its
-// directions (8u) stay inside the n beta.k bound, and its time error adds to
-// the detection-time bound e_d.  Returns false when the segment needs the
-// per-index binning or (kFilter) an exact evaluation, or when the trace has
-// 2^26 bins or more (staged counts then stay far inside 32 bits per warp);
-// the caller then discards whatever `out` holds.  The filter's ambiguity
-// test is applied at the end, after the samples are formed (the values it
-// declines are discarded): with the decision off the critical path the
-// kernel issues the staging arithmetic beside the bound arithmetic (7% off
-// the ZHS kernel on the 1e7 x 160 workload).
-template <bool kFilter, class Amp, bool kPre = false>
-__device__ __forceinline__ bool zhs_stage(double p1x, double p1y, double p1z, double p2x,
-                                          double p2y, double p2z, double t1, double t2,
+// accumulate_zhs_segment (RadioProjection.inl:412-480) evaluated exactly, as
+// zhs_segment<kRuns = true>, its samples staged instead of deposited.  The
+// segment's midpoint, its times and the time between them come from the
+// caller; kPre: the midpoint's source terms are `pre`, else they are looked
+// up.  Returns false when the segment needs the per-index binning or when the
+// trace has 2^26 bins or more (staged counts then stay far inside 32 bits per
+// warp); the caller then discards whatever `out` holds.
+template <bool kFixed, class Amp, bool kPre = false>
+__device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, double t1, double t2, double mt,
                                           Track const& t, Propagation const& p,
                                           ObserverCache const& o, bool subdivided,
                                           StagedSegment<Amp>& out,
                                           SourceTerms const& pre = SourceTerms{}) {
-  if (!(o.bins_d < 67108864.0)) return false;
-  bool decided = true;
-  double const mx = (p1x + p2x) * 0.5, my = (p1y + p2y) * 0.5, mz = (p1z + p2z) * 0.5;
-  FastPath const path = filtered_path<kFilter, kPre>(p, o, mx, my, mz, pre);
-  if (kFilter && !path.ok) return false;
+  if (!(o.bins_d < kMaxLeanBins)) return false;
+  Path const path = kPre ? propagate_with<true>(pre, o, mx, my, mz) : propagate<true>(p, o, mx, my, mz);
   double const bk = t.bx * path.kx + t.by * path.ky + t.bz * path.kz;
   double const nbk = path.n_src * bk;
-  double const mt = (t1 + t2) * 0.5;
   double d1 = t1 + path.time - nbk * (t1 - mt);
   double d2 = t2 + path.time - nbk * (t2 - mt);
-  double e_d = 0.;
-  if (kFilter) {
-    double const beta1 = fabs(t.bx) + fabs(t.by) + fabs(t.bz) + 1.;
-    double const e_nbk = path.n_src * beta1 * 0x1p-47 + 0x1p-50;
-    double const h = fabs(t1 - mt) + fabs(t2 - mt);
-    e_d = e_nbk * h + 0x1p-50 * (fabs(t1 + path.time) + fabs(t2 + path.time) + fabs(nbk) * h) +
-          path.time_err;
-  }
   double sign = 1.;
   if (d1 > d2) {
     double const swap = d1;
@@ -670,19 +800,8 @@ __device__ __forceinline__ bool zhs_stage(double p1x, double p1y, double p1z, do
   int const nb = x86_int(eb - sb);
   double const f1 = fabs(x1 - floor(x1) - 0.5);
   double const mag = fabs(x1) + static_cast<double>(nb) + fabs(d1 * fs) + fabs(o.start_time * fs) + 2.;
-  bool run_ok = mag < 0x1p50 && f1 > mag * 0x1p-48;
-  if (kFilter) {
-    double const e_x = (e_d + 0x1p-50 * (fabs(d1) + fabs(d2) + 2. * fabs(o.start_time))) * fs +
-                       0x1p-50 * (fabs(x1) + fabs(x2));
-    double const f2 = fabs(x2 - floor(x2) - 0.5);
-    run_ok = run_ok && f1 > mag * 0x1p-48 + e_x;
-    bool const ambiguous = fabs(d1 - d2) <= 2. * e_d || fabs(den) < 1.e-6 ||
-                           f1 <= e_x + 0x1p-50 * (fabs(x1) + 1.) ||
-                           f2 <= e_x + 0x1p-50 * (fabs(x2) + 1.) || (nb > 1 && !run_ok);
-    decided = !ambiguous;
-  } else if (nb > 1 && !run_ok) {
-    return false;
-  }
+  bool const run_ok = mag < 0x1p50 && f1 > mag * 0x1p-48;
+  if (nb > 1 && !run_ok) return false;
   Vec3<Amp> const k{static_cast<Amp>(path.kx), static_cast<Amp>(path.ky), static_cast<Amp>(path.kz)};
   Vec3<Amp> const beta{static_cast<Amp>(t.bx), static_cast<Amp>(t.by), static_cast<Amp>(t.bz)};
   out.perp = cross(k, cross(beta, k));
@@ -693,7 +812,9 @@ __device__ __forceinline__ bool zhs_stage(double p1x, double p1y, double p1z, do
   double const frac_last = single ? (tiny ? (t2 - t1) * fs : fabs(d2 * fs - d1 * fs))
                                   : fabs(x2 + 0.5 - eb);
   double const den_last = single && tiny ? path.dist : dd;
-  out.last = amp_div(static_cast<Amp>(sc * frac_last), static_cast<Amp>(den_last));
+  // FP32 values are staged in fixed-point units
+  Amp const unit = kFixed && sizeof(Amp) == sizeof(float) ? static_cast<Amp>(o.fixed_scale_f) : static_cast<Amp>(1);
+  out.last = amp_div(static_cast<Amp>(sc * frac_last), static_cast<Amp>(den_last)) * unit;
   out.flags = 0u;
   out.start = 0u;
   out.count = 0u;
@@ -704,11 +825,11 @@ __device__ __forceinline__ bool zhs_stage(double p1x, double p1y, double p1z, do
     out.last_bin = static_cast<uint32_t>(bv2);
     out.flags = 2u;
   }
-  if (single) return decided;
+  if (single) return true;
   double const frac_first = fabs(sb + 0.5 - x1);
-  out.first = amp_div(static_cast<Amp>(sc * frac_first), static_cast<Amp>(dd));
+  out.first = amp_div(static_cast<Amp>(sc * frac_first), static_cast<Amp>(dd)) * unit;
   double const mc = (subdivided ? 1. : sign) * t.constant;
-  out.mid = amp_div(static_cast<Amp>(mc), static_cast<Amp>(dd));
+  out.mid = amp_div(static_cast<Amp>(mc), static_cast<Amp>(dd)) * unit;
   // first sample, add_sample(detection_time1): bin nearest(x1)
   double const bv1 = nearest_bin(x1);
   bool const first_in = bv1 >= 0. && bv1 < o.bins_d;
@@ -732,7 +853,65 @@ __device__ __forceinline__ bool zhs_stage(double p1x, double p1y, double p1z, do
       }
     }
   }
-  return decided;
+  return true;
+}
+
+// The Fraunhofer number of an undivided track, (|beta|^2 - w^2) (h fs)^2 / |d|
+// times 8 pi c^2 / (wavelength fs^2) for the half duration h, surely below 1:
+// accumulate_zhs (RadioProjection.inl:483-503) then takes one segment.  The
+// difference |beta|^2 - w^2 is within 2^-46 of the reference's, so for a factor
+// below 2^18 the number is within 2^-26 of its FP64 value (the guard is
+// 2^-20); above it the caller defers.
+__device__ __forceinline__ bool surely_undivided(LeanPoint const& m, LeanObserver const& l, double half_bins,
+                                                 double bx, double by, double bz) {
+  double const square = fma(bz, bz, fma(by, by, bx * bx));
+  double const factor = half_bins * half_bins * (m.inverse * l.fraunhofer);
+  return (factor < 0x1p18) & (fma(-m.w, m.w, square) * factor < 1. - 0x1p-20);
+}
+
+// One ZHS segment (RadioProjection.inl:412-480) by the filtered arithmetic,
+// staged: `m` is its midpoint with the time in its middle, half_bins half its
+// duration in bins, `constant` the charge constant in the observer's units.
+// Its detection times are m.x -+ |half_bins (1 - n w)|, in time order, and the
+// potential's sign times 1 / (1 - n w) is 1 / |1 - n w|.  False when a guard
+// cannot decide (the caller evaluates the segment exactly).
+__device__ __forceinline__ bool zhs_lean(LeanPoint const& m, double half_bins, float constant, double bx, double by,
+                                         double bz, ObserverCache const& o, bool subdivided,
+                                         StagedSegment<float>& out) {
+  double const reach = fabs(half_bins * m.factor);
+  double const x1 = m.x - reach, x2 = m.x + reach;
+  out.flags = 0u;
+  out.start = 0u;
+  out.count = 0u;
+  out.last_bin = 0u;
+  int b1, b2;
+  double const r1 = lean_nearest(x1, b1), r2 = lean_nearest(x2, b2);
+  bool const decided = (fabs(r1) < 0.5 - kBinGuard) & (fabs(r2) < 0.5 - kBinGuard) & (reach > kBinGuard) &
+                       (fabs(m.factor) >= 1.e-6);
+  if ((x2 < -1.) | (x1 > o.bins_d + 1.)) return m.ok;  // off the trace
+  // from here |x1|, |x2| < 2^27: reach is below 2^25 and one of them is near the trace
+  float const amplitude = __fdividef(constant, static_cast<float>(fabs(m.factor) * m.dist));
+  out.perp = Vec3<float>{static_cast<float>(fma(-m.dx, m.along, bx)), static_cast<float>(fma(-m.dy, m.along, by)),
+                         static_cast<float>(fma(-m.dz, m.along, bz))};
+  bool const single = b1 == b2;
+  out.last = amplitude * static_cast<float>(single ? 2. * reach : r2 + 0.5);
+  out.first = amplitude * static_cast<float>(0.5 - r1);
+  out.mid = (subdivided & (m.factor < 0.)) ? -amplitude : amplitude;
+  unsigned const bins = static_cast<unsigned>(o.bins);
+  if (static_cast<unsigned>(b2) < bins) {
+    out.last_bin = static_cast<unsigned>(b2);
+    out.flags = 2u;
+  }
+  if (!single) {
+    bool const first_in = static_cast<unsigned>(b1) < bins;
+    int const low = b1 + 1 > 0 ? b1 + 1 : 0;
+    int const high = b2 < static_cast<int>(bins) ? b2 : static_cast<int>(bins);
+    int const mids = high > low ? high - low : 0;
+    out.start = static_cast<unsigned>(first_in ? b1 : low);
+    out.count = static_cast<unsigned>(mids) + (first_in ? 1u : 0u);
+    out.flags |= first_in ? 1u : 0u;
+  }
+  return decided & m.ok;
 }
 
 // Deposits the staged segments of a warp: every lane takes two bins of the
@@ -760,7 +939,7 @@ __device__ __forceinline__ void deposit_staged(StagedSegment<Amp>* staging,
   // window atomics below might alias as far as the compiler can tell
   ObserverCache grid;
   grid.fixed_scale = o.fixed_scale;
-  grid.fixed_scale_f = o.fixed_scale_f;
+  grid.fixed_scale_f = 1.f;  // staged FP32 values are in fixed-point units
   grid.count_samples = o.count_samples;
   for (uint32_t base = 0; base < total; base += 64u) {
     uint32_t const j0 = base + lane, j1 = j0 + 32u;
@@ -799,14 +978,6 @@ __device__ __forceinline__ void deposit_staged(StagedSegment<Amp>* staging,
   __syncwarp();
 }
 
-// The fixed-point value of one component, as to_fixed computes it.
-__device__ __forceinline__ long long fixed_value(float v, ObserverCache const& grid) {
-  return __float2ll_rn(v * grid.fixed_scale_f);
-}
-__device__ __forceinline__ long long fixed_value(double v, ObserverCache const& grid) {
-  return __double2ll_rn(v * grid.fixed_scale);
-}
-
 // The owner's half of the unchecked deposit of its staged segment (fixed
 // point, the whole trace in the window, whose adds are not checked): shows
 // once for the segment that every sample converts -- each component's
@@ -815,98 +986,136 @@ __device__ __forceinline__ long long fixed_value(double v, ObserverCache const& 
 // an upper bound of their |components| to the window bound (each factor's
 // roundings, at most nine of 2^-24, inside the 2^-20 margin).  The deposit
 // then converts and adds each sample with no check.  Returns false when a
-// sample might not convert (huge or non-finite values) or in the diagnostic
-// count-samples mode: the pair then goes to the checked drain.
+// sample might not convert (huge or non-finite values): the pair then goes to
+// the checked drain.
 template <class Amp>
 __device__ __forceinline__ bool account_staged(StagedSegment<Amp> const& seg, ObserverCache const& o,
                                                Counts& c) {
   uint32_t const samples = seg.count + ((seg.flags >> 1) & 1u);
   if (samples == 0u) return true;
-  if (o.count_samples) return false;
   bool const has_first = (seg.flags & 1u) != 0u;
   uint32_t const mids = seg.count - (has_first ? 1u : 0u);
   Amp const zero = static_cast<Amp>(0);
   Amp const af = has_first ? fabs(seg.first) : zero;
   Amp const am = mids ? fabs(seg.mid) : zero;
   Amp const al = (seg.flags & 2u) ? fabs(seg.last) : zero;
-  Amp const px = fabs(seg.perp.x), py = fabs(seg.perp.y), pz = fabs(seg.perp.z);
-  Amp const fs = sizeof(Amp) == sizeof(float) ? static_cast<Amp>(o.fixed_scale_f) : static_cast<Amp>(o.fixed_scale);
-  Amp const largest = fmax(fmax(px, py), pz) * fmax(fmax(af, am), al) * fs;
-  if (!(largest < static_cast<Amp>(0x1p62))) return false;  // also NaN and infinities
-  Amp const sum = (af + am * static_cast<Amp>(mids) + al) * (px + py + pz) * fs *
-                  static_cast<Amp>(1. + 0x1p-20);
+  // staged FP32 values are in fixed-point units; when counting samples each component adds 1
+  Amp const fs = sizeof(Amp) == sizeof(float) ? static_cast<Amp>(1) : static_cast<Amp>(o.fixed_scale);
+  Amp const width = (fabs(seg.perp.x) + fabs(seg.perp.y) + fabs(seg.perp.z)) * fs;
+  if (!(width * fmax(fmax(af, am), al) < static_cast<Amp>(0x1p62))) return false;  // also NaN and infinities
+  Amp const sum = o.count_samples ? static_cast<Amp>(3u * samples)
+                                  : (af + am * static_cast<Amp>(mids) + al) * width;
   c.zhs += samples;
-  c.mag += sizeof(Amp) == sizeof(float) ? static_cast<float>(sum)
-                                        : __double2float_ru(static_cast<double>(sum));
+  Amp const bound = sum * static_cast<Amp>(1. + 0x1p-20);
+  c.mag += sizeof(Amp) == sizeof(float) ? static_cast<float>(bound)
+                                        : __double2float_ru(static_cast<double>(bound));
   return true;
 }
 
-// The unchecked deposit of a warp's staged segments: deposit_staged's
-// redistribution (every lane takes two bins of the flattened list per step),
-// each sample converted and added to the window with no check, its counts
-// and bound already taken by account_staged.  Every bin is below the trace's
-// bins, which the window holds whole.
+// The fixed-point value of one staged component, as to_fixed computes it; 1
+// when counting samples (then scale 0, bias 1).
+__device__ __forceinline__ long long fixed_value(float v, float amplitude, float scale, float bias) {
+  return __float2ll_rn(fmaf(v * amplitude, scale, bias));
+}
+__device__ __forceinline__ long long fixed_value(double v, double amplitude, double scale, double bias) {
+  return __double2ll_rn(fma(v * amplitude, scale, bias));
+}
+
+// The unchecked deposit of a staged segment as differences: the window holds
+// the differences of consecutive bins and difference_window sums them before
+// the flush.  A segment's samples are constant between its first and its last
+// bin, so it touches at most four bins -- start, start + 1, the bin after the
+// run (its last sample) and the next -- whatever its length, each lane on its
+// own: no redistribution over the warp (a prefix sum, searches by shuffle and
+// 40 bytes staged a lane in the former version).  On the 1e7 x 160 workload 55% of the
+// segments have one sample, 26% two, 17% more (2.0 samples a pair, 2.6
+// differences).  The sums of differences are exact modulo 2^64, and the
+// item's bound (account_staged) shows that no bin's value leaves the int64
+// range.  The adds go through a generic pointer: where the compiler can tell
+// the window is shared memory it emits shared-space 64-bit atomics, which this
+// GPU executes as about one instruction per active lane (twice the atomic
+// wavefronts of generic adds on the same samples).
 template <class Amp>
-__device__ __forceinline__ void deposit_unchecked(StagedSegment<Amp>* staging, StagedSegment<Amp> const& seg,
-                                                  ObserverCache const& o, WindowSink const& sink) {
-  unsigned const lane = threadIdx.x & 31u;
-  uint32_t const cnt = seg.count + ((seg.flags >> 1) & 1u);
-  uint32_t incl = cnt;
-#pragma unroll
-  for (unsigned d = 1; d < 32u; d <<= 1) {
-    uint32_t const v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
-  }
-  uint32_t const total = __shfl_sync(0xffffffffu, incl, 31);
-  if (total == 0u) return;
-  staging[lane] = seg;
-  __syncwarp();
-  uint32_t const before_mine = incl - cnt;
-  ObserverCache grid;  // the converting fields in registers
-  grid.fixed_scale = o.fixed_scale;
-  grid.fixed_scale_f = o.fixed_scale_f;
-  // The adds go through a generic pointer: where the compiler can tell the
-  // window is shared memory it emits shared-space 64-bit atomics, which this
-  // GPU executes as about one instruction per active lane (the ZHS track
-  // loop alone, one pass of two, ran at twice the atomic wavefronts of the
-  // single-pass kernel's generic adds on the same samples).
+__device__ __forceinline__ void deposit_differences(StagedSegment<Amp> const& seg, ObserverCache const& o,
+                                                    WindowSink const& sink) {
+  bool const last = (seg.flags & 2u) != 0u;
+  if (seg.count == 0u && !last) return;
+  Amp const one = static_cast<Amp>(1);
+  Amp const bias = o.count_samples ? one : static_cast<Amp>(0);
+  Amp const unit = sizeof(Amp) == sizeof(float) ? one : static_cast<Amp>(o.fixed_scale);
+  Amp const scale = o.count_samples ? static_cast<Amp>(0) : unit;
   unsigned long long* win = sink.win;
   asm volatile("" : "+l"(win));
   uint32_t const width = sink.width;
-  // kPer bins per lane per step, their owner searches interleaved
-  constexpr int kPer = sizeof(Amp) == sizeof(float) ? 2 : 4;  // measured best of 2 and 4
-  for (uint32_t base = 0; base < total; base += 32u * kPer) {
-    uint32_t owner[kPer], before[kPer];
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) owner[u] = 0u;
-#pragma unroll
-    for (uint32_t step = 16; step >= 1u; step >>= 1) {
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        uint32_t const v = __shfl_sync(0xffffffffu, incl, owner[u] + step - 1u);
-        if (v <= base + lane + 32u * u) owner[u] += step;
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) before[u] = __shfl_sync(0xffffffffu, before_mine, owner[u] & 31u);
-#pragma unroll
-    for (int u = 0; u < kPer; ++u) {
-      uint32_t const j = base + lane + 32u * u;
-      if (j < total) {
-        StagedSegment<Amp> const& g = staging[owner[u]];
-        uint32_t const k = j - before[u];
-        bool const last = k >= g.count;
-        uint32_t const bin = last ? g.last_bin : g.start + k;
-        Amp const scale = last ? g.last : ((k == 0u && (g.flags & 1u)) ? g.first : g.mid);
-        Vec3<Amp> const v = scaled(g.perp, scale);
-        unsigned long long* const w = win + bin;
-        atomicAdd(w, static_cast<unsigned long long>(fixed_value(v.x, grid)));
-        atomicAdd(w + width, static_cast<unsigned long long>(fixed_value(v.y, grid)));
-        atomicAdd(w + 2 * width, static_cast<unsigned long long>(fixed_value(v.z, grid)));
-      }
+  auto value = [&](Amp amplitude) {
+    return Vec3<long long>{fixed_value(seg.perp.x, amplitude, scale, bias),
+                           fixed_value(seg.perp.y, amplitude, scale, bias),
+                           fixed_value(seg.perp.z, amplitude, scale, bias)};
+  };
+  auto add = [&](uint32_t bin, Vec3<long long> v) {
+    unsigned long long* const w = win + bin;
+    atomicAdd(w, static_cast<unsigned long long>(v.x));
+    atomicAdd(w + width, static_cast<unsigned long long>(v.y));
+    atomicAdd(w + 2 * width, static_cast<unsigned long long>(v.z));
+  };
+  Vec3<long long> run{0, 0, 0};  // the value up to the bin before `end`
+  uint32_t const end = seg.start + seg.count;
+  if (seg.count != 0u) {
+    bool const first = (seg.flags & 1u) != 0u;
+    run = value(first ? seg.first : seg.mid);
+    add(seg.start, run);
+    if (first && seg.count > 1u) {
+      Vec3<long long> const mid = value(seg.mid);
+      add(seg.start + 1u, Vec3<long long>{mid.x - run.x, mid.y - run.y, mid.z - run.z});
+      run = mid;
     }
   }
-  __syncwarp();
+  // the last sample is in the bin after the run (staged runs are clipped to
+  // the trace only at its start when the last sample is on it)
+  if (last) {
+    Vec3<long long> const v = value(seg.last);
+    add(seg.last_bin, Vec3<long long>{v.x - run.x, v.y - run.y, v.z - run.z});
+    run = v;
+  }
+  uint32_t const after = last ? seg.last_bin + 1u : end;
+  if (after < width) add(after, Vec3<long long>{-run.x, -run.y, -run.z});
+}
+
+// Turns a window of differences into the bins' values: a running sum over
+// each of its three rows.  Every thread of the CTA calls it.  Out of line, so
+// that its registers do not count in the track loops.
+__device__ __noinline__ void difference_window(unsigned long long* win, uint32_t width) {
+  __shared__ unsigned long long totals[3][32];
+  unsigned const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t per = (width + blockDim.x - 1) / blockDim.x;
+  per |= 1u;  // an odd stride keeps the lanes' 64-bit words on different banks
+  uint32_t const first = threadIdx.x * per < width ? threadIdx.x * per : width;
+  uint32_t const stop = first + per < width ? first + per : width;
+  unsigned long long before[3];
+  __syncthreads();
+  for (int row = 0; row < 3; ++row) {
+    unsigned long long const* const w = win + row * static_cast<size_t>(width);
+    unsigned long long sum = 0;
+    for (uint32_t j = first; j < stop; ++j) sum += w[j];
+    unsigned long long incl = sum;
+    for (unsigned d = 1; d < 32u; d <<= 1) {
+      unsigned long long const v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (lane == 31u) totals[row][warp] = incl;
+    before[row] = incl - sum;
+  }
+  __syncthreads();
+  for (int row = 0; row < 3; ++row) {
+    unsigned long long* const w = win + row * static_cast<size_t>(width);
+    unsigned long long sum = before[row];
+    for (unsigned k = 0; k < warp; ++k) sum += totals[row][k];
+    for (uint32_t j = first; j < stop; ++j) {
+      sum += w[j];
+      w[j] = sum;
+    }
+  }
+  __syncthreads();
 }
 
 // accumulate_zhs, RadioProjection.inl:483-529, every decision exact.
@@ -948,7 +1157,7 @@ __device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
 #pragma unroll 1
   for (long long index = 0; index < segments; ++index) {
     double const p2x = p1x + rx, p2y = p1y + ry, p2z = p1z + rz, t2 = t1 + rt;
-    zhs_segment<kFixed, kRuns, false, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, sink, c,
+    zhs_segment<kFixed, kRuns, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, sink, c,
                                            subdivided);
     p1x = p2x;
     p1y = p2y;
@@ -960,56 +1169,52 @@ __device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
         static_cast<long long>(subtracks * (refinement - 1)));
 }
 
-// The common ZHS pair of the windowed kernel: one undivided segment, staged
-// for the warp's cooperative deposit.  Returns false, staging nothing (`seg`
-// cleared), when the track is subdivided (Fraunhofer number above 1, or
-// refinement), when (kFilter) the Fraunhofer test is not surely below 1, or
-// when zhs_stage declines the segment; the kernel then defers the pair to
-// zhs_drain.  The FP32 Fraunhofer test and the staging of the one segment
-// are independent and both evaluated; the test decides at the end.
+// The common ZHS pair of the windowed kernel: one undivided segment, staged,
+// from the track's columns `r`.  Returns false, staging nothing (`seg`
+// cleared), when the track is or might be subdivided (the Fraunhofer number
+// not surely below 1, or refinement) or when the segment cannot be staged; the
+// kernel then defers the pair to zhs_drain.  Mixed precision (Amp = float)
+// stages by the filtered arithmetic, FP64 exactly; both decide "one segment"
+// from the filtered midpoint, which spares FP64 the exact Fraunhofer number
+// (a square root and seven divisions).  `row` addresses the same track's
+// columns from the work item's first one.
 //
-// kFilter: F is estimated in FP32 as sin^2(theta) K with
-// sin^2 = |beta x d|^2 / (|beta|^2 |d|^2) and K = 2 pi L^2 / (|d| lambda); its
-// distance from the reference's FP64 F is at most 1.7e-6 sqrt(K F) + 4e-6 F +
-// 1e-12 K (cross-product cancellation, the FP32 roundings and the approximate
-// reciprocals; used with margins of 2.3x and more), so an estimate surely
-// below 1 decides "one segment" exactly as the reference does.
-template <bool kFilter, bool kPre, class Amp>
-__device__ __forceinline__ bool zhs_common(Track const& t, Propagation const& p,
-                                           ObserverCache const& o, Counts& c,
-                                           StagedSegment<Amp>& seg, SourceTerms const& pre_mid) {
-  if (p.refinement != 1u) return false;
-  double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
-  bool surely_one = true;
-  if (kFilter) {
-    float const dx = static_cast<float>(o.px - mx), dy = static_cast<float>(o.py - my),
-                dz = static_cast<float>(o.pz - mz);
-    float const bx = static_cast<float>(t.bx), by = static_cast<float>(t.by),
-                bz = static_cast<float>(t.bz);
-    float const cx = by * dz - bz * dy, cy = bz * dx - bx * dz, cz = bx * dy - by * dx;
-    float const d2 = dx * dx + dy * dy + dz * dz;
-    float const b2 = bx * bx + by * by + bz * bz;
-    float const length = static_cast<float>(t.length);
-    // approximate reciprocals and square roots (relative errors near 2^-21,
-    // inside the 4e-5 (f + 1) term below)
-    float const s2 = __fdividef(cx * cx + cy * cy + cz * cz, b2 * d2);
-    float const k = __fdividef(6.2831853f * length * length * rsqrtf(d2), static_cast<float>(o.wavelength));
-    float const f = s2 * k;
-    float const kf = k * (f + 1.f);
-    float const root = kf > 0.f ? kf * rsqrtf(kf) : 0.f;
-    float const margin = 4.e-6f * root + 4.e-5f * (f + 1.f) + 4.e-12f * k;
-    surely_one = f + margin < 1.f;
+// With the filtered segment and its deposit as differences a pair takes 450
+// instead of 764 warp instructions: 1e7 x 160 x 8192 ZHS 59.4 -> 32.9 ms, FP64 at
+// 1e6 x 160 10.4 -> 7.3 ms.
+template <bool kFixed, bool kPre, class Amp>
+__device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propagation const& p,
+                                           ObserverCache const& o, LeanObserver const& l, Counts& c,
+                                           StagedSegment<Amp>& seg) {
+  constexpr unsigned T = kTrackTile;
+  double2 const cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T), cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T),
+                ch = __ldg(r + 11 * T);
+  unsigned const flags = pack_flags(ce.y);
+  SourceTerms st;
+  if (kPre) {
+    double2 const m = __ldg(r + kFactorMid / 2 * T);
+    st = SourceTerms{m.x, m.y, 0.};
   } else {
-    Path const pm = propagate<false>(p, o, mx, my, mz);
-    double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
-    double const s2 = 1. - uk * uk;
-    double const fraunhofer = s2 * t.length * t.length / pm.dist / o.wavelength * 2. * kPi;
-    if (fraunhofer > 1.) return false;
+    st = source_terms(p, destination_of(o), cn.x);
   }
-  bool const staged = zhs_stage<kFilter, Amp, kPre>(t.sx, t.sy, t.sz, t.sx + (t.ex - t.sx), t.sy + (t.ey - t.sy),
-                                     t.sz + (t.ez - t.sz), t.ts, t.ts + (t.te - t.ts), t, p, o, false,
-                                     seg, pre_mid);
-  if (!(staged && surely_one)) {
+  LeanPoint const m = lean_point(o, l, cm.x, cm.y, cn.x, cn.y, cd.x, cd.y, ce.x, st.factor, st.n_src);
+  double const half = ch.x * l.rate;
+  bool staged = ((flags & kTrackRegular & l.usable) != 0u) & (p.refinement == 1u) & m.ok &
+                surely_undivided(m, l, half, cd.x, cd.y, ce.x);
+  if (!kPre) staged = staged & lean_index(st.n_src);
+  if constexpr (sizeof(Amp) == sizeof(float)) {
+    staged = zhs_lean(m, half, pack_constant(ce.y) * l.scale, cd.x, cd.y, ce.x, o, false, seg) & staged;
+  } else if (staged) {
+    double2 const ct = __ldg(r + 3 * T);
+    Track t;
+    t.bx = cd.x;
+    t.by = cd.y;
+    t.bz = ce.x;
+    t.constant = ch.y;
+    staged = zhs_stage<kFixed, Amp, true>(cm.x, cm.y, cn.x, ct.x, ct.x + (ct.y - ct.x), cn.y, t, p, o, false, seg,
+                                          st);
+  }
+  if (!staged) {
     seg.count = 0u;
     seg.flags = 0u;
     return false;
@@ -1019,13 +1224,11 @@ __device__ __forceinline__ bool zhs_common(Track const& t, Propagation const& p,
 }
 
 // ---------------------------------------------------------------- helpers
-__device__ __forceinline__ Track load_track(const double* __restrict__ base, uint64_t stride,
-                                            uint64_t i) {
-  (void)stride;
-  double2 const* r = track_ref(base, i);
-  constexpr unsigned T = kTrackTile;
-  double2 const a = __ldg(r + 0 * T), b = __ldg(r + 1 * T), c = __ldg(r + 2 * T), d = __ldg(r + 3 * T);
-  double2 const e = __ldg(r + 4 * T), f = __ldg(r + 5 * T), g = __ldg(r + 6 * T);
+// The fields of a track, its columns read by `load`.
+template <class Load>
+__device__ __forceinline__ Track unpack_track(Load load) {
+  double2 const a = load(0), b = load(1), c = load(2), d = load(3);
+  double2 const e = load(4), f = load(5), g = load(kConst / 2);
   Track t;
   t.sx = a.x;
   t.sy = a.y;
@@ -1038,33 +1241,21 @@ __device__ __forceinline__ Track load_track(const double* __restrict__ base, uin
   t.bx = e.x;
   t.by = e.y;
   t.bz = f.x;
-  t.length = f.y;
-  t.beta_module = g.x;
   t.constant = g.y;
+  derive_track(t);
   return t;
+}
+
+__device__ __forceinline__ Track load_track(const double* __restrict__ base, uint64_t i) {
+  double2 const* r = track_ref(base, i);
+  return unpack_track([&](unsigned k) { return __ldg(r + k * kTrackTile); });
 }
 
 // A track staged in shared memory as one interleaved 192-byte record (plain
 // loads: __ldg reads the global space only).
 __device__ __forceinline__ Track load_staged_track(double const* base, unsigned i) {
   double2 const* r = reinterpret_cast<double2 const*>(base + i * kTrackDoubles);
-  double2 const a = r[0], b = r[1], c = r[2], d = r[3], e = r[4], f = r[5], g = r[6];
-  Track t;
-  t.sx = a.x;
-  t.sy = a.y;
-  t.sz = b.x;
-  t.ex = b.y;
-  t.ey = c.x;
-  t.ez = c.y;
-  t.ts = d.x;
-  t.te = d.y;
-  t.bx = e.x;
-  t.by = e.y;
-  t.bz = f.x;
-  t.length = f.y;
-  t.beta_module = g.x;
-  t.constant = g.y;
-  return t;
+  return unpack_track([&](unsigned k) { return r[k]; });
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
@@ -1078,6 +1269,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 __device__ __forceinline__ double warp_max(double v) {
   for (int d = 16; d > 0; d >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, d));
   return v;
+}
+
+__device__ __forceinline__ void add_counts(Counts& c, Counts const& d) {
+  c.coreas += d.coreas;
+  c.zhs += d.zhs;
+  c.subtracks += d.subtracks;
+  c.overflows += d.overflows;
+  c.mag += d.mag;
 }
 
 // Adds per-thread counts into the event counters: one atomic per warp.
@@ -1185,32 +1384,44 @@ __global__ void __launch_bounds__(256) ingest_kernel(
     uint64_t const j = base + __popc(ballot & ((1u << lane) - 1u));
     double2* r = track_ref(tracks, j);
     constexpr unsigned T = kTrackTile;
+    // the ZHS segment of an undivided track, with the reference's own
+    // arithmetic (RadioProjection.inl:418-425, :505-512): it ends at
+    // start + (end - start)
+    double const mx = (t.sx + (t.sx + (t.ex - t.sx))) * 0.5, my = (t.sy + (t.sy + (t.ey - t.sy))) * 0.5,
+                 mz = (t.sz + (t.sz + (t.ez - t.sz))) * 0.5;
+    double const t2 = t.ts + (t.te - t.ts);
+    double const tm = (t.ts + t2) * 0.5;
+    bool regular = fabs(t.bx) + fabs(t.by) + fabs(t.bz) <= 4. && fabs(t.ts) <= terms.limits.time &&
+                   fabs(t.te) <= terms.limits.time && duration <= terms.limits.duration;
+    unsigned flags = 0u;
+    if (terms.enabled) {
+      // the source points of the windowed kernels
+      Propagation const& p = terms.propagation;
+      Destination const& d = terms.destination;
+      SourceTerms const s = source_terms(p, d, t.sz);
+      SourceTerms const e = source_terms(p, d, t.ez);
+      SourceTerms const m = source_terms(p, d, mz);
+      // the CoREAS near-cone midpoint is (start + end) / 2 (:357-359)
+      SourceTerms const mc = source_terms(p, d, (t.sz + t.ez) * 0.5);
+      r[6 * T] = make_double2(s.factor, s.n_src);
+      r[7 * T] = make_double2(e.factor, e.n_src);
+      r[8 * T] = make_double2(m.factor, m.n_src);
+      regular = regular && lean_index(s.n_src) && lean_index(e.n_src) && lean_index(m.n_src);
+      if (s.n_dst > 1.) flags |= kTrackDense;
+      if (mc.factor == m.factor && mc.n_src == m.n_src) flags |= kTrackOneMid;
+    }
+    if (regular) flags |= kTrackRegular;
+    double const pack = __hiloint2double(
+        static_cast<int>(flags), __float_as_int(static_cast<float>(t.constant * kConstantShift)));
     r[0 * T] = make_double2(t.sx, t.sy);
     r[1 * T] = make_double2(t.sz, t.ex);
     r[2 * T] = make_double2(t.ey, t.ez);
     r[3 * T] = make_double2(t.ts, t.te);
     r[4 * T] = make_double2(t.bx, t.by);
-    r[5 * T] = make_double2(t.bz, t.length);
-    r[6 * T] = make_double2(t.beta_module, t.constant);
-    if (terms.enabled) {
-      // the source points of the windowed kernels, with the reference's own
-      // arithmetic: the ZHS segment of an undivided track ends at
-      // start + (end - start) (RadioProjection.inl:505-512), the CoREAS
-      // near-cone midpoint is (start + end) / 2 (:357-359)
-      Propagation const& p = terms.propagation;
-      Destination const& d = terms.destination;
-      SourceTerms const s = source_terms(p, d, t.sz);
-      SourceTerms const e = source_terms(p, d, t.ez);
-      SourceTerms const mz = source_terms(p, d, (t.sz + (t.sz + (t.ez - t.sz))) * 0.5);
-      SourceTerms const mc = source_terms(p, d, (t.sz + t.ez) * 0.5);
-      r[7 * T] = make_double2(s.n_dst, 0.);
-      r[8 * T] = make_double2(s.factor, s.n_src);
-      r[9 * T] = make_double2(e.factor, e.n_src);
-      r[10 * T] = make_double2(mz.factor, mz.n_src);
-      r[11 * T] = make_double2(mc.factor, mc.n_src);
-    } else {
-      r[7 * T] = make_double2(0., 0.);
-    }
+    r[5 * T] = make_double2(t.bz, pack);
+    r[9 * T] = make_double2(mx, my);
+    r[10 * T] = make_double2(mz, tm);
+    r[11 * T] = make_double2((t2 - t.ts) * 0.5, t.constant);
   }
   if (lane == 0 && ballot) atomicAdd(&counters->valid_tracks, static_cast<unsigned long long>(__popc(ballot)));
   if (!diagnostics) return;
@@ -1312,7 +1523,7 @@ __global__ void __launch_bounds__(256) direct_kernel(const __grid_constant__ Eve
        pair += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
     uint64_t const ti = pair / observers;
     uint32_t const oi = static_cast<uint32_t>(pair - ti * observers);
-    Track const t = load_track(ev.tracks, ev.stride, ti);
+    Track const t = load_track(ev.tracks, ti);
     if (kCoreas && oi < ev.observer_count[0]) {
       ObserverCache const& o = ev.observers[0][oi];
       GlobalSink sink;
@@ -1413,7 +1624,6 @@ __global__ void __launch_bounds__(kTileThreads) tiled_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------- windowed
-constexpr int kWindowThreadsMax = kWindowThreads;
 // Threads of a CTA of the one-pass ZHS kernel (floating traces, the
 // no-allocation entry point, launches past the two-pass storage cap, and the
 // third pass of two-pass launches).  Its drain's live state needs more
@@ -1425,13 +1635,12 @@ constexpr int kWindowThreadsMax = kWindowThreads;
 // 117.0, 480 128.5.
 constexpr int kZhsThreadsFloat = 768;
 constexpr int kZhsThreadsDouble = 384;
-// Two passes (fixed point): the track loop alone runs larger CTAs (FP32 768
-// threads, FP64 480: the most its 72-byte staging slots allow beside an
-// 8192-bin window), the drain pass FP32 512 (ZHS 62.0 -> 60.7 ms on the 1e7 x
-// 160 workload against 384; 768 ran slower), FP64 384.  FP64 track loops of
-// 512 threads with unpadded 64-byte slots ran 110.3 ms against 96.2.
-constexpr int kZhsLoopThreadsFloat = 768;
-constexpr int kZhsLoopThreadsDouble = 480;
+// Two passes (fixed point): the track loop alone runs larger CTAs.  FP32 1024
+// threads (1e7 x 160 workload, ZHS ms at 640 / 768 / 896 / 1024 threads: 39.8 /
+// 36.3 / 33.9 / 32.9), FP64 640 (1e6 x 160: 8.5 at 480, 7.3 at 640); the drain
+// pass FP32 512, FP64 384.
+constexpr int kZhsLoopThreadsFloat = 1024;
+constexpr int kZhsLoopThreadsDouble = 640;
 constexpr int kZhsDrainThreadsFloat = 512;
 constexpr int kZhsDrainThreadsDouble = 384;
 // kPass: 0 one pass; of a two-pass launch 1 the track loop, 2 the drain, 3
@@ -1450,12 +1659,12 @@ constexpr int zhs_block(int threads) {
              ? (threads < zhs_threads_max<Amp, kPass>() ? threads : zhs_threads_max<Amp, kPass>())
              : zhs_threads_max<Amp, kPass>();
 }
-// staging slots of the ZHS kernel: 32 per warp of its largest CTA
+// staging slots of the ZHS kernel: 32 per warp of its largest CTA that stages
+// (pass 1 does not)
 template <class Amp>
 constexpr size_t staging_bytes() {
-  int const a = zhs_threads_max<Amp, 0>(), b = zhs_threads_max<Amp, 1>(), c = zhs_threads_max<Amp, 2>();
-  int const most = a > b ? (a > c ? a : c) : (b > c ? b : c);
-  return static_cast<size_t>(most) * sizeof(StagedSegment<Amp>);
+  int const a = zhs_threads_max<Amp, 0>(), c = zhs_threads_max<Amp, 2>();
+  return static_cast<size_t>(a > c ? a : c) * sizeof(StagedSegment<Amp>);
 }
 constexpr size_t kStagingBytes =
     staging_bytes<float>() > staging_bytes<double>() ? staging_bytes<float>() : staging_bytes<double>();
@@ -1477,14 +1686,14 @@ __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t
 // one deferred pair each and evaluate its Fraunhofer number and subdivision
 // exactly; the warp then steps through segment index s = 0, 1, ...: every lane
 // whose pair has a segment s forms its endpoints by the reference's
-// sequential additions, stages it (kFilter: the filtered decisions first, the
-// exact ones where those are ambiguous), and the warp deposits the staged
+// sequential additions, stages it (mixed precision: by the filtered arithmetic
+// first, exactly where a guard cannot decide), and the warp deposits the staged
 // samples together.  A segment that needs the per-index binning deposits on
 // its own lane.  Every lane of the warp calls it.
-template <bool kFixed, bool kFilter, class Amp, class Sink>
+template <bool kFixed, class Amp, class Sink>
 __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint64_t begin,
                                          unsigned const* list, unsigned count,
-                                         Propagation const& p, ObserverCache const& o, Sink sink,
+                                         Propagation const& p, ObserverCache const& o, LeanObserver const& l, Sink sink,
                                          StagedSegment<Amp>* staging) {
   Counts c;
   unsigned const lane = threadIdx.x & 31u;
@@ -1494,7 +1703,7 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
   double p1x = 0., p1y = 0., p1z = 0., t1 = 0., rx = 0., ry = 0., rz = 0., rt = 0.;
   if (lane < count) {
     row = begin + list[lane];
-    Track const t = load_track(tracks, 0, row);
+    Track const t = load_track(tracks, row);
     double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
     Path const pm = propagate<false>(p, o, mx, my, mz);
     double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
@@ -1544,24 +1753,28 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
       // registers held across the warp's steps
       double2 const* r = track_ref(tracks, row);
       asm volatile("" : "+l"(r));
-      double2 const e = __ldg(r + 4 * kTrackTile), f = __ldg(r + 5 * kTrackTile), g = __ldg(r + 6 * kTrackTile);
+      double2 const e = __ldg(r + 4 * kTrackTile), f = __ldg(r + 5 * kTrackTile);
+      double const p2x = p1x + rx, p2y = p1y + ry, p2z = p1z + rz, t2 = t1 + rt;
+      double const mx = (p1x + p2x) * 0.5, my = (p1y + p2y) * 0.5, mz = (p1z + p2z) * 0.5, mt = (t1 + t2) * 0.5;
+      bool staged = false;
+      if constexpr (sizeof(Amp) == sizeof(float)) {
+        SourceTerms const st = source_terms(p, destination_of(o), mz);
+        LeanPoint const m = lean_point(o, l, mx, my, mz, mt, e.x, e.y, f.x, st.factor, st.n_src);
+        staged = zhs_lean(m, (t2 - t1) * l.half_rate, pack_constant(f.y) * l.scale, e.x, e.y, f.x, o, subdivided, seg) &
+                 ((pack_flags(f.y) & kTrackRegular & l.usable) != 0u) & lean_index(st.n_src);
+      }
       Track t;
       t.bx = e.x;
       t.by = e.y;
       t.bz = f.x;
-      t.length = f.y;
-      t.beta_module = g.x;
-      t.constant = g.y;
-      double const p2x = p1x + rx, p2y = p1y + ry, p2z = p1z + rz, t2 = t1 + rt;
-      bool staged =
-          zhs_stage<kFilter, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, subdivided, seg);
-      if (kFilter && !staged)
-        staged = zhs_stage<false, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, subdivided,
-                                       seg);
+      if (!staged) {
+        t.constant = __ldg(r + kConst / 2 * kTrackTile).y;
+        staged = zhs_stage<kFixed, Amp>(mx, my, mz, t1, t2, mt, t, p, o, subdivided, seg);
+      }
       if (!staged) {
         seg.count = 0u;
         seg.flags = 0u;
-        zhs_segment<kFixed, true, false, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, sink,
+        zhs_segment<kFixed, true, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, sink,
                                               c, subdivided);
       }
       p1x = p2x;
@@ -1581,49 +1794,97 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
 template <bool kFixed, class Amp, bool kPre, class Sink>
 __device__ __noinline__ Counts coreas_drain_pair(const double* __restrict__ tracks, uint64_t row,
                                                  unsigned hint, Propagation const& p,
-                                                 ObserverCache const& o, Sink sink) {
+                                                 ObserverCache const& o, LeanObserver const& l, Sink sink) {
   Counts c;
-  if (hint & static_cast<unsigned>(kCoreasNearCone)) {
-    SourceTerms mid{};
-    if (kPre) {
-      double2 const m = __ldg(track_ref(tracks, row) + kFactorMidCoreas / 2 * kTrackTile);
-      mid = SourceTerms{m.x, m.y, 0.};
-    }
-    return coreas_near_cone<kFixed, Amp, kPre>(load_track(tracks, 0, row), p, o, sink, (hint & 1u) != 0u, mid);
+  double2 const* r = track_ref(tracks, row);
+  if constexpr (kFixed && sizeof(Amp) == sizeof(float)) {
+    if ((hint & static_cast<unsigned>(kCoreasNearCone)) &&
+        near_cone_lean<kPre>(r, (hint & 1u) != 0u, p, o, l, sink, c))
+      return c;
   }
+  constexpr unsigned T = kTrackTile;
+  unsigned const flags = pack_flags(__ldg(r + kPack / 2 * T).y);
+  Track const t = load_track(tracks, row);
   if (kPre) {
-    double2 const* r = track_ref(tracks, row);
-    constexpr unsigned T = kTrackTile;
-    double2 const n = __ldg(r + kNdstStart / 2 * T), s = __ldg(r + kFactorStart / 2 * T),
-                  e = __ldg(r + kFactorEnd / 2 * T), m = __ldg(r + kFactorMidCoreas / 2 * T);
-    SourceTerms const pre[3] = {{s.x, s.y, n.x}, {e.x, e.y, 0.}, {m.x, m.y, 0.}};
-    coreas_pair<kFixed, Amp, Sink, true>(load_track(tracks, 0, row), p, o, sink, c, pre);
+    // the near-cone midpoint's terms are the ZHS midpoint's (kTrackOneMid) or looked up
+    double2 const m = __ldg(r + kFactorMid / 2 * T);
+    SourceTerms const mid = (flags & kTrackOneMid) ? SourceTerms{m.x, m.y, 0.}
+                                                   : source_terms(p, destination_of(o), (t.sz + t.ez) * 0.5);
+    if (hint & static_cast<unsigned>(kCoreasNearCone))
+      return coreas_near_cone<kFixed, Amp, true>(t, p, o, sink, (hint & 1u) != 0u, mid);
+    double2 const s = __ldg(r + kFactorStart / 2 * T), e = __ldg(r + kFactorEnd / 2 * T);
+    SourceTerms const pre[3] = {{s.x, s.y, dense_index(flags)}, {e.x, e.y, 0.}, mid};
+    coreas_pair<kFixed, Amp, Sink, true>(t, p, o, sink, c, pre);
   } else {
-    coreas_pair<kFixed, Amp>(load_track(tracks, 0, row), p, o, sink, c);
+    if (hint & static_cast<unsigned>(kCoreasNearCone))
+      return coreas_near_cone<kFixed, Amp, false>(t, p, o, sink, (hint & 1u) != 0u, SourceTerms{});
+    coreas_pair<kFixed, Amp>(t, p, o, sink, c);
   }
   return c;
 }
 
-// The precomputed source terms of a track's common path (kTrackDoubles):
-// CoREAS start and end (n_dst at the start), ZHS segment midpoint.
-template <int kAlgorithm>
-__device__ __forceinline__ void load_source_terms(const double* __restrict__ base, uint64_t i,
-                                                  SourceTerms& a, SourceTerms& b) {
+// The precomputed source terms of a track's end points (with the start's n_dst
+// as far as the path looks at it: above 1 or not).
+__device__ __forceinline__ void load_endpoint_terms(const double* __restrict__ base, uint64_t i, SourceTerms& start,
+                                                    SourceTerms& end) {
   double2 const* r = track_ref(base, i);
   constexpr unsigned T = kTrackTile;
-  if (kAlgorithm == 0) {
-    double2 const n = __ldg(r + kNdstStart / 2 * T), s = __ldg(r + kFactorStart / 2 * T),
-                  e = __ldg(r + kFactorEnd / 2 * T);
-    a = SourceTerms{s.x, s.y, n.x};
-    b = SourceTerms{e.x, e.y, 0.};
-  } else {
-    double2 const m = __ldg(r + kFactorMidZhs / 2 * T);
-    a = SourceTerms{m.x, m.y, 0.};
+  double2 const s = __ldg(r + kFactorStart / 2 * T), e = __ldg(r + kFactorEnd / 2 * T);
+  start = SourceTerms{s.x, s.y, dense_index(pack_flags(__ldg(r + kPack / 2 * T).y))};
+  end = SourceTerms{e.x, e.y, 0.};
+}
+
+// Appends a warp's deferred pairs to its CTA's list: `entry` of the lanes with
+// `deferred` set, one atomic on the shared counter.  Entries at or past
+// `capacity` are counted, not written.
+__device__ __forceinline__ void push_deferred(bool deferred, unsigned entry, unsigned* list, unsigned* total,
+                                              uint64_t used, uint64_t capacity) {
+  unsigned const ballot = __ballot_sync(0xffffffffu, deferred);
+  if (!ballot) return;
+  unsigned const lane = threadIdx.x & 31u;
+  unsigned slot = 0;
+  if (lane == 0) slot = atomicAdd(total, static_cast<unsigned>(__popc(ballot)));
+  slot = __shfl_sync(0xffffffffu, slot, 0);
+  uint64_t const at = used + slot + __popc(ballot & ((1u << lane) - 1u));
+  if (deferred && at < capacity) list[at] = entry;
+}
+
+// The CoREAS track loop in mixed precision and fixed point: `count` tracks from
+// `begin`, a thread each, the deferred ones appended to `list`.  A thread's
+// track advances by whole tiles, so its columns' address is one running
+// pointer.
+template <bool kPre, bool kUnchecked>
+__device__ __forceinline__ void coreas_lean_loop(const double* __restrict__ tracks, uint64_t begin, uint32_t count,
+                                                 Propagation const& p, ObserverCache const& o,
+                                                 LeanObserver const& l, WindowSink& sink, unsigned* list,
+                                                 unsigned* total, Counts& c) {
+  double2 const* r = track_ref(tracks, begin + threadIdx.x);
+  uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
+  for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
+    uint32_t const k = base + threadIdx.x;
+    int code = kCoreasDeposited;
+    if (k < count) code = coreas_lean<kPre, kUnchecked>(r, p, o, l, sink, c);
+    push_deferred(code != kCoreasDeposited,
+                  k | (code >= kCoreasNearCone ? static_cast<unsigned>(code) << kDeferredHintShift : 0u), list,
+                  total, 0, ~0ull);
   }
 }
 
+// The same with checked adds (an item run again, or a trace longer than the
+// window), out of line: its registers do not count in the unchecked loop.
+template <bool kPre>
+__device__ __noinline__ Counts coreas_lean_checked(const double* __restrict__ tracks, uint64_t begin,
+                                                   uint32_t count, Propagation const& p, ObserverCache const& o,
+                                                   LeanObserver const& l, WindowSink sink, unsigned* list,
+                                                   unsigned* total) {
+  Counts c;
+  coreas_lean_loop<kPre, false>(tracks, begin, count, p, o, l, sink, list, total, c);
+  return c;
+}
+
 // kPass 0: one pass over every item.  Two passes (fixed-point ZHS):
-// kPass 1 runs the track loop alone with unchecked window adds, appends the
+// kPass 1 runs the track loop alone, depositing differences with unchecked
+// window adds (deposit_differences), appends the
 // deferred pairs of all its items to its CTA's list, flushes each item whose
 // window bound holds and records where its deferred pairs are; an item whose
 // bound does not hold, whose trace is longer than the window or whose pairs
@@ -1634,12 +1895,13 @@ __device__ __forceinline__ void load_source_terms(const double* __restrict__ bas
 // registers than the track loop (168 against 80 FP32, 118 FP64), so apart
 // the track loop runs without spills in larger CTAs.
 template <bool kFixed, class Amp, int kAlgorithm, bool kPre, int kPass = 0>
-__global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>() : kWindowThreadsMax, 1)
+__global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>() : kWindowThreads, 1)
     windowed_kernel(const __grid_constant__ WorkPlan plan) {
   static_assert(kPass == 0 || (kFixed && kAlgorithm == 1), "two passes: fixed-point ZHS");
   extern __shared__ __align__(16) unsigned long long window[];
   __shared__ unsigned long long item_shared;
   __shared__ ObserverCache observer;
+  __shared__ LeanObserver lean;
   __shared__ float window_bound;
   __shared__ unsigned deferred_total;
   // this CTA's list of the deferred pairs of its current item (kPass 1: of
@@ -1687,7 +1949,10 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
       }
       continue;
     }
-    if (threadIdx.x == 0) observer = ev.observers[algorithm][oi];
+    if (threadIdx.x == 0) {
+      observer = ev.observers[algorithm][oi];
+      if (kAlgorithm == 1 || sizeof(Amp) == sizeof(float)) make_lean_observer<kAlgorithm>(observer, lean);
+    }
     ObserverCache const& o = observer;
 
     // zero the window (3 rows of width bins); the barrier also publishes `observer`
@@ -1739,48 +2004,57 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
       c.mag = 0.f;
       if (threadIdx.x == 0) deferred_total = 0u;
       __syncthreads();
-      for (uint64_t base = begin; !drain_only && base < end; base += blockDim.x) {
-        uint64_t const i = base + threadIdx.x;
-        bool deferred = false;
-        unsigned hint = 0u;  // CoREAS: the near-Cherenkov decision, in the list entry's top bits
-        StagedSegment<Amp> seg;
-        seg.count = 0u;
-        seg.flags = 0u;
-        if (i < end) {
-          Track const t = load_track(ev.tracks, ev.stride, i);
-          SourceTerms pa{}, pb{};
-          if (kPre) load_source_terms<kAlgorithm>(ev.tracks, i, pa, pb);
-          if constexpr (kAlgorithm == 0) {
-            int const code = coreas_common<kFixed, kFilter, kPre, Amp>(t, ev.propagation, o, sink, c, pa, pb);
-            deferred = code != kCoreasDeposited;
-            hint = code >= kCoreasNearCone ? static_cast<unsigned>(code) << kDeferredHintShift : 0u;
-          } else {
-            deferred = !zhs_common<kFilter, kPre, Amp>(t, ev.propagation, o, c, seg, pa);
+      if constexpr (kAlgorithm == 0 && kFixed && kFilter) {
+        uint32_t const count = static_cast<uint32_t>(end - begin);
+        if (sink.unchecked)
+          coreas_lean_loop<kPre, true>(ev.tracks, begin, count, ev.propagation, o, lean, sink, deferred_list,
+                                       &deferred_total, c);
+        else
+          add_counts(c, coreas_lean_checked<kPre>(ev.tracks, begin, count, ev.propagation, o, lean, sink,
+                                                  deferred_list, &deferred_total));
+      } else if constexpr (kAlgorithm == 0) {
+        for (uint64_t base = begin; base < end; base += blockDim.x) {
+          uint64_t const i = base + threadIdx.x;
+          int code = kCoreasDeposited;
+          if (i < end) {
+            Track const t = load_track(ev.tracks, i);
+            SourceTerms pa{}, pb{};
+            if (kPre) load_endpoint_terms(ev.tracks, i, pa, pb);
+            code = coreas_common<kFixed, kPre, Amp>(t, ev.propagation, o, sink, c, pa, pb);
           }
+          push_deferred(code != kCoreasDeposited,
+                        static_cast<unsigned>(i - begin) |
+                            (code >= kCoreasNearCone ? static_cast<unsigned>(code) << kDeferredHintShift : 0u),
+                        deferred_list, &deferred_total, 0, ~0ull);
         }
-        if (kAlgorithm == 1) {
-          if (kFixed && sink.unchecked) {
+      } else if (!drain_only) {
+        uint32_t const count = static_cast<uint32_t>(end - begin);
+        double2 const* r = track_ref(ev.tracks, begin + threadIdx.x);
+        uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
+        for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
+          uint32_t const k = base + threadIdx.x;
+          bool deferred = false;
+          StagedSegment<Amp> seg;
+          seg.count = 0u;
+          seg.flags = 0u;
+          if (k < count) deferred = !zhs_common<kFixed, kPre, Amp>(r, ev.propagation, o, lean, c, seg);
+          if (kFixed && (kPass == 1 || sink.unchecked)) {
             if (!deferred && !account_staged(seg, o, c)) {
               seg.count = 0u;
               seg.flags = 0u;
               deferred = true;
               c.subtracks -= 1ull;  // the drain counts the pair's subtracks
             }
-            deposit_unchecked(staging, seg, o, sink);
+            deposit_differences(seg, o, sink);
           } else {
             if constexpr (kPass != 1) deposit_staged<kFixed>(staging, seg, o, sink, c);
           }
+          push_deferred(deferred, k, deferred_list, &deferred_total, used,
+                        kPass == 1 ? plan.deferred_capacity : ~0ull);  // used: 0 but in kPass 1
         }
-        unsigned const ballot = __ballot_sync(0xffffffffu, deferred);
-        unsigned const rank = __popc(ballot & ((1u << lane) - 1u));
-        if (ballot) {
-          unsigned slot = 0;
-          if (lane == 0) slot = atomicAdd(&deferred_total, static_cast<unsigned>(__popc(ballot)));
-          slot = __shfl_sync(0xffffffffu, slot, 0);
-          uint64_t const at = static_cast<uint64_t>(used) + slot + rank;  // used: 0 but in kPass 1
-          if (deferred && (kPass != 1 || at < plan.deferred_capacity))
-            deferred_list[at] = static_cast<unsigned>(i - begin) | hint;
-        }
+      }
+      if constexpr (kAlgorithm == 1 && kFixed && kPass != 2) {
+        if (kPass == 1 || sink.unchecked) difference_window(window, width);
       }
       __syncthreads();
       // at most end - begin <= deferred_stride (kPass 1: over the list's end
@@ -1800,18 +2074,14 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
         if constexpr (kAlgorithm == 1 && kPass == 1) {
           (void)count;
         } else if (kAlgorithm == 1) {
-          d = zhs_drain<kFixed, kFilter, Amp>(ev.tracks, begin, list + from, count,
-                                              ev.propagation, o, sink, staging);
+          d = zhs_drain<kFixed, Amp>(ev.tracks, begin, list + from, count, ev.propagation, o, lean,
+                                     sink, staging);
         } else if (lane < count) {
           unsigned const entry = list[from + lane];
           d = coreas_drain_pair<kFixed, Amp, kPre>(ev.tracks, begin + (entry & kDeferredOffsetMask),
-                                                   entry >> kDeferredHintShift, ev.propagation, o, sink);
+                                                   entry >> kDeferredHintShift, ev.propagation, o, lean, sink);
         }
-        c.coreas += d.coreas;
-        c.zhs += d.zhs;
-        c.subtracks += d.subtracks;
-        c.overflows += d.overflows;
-        c.mag += d.mag;
+        add_counts(c, d);
         __syncwarp();
       }
       __syncthreads();
@@ -1954,11 +2224,11 @@ cudaError_t tiled_dispatch(EventPlan const& ev, uint64_t bound, bool coreas, boo
   return cudaGetLastError();
 }
 
-// window rows | (ZHS) per-warp staging slots
+// window rows | (ZHS, but for pass 1) per-warp staging slots
 template <class Amp>
-size_t windowed_smem_bytes(uint32_t window, int algorithm) {
+size_t windowed_smem_bytes(uint32_t window, int algorithm, int pass) {
   return static_cast<size_t>(window) * 3 * sizeof(unsigned long long) +
-         (algorithm == 1 ? staging_bytes<Amp>() : 0);
+         (algorithm == 1 && pass != 1 ? staging_bytes<Amp>() : 0);
 }
 
 // Every event of the plan carries precomputed source terms.
@@ -1971,7 +2241,7 @@ bool plan_precomputed(WorkPlan const& plan) {
 
 template <bool kFixed, class Amp, int kAlgorithm, bool kPre, int kPass = 0>
 cudaError_t windowed_launch(WorkPlan const& plan, int ctas, int threads, cudaStream_t stream) {
-  size_t const bytes = windowed_smem_bytes<Amp>(plan.window, kAlgorithm);
+  size_t const bytes = windowed_smem_bytes<Amp>(plan.window, kAlgorithm, kPass);
   cudaError_t err = cudaFuncSetAttribute(windowed_kernel<kFixed, Amp, kAlgorithm, kPre, kPass>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(bytes));
@@ -2030,8 +2300,8 @@ cudaError_t windowed_dispatch(WorkPlan const& plan, int ctas, int threads, cudaS
 template <bool kFixed, class Amp>
 int ctas_per_sm(int window, int threads) {
   int worst = 1 << 30;
-  auto probe = [&](auto kernel, int block, int algorithm) {
-    size_t const bytes = windowed_smem_bytes<Amp>(static_cast<uint32_t>(window), algorithm);
+  auto probe = [&](auto kernel, int block, int algorithm, int pass = 0) {
+    size_t const bytes = windowed_smem_bytes<Amp>(static_cast<uint32_t>(window), algorithm, pass);
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     int blocks = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, bytes) != cudaSuccess)
@@ -2043,12 +2313,12 @@ int ctas_per_sm(int window, int threads) {
   probe(windowed_kernel<kFixed, Amp, 1, false>, zhs_block<Amp>(threads), 1);
   probe(windowed_kernel<kFixed, Amp, 1, true>, zhs_block<Amp>(threads), 1);
   if constexpr (kFixed) {  // the two passes
-    probe(windowed_kernel<true, Amp, 1, false, 1>, zhs_block<Amp, 1>(threads), 1);
-    probe(windowed_kernel<true, Amp, 1, true, 1>, zhs_block<Amp, 1>(threads), 1);
-    probe(windowed_kernel<true, Amp, 1, false, 2>, zhs_block<Amp, 2>(threads), 1);
-    probe(windowed_kernel<true, Amp, 1, true, 2>, zhs_block<Amp, 2>(threads), 1);
-    probe(windowed_kernel<true, Amp, 1, false, 3>, zhs_block<Amp, 3>(threads), 1);
-    probe(windowed_kernel<true, Amp, 1, true, 3>, zhs_block<Amp, 3>(threads), 1);
+    probe(windowed_kernel<true, Amp, 1, false, 1>, zhs_block<Amp, 1>(threads), 1, 1);
+    probe(windowed_kernel<true, Amp, 1, true, 1>, zhs_block<Amp, 1>(threads), 1, 1);
+    probe(windowed_kernel<true, Amp, 1, false, 2>, zhs_block<Amp, 2>(threads), 1, 2);
+    probe(windowed_kernel<true, Amp, 1, true, 2>, zhs_block<Amp, 2>(threads), 1, 2);
+    probe(windowed_kernel<true, Amp, 1, false, 3>, zhs_block<Amp, 3>(threads), 1, 3);
+    probe(windowed_kernel<true, Amp, 1, true, 3>, zhs_block<Amp, 3>(threads), 1, 3);
   }
   return worst;
 }

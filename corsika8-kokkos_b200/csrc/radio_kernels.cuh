@@ -72,9 +72,22 @@ struct IngestTerms {
   int32_t pad_;
   Propagation propagation;
   Destination destination;
+  TrackLimits limits;  // times for which the filtered paths' error bounds hold
 };
 // The destination row shared by all `count` observers, if they share one.
 bool shared_destination(ObserverCache const* observers, std::size_t count, Destination& out);
+// The track limits of the filtered paths over `count` observers, narrowed from
+// `limits` (start from widest_limits()).
+inline TrackLimits widest_limits() { return TrackLimits{1e300, 1e300}; }
+inline void narrow_limits(ObserverCache const* observers, std::size_t count, TrackLimits& limits) {
+  for (std::size_t i = 0; i < count; ++i) {
+    ObserverCache const& o = observers[i];
+    double const start = o.start_time < 0. ? -o.start_time : o.start_time;
+    double const time = kMaxLeanBins / o.sample_rate - start, duration = 0x1p21 / o.sample_rate;
+    if (!(time >= limits.time)) limits.time = time;  // may be negative: no track then
+    if (!(duration >= limits.duration)) limits.duration = duration;
+  }
+}
 
 // Persistent windowed launch over a work list of (event, chunk, algorithm,
 // observer) items drawn from an atomic counter.  Passed as a __grid_constant__

@@ -356,6 +356,8 @@ class Server {
       ev->terms.enabled = shared_destination(all.data(), all.size(), d) ? 1 : 0;
       ev->terms.propagation = prop;
       ev->terms.destination = d;
+      ev->terms.limits = widest_limits();
+      narrow_limits(all.data(), all.size(), ev->terms.limits);
     }
     Block b = make_block(block);
     try {
