@@ -286,9 +286,10 @@ __device__ __forceinline__ Path propagate(Propagation const& p, ObserverCache co
 // or segment is evaluated exactly, operation by operation.  The guards hold
 // for "regular" tracks, whose magnitudes ingest has checked (regular_track):
 //
-//   |beta|_1 <= 4, 0 < n <= 4 at the source points; every time t of the track
-//   has (|t| + |t0|) fs <= 2^26 bins at every observer of the event, and the
-//   track lasts at most 2^21 bins (TrackLimits).
+//   |beta|_1 <= 4; 0 < n <= 4 and |factor| <= 4 at the source points; every time
+//   t of the track has (|t| + |t0|) fs <= 2^24 bins and every coordinate x has
+//   |x| fs / c <= 2^24 at every observer of the event, and the track lasts at
+//   most 2^21 bins (TrackLimits).
 //
 // With u = 2^-53, for a source point at displacement d from the observer
 // (the reference's own subtractions):
@@ -299,21 +300,34 @@ __device__ __forceinline__ Path propagate(Propagation const& p, ObserverCache co
 //   hence 1 - n w within kDopplerGuard = 2^-43.
 //   A detection time in bins, x = (t - t0) fs + |d| factor fs / c, lies within
 //   32u (|t| + |t0| + time) fs of the reference's (t + time - t0) fs; where x
-//   falls on the trace (fewer than 2^26 bins) that is below 32u 2^28 = 2^-20,
+//   falls on the trace (fewer than 2^26 bins) that is below 32u 2^27 = 2^-21,
 //   and the ZHS term n w (t - t_mid) adds at most 2^-43 2^20; kBinGuard =
-//   2^-19 covers both.  Where |x| is larger the error grows like 2^-46 |x|, so
+//   2^-19 covers both, and the 2^-20 of a divided track's segments
+//   (zhs_drain_lean).  Where |x| is larger the error grows like 2^-46 |x|, so
 //   such an x is off the trace in the reference as well.
 constexpr double kDopplerGuard = 0x1p-43;
 constexpr double kBinGuard = 0x1p-19;
-constexpr double kMaxLeanBins = 67108864.0;  // 2^26
+constexpr double kMaxLeanBins = 67108864.0;   // 2^26
+constexpr double kMaxLeanTime = 16777216.0;   // 2^24 bins
 
 // Limits on a track's times (s), from every observer of the event.
 struct TrackLimits {
   double time = 0.;      // |t_start|, |t_end| at most this
   double duration = 0.;  // t_end - t_start at most this
+  double length = 0.;    // |coordinates| (m) at most this
 };
 
-__device__ __forceinline__ bool lean_index(double n) { return (n > 0.) & (n <= 4.); }
+__device__ __forceinline__ bool lean_terms(SourceTerms const& st) {
+  return (st.n_src > 0.) & (st.n_src <= 4.) & (fabs(st.factor) <= 4.);
+}
+
+// Whether the track's own magnitudes are covered by the bounds above.
+__device__ __forceinline__ bool regular_track(Track const& t, double duration, TrackLimits const& limits) {
+  double const furthest = fmax(fmax(fmax(fabs(t.sx), fabs(t.sy)), fmax(fabs(t.sz), fabs(t.ex))),
+                               fmax(fabs(t.ey), fabs(t.ez)));
+  return fabs(t.bx) + fabs(t.by) + fabs(t.bz) <= 4. && fabs(t.ts) <= limits.time && fabs(t.te) <= limits.time &&
+         duration <= limits.duration && furthest <= limits.length;
+}
 
 // 1/sqrt(s2) from the hardware's approximate reciprocal square root (about 20
 // bits) and one third-order step: with r = 1 - s2 y0^2 and |r| <= 2^-17
@@ -345,26 +359,40 @@ __device__ __forceinline__ double lean_nearest(double x, int& bin) {
 constexpr double kConstantShift = 0x1p60;
 
 // Constants of the item's observer for the filtered paths, derived once per
-// work item from its ObserverCache.
-struct LeanObserver {
+// work item from its ObserverCache.  In 16-byte groups of what is used together:
+// the track loops read them from shared memory once a track, 16 bytes a load
+// (copy_words; as 8-byte loads they took a third of the ZHS loop's
+// shared-memory wavefronts).
+struct alignas(16) LeanObserver {
+  double px, py;
+  double pz, start_time;
   double rate;         // fs
   double rate_over_c;  // fs / c
-  double half_rate;    // fs / 2
-  double gate_in;      // a CoREAS sample at kBinGuard < x < gate_in is recorded,
+  double gate_in;      // CoREAS: a sample at kBinGuard < x < gate_in is recorded,
   double gate_out;     // one at x < -kBinGuard or x > gate_out is not
-  double start_bins;   // t0 fs
-  double fraunhofer;   // 8 pi c^2 / (wavelength fs^2)
+  double fraunhofer;   // ZHS: 8 pi c^2 / (wavelength fs^2)
+  double past;         // number of bins + 1: a segment that starts later is off the trace
   float scale;         // 2^-60 x fixed-point scale (x fs, CoREAS); 0 when counting samples
   float bias;          // 1 when counting samples, else 0
   uint32_t usable;     // the filtered paths may be used for this observer
+  uint32_t bins;
+  double start_bins;   // t0 fs
+  double half_rate;    // fs / 2
+  double bin_guard_m;  // kBinGuard bins of path
+  double fixed_scale;  // fixed-point scale; 0 when counting samples
 };
 
 template <int kAlgorithm>
 __device__ __forceinline__ void make_lean_observer(ObserverCache const& o, LeanObserver& l) {
   double const fs = o.sample_rate;
+  l.px = o.px;
+  l.py = o.py;
+  l.pz = o.pz;
+  l.start_time = o.start_time;
   l.rate = fs;
   l.rate_over_c = fs / kSpeedOfLight;
   l.half_rate = 0.5 * fs;
+  l.bin_guard_m = kBinGuard * kSpeedOfLight / fs;
   double const end = (o.end_time - o.start_time) * fs;
   double const last = o.bins_d - 0.5;
   double const gate = end < last ? end : last;
@@ -372,10 +400,24 @@ __device__ __forceinline__ void make_lean_observer(ObserverCache const& o, LeanO
   l.gate_out = gate + kBinGuard;
   l.start_bins = o.start_time * fs;
   l.fraunhofer = 8. * kPi * (kSpeedOfLight / fs) * (kSpeedOfLight / fs) / o.wavelength;
+  l.past = o.bins_d + 1.;
   double const scale = (kAlgorithm == 0 ? fs * o.fixed_scale : o.fixed_scale) / kConstantShift;
   l.scale = o.count_samples ? 0.f : static_cast<float>(scale);
+  l.fixed_scale = o.count_samples ? 0. : o.fixed_scale;
   l.bias = o.count_samples ? 1.f : 0.f;
   l.usable = o.bins_d < kMaxLeanBins && fs < 0x1p200 ? 1u : 0u;
+  l.bins = static_cast<uint32_t>(o.bins);
+}
+
+// A copy in registers, read from shared memory 16 bytes at a time.
+template <class T>
+__device__ __forceinline__ T copy_words(T const& shared) {
+  static_assert(sizeof(T) % sizeof(double2) == 0 && alignof(T) >= sizeof(double2), "16-byte words");
+  T copy;
+#pragma unroll
+  for (unsigned i = 0; i < sizeof(T) / sizeof(double2); ++i)
+    reinterpret_cast<double2*>(&copy)[i] = reinterpret_cast<double2 const*>(&shared)[i];
+  return copy;
 }
 
 // separate_same_bin_endpoints, RadioProjection.inl:303-336.

@@ -74,6 +74,31 @@ __device__ __forceinline__ Vec3<T> scaled(Vec3<T> v, T s) {
   return {v.x * s, v.y * s, v.z * s};
 }
 
+__device__ __forceinline__ void add_counts(Counts& c, Counts const& d) {
+  c.coreas += d.coreas;
+  c.zhs += d.zhs;
+  c.subtracks += d.subtracks;
+  c.overflows += d.overflows;
+  c.mag += d.mag;
+}
+
+// A thread's counts within one work item in 32 bits, which the track loops hold
+// in fewer registers: CoREAS adds two samples a track (2^30 tracks an item at
+// most), and a ZHS item whose threads might pass 2^32 samples is not given to
+// the loop that uses them (kPass 1).
+struct Tally {
+  unsigned coreas = 0, zhs = 0, overflows = 0;
+  float mag = 0.f;
+};
+__device__ __forceinline__ Counts counts_of(Tally const& t) {
+  Counts c;
+  c.coreas = t.coreas;
+  c.zhs = t.zhs;
+  c.overflows = t.overflows;
+  c.mag = t.mag;
+  return c;
+}
+
 // Signed overflow of the three adds previous + increment (two's complement),
 // the condition checked_radio_atomic_add tests; increments whose conversion
 // failed are passed as 0 and cannot overflow.
@@ -130,8 +155,10 @@ __device__ __forceinline__ void spillf3(double* r0, double* r1, double* r2, doub
   atomicAdd(r2, z);
 }
 
-// Shared-memory window of `width` bins starting at bin 0 (rows X|Y|Z), with
-// bins past the window spilled to the global rows.
+// Shared-memory window of `width` bins starting at bin 0, with bins past the
+// window spilled to the global rows.  A bin's three components are neighbours
+// (word 3 bin + component), so that a deposit forms one address and reaches the
+// others by immediate offsets.
 struct WindowSink {
   unsigned long long* win;
   double* fwin;
@@ -146,18 +173,17 @@ struct WindowSink {
                                        bool ox, bool oy, bool oz, float mag, float& bound) {
     if (bin >= width)
       return spill3(row[0] + bin, row[1] + bin, row[2] + bin, x, y, z, ox, oy, oz);
-    unsigned long long* const w = win + bin;
+    unsigned long long* const w = win + 3u * static_cast<uint32_t>(bin);
     if (unchecked) {
       if (ox) atomicAdd(w, static_cast<unsigned long long>(x));
-      if (oy) atomicAdd(w + width, static_cast<unsigned long long>(y));
-      if (oz) atomicAdd(w + 2 * width, static_cast<unsigned long long>(z));
+      if (oy) atomicAdd(w + 1, static_cast<unsigned long long>(y));
+      if (oz) atomicAdd(w + 2, static_cast<unsigned long long>(z));
       bound += mag;
       return ox && oy && oz;
     }
     unsigned long long const px = ox ? atomicAdd(w, static_cast<unsigned long long>(x)) : 0ull;
-    unsigned long long const py = oy ? atomicAdd(w + width, static_cast<unsigned long long>(y)) : 0ull;
-    unsigned long long const pz =
-        oz ? atomicAdd(w + 2 * width, static_cast<unsigned long long>(z)) : 0ull;
+    unsigned long long const py = oy ? atomicAdd(w + 1, static_cast<unsigned long long>(y)) : 0ull;
+    unsigned long long const pz = oz ? atomicAdd(w + 2, static_cast<unsigned long long>(z)) : 0ull;
     return ox && oy && oz && no_overflow3(px, x, py, y, pz, z);
   }
   __device__ __forceinline__ void addf3(uint64_t bin, double x, double y, double z) {
@@ -165,11 +191,34 @@ struct WindowSink {
       spillf3(frow[0] + bin, frow[1] + bin, frow[2] + bin, x, y, z);
       return;
     }
-    double* const w = fwin + bin;
+    double* const w = fwin + 3u * static_cast<uint32_t>(bin);
     atomicAdd(w, x);
-    atomicAdd(w + width, y);
-    atomicAdd(w + 2 * width, z);
+    atomicAdd(w + 1, y);
+    atomicAdd(w + 2, z);
   }
+};
+
+// A window of differences (see deposit_differences) that holds the whole
+// trace: a value at one bin is that value there and its negative at the next.
+struct DifferenceSink {
+  unsigned long long* win;
+  uint32_t width;
+  __device__ __forceinline__ void add(uint32_t bin, long long x, long long y, long long z) {
+    unsigned long long* w = win + 3u * bin;
+    asm volatile("" : "+l"(w));
+    atomicAdd(w, static_cast<unsigned long long>(x));
+    atomicAdd(w + 1, static_cast<unsigned long long>(y));
+    atomicAdd(w + 2, static_cast<unsigned long long>(z));
+  }
+  __device__ __forceinline__ bool add3(uint64_t bin, long long x, long long y, long long z,
+                                       bool ox, bool oy, bool oz, float mag, float& bound) {
+    uint32_t const b = static_cast<uint32_t>(bin);
+    add(b, x, y, z);
+    if (b + 1u < width) add(b + 1u, -x, -y, -z);
+    bound += mag;
+    return ox && oy && oz;
+  }
+  __device__ __forceinline__ void addf3(uint64_t, double, double, double) {}  // fixed point only
 };
 
 // ---------------------------------------------------------------- add_sample
@@ -395,6 +444,14 @@ __device__ __forceinline__ int coreas_common(Track const& t, Propagation const& 
   return kCoreasDeposited;
 }
 
+// The windowed kernels' work item in shared memory: its observer, the filtered
+// paths' constants of it, and the number of its deferred pairs.  At namespace
+// scope, so that the track loops, functions of their own, address them directly.
+__shared__ ObserverCache s_observer;
+__shared__ LeanObserver s_lean;
+__shared__ unsigned s_deferred_total;
+__shared__ unsigned* s_deferred_list;  // this CTA's list (global memory)
+
 // The packed word's flags (kTrackRegular, ...) and FP32 constant.
 __device__ __forceinline__ unsigned pack_flags(double pack) {
   return static_cast<unsigned>(__double2hiint(pack));
@@ -410,17 +467,17 @@ struct LeanPoint {
   double dx, dy, dz, dist, inverse, x, w, factor, along;
   bool ok;
 };
-__device__ __forceinline__ LeanPoint lean_point(ObserverCache const& o, LeanObserver const& l, double sx, double sy,
-                                                double sz, double t, double bx, double by, double bz,
+__device__ __forceinline__ LeanPoint lean_point(LeanObserver const& l, double sx, double sy, double sz,
+                                                double t, double bx, double by, double bz,
                                                 double factor, double index) {
   LeanPoint r;
-  r.dx = o.px - sx;
-  r.dy = o.py - sy;
-  r.dz = o.pz - sz;
+  r.dx = l.px - sx;
+  r.dy = l.py - sy;
+  r.dz = l.pz - sz;
   double const s2 = fma(r.dz, r.dz, fma(r.dy, r.dy, r.dx * r.dx));
   r.ok = lean_rsqrt(s2, r.inverse);
   r.dist = s2 * r.inverse;
-  r.x = fma(r.dist, factor * l.rate_over_c, (t - o.start_time) * l.rate);
+  r.x = fma(r.dist, factor * l.rate_over_c, (t - l.start_time) * l.rate);
   r.w = fma(bz, r.dz, fma(by, r.dy, bx * r.dx)) * r.inverse;
   r.factor = fma(-index, r.w, 1.);
   r.along = r.w * r.inverse;
@@ -461,16 +518,16 @@ __device__ __forceinline__ bool lean_gate(double x, LeanObserver const& l, int& 
 // component when counting samples).  Every component is below 2^61.
 template <bool kUnchecked>
 __device__ __forceinline__ void lean_add(WindowSink& sink, LeanObserver const& l, int bin, float vx, float vy,
-                                         float vz, float a, Counts& c) {
+                                         float vz, float a, Tally& c) {
   long long const x = __float2ll_rn(fmaf(vx, a, l.bias)), y = __float2ll_rn(fmaf(vy, a, l.bias)),
                   z = __float2ll_rn(fmaf(vz, a, l.bias));
   if (kUnchecked) {
     // through a generic pointer (see deposit_unchecked)
-    unsigned long long* w = sink.win + bin;
+    unsigned long long* w = sink.win + 3u * static_cast<unsigned>(bin);
     asm volatile("" : "+l"(w));
     atomicAdd(w, static_cast<unsigned long long>(x));
-    atomicAdd(w + sink.width, static_cast<unsigned long long>(y));
-    atomicAdd(w + 2 * sink.width, static_cast<unsigned long long>(z));
+    atomicAdd(w + 1, static_cast<unsigned long long>(y));
+    atomicAdd(w + 2, static_cast<unsigned long long>(z));
     ++c.coreas;
   } else {
     float const mag = (fabsf(vx) + fabsf(vy) + fabsf(vz)) * fabsf(a) + 3.f * l.bias;
@@ -487,7 +544,7 @@ __device__ __forceinline__ void lean_add(WindowSink& sink, LeanObserver const& l
 // |components| (each factor's roundings inside 2^-20).
 template <bool kUnchecked>
 __device__ __forceinline__ bool lean_samples(WindowSink& sink, LeanObserver const& l, double xs, double xe,
-                                             Vec3<float> s, float as, Vec3<float> e, float ae, Counts& c) {
+                                             Vec3<float> s, float as, Vec3<float> e, float ae, Tally& c) {
   int bs, be;
   bool ins, ine;
   bool decided = lean_gate(xs, l, bs, ins);
@@ -510,16 +567,14 @@ __device__ __forceinline__ bool lean_samples(WindowSink& sink, LeanObserver cons
 // deposited nothing.  kPre: the points' source terms are the track's columns.
 //
 // Against exact times (a square root and four divisions an endpoint) and an
-// FP32 cross product the pair takes 358 instead of 621 warp instructions:
-// 1e7 x 160 x 8192 CoREAS 41.6 -> 27.4 ms, 5e6 x 64 in ice 9.0 -> 5.2 ms, and the
+// FP32 cross product the pair takes 344 instead of 621 warp instructions:
+// 1e7 x 160 x 8192 CoREAS 41.6 -> 22.5 ms, 5e6 x 64 in ice 9.0 -> 3.9 ms, and the
 // traces' relative error falls from 6e-7 to 1.1e-7.  What bounds it now is the
-// latency of the FP64 chain and of the track loads at 20 warps an SM (46% of
-// issue slots), with the atomics at 60% of the shared-memory pipe; blocks of
-// 512 / 768 / 1024 threads ran 30.6 / 33.1 (spills) / 30.2 ms.
+// shared-memory pipe (74% busy, mostly the six 64-bit atomics) beside 58% of the
+// issue slots.
 template <bool kPre, bool kUnchecked>
 __device__ __forceinline__ int coreas_lean(double2 const* __restrict__ r, Propagation const& p,
-                                           ObserverCache const& o, LeanObserver const& l, WindowSink& sink,
-                                           Counts& c) {
+                                           LeanObserver const& l, WindowSink& sink, Tally& c) {
   constexpr unsigned T = kTrackTile;
   double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T),
                 cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
@@ -531,13 +586,13 @@ __device__ __forceinline__ int coreas_lean(double2 const* __restrict__ r, Propag
     ts = SourceTerms{s.x, s.y, dense_index(flags)};
     te = SourceTerms{e.x, e.y, 0.};
   } else {
-    Destination const d = destination_of(o);
+    Destination const d = destination_of(s_observer);
     ts = source_terms(p, d, cb.x);
     te = source_terms(p, d, cc.y);
-    ok = ok & lean_index(ts.n_src) & lean_index(te.n_src);
+    ok = ok & lean_terms(ts) & lean_terms(te);
   }
-  LeanPoint const s = lean_point(o, l, ca.x, ca.y, cb.x, ct.x, cd.x, cd.y, ce.x, ts.factor, ts.n_src);
-  LeanPoint const e = lean_point(o, l, cb.y, cc.x, cc.y, ct.y, cd.x, cd.y, ce.x, te.factor, te.n_src);
+  LeanPoint const s = lean_point(l, ca.x, ca.y, cb.x, ct.x, cd.x, cd.y, ce.x, ts.factor, ts.n_src);
+  LeanPoint const e = lean_point(l, cb.y, cc.x, cc.y, ct.y, cd.x, cd.y, ce.x, te.factor, te.n_src);
   bool const dense = ts.n_dst > 1.;
   ok = ok & s.ok & e.ok;
   double const least = fmin(fabs(s.factor), fabs(e.factor));
@@ -574,8 +629,8 @@ __device__ __forceinline__ int coreas_lean(double2 const* __restrict__ r, Propag
 // guard cannot decide.
 template <bool kPre>
 __device__ __forceinline__ bool near_cone_lean(double2 const* __restrict__ r, bool start_before_end,
-                                               Propagation const& p, ObserverCache const& o,
-                                               LeanObserver const& l, WindowSink& sink, Counts& c) {
+                                               Propagation const& p, LeanObserver const& l, WindowSink& sink,
+                                               Tally& c) {
   constexpr unsigned T = kTrackTile;
   double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T),
                 cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
@@ -586,15 +641,15 @@ __device__ __forceinline__ bool near_cone_lean(double2 const* __restrict__ r, bo
     double2 const mid = __ldg(r + kFactorMid / 2 * T);
     m = SourceTerms{mid.x, mid.y, 0.};
   } else {
-    m = source_terms(p, destination_of(o), mz);
+    m = source_terms(p, destination_of(s_observer), mz);
   }
-  LeanPoint const s = lean_point(o, l, (ca.x + cb.y) * 0.5, (ca.y + cc.x) * 0.5, mz, (ct.x + ct.y) * 0.5, cd.x,
+  LeanPoint const s = lean_point(l, (ca.x + cb.y) * 0.5, (ca.y + cc.x) * 0.5, mz, (ct.x + ct.y) * 0.5, cd.x,
                                  cd.y, ce.x, m.factor, m.n_src);
   double const dt = (ct.y - ct.x) * l.rate * fabs(s.factor);
   // |factor| > 8 guards: its sign and the field's are the reference's.  Where
   // the samples share a bin the field is scaled by dt, which carries the
   // same factor, so a small one costs no precision.
-  if (!((flags & kTrackRegular) && l.usable && s.ok && lean_index(m.n_src) && fabs(s.factor) > 8. * kDopplerGuard &&
+  if (!((flags & kTrackRegular) && l.usable && s.ok && lean_terms(m) && fabs(s.factor) > 8. * kDopplerGuard &&
         fabs(dt - 1.) > 2. * kBinGuard && dt > 2. * kBinGuard))
     return false;
   double low = fma(-0.5, dt, s.x), high = fma(0.5, dt, s.x);
@@ -876,7 +931,7 @@ __device__ __forceinline__ bool surely_undivided(LeanPoint const& m, LeanObserve
 // potential's sign times 1 / (1 - n w) is 1 / |1 - n w|.  False when a guard
 // cannot decide (the caller evaluates the segment exactly).
 __device__ __forceinline__ bool zhs_lean(LeanPoint const& m, double half_bins, float constant, double bx, double by,
-                                         double bz, ObserverCache const& o, bool subdivided,
+                                         double bz, LeanObserver const& l, bool subdivided,
                                          StagedSegment<float>& out) {
   double const reach = fabs(half_bins * m.factor);
   double const x1 = m.x - reach, x2 = m.x + reach;
@@ -888,7 +943,7 @@ __device__ __forceinline__ bool zhs_lean(LeanPoint const& m, double half_bins, f
   double const r1 = lean_nearest(x1, b1), r2 = lean_nearest(x2, b2);
   bool const decided = (fabs(r1) < 0.5 - kBinGuard) & (fabs(r2) < 0.5 - kBinGuard) & (reach > kBinGuard) &
                        (fabs(m.factor) >= 1.e-6);
-  if ((x2 < -1.) | (x1 > o.bins_d + 1.)) return m.ok;  // off the trace
+  if ((x2 < -1.) | (x1 > l.past)) return m.ok;  // off the trace
   // from here |x1|, |x2| < 2^27: reach is below 2^25 and one of them is near the trace
   float const amplitude = __fdividef(constant, static_cast<float>(fabs(m.factor) * m.dist));
   out.perp = Vec3<float>{static_cast<float>(fma(-m.dx, m.along, bx)), static_cast<float>(fma(-m.dy, m.along, by)),
@@ -897,7 +952,7 @@ __device__ __forceinline__ bool zhs_lean(LeanPoint const& m, double half_bins, f
   out.last = amplitude * static_cast<float>(single ? 2. * reach : r2 + 0.5);
   out.first = amplitude * static_cast<float>(0.5 - r1);
   out.mid = (subdivided & (m.factor < 0.)) ? -amplitude : amplitude;
-  unsigned const bins = static_cast<unsigned>(o.bins);
+  unsigned const bins = l.bins;
   if (static_cast<unsigned>(b2) < bins) {
     out.last_bin = static_cast<unsigned>(b2);
     out.flags = 2u;
@@ -988,9 +1043,9 @@ __device__ __forceinline__ void deposit_staged(StagedSegment<Amp>* staging,
 // then converts and adds each sample with no check.  Returns false when a
 // sample might not convert (huge or non-finite values): the pair then goes to
 // the checked drain.
-template <class Amp>
-__device__ __forceinline__ bool account_staged(StagedSegment<Amp> const& seg, ObserverCache const& o,
-                                               Counts& c) {
+template <class Amp, class Tallies>
+__device__ __forceinline__ bool account_staged(StagedSegment<Amp> const& seg, LeanObserver const& l,
+                                               Tallies& c) {
   uint32_t const samples = seg.count + ((seg.flags >> 1) & 1u);
   if (samples == 0u) return true;
   bool const has_first = (seg.flags & 1u) != 0u;
@@ -1000,11 +1055,11 @@ __device__ __forceinline__ bool account_staged(StagedSegment<Amp> const& seg, Ob
   Amp const am = mids ? fabs(seg.mid) : zero;
   Amp const al = (seg.flags & 2u) ? fabs(seg.last) : zero;
   // staged FP32 values are in fixed-point units; when counting samples each component adds 1
-  Amp const fs = sizeof(Amp) == sizeof(float) ? static_cast<Amp>(1) : static_cast<Amp>(o.fixed_scale);
+  Amp const fs = sizeof(Amp) == sizeof(float) ? static_cast<Amp>(1) : static_cast<Amp>(l.fixed_scale);
   Amp const width = (fabs(seg.perp.x) + fabs(seg.perp.y) + fabs(seg.perp.z)) * fs;
   if (!(width * fmax(fmax(af, am), al) < static_cast<Amp>(0x1p62))) return false;  // also NaN and infinities
-  Amp const sum = o.count_samples ? static_cast<Amp>(3u * samples)
-                                  : (af + am * static_cast<Amp>(mids) + al) * width;
+  Amp const sum = (af + am * static_cast<Amp>(mids) + al) * width +
+                  static_cast<Amp>(3u * samples) * static_cast<Amp>(l.bias);
   c.zhs += samples;
   Amp const bound = sum * static_cast<Amp>(1. + 0x1p-20);
   c.mag += sizeof(Amp) == sizeof(float) ? static_cast<float>(bound)
@@ -1013,12 +1068,19 @@ __device__ __forceinline__ bool account_staged(StagedSegment<Amp> const& seg, Ob
 }
 
 // The fixed-point value of one staged component, as to_fixed computes it; 1
-// when counting samples (then scale 0, bias 1).
-__device__ __forceinline__ long long fixed_value(float v, float amplitude, float scale, float bias) {
-  return __float2ll_rn(fmaf(v * amplitude, scale, bias));
+// when counting samples (the amplitude or the scale is 0 then, the bias 1).
+__device__ __forceinline__ long long fixed_value(float v, float amplitude, float, float bias) {
+  return __float2ll_rn(fmaf(v, amplitude, bias));
 }
 __device__ __forceinline__ long long fixed_value(double v, double amplitude, double scale, double bias) {
   return __double2ll_rn(fma(v * amplitude, scale, bias));
+}
+
+// Adds a bin's three components to its words of a window (a generic pointer).
+__device__ __forceinline__ void add_words(unsigned long long* words, Vec3<long long> v) {
+  atomicAdd(words, static_cast<unsigned long long>(v.x));
+  atomicAdd(words + 1, static_cast<unsigned long long>(v.y));
+  atomicAdd(words + 2, static_cast<unsigned long long>(v.z));
 }
 
 // The unchecked deposit of a staged segment as differences: the window holds
@@ -1027,7 +1089,9 @@ __device__ __forceinline__ long long fixed_value(double v, double amplitude, dou
 // bin, so it touches at most four bins -- start, start + 1, the bin after the
 // run (its last sample) and the next -- whatever its length, each lane on its
 // own: no redistribution over the warp (a prefix sum, searches by shuffle and
-// 40 bytes staged a lane in the former version).  On the 1e7 x 160 workload 55% of the
+// 40 bytes staged a lane in the former version, 764 and 143 warp instructions per
+// 32 pairs with the drain; with the filtered segment it takes 370 in all, ZHS of
+// the 1e7 x 160 workload 59.4 -> 23.0 ms).  On the 1e7 x 160 workload 55% of the
 // segments have one sample, 26% two, 17% more (2.0 samples a pair, 2.6
 // differences).  The sums of differences are exact modulo 2^64, and the
 // item's bound (account_staged) shows that no bin's value leaves the int64
@@ -1036,28 +1100,20 @@ __device__ __forceinline__ long long fixed_value(double v, double amplitude, dou
 // GPU executes as about one instruction per active lane (twice the atomic
 // wavefronts of generic adds on the same samples).
 template <class Amp>
-__device__ __forceinline__ void deposit_differences(StagedSegment<Amp> const& seg, ObserverCache const& o,
-                                                    WindowSink const& sink) {
+__device__ __forceinline__ void deposit_differences(StagedSegment<Amp> const& seg, LeanObserver const& l,
+                                                    unsigned long long* win, uint32_t width) {
   bool const last = (seg.flags & 2u) != 0u;
   if (seg.count == 0u && !last) return;
-  Amp const one = static_cast<Amp>(1);
-  Amp const bias = o.count_samples ? one : static_cast<Amp>(0);
-  Amp const unit = sizeof(Amp) == sizeof(float) ? one : static_cast<Amp>(o.fixed_scale);
-  Amp const scale = o.count_samples ? static_cast<Amp>(0) : unit;
-  unsigned long long* win = sink.win;
+  // FP32 values are staged in fixed-point units, 0 when counting samples
+  Amp const bias = static_cast<Amp>(l.bias);
+  Amp const scale = sizeof(Amp) == sizeof(float) ? static_cast<Amp>(1) : static_cast<Amp>(l.fixed_scale);
   asm volatile("" : "+l"(win));
-  uint32_t const width = sink.width;
   auto value = [&](Amp amplitude) {
     return Vec3<long long>{fixed_value(seg.perp.x, amplitude, scale, bias),
                            fixed_value(seg.perp.y, amplitude, scale, bias),
                            fixed_value(seg.perp.z, amplitude, scale, bias)};
   };
-  auto add = [&](uint32_t bin, Vec3<long long> v) {
-    unsigned long long* const w = win + bin;
-    atomicAdd(w, static_cast<unsigned long long>(v.x));
-    atomicAdd(w + width, static_cast<unsigned long long>(v.y));
-    atomicAdd(w + 2 * width, static_cast<unsigned long long>(v.z));
-  };
+  auto add = [&](uint32_t bin, Vec3<long long> v) { add_words(win + 3u * bin, v); };
   Vec3<long long> run{0, 0, 0};  // the value up to the bin before `end`
   uint32_t const end = seg.start + seg.count;
   if (seg.count != 0u) {
@@ -1081,41 +1137,194 @@ __device__ __forceinline__ void deposit_differences(StagedSegment<Amp> const& se
   if (after < width) add(after, Vec3<long long>{-run.x, -run.y, -run.z});
 }
 
-// Turns a window of differences into the bins' values: a running sum over
-// each of its three rows.  Every thread of the CTA calls it.  Out of line, so
+// The samples of a staged segment one by one, each component converted only if
+// it can be (fixed point).
+template <class Amp, class Sink>
+__device__ __noinline__ Counts deposit_samples(StagedSegment<Amp> const seg, ObserverCache const& o, Sink sink) {
+  Counts c;
+  ObserverCache grid;
+  grid.fixed_scale = o.fixed_scale;
+  grid.fixed_scale_f = 1.f;  // staged FP32 values are in fixed-point units
+  grid.count_samples = o.count_samples;
+  for (uint32_t k = 0; k < seg.count; ++k) {
+    Amp const amplitude = k == 0u && (seg.flags & 1u) ? seg.first : seg.mid;
+    deposit_bin<true>(sink, seg.start + k, make_deposit<true>(grid, scaled(seg.perp, amplitude)), c.zhs, c.overflows,
+                      c.mag);
+  }
+  if (seg.flags & 2u)
+    deposit_bin<true>(sink, seg.last_bin, make_deposit<true>(grid, scaled(seg.perp, seg.last)), c.zhs, c.overflows,
+                      c.mag);
+  return c;
+}
+
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
+  return v;
+}
+
+// Turns a window of differences into the bins' values: a running sum of each
+// component over the bins.  Every thread of the CTA calls it.  Out of line, so
 // that its registers do not count in the track loops.
 __device__ __noinline__ void difference_window(unsigned long long* win, uint32_t width) {
-  __shared__ unsigned long long totals[3][32];
+  __shared__ unsigned long long totals[32];  // of each warp's bins, one component at a time
   unsigned const lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t per = (width + blockDim.x - 1) / blockDim.x;
   per |= 1u;  // an odd stride keeps the lanes' 64-bit words on different banks
   uint32_t const first = threadIdx.x * per < width ? threadIdx.x * per : width;
   uint32_t const stop = first + per < width ? first + per : width;
-  unsigned long long before[3];
   __syncthreads();
-  for (int row = 0; row < 3; ++row) {
-    unsigned long long const* const w = win + row * static_cast<size_t>(width);
-    unsigned long long sum = 0;
-    for (uint32_t j = first; j < stop; ++j) sum += w[j];
-    unsigned long long incl = sum;
+  unsigned long long sum[3] = {0, 0, 0};
+  for (uint32_t j = first; j < stop; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) sum[k] += win[3u * j + k];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    unsigned long long incl = sum[k];
     for (unsigned d = 1; d < 32u; d <<= 1) {
       unsigned long long const v = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += v;
     }
-    if (lane == 31u) totals[row][warp] = incl;
-    before[row] = incl - sum;
+    if (lane == 31u) totals[warp] = incl;
+    __syncthreads();
+    // the warps before this one: a lane takes one total, the warp adds them
+    sum[k] = incl - sum[k] + __shfl_sync(0xffffffffu, warp_sum(lane < warp ? totals[lane] : 0ull), 0);
+    __syncthreads();
   }
+  for (uint32_t j = first; j < stop; ++j)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      sum[k] += win[3u * j + k];
+      win[3u * j + k] = sum[k];
+    }
   __syncthreads();
-  for (int row = 0; row < 3; ++row) {
-    unsigned long long* const w = win + row * static_cast<size_t>(width);
-    unsigned long long sum = before[row];
-    for (unsigned k = 0; k < warp; ++k) sum += totals[row][k];
-    for (uint32_t j = first; j < stop; ++j) {
-      sum += w[j];
-      w[j] = sum;
+}
+
+// An undivided segment evaluated and deposited as differences in one go, in mixed
+// precision with the whole trace in the window: zhs_lean and
+// deposit_differences without the staged form between them, for segments that
+// lie on the trace whole (or off it whole).  The amplitudes and conversions are
+// those of zhs_lean's segments.  False, having deposited nothing, when a guard
+// cannot decide, an end of the trace cuts the segment or a value might not
+// convert.
+__device__ __forceinline__ bool zhs_lean_differences(LeanPoint const& m, double half_bins, float constant, double bx,
+                                                     double by, double bz, LeanObserver const& l,
+                                                     unsigned long long* win, Tally& c) {
+  double const reach = fabs(half_bins * m.factor);
+  double const x1 = m.x - reach, x2 = m.x + reach;
+  if ((x2 < -1.) | (x1 > l.past)) return m.ok;  // off the trace
+  int b1, b2;
+  double const r1 = lean_nearest(x1, b1), r2 = lean_nearest(x2, b2);
+  bool const decided = (fabs(r1) < 0.5 - kBinGuard) & (fabs(r2) < 0.5 - kBinGuard) & (reach > kBinGuard) &
+                       (fabs(m.factor) >= 1.e-6) & (static_cast<unsigned>(b1) < l.bins) &
+                       (static_cast<unsigned>(b2) < l.bins) & m.ok;
+  float const amplitude = __fdividef(constant, static_cast<float>(fabs(m.factor) * m.dist));
+  Vec3<float> const perp{static_cast<float>(fma(-m.dx, m.along, bx)), static_cast<float>(fma(-m.dy, m.along, by)),
+                         static_cast<float>(fma(-m.dz, m.along, bz))};
+  int const bins = b2 - b1;  // after the first
+  float const first = amplitude * static_cast<float>(0.5 - r1);
+  float const last = amplitude * static_cast<float>(bins == 0 ? 2. * reach : r2 + 0.5);
+  // every |sample| is at most |perp|_1 |amplitude|; the roundings lie inside 2^-20
+  float const width = fabsf(perp.x) + fabsf(perp.y) + fabsf(perp.z);
+  if (!(decided & (width * fabsf(amplitude) < 0x1p60f))) return false;  // also NaN and infinities
+  unsigned const samples = static_cast<unsigned>(bins) + 1u;
+  float const between = bins == 0 ? fabsf(last) : fabsf(first) + fabsf(last) + static_cast<float>(bins - 1) * fabsf(amplitude);
+  c.zhs += samples;
+  c.mag = fmaf(between * width, 1.f + 0x1p-20f, c.mag) + static_cast<float>(3u * samples) * l.bias;
+  auto value = [&](float a) {
+    return Vec3<long long>{fixed_value(perp.x, a, 1.f, l.bias), fixed_value(perp.y, a, 1.f, l.bias),
+                           fixed_value(perp.z, a, 1.f, l.bias)};
+  };
+  // through a generic pointer (see deposit_differences)
+  unsigned long long* w = win + 3u * static_cast<unsigned>(b1);
+  asm volatile("" : "+l"(w));
+  Vec3<long long> run{0, 0, 0};
+  if (bins > 0) {
+    run = value(first);
+    add_words(w, run);
+    if (bins > 1) {
+      Vec3<long long> const mid = value(amplitude);
+      add_words(w + 3, Vec3<long long>{mid.x - run.x, mid.y - run.y, mid.z - run.z});
+      run = mid;
     }
   }
-  __syncthreads();
+  Vec3<long long> const v = value(last);
+  unsigned long long* const end = w + 3 * bins;
+  add_words(end, Vec3<long long>{v.x - run.x, v.y - run.y, v.z - run.z});
+  if (static_cast<unsigned>(b2) + 1u < l.bins) add_words(end + 3, Vec3<long long>{-v.x, -v.y, -v.z});
+  return true;
+}
+
+// The FP64 counterpart: an undivided segment evaluated exactly (zhs_stage's
+// operations and decisions) and deposited as differences in one go.  Its fields
+// are formed one at a time as they are deposited, where a staged segment holds
+// six FP64 values a lane at once (which spilled the track loop at 640 threads).
+__device__ __forceinline__ bool zhs_exact_differences(Path const& path, double t1, double t2, double mt, double bx,
+                                                      double by, double bz, double constant, ObserverCache const& o,
+                                                      LeanObserver const& l, unsigned long long* win, Tally& c) {
+  double const bk = bx * path.kx + by * path.ky + bz * path.kz;
+  double const nbk = path.n_src * bk;
+  double d1 = t1 + path.time - nbk * (t1 - mt);
+  double d2 = t2 + path.time - nbk * (t2 - mt);
+  double sign = 1.;
+  if (d1 > d2) {
+    double const swap = d1;
+    d1 = d2;
+    d2 = swap;
+    sign = -1.;
+  }
+  double const fs = o.sample_rate;
+  double const x1 = (d1 - o.start_time) * fs;
+  double const x2 = (d2 - o.start_time) * fs;
+  if ((x2 < -1.) | (x1 > l.past)) return true;  // off the trace
+  // on the trace whole (an end that cuts the segment is left to the drain); then
+  // floor(x + 0.5) is an int
+  double const sb = floor(x1 + 0.5), eb = floor(x2 + 0.5);
+  if (!((sb >= 0.) & (eb < o.bins_d) & (x1 >= -0.5) & (nearest_bin(x1) == sb) & (nearest_bin(x2) == eb))) return false;
+  int const b1 = static_cast<int>(sb), bins = static_cast<int>(eb) - b1;
+  double const f1 = fabs(x1 - floor(x1) - 0.5);
+  double const mag = fabs(x1) + static_cast<double>(bins) + fabs(d1 * fs) + fabs(l.start_bins) + 2.;
+  // the consecutive-run test of zhs_segment
+  if (bins > 1 && !(mag < 0x1p50 && f1 > mag * 0x1p-48)) return false;
+  double const den = 1. - nbk;
+  Vec3<double> const k{path.kx, path.ky, path.kz};
+  Vec3<double> const perp = cross(k, cross(Vec3<double>{bx, by, bz}, k));
+  double const sc = sign * constant;
+  double const dd = den * path.dist;
+  bool const tiny = !(fabs(den) > 1.e-15);
+  double const frac_last = bins == 0 ? (tiny ? (t2 - t1) * fs : fabs(d2 * fs - d1 * fs)) : fabs(x2 + 0.5 - eb);
+  double const last = sc * frac_last / (bins == 0 && tiny ? path.dist : dd);
+  double first = 0., mid = 0.;
+  if (bins > 0) first = sc * fabs(sb + 0.5 - x1) / dd;
+  if (bins > 1) mid = sc / dd;
+  double const width = (fabs(perp.x) + fabs(perp.y) + fabs(perp.z)) * l.fixed_scale;
+  if (!(width * fmax(fmax(fabs(first), fabs(mid)), fabs(last)) < 0x1p60)) return false;  // also NaN and infinities
+  unsigned const samples = static_cast<unsigned>(bins) + 1u;
+  c.zhs += samples;
+  c.mag += __double2float_ru((fabs(first) + fabs(last) + fabs(mid) * static_cast<double>(bins > 1 ? bins - 1 : 0)) *
+                                 width * (1. + 0x1p-20) +
+                             static_cast<double>(3u * samples) * static_cast<double>(l.bias));
+  double const bias = static_cast<double>(l.bias);
+  auto value = [&](double a) {
+    return Vec3<long long>{fixed_value(perp.x, a, l.fixed_scale, bias), fixed_value(perp.y, a, l.fixed_scale, bias),
+                           fixed_value(perp.z, a, l.fixed_scale, bias)};
+  };
+  unsigned long long* w = win + 3u * static_cast<unsigned>(b1);
+  asm volatile("" : "+l"(w));
+  Vec3<long long> run{0, 0, 0};
+  if (bins > 0) {
+    run = value(first);
+    add_words(w, run);
+    if (bins > 1) {
+      Vec3<long long> const v = value(mid);
+      add_words(w + 3, Vec3<long long>{v.x - run.x, v.y - run.y, v.z - run.z});
+      run = v;
+    }
+  }
+  Vec3<long long> const v = value(last);
+  unsigned long long* const end = w + 3 * bins;
+  add_words(end, Vec3<long long>{v.x - run.x, v.y - run.y, v.z - run.z});
+  if (static_cast<unsigned>(b1 + bins) + 1u < l.bins) add_words(end + 3, Vec3<long long>{-v.x, -v.y, -v.z});
+  return true;
 }
 
 // accumulate_zhs, RadioProjection.inl:483-529, every decision exact.
@@ -1169,58 +1378,73 @@ __device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
         static_cast<long long>(subtracks * (refinement - 1)));
 }
 
-// The common ZHS pair of the windowed kernel: one undivided segment, staged,
-// from the track's columns `r`.  Returns false, staging nothing (`seg`
-// cleared), when the track is or might be subdivided (the Fraunhofer number
-// not surely below 1, or refinement) or when the segment cannot be staged; the
-// kernel then defers the pair to zhs_drain.  Mixed precision (Amp = float)
-// stages by the filtered arithmetic, FP64 exactly; both decide "one segment"
-// from the filtered midpoint, which spares FP64 the exact Fraunhofer number
-// (a square root and seven divisions).  `row` addresses the same track's
-// columns from the work item's first one.
-//
-// With the filtered segment and its deposit as differences a pair takes 450
-// instead of 764 warp instructions: 1e7 x 160 x 8192 ZHS 59.4 -> 32.9 ms, FP64 at
-// 1e6 x 160 10.4 -> 7.3 ms.
-template <bool kFixed, bool kPre, class Amp>
-__device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propagation const& p,
-                                           ObserverCache const& o, LeanObserver const& l, Counts& c,
-                                           StagedSegment<Amp>& seg) {
+// The segment of an undivided track seen from the item's observer, from the
+// track's columns `r`, by the filtered arithmetic.  `one`: the track is surely
+// one segment (the Fraunhofer number surely below 1, no refinement) and inside
+// the filtered paths' bounds.
+struct ZhsPoint {
+  LeanPoint m;
+  double half_bins, bx, by, bz;
+  float constant;
+  SourceTerms terms;
+  bool one;
+};
+template <bool kPre, bool kMayRefine>
+__device__ __forceinline__ ZhsPoint zhs_point(double2 const* __restrict__ r, Propagation const& p,
+                                              LeanObserver const& l) {
   constexpr unsigned T = kTrackTile;
-  double2 const cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T), cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T),
-                ch = __ldg(r + 11 * T);
+  double2 const cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T), cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T);
+  double const half = __ldg(reinterpret_cast<double const*>(r + kHalf / 2 * T));
   unsigned const flags = pack_flags(ce.y);
-  SourceTerms st;
+  ZhsPoint z;
   if (kPre) {
     double2 const m = __ldg(r + kFactorMid / 2 * T);
-    st = SourceTerms{m.x, m.y, 0.};
+    z.terms = SourceTerms{m.x, m.y, 0.};
   } else {
-    st = source_terms(p, destination_of(o), cn.x);
+    z.terms = source_terms(p, destination_of(s_observer), cn.x);
   }
-  LeanPoint const m = lean_point(o, l, cm.x, cm.y, cn.x, cn.y, cd.x, cd.y, ce.x, st.factor, st.n_src);
-  double const half = ch.x * l.rate;
-  bool staged = ((flags & kTrackRegular & l.usable) != 0u) & (p.refinement == 1u) & m.ok &
-                surely_undivided(m, l, half, cd.x, cd.y, ce.x);
-  if (!kPre) staged = staged & lean_index(st.n_src);
+  z.bx = cd.x;
+  z.by = cd.y;
+  z.bz = ce.x;
+  z.m = lean_point(l, cm.x, cm.y, cn.x, cn.y, cd.x, cd.y, ce.x, z.terms.factor, z.terms.n_src);
+  z.half_bins = half * l.rate;
+  z.constant = pack_constant(ce.y) * l.scale;
+  z.one = ((flags & kTrackRegular & l.usable) != 0u) & (!kMayRefine || p.refinement == 1u) & z.m.ok &
+          surely_undivided(z.m, l, z.half_bins, cd.x, cd.y, ce.x);
+  if (!kPre) z.one = z.one & lean_terms(z.terms);
+  return z;
+}
+
+// The common ZHS pair of the windowed kernel: one undivided segment, staged.
+// Returns false, staging nothing (`seg` cleared), when the track is or might be
+// subdivided or when the segment cannot be staged; the kernel then defers the
+// pair to a drain.  Mixed precision (Amp = float) stages by the filtered
+// arithmetic, FP64 exactly; both decide "one segment" from the filtered
+// midpoint, which spares FP64 the exact Fraunhofer number (a square root and
+// seven divisions).
+template <bool kFixed, bool kPre, bool kMayRefine, class Amp>
+__device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propagation const& p,
+                                           LeanObserver const& l, StagedSegment<Amp>& seg) {
+  constexpr unsigned T = kTrackTile;
+  ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
+  bool staged = z.one;
   if constexpr (sizeof(Amp) == sizeof(float)) {
-    staged = zhs_lean(m, half, pack_constant(ce.y) * l.scale, cd.x, cd.y, ce.x, o, false, seg) & staged;
+    staged = zhs_lean(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, false, seg) & staged;
   } else if (staged) {
-    double2 const ct = __ldg(r + 3 * T);
+    double2 const cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T), ct = __ldg(r + 3 * T);
     Track t;
-    t.bx = cd.x;
-    t.by = cd.y;
-    t.bz = ce.x;
-    t.constant = ch.y;
-    staged = zhs_stage<kFixed, Amp, true>(cm.x, cm.y, cn.x, ct.x, ct.x + (ct.y - ct.x), cn.y, t, p, o, false, seg,
-                                          st);
+    t.bx = z.bx;
+    t.by = z.by;
+    t.bz = z.bz;
+    t.constant = __ldg(r + kConst / 2 * T).y;
+    staged = zhs_stage<kFixed, Amp, true>(cm.x, cm.y, cn.x, ct.x, ct.x + (ct.y - ct.x), cn.y, t, p,
+                                          copy_words(s_observer), false, seg, z.terms);
   }
   if (!staged) {
     seg.count = 0u;
     seg.flags = 0u;
-    return false;
   }
-  c.subtracks += 1ull;
-  return true;
+  return staged;
 }
 
 // ---------------------------------------------------------------- helpers
@@ -1258,10 +1482,6 @@ __device__ __forceinline__ Track load_staged_track(double const* base, unsigned 
   return unpack_track([&](unsigned k) { return r[k]; });
 }
 
-__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
-  for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
-  return v;
-}
 __device__ __forceinline__ double warp_sum(double v) {
   for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(0xffffffffu, v, d);
   return v;
@@ -1269,14 +1489,6 @@ __device__ __forceinline__ double warp_sum(double v) {
 __device__ __forceinline__ double warp_max(double v) {
   for (int d = 16; d > 0; d >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, d));
   return v;
-}
-
-__device__ __forceinline__ void add_counts(Counts& c, Counts const& d) {
-  c.coreas += d.coreas;
-  c.zhs += d.zhs;
-  c.subtracks += d.subtracks;
-  c.overflows += d.overflows;
-  c.mag += d.mag;
 }
 
 // Adds per-thread counts into the event counters: one atomic per warp.
@@ -1391,8 +1603,7 @@ __global__ void __launch_bounds__(256) ingest_kernel(
                  mz = (t.sz + (t.sz + (t.ez - t.sz))) * 0.5;
     double const t2 = t.ts + (t.te - t.ts);
     double const tm = (t.ts + t2) * 0.5;
-    bool regular = fabs(t.bx) + fabs(t.by) + fabs(t.bz) <= 4. && fabs(t.ts) <= terms.limits.time &&
-                   fabs(t.te) <= terms.limits.time && duration <= terms.limits.duration;
+    bool regular = regular_track(t, duration, terms.limits);
     unsigned flags = 0u;
     if (terms.enabled) {
       // the source points of the windowed kernels
@@ -1406,7 +1617,7 @@ __global__ void __launch_bounds__(256) ingest_kernel(
       r[6 * T] = make_double2(s.factor, s.n_src);
       r[7 * T] = make_double2(e.factor, e.n_src);
       r[8 * T] = make_double2(m.factor, m.n_src);
-      regular = regular && lean_index(s.n_src) && lean_index(e.n_src) && lean_index(m.n_src);
+      regular = regular && lean_terms(s) && lean_terms(e) && lean_terms(m);
       if (s.n_dst > 1.) flags |= kTrackDense;
       if (mc.factor == m.factor && mc.n_src == m.n_src) flags |= kTrackOneMid;
     }
@@ -1635,21 +1846,17 @@ __global__ void __launch_bounds__(kTileThreads) tiled_kernel(const __grid_consta
 // 117.0, 480 128.5.
 constexpr int kZhsThreadsFloat = 768;
 constexpr int kZhsThreadsDouble = 384;
-// Two passes (fixed point): the track loop alone runs larger CTAs.  FP32 1024
-// threads (1e7 x 160 workload, ZHS ms at 640 / 768 / 896 / 1024 threads: 39.8 /
-// 36.3 / 33.9 / 32.9), FP64 640 (1e6 x 160: 8.5 at 480, 7.3 at 640); the drain
-// pass FP32 512, FP64 384.
+// Two passes (fixed point): the first, whose track loop is a function of its own,
+// runs larger CTAs.  FP32 1024 threads (1e7 x 160 workload: 23.0 ms, 24.0 at 896),
+// FP64 640.
 constexpr int kZhsLoopThreadsFloat = 1024;
 constexpr int kZhsLoopThreadsDouble = 640;
-constexpr int kZhsDrainThreadsFloat = 512;
-constexpr int kZhsDrainThreadsDouble = 384;
-// kPass: 0 one pass; of a two-pass launch 1 the track loop, 2 the drain, 3
-// the handed-back items in full (as one pass).
+// kPass: 0 one pass; of a two-pass launch 1 the first, 3 the handed-back items
+// in full (as one pass).
 template <class Amp, int kPass = 0>
 constexpr int zhs_threads_max() {
-  return kPass == 2   ? (sizeof(Amp) == sizeof(float) ? kZhsDrainThreadsFloat : kZhsDrainThreadsDouble)
-         : kPass == 1 ? (sizeof(Amp) == sizeof(float) ? kZhsLoopThreadsFloat : kZhsLoopThreadsDouble)
-                      : (sizeof(Amp) == sizeof(float) ? kZhsThreadsFloat : kZhsThreadsDouble);
+  return kPass == 1 ? (sizeof(Amp) == sizeof(float) ? kZhsLoopThreadsFloat : kZhsLoopThreadsDouble)
+                    : (sizeof(Amp) == sizeof(float) ? kZhsThreadsFloat : kZhsThreadsDouble);
 }
 // The ZHS block for a team of `threads`: the team when it is smaller than the
 // default team, else the largest block of the amplitude type and pass.
@@ -1659,12 +1866,26 @@ constexpr int zhs_block(int threads) {
              ? (threads < zhs_threads_max<Amp, kPass>() ? threads : zhs_threads_max<Amp, kPass>())
              : zhs_threads_max<Amp, kPass>();
 }
+// CoREAS in mixed precision and fixed point: ms of the 1e7 x 160 workload at 640 /
+// 768 / 896 / 1024 threads 26.4 / 24.3 / 23.9 / 22.5, in ice (5e6 x 64) 5.1 / 4.4 /
+// 4.2 / 3.9.  Where each endpoint looks its source terms up (no shared
+// destination row) 1024 threads spill the loop.
+constexpr int kCoreasLeanThreads = 1024, kCoreasLeanLookupThreads = 768;
+template <bool kFixed, class Amp, bool kPre>
+constexpr int coreas_threads_max() {
+  return kFixed && sizeof(Amp) == sizeof(float) ? (kPre ? kCoreasLeanThreads : kCoreasLeanLookupThreads)
+                                                : kWindowThreads;
+}
+// The CoREAS block for a team of `threads`, by the same rule.
+template <bool kFixed, class Amp, bool kPre>
+constexpr int coreas_block(int threads) {
+  return threads < kWindowThreads ? threads : coreas_threads_max<kFixed, Amp, kPre>();
+}
 // staging slots of the ZHS kernel: 32 per warp of its largest CTA that stages
 // (pass 1 does not)
 template <class Amp>
 constexpr size_t staging_bytes() {
-  int const a = zhs_threads_max<Amp, 0>(), c = zhs_threads_max<Amp, 2>();
-  return static_cast<size_t>(a > c ? a : c) * sizeof(StagedSegment<Amp>);
+  return static_cast<size_t>(zhs_threads_max<Amp, 0>()) * sizeof(StagedSegment<Amp>);
 }
 constexpr size_t kStagingBytes =
     staging_bytes<float>() > staging_bytes<double>() ? staging_bytes<float>() : staging_bytes<double>();
@@ -1681,6 +1902,170 @@ __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t
   return lo;
 }
 
+// The subdivision of a track seen from an observer (accumulate_zhs,
+// RadioProjection.inl:483-503), every operation exact.
+struct Subdivision {
+  double divisor;
+  int subtracks;
+};
+__device__ __forceinline__ Subdivision subdivide(Track const& t, Propagation const& p, ObserverCache const& o) {
+  double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
+  Path const pm = propagate<false>(p, o, mx, my, mz);
+  double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
+  double const s2 = 1. - uk * uk;
+  double const fraunhofer = s2 * t.length * t.length / pm.dist / o.wavelength * 2. * kPi;
+  Subdivision d{1., 1};
+  if (fraunhofer > 1.) {
+    d.divisor = sqrt(fraunhofer) + 1.;
+    d.subtracks = x86_int(ceil(d.divisor));
+  }
+  return d;
+}
+__device__ __noinline__ Subdivision subdivide_row(const double* __restrict__ tracks, uint64_t row,
+                                                  Propagation const& p, ObserverCache const& o) {
+  return subdivide(load_track(tracks, row), p, o);
+}
+
+// The step of a divided track's sequential additions (RadioProjection.inl:505-512).
+struct Steps {
+  double x, y, z, t;
+};
+__device__ __forceinline__ Steps subtrack_steps(Track const& t, double divisor, int refinement) {
+  Steps r{t.ex - t.sx, t.ey - t.sy, t.ez - t.sz, t.te - t.ts};
+  if (divisor != 1. || refinement > 1) {  // x / 1 == x exactly: undivided tracks skip the divisions
+    r.x = r.x / divisor;
+    r.y = r.y / divisor;
+    r.z = r.z / divisor;
+    r.t = r.t / divisor;
+  }
+  if (refinement > 1) {
+    double const rd = static_cast<double>(refinement);
+    r.x = r.x / rd;
+    r.y = r.y / rd;
+    r.z = r.z / rd;
+    r.t = r.t / rd;
+  }
+  return r;
+}
+
+// Segments [from, to) of a divided track evaluated exactly, sample by sample, by
+// one lane: what the filtered drain leaves undecided.
+template <class Amp>
+__device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tracks, uint64_t row, long long from,
+                                                  long long to, Propagation const& p, ObserverCache const& o,
+                                                  DifferenceSink sink) {
+  Counts c;
+  Track const t = load_track(tracks, row);
+  Subdivision const d = subdivide(t, p, o);
+  int const refinement = static_cast<int>(p.refinement);
+  Steps const r = subtrack_steps(t, d.divisor, refinement);
+  bool const subdivided = d.subtracks > 1 || refinement > 1;
+  double x = t.sx, y = t.sy, z = t.sz, time = t.ts;
+#pragma unroll 1
+  for (long long s = 0; s < to; ++s) {
+    double const nx = x + r.x, ny = y + r.y, nz = z + r.z, next = time + r.t;
+    if (s >= from) zhs_segment<true, true, Amp>(x, y, z, nx, ny, nz, time, next, t, p, o, sink, c, subdivided);
+    x = nx;
+    y = ny;
+    z = nz;
+    time = next;
+  }
+  return c;
+}
+
+// Deferred ZHS pairs in mixed precision and fixed point, the whole trace in the
+// window: the warp's pairs (a lane each, below `count`) are divided exactly,
+// then their segments are dealt out to the lanes in turn -- lane j of a step
+// takes segment base + j of the flattened list, its owner found by shuffles --
+// and each lane evaluates and deposits its segment on its own by the filtered
+// arithmetic, at start + (index + 1/2) (end - start) / divisor.  That is within
+// s 2u of the coordinates' and times' magnitudes of the reference's s sequential
+// additions: with those below 2^24 bins (regular_track) and s <= 64, below 2^-20
+// bins, inside kBinGuard.  Longer divisions, irregular tracks and segments that
+// a guard cannot decide are evaluated exactly.  Little is held per lane (a row,
+// an index, one FP64 number), so the function fits the registers of the track
+// loop's kernel: the pair-per-lane drain it replaces there spilled 1700 words a
+// pair at 64 registers.
+constexpr long long kLeanSegments = 64;
+// The table row at height z is that of every height within kBinGuard bins.
+__device__ __forceinline__ bool table_row_decided(Propagation const& p, LeanObserver const& l, double z) {
+  if (p.homogeneous > 0.) return true;
+  double const height = (z - p.min_height) * p.inv_step, guard = l.bin_guard_m * p.inv_step;
+  int row;
+  return (fabs(lean_nearest(height + 0.5, row)) > guard) & (fabs(height) > guard);
+}
+__device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks, uint64_t begin, unsigned const* list,
+                                              unsigned count, Propagation const& p, unsigned long long* win,
+                                              uint32_t width) {
+  Tally c;
+  Counts rare;  // counts of the exact evaluations, and the subtracks
+  unsigned const lane = threadIdx.x & 31u;
+  uint64_t row = 0;
+  double fraction = 1.;
+  unsigned mine = 0;
+  if (lane < count) {
+    row = begin + list[lane];
+    Subdivision const d = subdivide_row(tracks, row, p, s_observer);
+    int const refinement = static_cast<int>(p.refinement);
+    // both products as the reference forms them (RadioProjection.inl:503, :527)
+    rare.subtracks = static_cast<unsigned long long>(static_cast<long long>(d.subtracks));
+    if (refinement > 1)
+      rare.subtracks += static_cast<unsigned long long>(static_cast<long long>(d.subtracks * (refinement - 1)));
+    long long const segments = static_cast<long long>(d.subtracks) * refinement;
+    fraction = 1. / (d.divisor * static_cast<double>(refinement));
+    unsigned const flags = pack_flags(__ldg(track_ref(tracks, row) + kPack / 2 * kTrackTile).y);
+    if (segments > kLeanSegments || !(flags & kTrackRegular & s_lean.usable))
+      add_counts(rare, zhs_exact_segments<float>(tracks, row, 0, segments, p, s_observer, DifferenceSink{win, width}));
+    else if (segments > 0)
+      mine = static_cast<unsigned>(segments);
+  }
+  unsigned incl = mine;
+#pragma unroll
+  for (unsigned d = 1; d < 32u; d <<= 1) {
+    unsigned const v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  unsigned const total = __shfl_sync(0xffffffffu, incl, 31);
+  for (unsigned base = 0; base < total; base += 32u) {
+    unsigned const j = base + lane;
+    unsigned owner = 0;
+#pragma unroll
+    for (unsigned step = 16; step >= 1u; step >>= 1) {
+      unsigned const v = __shfl_sync(0xffffffffu, incl, owner + step - 1u);
+      if (v <= j) owner += step;
+    }
+    owner &= 31u;
+    unsigned const index = j - __shfl_sync(0xffffffffu, incl - mine, owner);
+    uint64_t const its_row = __shfl_sync(0xffffffffu, row, owner);
+    double const its_fraction = __shfl_sync(0xffffffffu, fraction, owner);
+    bool const subdivided = __shfl_sync(0xffffffffu, mine, owner) > 1u;
+    bool deposited = true;
+    if (j < total) {
+      LeanObserver const l = copy_words(s_lean);
+      double2 const* r = track_ref(tracks, its_row);
+      constexpr unsigned T = kTrackTile;
+      double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T);
+      double2 const cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
+      double const at = (static_cast<double>(index) + 0.5) * its_fraction;
+      double const z = fma(cc.y - cb.x, at, cb.x), duration = ct.y - ct.x;
+      double const half_bins = duration * its_fraction * l.half_rate;
+      SourceTerms const st = source_terms(p, destination_of(s_observer), z);
+      LeanPoint const m = lean_point(l, fma(cb.y - ca.x, at, ca.x), fma(cc.x - ca.y, at, ca.y), z,
+                                     fma(duration, at, ct.x), cd.x, cd.y, ce.x, st.factor, st.n_src);
+      StagedSegment<float> seg;
+      deposited = zhs_lean(m, half_bins, pack_constant(ce.y) * l.scale, cd.x, cd.y, ce.x, l, subdivided, seg) &
+                  lean_terms(st) & table_row_decided(p, l, z) & (m.dist * l.rate_over_c >= 4. * half_bins);
+      deposited = deposited && account_staged(seg, l, c);
+      if (deposited) deposit_differences(seg, l, win, width);
+    }
+    if (__any_sync(0xffffffffu, !deposited) && !deposited)
+      add_counts(rare, zhs_exact_segments<float>(tracks, its_row, index, static_cast<long long>(index) + 1, p,
+                                                 s_observer, DifferenceSink{win, width}));
+  }
+  add_counts(rare, counts_of(c));
+  return rare;
+}
+
 // Deferred ZHS pairs of the windowed kernel, drained by the whole warp
 // (accumulate_zhs, RadioProjection.inl:483-529).  Lanes below `count` take
 // one deferred pair each and evaluate its Fraunhofer number and subdivision
@@ -1690,7 +2075,7 @@ __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t
 // first, exactly where a guard cannot decide), and the warp deposits the staged
 // samples together.  A segment that needs the per-index binning deposits on
 // its own lane.  Every lane of the warp calls it.
-template <bool kFixed, class Amp, class Sink>
+template <bool kFixed, bool kDifferences, class Amp, class Sink>
 __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint64_t begin,
                                          unsigned const* list, unsigned count,
                                          Propagation const& p, ObserverCache const& o, LeanObserver const& l, Sink sink,
@@ -1704,40 +2089,18 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
   if (lane < count) {
     row = begin + list[lane];
     Track const t = load_track(tracks, row);
-    double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
-    Path const pm = propagate<false>(p, o, mx, my, mz);
-    double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
-    double const s2 = 1. - uk * uk;
-    double const fraunhofer = s2 * t.length * t.length / pm.dist / o.wavelength * 2. * kPi;
-    double divisor = 1.;
-    int subtracks = 1;
-    if (fraunhofer > 1.) {
-      divisor = sqrt(fraunhofer) + 1.;
-      subtracks = x86_int(ceil(divisor));
-    }
+    Subdivision const d = subdivide(t, p, o);
     int const refinement = static_cast<int>(p.refinement);
-    c.subtracks += static_cast<unsigned long long>(static_cast<long long>(subtracks));
+    c.subtracks += static_cast<unsigned long long>(static_cast<long long>(d.subtracks));
     if (refinement > 1)
-      c.subtracks += static_cast<unsigned long long>(
-          static_cast<long long>(subtracks * (refinement - 1)));
-    subdivided = subtracks > 1 || refinement > 1;
-    rx = t.ex - t.sx;
-    ry = t.ey - t.sy;
-    rz = t.ez - t.sz;
-    rt = t.te - t.ts;
-    if (refinement > 1) {  // x / 1 == x exactly: undivided tracks skip the divisions
-      double const rd = static_cast<double>(refinement);
-      rx = rx / divisor / rd;
-      ry = ry / divisor / rd;
-      rz = rz / divisor / rd;
-      rt = rt / divisor / rd;
-    } else if (subdivided) {
-      rx = rx / divisor;
-      ry = ry / divisor;
-      rz = rz / divisor;
-      rt = rt / divisor;
-    }
-    segments = static_cast<long long>(subtracks) * refinement;
+      c.subtracks += static_cast<unsigned long long>(static_cast<long long>(d.subtracks * (refinement - 1)));
+    subdivided = d.subtracks > 1 || refinement > 1;
+    Steps const step = subtrack_steps(t, d.divisor, refinement);
+    rx = step.x;
+    ry = step.y;
+    rz = step.z;
+    rt = step.t;
+    segments = static_cast<long long>(d.subtracks) * refinement;
     p1x = t.sx;
     p1y = t.sy;
     p1z = t.sz;
@@ -1759,9 +2122,9 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
       bool staged = false;
       if constexpr (sizeof(Amp) == sizeof(float)) {
         SourceTerms const st = source_terms(p, destination_of(o), mz);
-        LeanPoint const m = lean_point(o, l, mx, my, mz, mt, e.x, e.y, f.x, st.factor, st.n_src);
-        staged = zhs_lean(m, (t2 - t1) * l.half_rate, pack_constant(f.y) * l.scale, e.x, e.y, f.x, o, subdivided, seg) &
-                 ((pack_flags(f.y) & kTrackRegular & l.usable) != 0u) & lean_index(st.n_src);
+        LeanPoint const m = lean_point(l, mx, my, mz, mt, e.x, e.y, f.x, st.factor, st.n_src);
+        staged = zhs_lean(m, (t2 - t1) * l.half_rate, pack_constant(f.y) * l.scale, e.x, e.y, f.x, l, subdivided, seg) &
+                 ((pack_flags(f.y) & kTrackRegular & l.usable) != 0u) & lean_terms(st);
       }
       Track t;
       t.bx = e.x;
@@ -1782,7 +2145,15 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
       p1z = p2z;
       t1 = t2;
     }
-    deposit_staged<kFixed>(staging, seg, o, sink, c);
+    if constexpr (kDifferences) {
+      // a segment whose values might not convert: sample by sample, checked
+      if (!account_staged(seg, l, c))
+        add_counts(c, deposit_samples(seg, o, sink));
+      else
+        deposit_differences(seg, l, sink.win, sink.width);
+    } else {
+      deposit_staged<kFixed>(staging, seg, o, sink, c);
+    }
   }
   return c;
 }
@@ -1798,9 +2169,10 @@ __device__ __noinline__ Counts coreas_drain_pair(const double* __restrict__ trac
   Counts c;
   double2 const* r = track_ref(tracks, row);
   if constexpr (kFixed && sizeof(Amp) == sizeof(float)) {
+    Tally t;
     if ((hint & static_cast<unsigned>(kCoreasNearCone)) &&
-        near_cone_lean<kPre>(r, (hint & 1u) != 0u, p, o, l, sink, c))
-      return c;
+        near_cone_lean<kPre>(r, (hint & 1u) != 0u, p, s_lean, sink, t))
+      return counts_of(t);
   }
   constexpr unsigned T = kTrackTile;
   unsigned const flags = pack_flags(__ldg(r + kPack / 2 * T).y);
@@ -1834,91 +2206,220 @@ __device__ __forceinline__ void load_endpoint_terms(const double* __restrict__ b
   end = SourceTerms{e.x, e.y, 0.};
 }
 
+// A deferred-list entry: the track's offset in the item and, for CoREAS, the
+// track loop's decision in the top bits.
+__device__ __forceinline__ unsigned deferred_entry(uint32_t offset, int code) {
+  return offset | (code >= kCoreasNearCone ? static_cast<unsigned>(code) << kDeferredHintShift : 0u);
+}
+
 // Appends a warp's deferred pairs to its CTA's list: `entry` of the lanes with
-// `deferred` set, one atomic on the shared counter.  Entries at or past
-// `capacity` are counted, not written.
-__device__ __forceinline__ void push_deferred(bool deferred, unsigned entry, unsigned* list, unsigned* total,
-                                              uint64_t used, uint64_t capacity) {
+// `deferred` set, one atomic on the shared counter.
+__device__ __forceinline__ void push_deferred(bool deferred, unsigned entry) {
   unsigned const ballot = __ballot_sync(0xffffffffu, deferred);
   if (!ballot) return;
   unsigned const lane = threadIdx.x & 31u;
   unsigned slot = 0;
-  if (lane == 0) slot = atomicAdd(total, static_cast<unsigned>(__popc(ballot)));
+  if (lane == 0) slot = atomicAdd(&s_deferred_total, static_cast<unsigned>(__popc(ballot)));
   slot = __shfl_sync(0xffffffffu, slot, 0);
-  uint64_t const at = used + slot + __popc(ballot & ((1u << lane) - 1u));
-  if (deferred && at < capacity) list[at] = entry;
+  if (deferred) s_deferred_list[slot + __popc(ballot & ((1u << lane) - 1u))] = entry;
 }
 
-// The CoREAS track loop in mixed precision and fixed point: `count` tracks from
-// `begin`, a thread each, the deferred ones appended to `list`.  A thread's
-// track advances by whole tiles, so its columns' address is one running
-// pointer.
+// The track loops run out of line, each a function of its own: what the kernel
+// holds across an item (the plan, the calls of the drain and the flush) then
+// takes no registers from the loop, whose speed turns on its register
+// allocation (inlined beside them, the loops of the 1e7 x 160 workload ran 31.1
+// (CoREAS) and 42.7 ms (ZHS) where they run 26.8 and 34.3 as functions).  `count` tracks from `begin`, a
+// thread each; a thread's track advances by whole tiles, so its columns'
+// address is one running pointer.  Deferred pairs go to `list`.
+
+// CoREAS in mixed precision and fixed point.
 template <bool kPre, bool kUnchecked>
-__device__ __forceinline__ void coreas_lean_loop(const double* __restrict__ tracks, uint64_t begin, uint32_t count,
-                                                 Propagation const& p, ObserverCache const& o,
-                                                 LeanObserver const& l, WindowSink& sink, unsigned* list,
-                                                 unsigned* total, Counts& c) {
+__device__ __noinline__ Counts coreas_lean_loop(const double* __restrict__ tracks, uint64_t begin, uint32_t count,
+                                                Propagation const& p, WindowSink sink) {
+  Tally c;
   double2 const* r = track_ref(tracks, begin + threadIdx.x);
   uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
   for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
     uint32_t const k = base + threadIdx.x;
     int code = kCoreasDeposited;
-    if (k < count) code = coreas_lean<kPre, kUnchecked>(r, p, o, l, sink, c);
-    push_deferred(code != kCoreasDeposited,
-                  k | (code >= kCoreasNearCone ? static_cast<unsigned>(code) << kDeferredHintShift : 0u), list,
-                  total, 0, ~0ull);
+    if (k < count) code = coreas_lean<kPre, kUnchecked>(r, p, copy_words(s_lean), sink, c);
+    push_deferred(code != kCoreasDeposited, deferred_entry(k, code));
   }
+  return counts_of(c);
 }
 
-// The same with checked adds (an item run again, or a trace longer than the
-// window), out of line: its registers do not count in the unchecked loop.
-template <bool kPre>
-__device__ __noinline__ Counts coreas_lean_checked(const double* __restrict__ tracks, uint64_t begin,
-                                                   uint32_t count, Propagation const& p, ObserverCache const& o,
-                                                   LeanObserver const& l, WindowSink sink, unsigned* list,
-                                                   unsigned* total) {
+// CoREAS in FP64 or with floating traces.
+template <bool kFixed, bool kPre, class Amp>
+__device__ __noinline__ Counts coreas_loop(const double* __restrict__ tracks, uint64_t begin, uint32_t count,
+                                           Propagation const& p, WindowSink sink) {
   Counts c;
-  coreas_lean_loop<kPre, false>(tracks, begin, count, p, o, l, sink, list, total, c);
+  for (uint32_t base = 0; base < count; base += blockDim.x) {
+    uint32_t const k = base + threadIdx.x;
+    int code = kCoreasDeposited;
+    if (k < count) {
+      Track const t = load_track(tracks, begin + k);
+      SourceTerms start{}, end{};
+      if (kPre) load_endpoint_terms(tracks, begin + k, start, end);
+      code = coreas_common<kFixed, kPre, Amp>(t, p, s_observer, sink, c, start, end);
+    }
+    push_deferred(code != kCoreasDeposited, deferred_entry(k, code));
+  }
   return c;
 }
 
-// kPass 0: one pass over every item.  Two passes (fixed-point ZHS):
-// kPass 1 runs the track loop alone, depositing differences with unchecked
-// window adds (deposit_differences), appends the
-// deferred pairs of all its items to its CTA's list, flushes each item whose
-// window bound holds and records where its deferred pairs are; an item whose
-// bound does not hold, whose trace is longer than the window or whose pairs
-// do not fit in the list is handed back unflushed, and once its list has
-// overflowed a CTA hands back its later items unprojected.  kPass 2 drains
-// each recorded item's pairs into a fresh window; kPass 3 projects the
-// handed-back items in full, as kPass 0 does.  The drain needs more
-// registers than the track loop (168 against 80 FP32, 118 FP64), so apart
-// the track loop runs without spills in larger CTAs.
+// ZHS in fixed point with the whole trace in the window: deposited lane by lane
+// as differences.
+template <bool kPre, bool kMayRefine, class Amp>
+__device__ __noinline__ Counts zhs_difference_loop(const double* __restrict__ tracks, uint64_t begin,
+                                                   uint32_t count, Propagation const& p, unsigned long long* win,
+                                                   uint32_t width) {
+  Tally c;
+  double2 const* r = track_ref(tracks, begin + threadIdx.x);
+  uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
+  for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
+    uint32_t const k = base + threadIdx.x;
+    bool deferred = false;
+    LeanObserver const l = copy_words(s_lean);
+    if constexpr (sizeof(Amp) == sizeof(float)) {
+      if (k < count) {
+        ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
+        deferred = !(z.one && zhs_lean_differences(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, win, c));
+      }
+    } else if (k < count) {
+      ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
+      deferred = !z.one;
+      if (z.one) {
+        constexpr unsigned T = kTrackTile;
+        ObserverCache const o = copy_words(s_observer);
+        double2 const cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T), ct = __ldg(r + 3 * T);
+        deferred = !zhs_exact_differences(propagate_with<true>(z.terms, o, cm.x, cm.y, cn.x), ct.x,
+                                          ct.x + (ct.y - ct.x), cn.y, z.bx, z.by, z.bz,
+                                          __ldg(r + kConst / 2 * T).y, o, l, win, c);
+      }
+    }
+    push_deferred(deferred, k);
+  }
+  return counts_of(c);
+}
+
+// ZHS with the segments staged for the warp (floating traces, checked runs).
+template <bool kFixed, bool kPre, class Amp>
+__device__ __noinline__ Counts zhs_staged_loop(const double* __restrict__ tracks, uint64_t begin, uint32_t count,
+                                               Propagation const& p, WindowSink sink,
+                                               StagedSegment<Amp>* staging) {
+  Counts c;
+  double2 const* r = track_ref(tracks, begin + threadIdx.x);
+  uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
+  for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
+    uint32_t const k = base + threadIdx.x;
+    bool deferred = false;
+    StagedSegment<Amp> seg;
+    seg.count = 0u;
+    seg.flags = 0u;
+    if (k < count) deferred = !zhs_common<kFixed, kPre, true, Amp>(r, p, s_lean, seg);
+    deposit_staged<kFixed>(staging, seg, s_observer, sink, c);
+    push_deferred(deferred, k);
+  }
+  return c;
+}
+
+// No thread of the CTA can count 2^32 samples in an item of `count` tracks.
+__device__ __forceinline__ bool tally_fits(uint64_t count, uint32_t width) {
+  return (count / blockDim.x + 1u) * width < 0xffffffffull;
+}
+
+// Notes an item for the third pass; one thread of the CTA writes it.
+__device__ __forceinline__ void hand_back(WorkPlan const& plan, uint64_t item) {
+  if (threadIdx.x != 0) return;
+  plan.item_state[atomicAdd(plan.drain_next_item, 1u)].item = item;
+  if (plan.handbacks) atomicAdd(plan.handbacks, 1ull);
+}
+
+// Zeroes 3 * width words of the window.  Every thread of the CTA calls it.
+__device__ __forceinline__ void zero_window(unsigned long long* win, uint32_t width) {
+  uint32_t const words = 3u * width;
+  for (uint32_t j = threadIdx.x; j < words / 2u; j += blockDim.x)
+    reinterpret_cast<ulonglong2*>(win)[j] = make_ulonglong2(0ull, 0ull);
+  if (threadIdx.x == 0 && (words & 1u)) win[words - 1u] = 0ull;
+}
+
+// Adds the window's non-zero bins to the observer's trace rows with checked
+// global atomics; returns this thread's overflows.  A thread issues the adds
+// of four bins' three components before it looks at what they returned: one
+// add at a time waits for the L2 at every bin (24576 adds an item of 8192
+// bins).  Out of line, so that its registers do not count in the track loops.
+__device__ __noinline__ unsigned flush_window(unsigned long long const* win, uint32_t width,
+                                              unsigned long long* row0, unsigned long long* row1,
+                                              unsigned long long* row2) {
+  constexpr uint32_t kDepth = 4;
+  unsigned overflows = 0;
+  for (uint32_t base = threadIdx.x; base < width; base += kDepth * blockDim.x) {
+    unsigned long long v[kDepth][3], before[kDepth][3];
+#pragma unroll
+    for (uint32_t d = 0; d < kDepth; ++d) {
+      uint32_t const j = base + d * blockDim.x;
+#pragma unroll
+      for (uint32_t row = 0; row < 3; ++row) v[d][row] = j < width ? win[3u * j + row] : 0ull;
+    }
+#pragma unroll
+    for (uint32_t d = 0; d < kDepth; ++d) {
+      uint32_t const j = base + d * blockDim.x;
+      before[d][0] = v[d][0] ? atomicAdd(row0 + j, v[d][0]) : 0ull;
+      before[d][1] = v[d][1] ? atomicAdd(row1 + j, v[d][1]) : 0ull;
+      before[d][2] = v[d][2] ? atomicAdd(row2 + j, v[d][2]) : 0ull;
+    }
+#pragma unroll
+    for (uint32_t d = 0; d < kDepth; ++d)
+#pragma unroll
+      for (uint32_t row = 0; row < 3; ++row)
+        overflows += checked(before[d][row], static_cast<long long>(v[d][row])) ? 0u : 1u;
+  }
+  return overflows;
+}
+
+__device__ __noinline__ void flush_window_floating(double const* win, uint32_t width, double* row0, double* row1,
+                                                   double* row2) {
+  for (uint32_t j = threadIdx.x; j < width; j += blockDim.x) {
+    double const x = win[3u * j], y = win[3u * j + 1u], z = win[3u * j + 2u];
+    if (x != 0.) atomicAdd(row0 + j, x);
+    if (y != 0.) atomicAdd(row1 + j, y);
+    if (z != 0.) atomicAdd(row2 + j, z);
+  }
+}
+
+// kPass 0: every item in one pass.  Two passes (fixed-point ZHS): kPass 1
+// projects an item's tracks and then its deferred pairs with unchecked window
+// adds, all as differences (deposit_differences), and hands back, unflushed and
+// uncounted, the items it cannot: traces longer than the window, refined
+// tracks (each pair is divided) and items whose window bound does not hold;
+// kPass 3 projects those in full, as kPass 0 does.  With the general path in a
+// kernel of its own, the first pass holds nothing but the track loop and runs
+// it without spills in larger CTAs.
 template <bool kFixed, class Amp, int kAlgorithm, bool kPre, int kPass = 0>
-__global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>() : kWindowThreads, 1)
+__global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>() : coreas_threads_max<kFixed, Amp, kPre>(), 1)
     windowed_kernel(const __grid_constant__ WorkPlan plan) {
   static_assert(kPass == 0 || (kFixed && kAlgorithm == 1), "two passes: fixed-point ZHS");
   extern __shared__ __align__(16) unsigned long long window[];
   __shared__ unsigned long long item_shared;
-  __shared__ ObserverCache observer;
-  __shared__ LeanObserver lean;
   __shared__ float window_bound;
-  __shared__ unsigned deferred_total;
-  // this CTA's list of the deferred pairs of its current item (kPass 1: of
-  // all its items, from `used` on; kPass 2: of the items it projects in full)
-  unsigned* const deferred_list =
-      kPass >= 2 ? plan.drain_deferred + static_cast<size_t>(blockIdx.x) * plan.deferred_stride
-      : kPass == 1 ? plan.deferred + static_cast<size_t>(blockIdx.x) * plan.deferred_capacity
-                   : plan.deferred + static_cast<size_t>(blockIdx.x) * plan.deferred_stride;
-  uint32_t used = 0;  // kPass 1: entries of the list taken by earlier items
-  bool full = false;  // kPass 1: the list overflowed; later items are handed back
+  // this CTA's list of the deferred pairs of its current item
+  if (threadIdx.x == 0)
+    s_deferred_list = (kPass == 3 ? plan.drain_deferred : plan.deferred) +
+                      static_cast<size_t>(blockIdx.x) * plan.deferred_stride;
   Counts c;
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) item_shared = atomicAdd(plan.next_item, 1u);
-    __syncthreads();
-    uint64_t const item = item_shared;
-    if (item >= plan.total_items) break;
+  for (uint64_t turn = blockIdx.x;; turn += gridDim.x) {
+    uint64_t item;
+    if constexpr (kPass == 3) {  // the handed-back items, every gridDim.x-th
+      if (turn >= *plan.drain_next_item) break;
+      item = plan.item_state[turn].item;
+      __syncthreads();
+    } else {
+      __syncthreads();
+      if (threadIdx.x == 0) item_shared = atomicAdd(plan.next_item, 1u);
+      __syncthreads();
+      item = item_shared;
+      if (item >= plan.total_items) break;
+    }
     EventPlan const& ev = plan.events[find_event(plan.events, plan.event_count, item)];
     constexpr int algorithm = kAlgorithm;
     uint64_t const local = item - ev.first_item;
@@ -1928,166 +2429,116 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
     uint64_t const valid = *ev.valid_tracks;
     uint64_t const track_count = valid < ev.last_track ? valid : ev.last_track;
     uint64_t const begin = ev.first_track + slice_chunk * ev.chunk_size;
-    ItemState state{blockIdx.x, used, 0u, 0u};
-    if constexpr (kPass >= 2) {
-      state = plan.item_state[item];
-      if (kPass == 2 && (state.redo || state.count == 0u)) continue;  // nothing to drain
-      if (kPass == 3 && !state.redo) continue;                          // done by passes 1-2
-    }
-    bool const drain_only = kPass == 2;
-    if (begin >= track_count) {
-      if (kPass == 1 && threadIdx.x == 0) plan.item_state[item] = state;
-      continue;
-    }
+    if (begin >= track_count) continue;
     uint64_t const end = begin + ev.chunk_size < track_count ? begin + ev.chunk_size : track_count;
     uint64_t const bins = ev.observers[algorithm][oi].bins;
     uint32_t const width = static_cast<uint32_t>(bins < ev.window ? bins : ev.window);
-    if (kPass == 1 && (full || bins > width)) {  // handed back unprojected
-      if (threadIdx.x == 0) {
-        plan.item_state[item] = ItemState{blockIdx.x, used, 0u, 1u};
-        if (plan.handbacks) atomicAdd(plan.handbacks, 1ull);
-      }
+    if (kPass == 1 && (bins > width || ev.propagation.refinement != 1u || !tally_fits(end - begin, width))) {
+      hand_back(plan, item);
       continue;
     }
     if (threadIdx.x == 0) {
-      observer = ev.observers[algorithm][oi];
-      if (kAlgorithm == 1 || sizeof(Amp) == sizeof(float)) make_lean_observer<kAlgorithm>(observer, lean);
+      s_observer = ev.observers[algorithm][oi];
+      if (kAlgorithm == 1 || sizeof(Amp) == sizeof(float)) make_lean_observer<kAlgorithm>(s_observer, s_lean);
     }
-    ObserverCache const& o = observer;
 
-    // zero the window (3 rows of width bins); the barrier also publishes `observer`
-    for (uint32_t j = threadIdx.x; j < 3 * width; j += blockDim.x) window[j] = 0ull;
+    // zero the window (3 words for each of width bins); the barrier also publishes the observer
+    zero_window(window, width);
     if (threadIdx.x == 0) window_bound = 0.f;
     __syncthreads();
 
-    WindowSink sink;
-    sink.win = window;
-    sink.fwin = reinterpret_cast<double*>(window);
-    sink.width = width;
-    uint64_t const total = ev.total_bins[algorithm];
-    for (int row = 0; row < 3; ++row) {
-      sink.row[row] = kFixed ? ev.fixed[algorithm] + row * total + o.offset : nullptr;
-      sink.frow[row] = kFixed ? nullptr : ev.floating[algorithm] + row * total + o.offset;
-    }
     constexpr bool kFilter = sizeof(Amp) == sizeof(float);  // mixed precision
     // Deferred pairs (track offsets in the chunk: CoREAS pairs for the
     // near-Cherenkov branch or an exact evaluation, ZHS pairs with subdivided
     // tracks or an exact evaluation) leave the common path, so rare paths do
     // not hold up the other lanes: they go to the CTA's list in global memory
     // and all warps drain it, 32 pairs at a time, after the item's tracks.
-    // The track loop then holds no call, which keeps its registers free.
     // per-warp staging slots of the ZHS kernel's cooperative deposit
     StagedSegment<Amp>* const staging =
         reinterpret_cast<StagedSegment<Amp>*>(window + 3 * static_cast<size_t>(plan.window)) +
         (threadIdx.x >> 5) * 32u;
     unsigned const lane = threadIdx.x & 31u;
-    Counts const saved = c;
-    bool redo = false;  // kPass 1: the item goes back to the second pass
-    unsigned n = 0;     // deferred pairs of the item
+    uint32_t const count = static_cast<uint32_t>(end - begin);
+    bool handed_back = false, whole = false;  // whole: the window's adds were unchecked
+    // The trace rows' addresses are formed again wherever they are used
+    // (`fresh` hides that they are the same), not held across the track loop.
+    auto make_sink = [&](bool unchecked) {
+      uint64_t offset = s_observer.offset;
+      asm volatile("" : "+l"(offset));  // fresh
+      WindowSink k;
+      k.win = window;
+      k.fwin = reinterpret_cast<double*>(window);
+      k.width = width;
+      k.unchecked = unchecked;
+      for (int row = 0; row < 3; ++row) {
+        uint64_t const at = row * ev.total_bins[algorithm] + offset;
+        k.row[row] = kFixed ? ev.fixed[algorithm] + at : nullptr;
+        k.frow[row] = kFixed ? nullptr : ev.floating[algorithm] + at;
+      }
+      return k;
+    };
     // Fixed point, whole trace in the window: the window takes unchecked
     // adds, and `c.mag` bounds the sum of |increments| of this thread.  If the
     // block's bound stays below 2^61, no partial sum of any bin can have left
     // the int64 range in any order, so no add overflowed; else the item is
-    // run again with checked adds.  An FP32 sum of n terms is off by a factor
-    // below 1 + n 2^-24, so a thread's sum counts only while the thread made
-    // fewer than 2^22 adds (factor below 1 + 2^-2); a thread with more (its
-    // deposits since the attempt began: contributions plus failed
-    // conversions, an upper bound of its window adds) sends the item to the
-    // checked run.  Bins past the window and the flush below are always
-    // checked.
+    // run again with checked adds (kPass 1: handed back).  An FP32 sum of n
+    // terms is off by a factor below 1 + n 2^-24, so a thread's sum counts only
+    // while the thread made fewer than 2^22 adds (factor below 1 + 2^-2); a
+    // thread with more (its deposits since the attempt began: contributions
+    // plus failed conversions, an upper bound of its window adds) sends the
+    // item to the checked run.  Bins past the window and the flush below are
+    // always checked.
     for (int attempt = 0;; ++attempt) {
       if (attempt > 0) {
-        for (uint32_t j = threadIdx.x; j < 3 * width; j += blockDim.x) window[j] = 0ull;
+        zero_window(window, width);
         __syncthreads();
       }
-      sink.unchecked = kFixed && attempt == 0 && bins <= width;
-      c.mag = 0.f;
-      if (threadIdx.x == 0) deferred_total = 0u;
+      bool const unchecked = kFixed && attempt == 0 && bins <= width && (kAlgorithm == 0 || tally_fits(count, width));
+      c = Counts{};
+      if (threadIdx.x == 0) s_deferred_total = 0u;
       __syncthreads();
+      Propagation const& p = ev.propagation;
       if constexpr (kAlgorithm == 0 && kFixed && kFilter) {
-        uint32_t const count = static_cast<uint32_t>(end - begin);
-        if (sink.unchecked)
-          coreas_lean_loop<kPre, true>(ev.tracks, begin, count, ev.propagation, o, lean, sink, deferred_list,
-                                       &deferred_total, c);
-        else
-          add_counts(c, coreas_lean_checked<kPre>(ev.tracks, begin, count, ev.propagation, o, lean, sink,
-                                                  deferred_list, &deferred_total));
+        c = unchecked ? coreas_lean_loop<kPre, true>(ev.tracks, begin, count, p, make_sink(true))
+                      : coreas_lean_loop<kPre, false>(ev.tracks, begin, count, p, make_sink(false));
       } else if constexpr (kAlgorithm == 0) {
-        for (uint64_t base = begin; base < end; base += blockDim.x) {
-          uint64_t const i = base + threadIdx.x;
-          int code = kCoreasDeposited;
-          if (i < end) {
-            Track const t = load_track(ev.tracks, i);
-            SourceTerms pa{}, pb{};
-            if (kPre) load_endpoint_terms(ev.tracks, i, pa, pb);
-            code = coreas_common<kFixed, kPre, Amp>(t, ev.propagation, o, sink, c, pa, pb);
-          }
-          push_deferred(code != kCoreasDeposited,
-                        static_cast<unsigned>(i - begin) |
-                            (code >= kCoreasNearCone ? static_cast<unsigned>(code) << kDeferredHintShift : 0u),
-                        deferred_list, &deferred_total, 0, ~0ull);
-        }
-      } else if (!drain_only) {
-        uint32_t const count = static_cast<uint32_t>(end - begin);
-        double2 const* r = track_ref(ev.tracks, begin + threadIdx.x);
-        uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
-        for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
-          uint32_t const k = base + threadIdx.x;
-          bool deferred = false;
-          StagedSegment<Amp> seg;
-          seg.count = 0u;
-          seg.flags = 0u;
-          if (k < count) deferred = !zhs_common<kFixed, kPre, Amp>(r, ev.propagation, o, lean, c, seg);
-          if (kFixed && (kPass == 1 || sink.unchecked)) {
-            if (!deferred && !account_staged(seg, o, c)) {
-              seg.count = 0u;
-              seg.flags = 0u;
-              deferred = true;
-              c.subtracks -= 1ull;  // the drain counts the pair's subtracks
-            }
-            deposit_differences(seg, o, sink);
-          } else {
-            if constexpr (kPass != 1) deposit_staged<kFixed>(staging, seg, o, sink, c);
-          }
-          push_deferred(deferred, k, deferred_list, &deferred_total, used,
-                        kPass == 1 ? plan.deferred_capacity : ~0ull);  // used: 0 but in kPass 1
-        }
-      }
-      if constexpr (kAlgorithm == 1 && kFixed && kPass != 2) {
-        if (kPass == 1 || sink.unchecked) difference_window(window, width);
+        c = coreas_loop<kFixed, kPre, Amp>(ev.tracks, begin, count, p, make_sink(unchecked));
+      } else if (kFixed && (kPass == 1 || unchecked)) {
+        c = zhs_difference_loop<kPre, kPass != 1, Amp>(ev.tracks, begin, count, p, window, width);
+      } else if constexpr (kPass != 1) {
+        c = zhs_staged_loop<kFixed, kPre, Amp>(ev.tracks, begin, count, p, make_sink(false), staging);
       }
       __syncthreads();
-      // at most end - begin <= deferred_stride (kPass 1: over the list's end
-      // when used + n is)
-      n = drain_only ? state.count : deferred_total;
-      if (kPass == 1 && static_cast<uint64_t>(used) + n > plan.deferred_capacity) {
-        redo = true;
-        full = true;
-        break;
-      }
-      unsigned const* const list =
-          drain_only ? plan.deferred + static_cast<size_t>(state.cta) * plan.deferred_capacity + state.begin
-                     : deferred_list;
-      for (unsigned from = (threadIdx.x >> 5) * 32u; kPass != 1 && from < n; from += (blockDim.x >> 5) * 32u) {
-        unsigned const count = n - from < 32u ? n - from : 32u;
+      unsigned const n = s_deferred_total;  // at most end - begin <= deferred_stride
+      // one subtrack for each pair that the track loop deposited; the drain counts the others'
+      if (kAlgorithm == 1 && threadIdx.x == 0) c.subtracks += count - n;
+      for (unsigned from = (threadIdx.x >> 5) * 32u; from < n; from += (blockDim.x >> 5) * 32u) {
+        unsigned const left = n - from < 32u ? n - from : 32u;
         Counts d;
-        if constexpr (kAlgorithm == 1 && kPass == 1) {
-          (void)count;
-        } else if (kAlgorithm == 1) {
-          d = zhs_drain<kFixed, Amp>(ev.tracks, begin, list + from, count, ev.propagation, o, lean,
-                                     sink, staging);
-        } else if (lane < count) {
-          unsigned const entry = list[from + lane];
+        if constexpr (kAlgorithm == 1) {
+          if (kFixed && (kPass == 1 || unchecked)) {
+            if constexpr (sizeof(Amp) == sizeof(float))
+              d = zhs_drain_lean(ev.tracks, begin, s_deferred_list + from, left, p, window, width);
+            else
+              d = zhs_drain<kFixed, true, Amp>(ev.tracks, begin, s_deferred_list + from, left, p, s_observer, s_lean,
+                                               DifferenceSink{window, width}, staging);
+          }
+          else if constexpr (kPass != 1)
+            d = zhs_drain<kFixed, false, Amp>(ev.tracks, begin, s_deferred_list + from, left, p, s_observer, s_lean,
+                                              make_sink(false), staging);
+        } else if (lane < left) {
+          unsigned const entry = s_deferred_list[from + lane];
           d = coreas_drain_pair<kFixed, Amp, kPre>(ev.tracks, begin + (entry & kDeferredOffsetMask),
-                                                   entry >> kDeferredHintShift, ev.propagation, o, lean, sink);
+                                                   entry >> kDeferredHintShift, p, s_observer, s_lean,
+                                                   make_sink(unchecked));
         }
         add_counts(c, d);
         __syncwarp();
       }
       __syncthreads();
-      if (!sink.unchecked) break;
-      unsigned long long const adds = (c.coreas - saved.coreas) + (c.zhs - saved.zhs) +
-                                      (c.overflows - saved.overflows);
+      if (!unchecked) break;
+      whole = true;
+      unsigned long long const adds = c.coreas + c.zhs + c.overflows;
       double const mine = adds < (1ull << 22) ? static_cast<double>(c.mag) : static_cast<double>(INFINITY);
       float const thread_bound = static_cast<float>(warp_sum(mine));
       if (lane == 0) atomicAdd(&window_bound, thread_bound);
@@ -2095,39 +2546,23 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
       float const block_bound = window_bound;
       __syncthreads();
       if (block_bound < 0x1p61f) break;
+      whole = false;
       if (kPass == 1) {
-        redo = true;
+        handed_back = true;
         break;
       }
       if (threadIdx.x == 0 && plan.reruns) atomicAdd(plan.reruns, 1ull);
-      c = saved;
     }
-    if constexpr (kPass == 1) {
-      if (redo) {  // unflushed: the second pass projects the item in full
-        c = saved;
-        if (threadIdx.x == 0) {
-          plan.item_state[item] = ItemState{blockIdx.x, used, 0u, 1u};
-          if (plan.handbacks) atomicAdd(plan.handbacks, 1ull);
-        }
-        continue;
-      }
-      if (threadIdx.x == 0) plan.item_state[item] = ItemState{blockIdx.x, used, n, 0u};
-      used += n;
+    if (kPass == 1 && handed_back) {
+      hand_back(plan, item);
+      continue;
     }
-
-    // flush: non-zero bins, checked global adds
-    for (uint32_t j = threadIdx.x; j < 3 * width; j += blockDim.x) {
-      unsigned long long const v = window[j];
-      if (v == 0ull) continue;
-      uint32_t const row = j / width;
-      uint32_t const bin = j - row * width;
-      if (kFixed) {
-        long long const inc = static_cast<long long>(v);
-        if (!checked(atomicAdd(sink.row[row] + bin, v), inc)) ++c.overflows;
-      } else {
-        atomicAdd(sink.frow[row] + bin, __longlong_as_double(static_cast<long long>(v)));
-      }
-    }
+    if (kAlgorithm == 1 && kFixed && whole) difference_window(window, width);
+    WindowSink const sink = make_sink(false);
+    if (kFixed)
+      c.overflows += flush_window(window, width, sink.row[0], sink.row[1], sink.row[2]);
+    else
+      flush_window_floating(sink.fwin, width, sink.frow[0], sink.frow[1], sink.frow[2]);
     flush_counts(c, ev.counters);
   }
 }
@@ -2224,7 +2659,7 @@ cudaError_t tiled_dispatch(EventPlan const& ev, uint64_t bound, bool coreas, boo
   return cudaGetLastError();
 }
 
-// window rows | (ZHS, but for pass 1) per-warp staging slots
+// window | (ZHS, but for pass 1) per-warp staging slots
 template <class Amp>
 size_t windowed_smem_bytes(uint32_t window, int algorithm, int pass) {
   return static_cast<size_t>(window) * 3 * sizeof(unsigned long long) +
@@ -2246,27 +2681,20 @@ cudaError_t windowed_launch(WorkPlan const& plan, int ctas, int threads, cudaStr
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(bytes));
   if (err != cudaSuccess) return err;
-  int const block = kAlgorithm == 1 ? zhs_block<Amp, kPass>(threads) : threads;
+  int const block = kAlgorithm == 1 ? zhs_block<Amp, kPass>(threads) : coreas_block<kFixed, Amp, kPre>(threads);
   windowed_kernel<kFixed, Amp, kAlgorithm, kPre, kPass><<<ctas, block, bytes, stream>>>(plan);
   return cudaGetLastError();
 }
 
 // The passes of a two-pass fixed-point ZHS launch, one after the other on
-// the stream: the track loop, the drain, and the handed-back items in full;
-// the last two draw items from their own counter.
+// the stream; drain_next_item counts the items the first hands back.
 template <class Amp, bool kPre>
 cudaError_t windowed_two_pass(WorkPlan const& plan, int ctas, int threads, cudaStream_t stream) {
-  cudaError_t err = windowed_launch<true, Amp, 1, kPre, 1>(plan, ctas, threads, stream);
+  cudaError_t err = cudaMemsetAsync(plan.drain_next_item, 0, sizeof(unsigned), stream);
   if (err != cudaSuccess) return err;
-  WorkPlan later = plan;
-  later.next_item = plan.drain_next_item;
-  err = cudaMemsetAsync(plan.drain_next_item, 0, sizeof(unsigned), stream);
+  err = windowed_launch<true, Amp, 1, kPre, 1>(plan, ctas, threads, stream);
   if (err != cudaSuccess) return err;
-  err = windowed_launch<true, Amp, 1, kPre, 2>(later, ctas, threads, stream);
-  if (err != cudaSuccess) return err;
-  err = cudaMemsetAsync(plan.drain_next_item, 0, sizeof(unsigned), stream);
-  if (err != cudaSuccess) return err;
-  return windowed_launch<true, Amp, 1, kPre, 3>(later, ctas, threads, stream);
+  return windowed_launch<true, Amp, 1, kPre, 3>(plan, ctas, threads, stream);
 }
 
 template <bool kFixed, class Amp, int kAlgorithm>
@@ -2308,15 +2736,13 @@ int ctas_per_sm(int window, int threads) {
       blocks = 0;
     worst = blocks < worst ? blocks : worst;
   };
-  probe(windowed_kernel<kFixed, Amp, 0, false>, threads, 0);
-  probe(windowed_kernel<kFixed, Amp, 0, true>, threads, 0);
+  probe(windowed_kernel<kFixed, Amp, 0, false>, coreas_block<kFixed, Amp, false>(threads), 0);
+  probe(windowed_kernel<kFixed, Amp, 0, true>, coreas_block<kFixed, Amp, true>(threads), 0);
   probe(windowed_kernel<kFixed, Amp, 1, false>, zhs_block<Amp>(threads), 1);
   probe(windowed_kernel<kFixed, Amp, 1, true>, zhs_block<Amp>(threads), 1);
   if constexpr (kFixed) {  // the two passes
     probe(windowed_kernel<true, Amp, 1, false, 1>, zhs_block<Amp, 1>(threads), 1, 1);
     probe(windowed_kernel<true, Amp, 1, true, 1>, zhs_block<Amp, 1>(threads), 1, 1);
-    probe(windowed_kernel<true, Amp, 1, false, 2>, zhs_block<Amp, 2>(threads), 1, 2);
-    probe(windowed_kernel<true, Amp, 1, true, 2>, zhs_block<Amp, 2>(threads), 1, 2);
     probe(windowed_kernel<true, Amp, 1, false, 3>, zhs_block<Amp, 3>(threads), 1, 3);
     probe(windowed_kernel<true, Amp, 1, true, 3>, zhs_block<Amp, 3>(threads), 1, 3);
   }

@@ -78,14 +78,16 @@ struct IngestTerms {
 bool shared_destination(ObserverCache const* observers, std::size_t count, Destination& out);
 // The track limits of the filtered paths over `count` observers, narrowed from
 // `limits` (start from widest_limits()).
-inline TrackLimits widest_limits() { return TrackLimits{1e300, 1e300}; }
+inline TrackLimits widest_limits() { return TrackLimits{1e300, 1e300, 1e300}; }
 inline void narrow_limits(ObserverCache const* observers, std::size_t count, TrackLimits& limits) {
   for (std::size_t i = 0; i < count; ++i) {
     ObserverCache const& o = observers[i];
     double const start = o.start_time < 0. ? -o.start_time : o.start_time;
-    double const time = kMaxLeanBins / o.sample_rate - start, duration = 0x1p21 / o.sample_rate;
+    double const time = kMaxLeanTime / o.sample_rate - start, duration = 0x1p21 / o.sample_rate;
+    double const length = kMaxLeanTime * kSpeedOfLight / o.sample_rate;
     if (!(time >= limits.time)) limits.time = time;  // may be negative: no track then
     if (!(duration >= limits.duration)) limits.duration = duration;
+    if (!(length >= limits.length)) limits.length = length;
   }
 }
 
@@ -93,18 +95,12 @@ inline void narrow_limits(ObserverCache const* observers, std::size_t count, Tra
 // observer) items drawn from an atomic counter.  Passed as a __grid_constant__
 // kernel parameter (no host-to-device copy; graph-capturable).
 constexpr int kMaxEventsPerLaunch = 64;
-// Pairs a batched launch takes beyond its first event (its two-pass ZHS
-// storage stays near 8% of them).
-constexpr uint64_t kMaxPairsPerLaunch = 4000000000ull;
 constexpr int kPlanEntries = kMaxEventsPerLaunch + 1;  // + the short-chunk tail of the last event
 constexpr int kWindowThreads = 640;  // upper bound (and default) of the windowed block size
-// Where the first pass of a two-pass ZHS launch left a work item's deferred
-// pairs: `count` entries from `begin` of CTA `cta`'s list; `redo` when the
-// second pass projects the item in full (its window could not be shown free
-// of overflow, its trace was longer than the window, or the CTA's list was
-// full).
+// A work item that the first pass of a two-pass ZHS launch handed back.
 struct ItemState {
-  uint32_t cta, begin, count, redo;
+  uint64_t item;
+  uint64_t pad_;
 };
 
 struct WorkPlan {
@@ -124,14 +120,11 @@ struct WorkPlan {
   unsigned long long* reruns;
   // Items the first pass of two handed to the second; counted when not null.
   unsigned long long* handbacks;
-  // Two-pass ZHS (fixed point), when item_state is set: the first pass runs
-  // the track loop alone and keeps each CTA's deferred pairs of all its items
-  // in its list (`deferred`), the second drains them item by item and
-  // projects in full the items the first handed back, with its own lists
-  // (`drain_deferred`, deferred_stride entries a CTA) and work counter.
-  // The drain needs more registers than the track loop, so the track loop
-  // runs larger CTAs on its own (attach_deferred sets these).  The first
-  // pass's lists hold `deferred_capacity` entries a CTA.
+  // Two-pass ZHS (fixed point), when item_state is set: the first pass projects
+  // the items it can with unchecked window adds and appends the others to
+  // item_state, counted by drain_next_item; the second projects those in full,
+  // with its own lists (`drain_deferred`, deferred_stride entries a CTA).
+  // attach_deferred sets these; deferred_capacity is the stride of `deferred`.
   ItemState* item_state;
   unsigned int* drain_deferred;
   unsigned int* drain_next_item;
@@ -153,33 +146,11 @@ inline uint32_t deferred_list_stride(WorkPlan const& plan) {
   return stride;
 }
 
-// Pairs a launch of `plan` covers at most (its items' chunks at full length).
-inline uint64_t plan_pairs(WorkPlan const& plan) {
-  uint64_t pairs = 0;
-  for (uint32_t e = 0; e < plan.event_count; ++e) {
-    EventPlan const& ev = plan.events[e];
-    pairs += static_cast<uint64_t>(ev.chunks) * ev.chunk_size * ev.observer_count[plan.algorithm];
-  }
-  return pairs;
-}
-
-// First-pass list entries a CTA of a two-pass launch holds: the deferred
-// pairs of all its items, sized for 8% of its share of the launch's pairs
-// (ZHS defers 3% on the 1e7 x 160 workload) and at least one chunk; an item
-// past the end is handed back to the second pass (correct, slower).
-constexpr double kTwoPassDeferredShare = 0.08;
 // Launches whose two-pass storage would pass 2^30 words (4 GiB) run one pass.
 constexpr uint64_t kTwoPassMaxWords = 1ull << 30;
 
-inline uint64_t pass1_capacity(WorkPlan const& plan, uint64_t ctas) {
-  uint64_t const share = static_cast<uint64_t>(kTwoPassDeferredShare * static_cast<double>(plan_pairs(plan)) /
-                                               static_cast<double>(ctas > 0 ? ctas : 1)) + 1;
-  uint64_t const capacity = share > plan.deferred_stride ? share : plan.deferred_stride;
-  return capacity < 0xffffffffull ? capacity : 0xffffffffull;
-}
-
 inline uint64_t two_pass_words(WorkPlan const& plan, uint64_t ctas) {
-  return ctas * pass1_capacity(plan, ctas) + ctas * plan.deferred_stride +
+  return 2 * ctas * plan.deferred_stride +
          plan.total_items * (sizeof(ItemState) / sizeof(unsigned)) + 1;
 }
 
@@ -205,8 +176,7 @@ inline void attach_deferred(WorkPlan& plan, unsigned* words, uint64_t ctas, bool
   plan.drain_next_item = nullptr;
   plan.deferred_capacity = plan.deferred_stride;
   if (!two_pass(plan, ctas, fixed)) return;
-  uint64_t const first = ctas * pass1_capacity(plan, ctas);
-  plan.deferred_capacity = static_cast<uint32_t>(pass1_capacity(plan, ctas));
+  uint64_t const first = ctas * plan.deferred_stride;
   plan.drain_deferred = words + first;
   plan.item_state = reinterpret_cast<ItemState*>(words + first + ctas * plan.deferred_stride);
   plan.drain_next_item = reinterpret_cast<unsigned*>(plan.item_state + plan.total_items);

@@ -1,0 +1,84 @@
+"""The filtered mixed-precision paths and the ZHS deposits as differences, where
+their bins sit on an edge: traces of one, two and odd numbers of bins, cut
+through the pulse at either end, samples at whole and half bins, and antennas
+inside a track's reach.  FP64 traces equal the oracle's bit for bit; mixed
+precision's sample counts per bin and counters equal the oracle's."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+COUNTERS = ("coreas_contributions", "zhs_contributions", "zhs_subtracks", "valid_tracks", "fixed_point_overflows")
+
+
+def project(pkg, config, records, tuning=None):
+    import torch
+
+    raw = torch.from_numpy(np.ascontiguousarray(records).view(np.uint8).reshape(-1)).cuda()
+    acc = pkg.RadioAccumulator(config, tuning)
+    acc.accumulate_lepton_tracks(raw.data_ptr(), records.size)
+    got = acc.download_fixed()
+    acc.close()
+    return got
+
+
+def check(pkg, oracle, showers, workload, records, tuning=None, **extra):
+    for precision, counting in ((0, False), (0, True), (1, True)):
+        config = showers.make_config(workload, precision=precision, kernel=2, count_samples=counting, **extra)
+        got = project(pkg, config, records, tuning)
+        want = oracle.restatement().project(showers.make_config(workload, count_samples=counting, **extra), records,
+                                            threads=16)
+        for k in range(2):
+            assert np.array_equal(got[k], want[k]), (precision, counting, k, np.count_nonzero(got[k] != want[k]))
+        for key in COUNTERS:
+            assert got[2][key] == want[2][key], (precision, counting, key)
+
+
+@pytest.mark.parametrize("bins", [1, 2, 31, 32, 33, 97, 1023, 4099])
+def test_traces_cut_through_the_pulse(pkg, oracle, showers, bins):
+    wl, gen, _ = showers.workload_config("plain_c0", bins=bins)
+    records = showers.shower_records(20_003, seed=17 + bins, **gen)
+    observers = wl["observers"].copy()
+    observers["start_time_s"] += np.linspace(30e-9, 70e-9, len(observers))  # from before the pulse into it
+    wl["observers"] = observers
+    check(pkg, oracle, showers, wl, records, pkg.TuningParameters(track_tile_size=4000))
+
+
+def test_samples_at_whole_and_half_bins(pkg, oracle, showers):
+    """Tracks along one line towards an antenna in vacuum: every arrival is a
+    whole or half number of bins, so no guard can decide and each pair takes the
+    exact evaluation."""
+    c = showers.SPEED_OF_LIGHT
+    count = 4096
+    step = c / 1e10  # one bin of path
+    start = np.zeros((count, 3))
+    start[:, 2] = 1000.0 + 0.5 * step * np.arange(count)
+    direction = np.tile([0.0, 0.0, -1.0], (count, 1))
+    length = np.full(count, 8 * step)
+    t0 = np.zeros(count)
+    seg = dict(start=start, end=start + length[:, None] * direction, t_start=t0, t_end=t0 + length / (0.5 * c),
+               pid=np.where(np.arange(count) % 2, 11, -11).astype(np.int32), energy_gev=np.full(count, 1e-3),
+               direction=direction, weight=np.ones(count))
+    observers = np.zeros(3, pkg.abi.OBSERVER)
+    observers["position_m"][1] = (3.0, 0.0, 0.0)
+    observers["position_m"][2] = (0.0, 0.0, 1200.0)  # between the tracks
+    observers["start_time_s"] = (1000.0 / c, 1000.0 / c, 0.0)
+    observers["duration_s"] = 2047 / 1e10
+    observers["sample_rate_hz"] = 1e10
+    observers["number_of_bins"] = 2048
+    wl = dict(observers=observers, homogeneous=1.0, table=None)
+    check(pkg, oracle, showers, wl, showers.to_records(seg))
+
+
+@pytest.mark.parametrize("scale", [1e-6, 1e3, 1e6])
+def test_times_outside_the_guards_reach(pkg, oracle, showers, scale):
+    """Track times shifted until the filtered paths' bounds no longer cover them
+    (the last scales): those tracks are evaluated exactly."""
+    wl, gen, _ = showers.workload_config("ice_c2", bins=1000)
+    records = showers.ice_records(6_001, seed=5, **gen)
+    shift = 3.7e-6 * scale
+    records["start"]["time_s"] += shift
+    records["end"]["time_s"] += shift
+    wl["observers"] = wl["observers"][::5].copy()
+    wl["observers"]["start_time_s"] += shift
+    check(pkg, oracle, showers, wl, records)
