@@ -326,8 +326,8 @@ class RadioAccumulator:
             self._h, C.c_void_p(device_pointer), count, count if extent is None else extent))
 
     def download(self) -> RadioWaveforms:
-        coreas = np.zeros((3, self.coreas_bins), np.float64)
-        zhs = np.zeros((3, self.zhs_bins), np.float64)
+        coreas = np.empty((3, self.coreas_bins), np.float64)
+        zhs = np.empty((3, self.zhs_bins), np.float64)
         counters = abi.Counters()
         self._check(self._lib.c8r_download(
             self._h, coreas.ctypes.data if coreas.size else None,
@@ -343,8 +343,8 @@ class RadioAccumulator:
         return counters.as_dict()
 
     def download_fixed(self):
-        coreas = np.zeros((3, self.coreas_bins), np.int64)
-        zhs = np.zeros((3, self.zhs_bins), np.int64)
+        coreas = np.empty((3, self.coreas_bins), np.int64)
+        zhs = np.empty((3, self.zhs_bins), np.int64)
         counters = abi.Counters()
         self._check(self._lib.c8r_download_fixed(
             self._h, coreas.ctypes.data if coreas.size else None,
@@ -512,8 +512,8 @@ class RadioServer:
     def fetch_fixed(self, event: int):
         """(coreas int64 (3, bins), zhs int64 (3, bins), counters, info); releases the event."""
         nc, nz = self._configs[event]
-        coreas = np.zeros((3, nc), np.int64)
-        zhs = np.zeros((3, nz), np.int64)
+        coreas = np.empty((3, nc), np.int64)
+        zhs = np.empty((3, nz), np.int64)
         counters, info = abi.Counters(), abi.ServerEventInfo()
         self._check(self._lib.c8r_server_fetch_fixed(
             self._h, event, coreas.ctypes.data if coreas.size else None,
@@ -524,8 +524,8 @@ class RadioServer:
     def fetch(self, event: int):
         """(RadioWaveforms decoded to V/m and V s/m, info); releases the event."""
         nc, nz = self._configs[event]
-        coreas = np.zeros((3, nc), np.float64)
-        zhs = np.zeros((3, nz), np.float64)
+        coreas = np.empty((3, nc), np.float64)
+        zhs = np.empty((3, nz), np.float64)
         counters, info = abi.Counters(), abi.ServerEventInfo()
         try:
             self._check(self._lib.c8r_server_fetch(

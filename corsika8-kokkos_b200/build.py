@@ -17,7 +17,7 @@ CSRC = HERE / "csrc"
 LIBRARY = HERE / "libc8radio.so"
 SOURCES = ["radio_kernels.cu", "accumulator.cu", "probes.cu", "no_alloc.cu", "server.cu",
            "precision_study.cu", "spool.cu", "snapshot.cu", "tuning.cu"]
-HEADERS = ["radio_device.cuh", "radio_kernels.cuh", "host_setup.hpp", "status.hpp"]
+HEADERS = ["radio_device.cuh", "radio_kernels.cuh", "host_setup.hpp", "status.hpp", "transfer.hpp"]
 
 NVCC_FLAGS = [
     "-std=c++17",

@@ -23,12 +23,20 @@
 #include "host_setup.hpp"
 #include "radio_kernels.cuh"
 #include "status.hpp"
+#include "transfer.hpp"
 
 namespace c8r {
 namespace {
 
 constexpr std::size_t kDefaultHostBatch = 4096;   // RadioAccumulator.hpp:49
 constexpr std::size_t kDirectThreshold = 16384;   // RadioAccumulator.hpp:101
+// Full batches of one pageable host call are ingested as they fill and
+// projected together, at most so many records at a time: a projection costs
+// its launches and a pass over every antenna's window whatever its size.
+constexpr std::size_t kProjectRecords = 65536;
+// Least size of a host staging half: the two also serve as the pinned slots
+// through which results are copied out (SlotRing).
+constexpr std::size_t kHostHalfBytes = 4 * SlotRing::kSlotBytes;
 
 void check(cudaError_t err, char const* what) {
   if (err != cudaSuccess)
@@ -216,8 +224,11 @@ class Accumulator {
     slot_.allocate(1);
     next_item_.allocate(2);  // one work counter per algorithm
     reruns_.allocate(2);  // items re-run with checked adds, items handed to a drain pass
-    staging_.allocate(host_batch_);
-    for (auto& h : host_) h.allocate(host_batch_);
+    staging_.allocate(checked_mul(host_batch_, sizeof(c8r_lepton_transport_record)));
+    for (auto& h : host_) {
+      h.allocate(std::max(checked_mul(host_batch_, kUsedBytes), kHostHalfBytes));
+      check(ring_.use(h.ptr, kHostHalfBytes), "event");
+    }
     for (auto& e : host_ready_) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
     fuse_ = coreas_enabled_ && zhs_enabled_ && observers_share_grid();
     initialized_ = true;
@@ -282,16 +293,21 @@ class Accumulator {
       enqueue_pinned(records, count);
       return;
     }
+    if (count >= host_batch_ && staged_ == 0)  // room for the batches projected together, in one go
+      ensure_capacity(std::max(host_batch_, std::min(host_count_ + count, kProjectRecords)));
     while (count != 0) {
       if (host_count_ == 0) check(cudaEventSynchronize(host_ready_[host_index_]), "staging wait");
       std::size_t const copied = std::min(count, host_batch_ - host_count_);
-      std::memcpy(host_[host_index_].ptr + host_count_, records, copied * sizeof(*records));
+      pack_used(host_[host_index_].ptr + host_count_ * kUsedBytes, records, copied);
       host_count_ += copied;
       stats_.host_tracks_enqueued += copied;
       records += copied;
       count -= copied;
-      if (host_count_ == host_batch_) flush();
+      if (host_count_ != host_batch_) break;
+      ingest_host_batch();
+      if (staged_ > kProjectRecords - std::min(kProjectRecords, host_batch_)) project_staged(true);
     }
+    project_staged(true);
   }
 
   static bool is_pinned(void const* p) {
@@ -306,22 +322,23 @@ class Accumulator {
   // The bytes of a record the ingest reads: start.pid through start.weight
   // and end.position through end.time (with the diagnostics' energy and
   // directions), one span of 208 of the record's 752 bytes.  Host records are
-  // uploaded as that span alone, a pitched copy to the same offsets of the
-  // device staging records (whose other bytes the ingest never reads).
+  // staged, uploaded and ingested as that span alone: pageable ones packed by the
+  // caller's copy (60001 records 1.1 ms, whole 2.6) and uploaded in one piece (4096
+  // spans 19 us), pinned ones by a copy of equal pitches (24 us; one that changes
+  // the pitch moves a row in 89 ns, 364 us).
   static constexpr std::size_t kUsedBegin = offsetof(c8r_lepton_transport_record, start);
   static constexpr std::size_t kUsedEnd =
       offsetof(c8r_lepton_transport_record, end) + offsetof(c8r_particle_state, time_s) + sizeof(double);
+  static constexpr std::size_t kUsedBytes = kUsedEnd - kUsedBegin;
   static_assert(offsetof(c8r_particle_state, weight) + sizeof(double) <=
                     offsetof(c8r_lepton_transport_record, end) - offsetof(c8r_lepton_transport_record, start),
                 "start fields inside the span");
-  static_assert(kUsedEnd - kUsedBegin == 208, "208-byte span of the 752-byte record");
+  static_assert(kUsedBytes == 208, "208-byte span of the 752-byte record");
 
-  cudaError_t upload_used(c8r_lepton_transport_record* dst, c8r_lepton_transport_record const* src,
-                          std::size_t n, cudaStream_t stream) {
-    constexpr std::size_t kPitch = sizeof(c8r_lepton_transport_record);
-    return cudaMemcpy2DAsync(reinterpret_cast<unsigned char*>(dst) + kUsedBegin, kPitch,
-                             reinterpret_cast<unsigned char const*>(src) + kUsedBegin, kPitch,
-                             kUsedEnd - kUsedBegin, n, cudaMemcpyHostToDevice, stream);
+  static void pack_used(unsigned char* out, c8r_lepton_transport_record const* records, std::size_t n) {
+    auto const* in = reinterpret_cast<unsigned char const*>(records) + kUsedBegin;
+    for (std::size_t i = 0; i < n; ++i)
+      std::memcpy(out + i * kUsedBytes, in + i * sizeof(c8r_lepton_transport_record), kUsedBytes);
   }
 
   // Batches of host_batch_ records (the last one partial) copied from pinned
@@ -339,7 +356,7 @@ class Accumulator {
       check(cudaStreamCreateWithFlags(&copy_stream_, cudaStreamNonBlocking), "copy stream");
       for (auto& e : copy_done_) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
       for (auto& e : consumed_) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-      staging2_.allocate(host_batch_);
+      staging2_.allocate(checked_mul(host_batch_, sizeof(c8r_lepton_transport_record)));
     }
     // earlier work on the accumulator stream may still read staging_
     for (auto& e : consumed_) check(cudaEventRecord(e, stream_), "event");
@@ -349,17 +366,20 @@ class Accumulator {
       std::size_t const n = std::min(count - offset, size);
       size = std::min(host_batch_, 2 * size);
       int const k = static_cast<int>(b & 1);
-      c8r_lepton_transport_record* dst = k ? staging2_.ptr : staging_.ptr;
+      unsigned char* const dst = k ? staging2_.ptr : staging_.ptr;
       // the staging buffer is free once the ingest that read it has run
       check(cudaStreamWaitEvent(copy_stream_, consumed_[k], 0), "wait");
-      check(upload_used(dst, records + offset, n, copy_stream_), "host track upload");
+      constexpr std::size_t kPitch = sizeof(c8r_lepton_transport_record);
+      check(cudaMemcpy2DAsync(dst, kPitch, reinterpret_cast<unsigned char const*>(records + offset) + kUsedBegin,
+                              kPitch, kUsedBytes, n, cudaMemcpyHostToDevice, copy_stream_),
+            "host track upload");
       check(cudaEventRecord(copy_done_[k], copy_stream_), "event");
       check(cudaStreamWaitEvent(stream_, copy_done_[k], 0), "wait");
-      stage_device(dst, n, host_batch_);
+      stage_spans(dst, kPitch, n);
       check(cudaEventRecord(consumed_[k], stream_), "event");
       project_staged(true);
       offset += n;
-      stats_.host_to_device_bytes += n * (kUsedEnd - kUsedBegin);
+      stats_.host_to_device_bytes += n * kUsedBytes;
       ++stats_.host_track_batches;
       stats_.host_tracks_enqueued += n;
     }
@@ -371,13 +391,20 @@ class Accumulator {
   // filled while it uploads (double buffering replaces the reference's fence).
   void flush() {
     if (host_count_ == 0) return;
+    ingest_host_batch();
+    project_staged(true);
+  }
+
+  // Uploads and ingests the staging half just filled.
+  void ingest_host_batch() {
     std::size_t const n = host_count_;
-    check(upload_used(staging_.ptr, host_[host_index_].ptr, n, stream_), "host track upload");
+    check(cudaMemcpyAsync(staging_.ptr, host_[host_index_].ptr, n * kUsedBytes, cudaMemcpyHostToDevice, stream_),
+          "host track upload");
     check(cudaEventRecord(host_ready_[host_index_], stream_), "event");
     host_index_ ^= 1;
     host_count_ = 0;
-    accumulate_device(staging_.ptr, n, staging_.count);
-    stats_.host_to_device_bytes += n * (kUsedEnd - kUsedBegin);
+    stage_spans(staging_.ptr, kUsedBytes, n);
+    stats_.host_to_device_bytes += n * kUsedBytes;
     ++stats_.host_track_batches;
   }
 
@@ -398,12 +425,18 @@ class Accumulator {
     if (sealed_) throw std::logic_error("radio endpoint already committed; reset before new tracks");
     if (count > extent) throw std::out_of_range("radio track count exceeds input view");
     if (records == nullptr) throw std::invalid_argument("null device radio track input");
+    stage_spans(reinterpret_cast<unsigned char const*>(records) + kUsedBegin, sizeof(*records), count);
+  }
+
+  // The same from the records' used spans, `pitch` bytes apart, in device memory.
+  void stage_spans(void const* spans, std::size_t pitch, std::size_t count) {
+    if (sealed_) throw std::logic_error("radio endpoint already committed; reset before new tracks");
     if (staged_ > std::numeric_limits<std::size_t>::max() - count)
       throw std::length_error("radio staged track count overflow");
     ensure_capacity(staged_ + count);
     if (staged_ == 0) check(cudaMemsetAsync(slot_.ptr, 0, sizeof(unsigned long long), stream_), "memset");
-    check(launch_ingest(records, count, tracks_.ptr, capacity_, slot_.ptr, counters_.ptr,
-                        diagnostics_, terms_, stream_),
+    check(launch_ingest_spans(spans, pitch, count, tracks_.ptr, capacity_, slot_.ptr, counters_.ptr, diagnostics_,
+                              terms_, stream_),
           "ingest launch");
     staged_ += count;
     ++stats_.track_precompute_batches;
@@ -548,6 +581,7 @@ class Accumulator {
     if (host.fixed_point_overflows != 0)
       throw std::runtime_error(
           "radio fixed-point accumulator overflowed; increase fixed_point_field_limit_V_per_m");
+    Transfers transfers;
     for (int a = 0; a < 2; ++a) {
       double* out = a == 0 ? coreas : zhs;
       std::size_t const values = 3 * bins_[a];
@@ -558,16 +592,12 @@ class Accumulator {
                             static_cast<uint32_t>(observers_host_[a].size()), max_observer_bins_[a],
                             stream_),
               "decode launch");
-        check(cudaMemcpyAsync(out, decoded_[a].ptr, values * sizeof(double), cudaMemcpyDeviceToHost,
-                              stream_),
-              "trace download");
+        transfers.add(out, decoded_[a].ptr, values * sizeof(double));
       } else {
-        check(cudaMemcpyAsync(out, float_traces_[a].ptr, values * sizeof(double),
-                              cudaMemcpyDeviceToHost, stream_),
-              "trace download");
+        transfers.add(out, float_traces_[a].ptr, values * sizeof(double));
       }
-      stats_.device_to_host_bytes += values * sizeof(double);
     }
+    copy_out(transfers);
     check(cudaStreamSynchronize(stream_), "download fence");
     if (counters) std::memcpy(counters, &host, sizeof(host));
     downloaded_ = true;
@@ -613,15 +643,14 @@ class Accumulator {
     sealed_ = true;
     DeviceCounters host{};
     fetch_counters(host);
+    Transfers transfers;
     for (int a = 0; a < 2; ++a) {
       long long* out = a == 0 ? coreas : zhs;
       std::size_t const values = 3 * bins_[a];
       if (values == 0 || out == nullptr) continue;
-      check(cudaMemcpyAsync(out, fixed_traces_[a].ptr, values * sizeof(long long),
-                            cudaMemcpyDeviceToHost, stream_),
-            "fixed trace download");
-      stats_.device_to_host_bytes += values * sizeof(long long);
+      transfers.add(out, fixed_traces_[a].ptr, values * sizeof(long long));
     }
+    copy_out(transfers);
     check(cudaStreamSynchronize(stream_), "download fence");
     if (counters) std::memcpy(counters, &host, sizeof(host));
     downloaded_ = true;
@@ -648,19 +677,17 @@ class Accumulator {
     sealed_ = true;
     DeviceCounters host{};
     fetch_counters(host);
+    Transfers transfers;
     for (int a = 0; a < 2; ++a) {
       long long* out = a == 0 ? coreas : zhs;
       std::size_t const values = 3 * config_bins_[a];
       if (values == 0) continue;
-      if (fixed_traces_[a].ptr && bins_[a] == config_bins_[a]) {
-        check(cudaMemcpyAsync(out, fixed_traces_[a].ptr, values * sizeof(long long),
-                              cudaMemcpyDeviceToHost, stream_),
-              "fixed trace download");
-        stats_.device_to_host_bytes += values * sizeof(long long);
-      } else {
+      if (fixed_traces_[a].ptr && bins_[a] == config_bins_[a])
+        transfers.add(out, fixed_traces_[a].ptr, values * sizeof(long long));
+      else
         std::memset(out, 0, values * sizeof(long long));  // algorithm disabled
-      }
     }
+    copy_out(transfers);
     check(cudaStreamSynchronize(stream_), "download fence");
     if (counters) std::memcpy(counters, &host, sizeof(host));
     if (host.fixed_point_overflows != 0)
@@ -669,6 +696,39 @@ class Accumulator {
   }
 
   std::size_t config_bins(int a) const { return config_bins_[a]; }
+
+  // Device buffers and the host memory that takes them.
+  struct Transfers {
+    std::vector<SlotRing::Segment> out;
+    std::vector<unsigned char const*> from;
+    void add(void* destination, void const* source, std::size_t bytes) {
+      out.push_back({destination, bytes});
+      from.push_back(static_cast<unsigned char const*>(source));
+    }
+  };
+
+  // Copies after the stream's earlier work and returns when they are done:
+  // page-locked destinations directly, pageable ones through the slots.
+  void copy_out(Transfers const& transfers) {
+    Transfers pageable;
+    for (std::size_t k = 0; k < transfers.out.size(); ++k) {
+      SlotRing::Segment const& d = transfers.out[k];
+      stats_.device_to_host_bytes += d.bytes;
+      if (ring_.usable() && !is_pinned(d.destination))
+        pageable.add(d.destination, transfers.from[k], d.bytes);
+      else
+        check(cudaMemcpyAsync(d.destination, transfers.from[k], d.bytes, cudaMemcpyDeviceToHost, stream_),
+              "trace download");
+    }
+    if (pageable.out.empty()) return;
+    // the slots are the host staging halves: no batch is filling (flushed), none is being uploaded
+    for (auto& e : host_ready_) check(cudaEventSynchronize(e), "staging wait");
+    check(ring_.run(pageable.out, stream_,
+                    [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
+                      return cudaMemcpyAsync(slot, pageable.from[k] + offset, bytes, cudaMemcpyDeviceToHost, stream_);
+                    }),
+          "trace download");
+  }
 
   void statistics(c8r_statistics& out) {
     resolve_timing();
@@ -1115,13 +1175,14 @@ class Accumulator {
   DeviceBuffer<double> tracks_;
   std::size_t capacity_ = 0;
   std::size_t staged_ = 0;  // records ingested since the last projection (upper bound of tracks)
-  DeviceBuffer<c8r_lepton_transport_record> staging_, staging2_;
+  DeviceBuffer<unsigned char> staging_, staging2_;  // used spans of host_batch_ records, a record apart at most
   cudaStream_t copy_stream_ = nullptr;
   cudaEvent_t copy_done_[2] = {nullptr, nullptr};
   cudaEvent_t consumed_[2] = {nullptr, nullptr};
   cudaStream_t side_stream_ = nullptr;               // ZHS launches beside CoREAS
   cudaEvent_t side_events_[2] = {nullptr, nullptr};  // tracks ingested, ZHS done
-  PinnedBuffer<c8r_lepton_transport_record> host_[2];
+  PinnedBuffer<unsigned char> host_[2];  // used spans of host_batch_ records; slots of ring_
+  SlotRing ring_;
   cudaEvent_t host_ready_[2] = {nullptr, nullptr};
   // (begin, end) event pairs; tag -1 = a whole accumulate's projection,
   // 0 / 1 = the windowed CoREAS / ZHS launch inside it

@@ -19,6 +19,7 @@
 
 #include <cuda_runtime.h>
 
+#include <cstddef>
 #include <cstring>
 
 #include "../../include/c8radio.h"
@@ -1525,17 +1526,25 @@ __device__ __forceinline__ int energy_bin(double kinetic) {
 // The fields radio reads from a track step, from 752-byte records or from
 // columns (one device array per field): the same arithmetic follows.
 struct RecordSource {
-  const c8r_lepton_transport_record* records;
-  __device__ int pid(uint64_t i) const { return records[i].start.pid; }
-  __device__ double weight(uint64_t i) const { return records[i].start.weight; }
-  __device__ double start_energy(uint64_t i) const { return records[i].start.energy_gev; }
-  __device__ double start_position(uint64_t i, int a) const { return records[i].start.position_m[a]; }
-  __device__ double end_position(uint64_t i, int a) const { return records[i].end.position_m[a]; }
-  __device__ double start_time(uint64_t i) const { return records[i].start.time_s; }
-  __device__ double end_time(uint64_t i) const { return records[i].end.time_s; }
-  __device__ double start_direction(uint64_t i, int a) const { return records[i].start.direction[a]; }
-  __device__ double end_direction(uint64_t i, int a) const { return records[i].end.direction[a]; }
+  const unsigned char* starts;  // the first record's start state, its end state after it
+  uint64_t pitch;               // bytes from one record's to the next's
+  __device__ const c8r_particle_state& start(uint64_t i) const {
+    return *reinterpret_cast<const c8r_particle_state*>(starts + i * pitch);
+  }
+  __device__ const c8r_particle_state& end(uint64_t i) const { return (&start(i))[1]; }
+  __device__ int pid(uint64_t i) const { return start(i).pid; }
+  __device__ double weight(uint64_t i) const { return start(i).weight; }
+  __device__ double start_energy(uint64_t i) const { return start(i).energy_gev; }
+  __device__ double start_position(uint64_t i, int a) const { return start(i).position_m[a]; }
+  __device__ double end_position(uint64_t i, int a) const { return end(i).position_m[a]; }
+  __device__ double start_time(uint64_t i) const { return start(i).time_s; }
+  __device__ double end_time(uint64_t i) const { return end(i).time_s; }
+  __device__ double start_direction(uint64_t i, int a) const { return start(i).direction[a]; }
+  __device__ double end_direction(uint64_t i, int a) const { return end(i).direction[a]; }
 };
+static_assert(offsetof(c8r_lepton_transport_record, end) ==
+                  offsetof(c8r_lepton_transport_record, start) + sizeof(c8r_particle_state),
+              "a record's end state follows its start state");
 
 struct ColumnSource {
   c8r_track_columns columns;
@@ -2582,6 +2591,29 @@ __global__ void decode_kernel(const long long* __restrict__ fixed, double* __res
   }
 }
 
+// A run of decoded values, [begin, begin + count) of a trace buffer's rows
+// [X | Y | Z], into `out` (page-locked host memory): value times the decode
+// factor of its observer (downloadSet, RadioAccumulator.inl:865-867), found by
+// its waveform offset.
+__global__ void decode_run_kernel(const long long* __restrict__ fixed, double* __restrict__ out, uint64_t total_bins,
+                                  uint64_t begin, uint64_t count, const ObserverCache* __restrict__ observers,
+                                  uint32_t observer_count, double limit, int differentiated) {
+  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
+       i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
+    uint64_t const bin = (begin + i) % total_bins;
+    uint32_t lo = 0, hi = observer_count;  // last observer whose offset is at most bin
+    while (hi - lo > 1) {
+      uint32_t const mid = (lo + hi) >> 1;
+      if (observers[mid].offset <= bin)
+        lo = mid;
+      else
+        hi = mid;
+    }
+    double const scale = differentiated ? observers[lo].sample_rate : 1.;
+    out[i] = static_cast<double>(fixed[begin + i]) * (limit / (kHeadroom * scale));
+  }
+}
+
 // The output step on the device: CoREAS fields added as they are, ZHS
 // potentials differentiated into fields E_i = -(A_{i+1} - A_i) fs at the bin
 // midpoints (RadioProcess.inl:213-223; one sample fewer per observer), both
@@ -2751,15 +2783,25 @@ int ctas_per_sm(int window, int threads) {
 
 }  // namespace
 
+cudaError_t launch_ingest_spans(const void* starts, uint64_t pitch, uint64_t count, double* tracks,
+                                uint64_t stride, unsigned long long* slot, DeviceCounters* counters,
+                                bool diagnostics, IngestTerms const& terms, cudaStream_t stream) {
+  if (count == 0) return cudaSuccess;
+  uint64_t const blocks = (count + 255) / 256;
+  ingest_kernel<RecordSource><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
+      RecordSource{static_cast<const unsigned char*>(starts), pitch}, count, tracks, stride, slot, counters,
+      diagnostics, terms);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_ingest(const c8r_lepton_transport_record* records, uint64_t count,
                           double* tracks, uint64_t stride, unsigned long long* slot,
                           DeviceCounters* counters, bool diagnostics, IngestTerms const& terms,
                           cudaStream_t stream) {
-  if (count == 0) return cudaSuccess;
-  uint64_t const blocks = (count + 255) / 256;
-  ingest_kernel<RecordSource><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-      RecordSource{records}, count, tracks, stride, slot, counters, diagnostics, terms);
-  return cudaGetLastError();
+  return launch_ingest_spans(reinterpret_cast<const unsigned char*>(records) +
+                                 offsetof(c8r_lepton_transport_record, start),
+                             sizeof(c8r_lepton_transport_record), count, tracks, stride, slot, counters, diagnostics,
+                             terms, stream);
 }
 
 cudaError_t launch_ingest_columns(c8r_track_columns const& columns, uint64_t count, double* tracks,
@@ -2846,6 +2888,16 @@ cudaError_t launch_output(const long long* fixed, const double* floating, double
   dim3 const grid(static_cast<unsigned>(bx), observer_count);
   output_kernel<<<grid, 256, 0, stream>>>(fixed, floating, out, total_bins, observers, factors,
                                           observer_count, differentiate ? 1 : 0);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_decode_run(const long long* fixed, double* out, uint64_t total_bins, uint64_t begin,
+                              uint64_t count, const ObserverCache* observers, uint32_t observer_count, double limit,
+                              int algorithm, cudaStream_t stream) {
+  if (count == 0) return cudaSuccess;
+  uint64_t const blocks = (count + 255) / 256;
+  decode_run_kernel<<<static_cast<unsigned>(blocks < 1024 ? blocks : 1024), 256, 0, stream>>>(
+      fixed, out, total_bins, begin, count, observers, observer_count, limit, algorithm == 1 ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -235,6 +235,12 @@ cudaError_t launch_ingest(const c8r_lepton_transport_record* records, uint64_t c
                           DeviceCounters* counters, bool diagnostics, IngestTerms const& terms,
                           cudaStream_t stream);
 
+// The same from records' start and end states `pitch` bytes apart, the first
+// record's at `starts`.
+cudaError_t launch_ingest_spans(const void* starts, uint64_t pitch, uint64_t count, double* tracks,
+                                uint64_t stride, unsigned long long* slot, DeviceCounters* counters,
+                                bool diagnostics, IngestTerms const& terms, cudaStream_t stream);
+
 // The same ingest from a structure-of-arrays view of the steps.
 cudaError_t launch_ingest_columns(c8r_track_columns const& columns, uint64_t count, double* tracks,
                                   uint64_t stride, unsigned long long* slot, DeviceCounters* counters,
@@ -274,6 +280,11 @@ cudaError_t launch_study(EventPlan const& event, uint64_t track_bound, bool core
 cudaError_t launch_output(const long long* fixed, const double* floating, double* out, uint64_t total_bins,
                           const ObserverCache* observers, const double* factors, uint32_t observer_count,
                           uint64_t max_bins, bool differentiate, cudaStream_t stream);
+
+// Decodes values [begin, begin + count) of a trace buffer into `out`.
+cudaError_t launch_decode_run(const long long* fixed, double* out, uint64_t total_bins, uint64_t begin,
+                              uint64_t count, const ObserverCache* observers, uint32_t observer_count, double limit,
+                              int algorithm, cudaStream_t stream);
 
 // Fixed-point decode on the device: out[r*bins + i] = in[r*bins + i] * factor(observer).
 cudaError_t launch_decode(const long long* fixed, double* out, uint64_t total_bins,

@@ -37,6 +37,7 @@
 #include "../../include/c8radio.h"
 #include "host_setup.hpp"
 #include "radio_kernels.cuh"
+#include "transfer.hpp"
 
 namespace c8r {
 void set_global_error(char const* message);  // accumulator.cu
@@ -55,6 +56,8 @@ void check(cudaError_t err, char const* what) {
 }
 
 constexpr std::size_t kGranule = 256;
+// Pinned slots of the fetches: page-locking costs about a millisecond a megabyte.
+constexpr std::size_t kFetchBytes = 4 * SlotRing::kSlotBytes;
 std::size_t round_up(std::size_t bytes) { return (bytes + kGranule - 1) / kGranule * kGranule; }
 
 // First-fit sub-allocator over one device reservation, coalescing on release.
@@ -209,6 +212,8 @@ class Server {
     check(cudaStreamCreateWithFlags(&admit_, cudaStreamNonBlocking), "stream");
     check(cudaStreamCreateWithFlags(&fetch_, cudaStreamNonBlocking), "stream");
     check(cudaMalloc(&next_item_, 64 * sizeof(unsigned)), "work counters");
+    check(cudaMallocHost(&fetch_slots_, kFetchBytes), "fetch slots");
+    check(ring_.use(fetch_slots_, kFetchBytes), "fetch slots");
     epoch_ = std::chrono::steady_clock::now();
     scheduler_ = std::thread([this] { run(); });
   }
@@ -235,6 +240,7 @@ class Server {
     cudaStreamDestroy(admit_);
     cudaStreamDestroy(fetch_);
     cudaFree(next_item_);
+    cudaFreeHost(fetch_slots_);
     if (deferred_) cudaFree(deferred_);
     arena_.free_all();
     if (previous >= 0) cudaSetDevice(previous);
@@ -477,27 +483,31 @@ class Server {
     ev.fetching = true;
     lock.unlock();
     DeviceCounters host{};
-    std::vector<long long> staging;
     try {
       std::lock_guard<std::mutex> copy_lock(fetch_mu_);
       check(cudaMemcpyAsync(&host, ev.counters, sizeof host, cudaMemcpyDeviceToHost, fetch_), "server fetch");
+      // through the pinned slots: copied, or decoded by a kernel straight into them
+      std::vector<SlotRing::Segment> out;
+      std::vector<int> of;
       for (int a = 0; a < 2; ++a) {
-        void* out = a == 0 ? coreas : zhs;
-        std::size_t const values = 3 * ev.bins[a];
-        if (values == 0 || out == nullptr) continue;
-        void const* src = ev.fixed ? static_cast<void const*>(ev.fixed_traces[a])
-                                   : static_cast<void const*>(ev.float_traces[a]);
-        if (ev.fixed && !fixed_out) {
-          staging.resize(values);
-          check(cudaMemcpyAsync(staging.data(), src, values * sizeof(long long), cudaMemcpyDeviceToHost, fetch_),
-                "server fetch");
-          check(cudaStreamSynchronize(fetch_), "server fetch");
-          decode(ev, a, staging.data(), static_cast<double*>(out));
-        } else {
-          check(cudaMemcpyAsync(out, src, values * sizeof(double), cudaMemcpyDeviceToHost, fetch_),
-                "server fetch");
-        }
+        void* const to = a == 0 ? coreas : zhs;
+        if (ev.bins[a] == 0 || to == nullptr) continue;
+        out.push_back({to, 3 * ev.bins[a] * sizeof(double)});
+        of.push_back(a);
       }
+      check(ring_.run(out, fetch_,
+                      [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
+                        int const a = of[k];
+                        std::size_t const first = offset / sizeof(double), n = bytes / sizeof(double);
+                        if (ev.fixed && !fixed_out)
+                          return launch_decode_run(reinterpret_cast<long long const*>(ev.fixed_traces[a]),
+                                                   static_cast<double*>(slot), ev.bins[a], first, n, ev.caches[a],
+                                                   ev.observers[a], ev.limit, a, fetch_);
+                        void const* src = ev.fixed ? static_cast<void const*>(ev.fixed_traces[a] + first)
+                                                   : static_cast<void const*>(ev.float_traces[a] + first);
+                        return cudaMemcpyAsync(slot, src, bytes, cudaMemcpyDeviceToHost, fetch_);
+                      }),
+            "server fetch");
       check(cudaStreamSynchronize(fetch_), "server fetch");
     } catch (...) {
       lock.lock();
@@ -560,20 +570,6 @@ class Server {
   void seal(Block& b) {
     b.sealed = true;
     b.chunks = static_cast<uint32_t>((b.records + chunk_tracks_ - 1) / chunk_tracks_);
-  }
-
-  // downloadSet's decode (RadioAccumulator.inl:849-898), value x factor per observer.
-  static void decode(ServedEvent const& ev, int a, long long const* in, double* out) {
-    std::size_t const total = ev.bins[a];
-    std::size_t offset = 0;
-    for (auto const& s : ev.snapshots[a]) {
-      double const f = decode_factor(s, a, ev.limit);
-      std::size_t const n = static_cast<std::size_t>(s.number_of_bins);
-      for (int row = 0; row < 3; ++row)
-        for (std::size_t i = 0; i < n; ++i)
-          out[row * total + offset + i] = static_cast<double>(in[row * total + offset + i]) * f;
-      offset += n;
-    }
   }
 
   // ------------------------------------------------------------ scheduler
@@ -808,6 +804,8 @@ class Server {
   uint64_t deferred_entries_ = 0;
   std::chrono::steady_clock::time_point epoch_;
   std::mutex mu_, fetch_mu_;
+  void* fetch_slots_ = nullptr;  // pinned, for ring_ (under fetch_mu_)
+  SlotRing ring_;
   std::condition_variable work_cv_, memory_cv_, done_cv_;
   std::map<uint64_t, std::unique_ptr<ServedEvent>> events_;
   std::deque<Round> inflight_;

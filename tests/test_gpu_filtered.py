@@ -82,3 +82,54 @@ def test_times_outside_the_guards_reach(pkg, oracle, showers, scale):
     wl["observers"] = wl["observers"][::5].copy()
     wl["observers"]["start_time_s"] += shift
     check(pkg, oracle, showers, wl, records)
+
+
+@pytest.mark.parametrize("count", [1, 255, 256, 257, 1500, 16_385])
+@pytest.mark.parametrize("deterministic", [True, False])
+def test_automatic_route_at_every_size(pkg, oracle, showers, count, deterministic):
+    """The automatic choice (direct below 256 tracks, windowed above, items cut
+    evenly over the GPU) gives the oracle's traces: bit for bit in fixed point, to
+    the order of FP64 sums in floating point."""
+    wl, gen, _ = showers.workload_config("plain_c0", bins=1500)
+    wl["observers"] = wl["observers"][:5].copy()
+    records = showers.shower_records(count, seed=91, **gen)
+    config = showers.make_config(wl, deterministic=deterministic)
+    want = oracle.restatement().project(config, records, threads=8)
+    if deterministic:
+        got = project(pkg, config, records)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+        counters = got[2]
+    else:
+        import torch
+
+        raw = torch.from_numpy(records.view(np.uint8).reshape(-1)).cuda()
+        acc = pkg.RadioAccumulator(config)
+        acc.accumulate_lepton_tracks(raw.data_ptr(), records.size)
+        waveforms = acc.download()
+        acc.close()
+        for g, w in ((waveforms.coreas, want[0]), (waveforms.zhs, want[1])):
+            assert np.abs(g - w).max(initial=0.0) <= 1e-28 + 2e-12 * np.abs(w).max(initial=0.0)
+        counters = waveforms.counters
+    for key in COUNTERS:
+        assert counters[key] == want[2][key], key
+
+
+@pytest.mark.parametrize("sizes", [(20_011,), (100, 9_000, 4_096, 1), (70_003,)])
+def test_pageable_host_calls_of_many_records(pkg, oracle, showers, sizes):
+    """Host calls that fill several batches (ingested as they fill, projected
+    together) and calls that leave a batch part full."""
+    wl, gen, _ = showers.workload_config("plain_c0", bins=2048)
+    records = showers.shower_records(sum(sizes), seed=95, **gen)
+    config = showers.make_config(wl)
+    want = oracle.restatement().project(config, records, threads=16)
+    acc = pkg.RadioAccumulator(config)
+    begin = 0
+    for size in sizes:
+        acc.enqueue_host_lepton_tracks(records[begin:begin + size])
+        begin += size
+    got = acc.download_fixed()
+    stats = acc.statistics()
+    acc.close()
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert stats.host_tracks_enqueued == records.size
+    assert stats.host_track_batches == -(-records.size // 4096)
