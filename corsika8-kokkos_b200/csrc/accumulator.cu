@@ -29,7 +29,13 @@ namespace c8r {
 namespace {
 
 constexpr std::size_t kDefaultHostBatch = 4096;   // RadioAccumulator.hpp:49
-constexpr std::size_t kDirectThreshold = 16384;   // RadioAccumulator.hpp:101
+// Fewer tracks than this run the direct kernel (the reference's threshold is
+// 16384, RadioAccumulator.hpp:101).  The windowed launches cost 45 to 55 us
+// whatever their size, the direct kernel's time is its serial chain of atomics:
+// direct / windowed us at 1, 64, 512, 4096, 16000 FP64 tracks x 16 antennas: 20/55,
+// 33/55, 98/57, 170/67, 242/91, x 160: 20/51, 32/57, 185/82, 339/137, 1029/292;
+// floating traces x 16: 17/24, 25/26, 57/39, 97/59, 147/107.
+constexpr std::size_t kDirectThreshold = 256;
 // Full batches of one pageable host call are ingested as they fill and
 // projected together, at most so many records at a time: a projection costs
 // its launches and a pass over every antenna's window whatever its size.
@@ -974,19 +980,9 @@ class Accumulator {
     ev.propagation = propagation_;
     ev.counters = counters_.ptr;
     ev.window = static_cast<uint32_t>(window_bins_);
-    uint32_t const per_chunk = ev.observer_count[0] + ev.observer_count[1];
     std::size_t chunk = tuning_.track_tile_size;
-    if (chunk == 0) {
-      // about 16 work items per CTA of each launch (one CTA per SM), at least
-      // 8192 tracks each; smaller launches take chunks of an eighth of their
-      // tracks up to 262144 (fewer items, so fewer window zero/flush passes:
-      // the work list ends on quarter-size chunks anyway)
-      std::size_t const ctas = static_cast<std::size_t>(sms_) * 2;
-      std::size_t const target_chunks = std::max<std::size_t>(1, (16 * ctas + per_chunk - 1) / std::max<uint32_t>(per_chunk, 1));
-      chunk = std::max<std::size_t>(8192, (count + target_chunks - 1) / target_chunks);
-      chunk = std::max<std::size_t>(chunk, std::min<std::size_t>((count + 7) / 8, 262144));
-      chunk = track_capacity(chunk);  // items start on a track tile
-    }
+    if (chunk == 0)
+      chunk = auto_chunk(count, std::max(ev.observer_count[0], ev.observer_count[1]), static_cast<uint64_t>(sms_));
     chunk = std::min<std::size_t>(chunk, kMaxChunkTracks);
     ev.chunk_size = static_cast<uint32_t>(chunk);
     ev.chunks = static_cast<uint32_t>((count + chunk - 1) / chunk);
@@ -1087,7 +1083,8 @@ class Accumulator {
       plan.reruns = reruns_.ptr;
       plan.handbacks = reruns_.ptr + 1;
       uint64_t ctas = static_cast<uint64_t>(per_sm) * sms_;
-      append_work(plan, ev, ctas, true);
+      // a launch of few rounds is planned to end evenly; a tail would add a round
+      append_work(plan, ev, ctas, static_cast<uint64_t>(ev.chunks) * ev.observer_count[algorithm] > 4 * ctas);
       if (ctas > plan.total_items) ctas = plan.total_items;
       plan.deferred_stride = deferred_list_stride(plan);
       attach_deferred(plan, deferred_lists(algorithm, deferred_words(plan, ctas, fixed_)), ctas, fixed_);

@@ -225,6 +225,39 @@ inline uint64_t append_work(WorkPlan& plan, EventPlan ev, uint64_t ctas, bool fi
   return plan.total_items - before;
 }
 
+// Tracks per work item for `count` tracks at `observers` observers of one
+// algorithm's launch on `ctas` persistent CTAs.  An item
+// costs a pass over its antenna's window (zeroed, summed and flushed: as long as
+// about 4400 tracks take) beside its tracks, and the launch lasts as many rounds
+// as the busiest CTA has items.  Up to 262144 tracks a CTA the number of chunks
+// is the one with the least rounds x (4400 + tracks); above that, items of about
+// a sixteenth of a CTA's share (at least an eighth of the launch up to 262144
+// tracks) and a tail of short ones even out what the antennas' different loads
+// leave (append_work).
+inline uint64_t auto_chunk(uint64_t count, uint64_t observers, uint64_t ctas) {
+  constexpr uint64_t kItemCost = 4400, kFewTracks = 262144, kMostChunks = 64;
+  if (count == 0 || observers == 0 || ctas == 0) return kTrackTile;
+  uint64_t chunk = 0;
+  if (count <= kFewTracks * ctas / observers) {
+    uint64_t least = ~0ull;
+    for (uint64_t chunks = 1; chunks <= kMostChunks; ++chunks) {
+      uint64_t const tracks = track_capacity((count + chunks - 1) / chunks);
+      uint64_t const items = (count + tracks - 1) / tracks * observers;
+      uint64_t const cost = (items + ctas - 1) / ctas * (kItemCost + tracks);
+      if (cost < least) {
+        least = cost;
+        chunk = tracks;
+      }
+    }
+    return chunk;
+  }
+  uint64_t const target = (16 * ctas + observers - 1) / observers;
+  chunk = (count + target - 1) / target;
+  chunk = chunk > 8192 ? chunk : 8192;
+  uint64_t const eighth = (count + 7) / 8 < kFewTracks ? (count + 7) / 8 : kFewTracks;
+  return track_capacity(chunk > eighth ? chunk : eighth);
+}
+
 enum class Precision : int { kFP64 = 0, kMixed = 1 };
 
 // Record ingest: LeptonTransportRecord AoS -> compacted SoA kinematics
