@@ -237,33 +237,64 @@ __device__ __forceinline__ SourceTerms source_terms(Propagation const& p, Destin
   return SourceTerms{1. + (i_src - d.integral) / height, n_src, n_dst};
 }
 
+// x / c, correctly rounded, without a division (P. Markstein, IBM J. Res. Dev. 34,
+// 1990): with z = RN(1/c), q = RN(x z) and the exact remainder r = x - q c,
+// RN(q + r z) is RN(x / c) when q is within one unit in the last place of x / c.
+// z is within 0.187 2^-53 of 1/c here, so q is within 0.69 units.  Outside the
+// range in which no step can underflow or overflow the division is used.
+__device__ __forceinline__ double over_light_speed(double x) {
+  constexpr double z = 1. / kSpeedOfLight;
+  unsigned const high = (static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu) - 0x1a700000u;  // 2^-600
+  if (high > 0x65700000u - 0x1a700000u) return x / kSpeedOfLight;                                // 2^600
+  double const q = x * z;
+  return fma(fma(-q, kSpeedOfLight, x), z, q);
+}
+
+// (x, y, z) / d, each correctly rounded, from one reciprocal (the same theorem):
+// r = RN(1/d); a r is within 1.5 units in the last place of a / d, one
+// correction by its remainder brings it within one, and the second one rounds
+// correctly.  Outside the range in which no step can underflow or overflow, or
+// with a zero among them, three divisions.
+__device__ __forceinline__ void divide3(double& x, double& y, double& z, double d) {
+  unsigned const hx = static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu,
+                 hy = static_cast<unsigned>(__double2hiint(y)) & 0x7fffffffu,
+                 hz = static_cast<unsigned>(__double2hiint(z)) & 0x7fffffffu;
+  unsigned const least = min(min(hx, hy), hz);
+  if (least < 0x1a700000u || static_cast<unsigned>(__double2hiint(d)) > 0x65700000u) {  // 2^-600, 2^600
+    x = x / d;
+    y = y / d;
+    z = z / d;
+    return;
+  }
+  double const r = 1. / d;
+  auto quotient = [&](double a) {
+    double const q0 = a * r;
+    double const q1 = fma(fma(-q0, d, a), r, q0);
+    return fma(fma(-q1, d, a), r, q1);
+  };
+  x = quotient(x);
+  y = quotient(y);
+  z = quotient(z);
+}
+
 // propagate, RadioProjection.inl:170-238, given the source terms of the
 // point: the reference's (1 + (I_src - I_dst) / height) * dist / c with the
 // parenthesised factor taken from `st` (the same IEEE value), or n dist / c.
 // kTime = false skips the refractive index and travel time (the Fraunhofer
-// midpoint uses only k and distance).  kApproxDirection = true returns
-// k = d * RN(1/|d|): each component within 3.01 u |k| of the reference's
-// RN(d/|d|) (u = 2^-53); distance, refractive indices and travel time are
-// exact in both forms.
-template <bool kTime, bool kApproxDirection = false>
+// midpoint uses only k and distance).
+template <bool kTime>
 __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCache const& o,
                                                double sx, double sy, double sz) {
   Path r;
   double const dx = o.px - sx, dy = o.py - sy, dz = o.pz - sz;
   double const dist = sqrt(dx * dx + dy * dy + dz * dz);
-  if (kApproxDirection) {
-    double const inverse = 1. / dist;
-    r.kx = dx * inverse;
-    r.ky = dy * inverse;
-    r.kz = dz * inverse;
-  } else {
-    r.kx = dx / dist;
-    r.ky = dy / dist;
-    r.kz = dz / dist;
-  }
+  r.kx = dx;
+  r.ky = dy;
+  r.kz = dz;
+  divide3(r.kx, r.ky, r.kz, dist);
   r.dist = dist;
   if (!kTime) return r;
-  r.time = st.factor * dist / kSpeedOfLight;
+  r.time = over_light_speed(st.factor * dist);
   r.n_src = st.n_src;
   r.n_dst = st.n_dst;
   return r;
@@ -271,11 +302,11 @@ __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCa
 
 // propagate, RadioProjection.inl:170-238: the source terms looked up in the
 // table for this observer, then the path.
-template <bool kTime, bool kApproxDirection = false>
+template <bool kTime>
 __device__ __forceinline__ Path propagate(Propagation const& p, ObserverCache const& o,
                                           double sx, double sy, double sz) {
   SourceTerms const st = kTime ? source_terms(p, destination_of(o), sz) : SourceTerms{0., 0., 0.};
-  return propagate_with<kTime, kApproxDirection>(st, o, sx, sy, sz);
+  return propagate_with<kTime>(st, o, sx, sy, sz);
 }
 
 // ---------------------------------------------------------------- filtered paths
