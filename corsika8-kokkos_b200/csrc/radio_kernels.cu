@@ -2014,8 +2014,12 @@ __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks,
   unsigned mine = 0;
   if (lane < count) {
     row = begin + list[lane];
-    Subdivision const d = subdivide_row(tracks, row, p, s_observer);
     int const refinement = static_cast<int>(p.refinement);
+    // refined tracks all come here, most of them undivided but for that: their
+    // Fraunhofer number is surely below 1
+    Subdivision d{1., 1};
+    if (refinement == 1 || !zhs_point<false, false>(track_ref(tracks, row), p, copy_words(s_lean)).one)
+      d = subdivide_row(tracks, row, p, s_observer);
     // both products as the reference forms them (RadioProjection.inl:503, :527)
     rare.subtracks = static_cast<unsigned long long>(static_cast<long long>(d.subtracks));
     if (refinement > 1)
