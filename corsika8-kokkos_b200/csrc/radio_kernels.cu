@@ -333,7 +333,9 @@ __device__ __noinline__ Counts coreas_near_cone(Track const t, Propagation const
   Vec3<Amp> fstart =
       scaled(cross(k, cross(k, beta)), amp_div(static_cast<Amp>(cf), static_cast<Amp>(md * pm.dist)));
   Vec3<Amp> fend = scaled(fstart, static_cast<Amp>(-1.));
-  double dt = t.length / (kSpeedOfLight * t.beta_module) * fabs(md);
+  Track whole = t;
+  derive_track(whole);
+  double dt = whole.length / (kSpeedOfLight * whole.beta_module) * fabs(md);
   double sr, er;
   if (start_before_end) {
     sr = mr - 0.5 * dt;
@@ -1328,20 +1330,51 @@ __device__ __forceinline__ bool zhs_exact_differences(Path const& path, double t
   return true;
 }
 
-// accumulate_zhs, RadioProjection.inl:483-529, every decision exact.
-template <bool kFixed, bool kRuns, class Amp, class Sink>
-__device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
-                                         ObserverCache const& o, Sink& sink, Counts& c) {
+// The subdivision of a track seen from an observer (accumulate_zhs,
+// RadioProjection.inl:483-503), every operation exact.
+struct Subdivision {
+  double divisor;
+  int subtracks;
+};
+__device__ __forceinline__ Subdivision subdivide(Track t, Propagation const& p, ObserverCache const& o) {
+  derive_track(t);
   double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
   Path const pm = propagate<false>(p, o, mx, my, mz);
   double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
   double const s2 = 1. - uk * uk;
   double const fraunhofer = s2 * t.length * t.length / pm.dist / o.wavelength * 2. * kPi;
+  Subdivision d{1., 1};
+  if (fraunhofer > 1.) {
+    d.divisor = sqrt(fraunhofer) + 1.;
+    d.subtracks = x86_int(ceil(d.divisor));
+  }
+  return d;
+}
+// Whether a track seen from an observer is surely one segment: the Fraunhofer
+// number as surely_undivided estimates it, 8 pi c^2 / (wavelength fs^2) being
+// 8 pi wavelength (wavelength = c / fs).
+__device__ __forceinline__ bool surely_one_segment(Track const& t, ObserverCache const& o) {
+  double const dx = o.px - (t.sx + t.ex) * 0.5, dy = o.py - (t.sy + t.ey) * 0.5, dz = o.pz - (t.sz + t.ez) * 0.5;
+  double inverse;
+  bool const ok = lean_rsqrt(fma(dz, dz, fma(dy, dy, dx * dx)), inverse);
+  double const w = fma(t.bz, dz, fma(t.by, dy, t.bx * dx)) * inverse;
+  double const square = fma(t.bz, t.bz, fma(t.by, t.by, t.bx * t.bx));
+  double const half_bins = (t.te - t.ts) * 0.5 * o.sample_rate;
+  double const factor = half_bins * half_bins * (inverse * (8. * kPi) * o.wavelength);
+  return ok & (fabs(t.bx) + fabs(t.by) + fabs(t.bz) <= 4.) & (factor < 0x1p18) &
+         (fma(-w, w, square) * factor < 1. - 0x1p-20);
+}
+
+// accumulate_zhs, RadioProjection.inl:483-529, every decision exact.
+template <bool kFixed, bool kRuns, class Amp, class Sink>
+__device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
+                                         ObserverCache const& o, Sink& sink, Counts& c) {
   double divisor = 1.;
   int subtracks = 1;
-  if (fraunhofer > 1.) {
-    divisor = sqrt(fraunhofer) + 1.;
-    subtracks = x86_int(ceil(divisor));
+  if (!surely_one_segment(t, o)) {
+    Subdivision const d = subdivide(t, p, o);
+    divisor = d.divisor;
+    subtracks = d.subtracks;
   }
   c.subtracks += static_cast<unsigned long long>(static_cast<long long>(subtracks));
   int const refinement = static_cast<int>(p.refinement);
@@ -1449,7 +1482,8 @@ __device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propag
 }
 
 // ---------------------------------------------------------------- helpers
-// The fields of a track, its columns read by `load`.
+// The fields of a track, its columns read by `load`; length and |beta| are left
+// to derive_track, where an exact evaluation needs them.
 template <class Load>
 __device__ __forceinline__ Track unpack_track(Load load) {
   double2 const a = load(0), b = load(1), c = load(2), d = load(3);
@@ -1467,7 +1501,6 @@ __device__ __forceinline__ Track unpack_track(Load load) {
   t.by = e.y;
   t.bz = f.x;
   t.constant = g.y;
-  derive_track(t);
   return t;
 }
 
@@ -1911,25 +1944,6 @@ __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t
   return lo;
 }
 
-// The subdivision of a track seen from an observer (accumulate_zhs,
-// RadioProjection.inl:483-503), every operation exact.
-struct Subdivision {
-  double divisor;
-  int subtracks;
-};
-__device__ __forceinline__ Subdivision subdivide(Track const& t, Propagation const& p, ObserverCache const& o) {
-  double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
-  Path const pm = propagate<false>(p, o, mx, my, mz);
-  double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
-  double const s2 = 1. - uk * uk;
-  double const fraunhofer = s2 * t.length * t.length / pm.dist / o.wavelength * 2. * kPi;
-  Subdivision d{1., 1};
-  if (fraunhofer > 1.) {
-    d.divisor = sqrt(fraunhofer) + 1.;
-    d.subtracks = x86_int(ceil(d.divisor));
-  }
-  return d;
-}
 __device__ __noinline__ Subdivision subdivide_row(const double* __restrict__ tracks, uint64_t row,
                                                   Propagation const& p, ObserverCache const& o) {
   return subdivide(load_track(tracks, row), p, o);
