@@ -827,9 +827,12 @@ struct StagedSegment<double> {
 // zhs_segment<kRuns = true>, its samples staged instead of deposited.  The
 // segment's midpoint, its times and the time between them come from the
 // caller; kPre: the midpoint's source terms are `pre`, else they are looked
-// up.  Returns false when the segment needs the per-index binning or when the
+// up.  Returns false when the segment needs the per-index binning, when the
 // trace has 2^26 bins or more (staged counts then stay far inside 32 bits per
-// warp); the caller then discards whatever `out` holds.
+// warp), or when a detection time's nearest bin is not the floor(x + 1/2) that
+// counts the bins between (x just below 1/2, where x + 1/2 rounds to 1): the
+// last sample then would not be in the bin after the run, as
+// deposit_differences takes it.  The caller discards whatever `out` holds.
 template <bool kFixed, class Amp, bool kPre = false>
 __device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, double t1, double t2, double mt,
                                           Track const& t, Propagation const& p,
@@ -879,6 +882,7 @@ __device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, doubl
   out.last_bin = 0u;
   // last sample, add_sample(detection_time2): bin nearest((d2 - t0) fs) = nearest(x2)
   double const bv2 = nearest_bin(x2);
+  if (bv2 != eb) return false;
   if (bv2 >= 0. && bv2 < o.bins_d) {
     out.last_bin = static_cast<uint32_t>(bv2);
     out.flags = 2u;
@@ -890,6 +894,7 @@ __device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, doubl
   out.mid = amp_div(static_cast<Amp>(mc), static_cast<Amp>(dd)) * unit;
   // first sample, add_sample(detection_time1): bin nearest(x1)
   double const bv1 = nearest_bin(x1);
+  if (bv1 != sb) return false;
   bool const first_in = bv1 >= 0. && bv1 < o.bins_d;
   if (first_in) {
     out.start = static_cast<uint32_t>(bv1);

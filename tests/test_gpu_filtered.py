@@ -70,6 +70,35 @@ def test_samples_at_whole_and_half_bins(pkg, oracle, showers):
     check(pkg, oracle, showers, wl, showers.to_records(seg))
 
 
+@pytest.mark.parametrize("edge,duration", [("end", 1e-3), ("end", 1.3), ("start", 1e-3), ("start", 1.1), ("start", 2.7)])
+def test_detection_time_just_below_the_first_half_bin(pkg, oracle, showers, edge, duration):
+    """The one detection time x (in bins) whose floor(x + 1/2) is not its nearest
+    bin: 1/2 less a unit in the last place, at which x + 1/2 rounds to 1.  The
+    track passes its antenna at a right angle (k.beta = 0), so a detection time is
+    a track time plus the travel time and can be placed there exactly."""
+    below = np.nextafter(0.5, 0.0)
+    height = 1.0e6
+    travel = height / showers.SPEED_OF_LIGHT
+    if edge == "end":
+        t_end = below - travel
+        t_start = t_end - duration
+        t_end = t_start + (t_end - t_start)
+        assert t_end + travel == below
+    else:
+        t_start = below - travel
+        t_end = t_start + duration
+        assert t_start + travel == below
+    seg = dict(start=np.array([[-500.0, 0.0, height]]), end=np.array([[500.0, 0.0, height]]),
+               t_start=np.array([t_start]), t_end=np.array([t_end]), pid=np.array([11], np.int32),
+               energy_gev=np.array([1e-3]), direction=np.array([[1.0, 0.0, 0.0]]), weight=np.array([1e18]))
+    observers = np.zeros(1, pkg.abi.OBSERVER)
+    observers["duration_s"] = 7.0
+    observers["sample_rate_hz"] = 1.0
+    observers["number_of_bins"] = 8
+    wl = dict(observers=observers, homogeneous=1.0, table=None)
+    check(pkg, oracle, showers, wl, showers.to_records(seg))
+
+
 @pytest.mark.parametrize("scale", [1e-6, 1e3, 1e6])
 def test_times_outside_the_guards_reach(pkg, oracle, showers, scale):
     """Track times shifted until the filtered paths' bounds no longer cover them
