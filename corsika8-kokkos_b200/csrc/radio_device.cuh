@@ -11,6 +11,8 @@
 
 #include <cstdint>
 #include <climits>
+#include <cmath>
+#include <cstring>
 
 namespace c8r {
 
@@ -237,30 +239,41 @@ __device__ __forceinline__ SourceTerms source_terms(Propagation const& p, Destin
   return SourceTerms{1. + (i_src - d.integral) / height, n_src, n_dst};
 }
 
+// The high word of |x|: sign cleared, exponent on top.
+__host__ __device__ __forceinline__ unsigned magnitude_word(double x) {
+#ifdef __CUDA_ARCH__
+  return static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu;
+#else
+  uint64_t bits;
+  std::memcpy(&bits, &x, sizeof bits);
+  return static_cast<unsigned>(bits >> 32) & 0x7fffffffu;
+#endif
+}
+
+// The operands of the quotients below lie in [2^-400, 2^400): a quotient is then
+// a normal number above 2^-801, and its remainder, a multiple of 2^-1000, exact.  Outside (zeros, infinities and NaN among them) the division is used.
+constexpr unsigned kQuotientLow = 0x26f00000u, kQuotientHigh = 0x58f00000u;  // 2^-400, 2^400
+
 // x / c, correctly rounded, without a division (P. Markstein, IBM J. Res. Dev. 34,
 // 1990): with z = RN(1/c), q = RN(x z) and the exact remainder r = x - q c,
 // RN(q + r z) is RN(x / c) when q is within one unit in the last place of x / c.
-// z is within 0.187 2^-53 of 1/c here, so q is within 0.69 units.  Outside the
-// range in which no step can underflow or overflow the division is used.
-__device__ __forceinline__ double over_light_speed(double x) {
+// z is within 0.187 2^-53 of 1/c here, so q is within 0.69 units.
+__host__ __device__ __forceinline__ double over_light_speed(double x) {
   constexpr double z = 1. / kSpeedOfLight;
-  unsigned const high = (static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu) - 0x1a700000u;  // 2^-600
-  if (high > 0x65700000u - 0x1a700000u) return x / kSpeedOfLight;                                // 2^600
+  if (magnitude_word(x) - kQuotientLow >= kQuotientHigh - kQuotientLow) return x / kSpeedOfLight;
   double const q = x * z;
   return fma(fma(-q, kSpeedOfLight, x), z, q);
 }
 
-// (x, y, z) / d, each correctly rounded, from one reciprocal (the same theorem):
+// (x, y, z) / d for d = |(x, y, z)|, each correctly rounded, from one reciprocal
+// (the same theorem):
 // r = RN(1/d); a r is within 1.5 units in the last place of a / d, one
 // correction by its remainder brings it within one, and the second one rounds
-// correctly.  Outside the range in which no step can underflow or overflow, or
-// with a zero among them, three divisions.
-__device__ __forceinline__ void divide3(double& x, double& y, double& z, double d) {
-  unsigned const hx = static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu,
-                 hy = static_cast<unsigned>(__double2hiint(y)) & 0x7fffffffu,
-                 hz = static_cast<unsigned>(__double2hiint(z)) & 0x7fffffffu;
+// correctly.
+__host__ __device__ __forceinline__ void divide3(double& x, double& y, double& z, double d) {
+  unsigned const hx = magnitude_word(x), hy = magnitude_word(y), hz = magnitude_word(z);
   unsigned const least = min(min(hx, hy), hz);
-  if (least < 0x1a700000u || static_cast<unsigned>(__double2hiint(d)) > 0x65700000u) {  // 2^-600, 2^600
+  if (least < kQuotientLow || magnitude_word(d) >= kQuotientHigh) {
     x = x / d;
     y = y / d;
     z = z / d;
