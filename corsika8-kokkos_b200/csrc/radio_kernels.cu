@@ -2015,12 +2015,34 @@ __device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tra
 // loop's kernel: the pair-per-lane drain it replaces there spilled 1700 words a
 // pair at 64 registers.
 constexpr long long kLeanSegments = 64;
-// The table row at height z is that of every height within kBinGuard bins.
-__device__ __forceinline__ bool table_row_decided(Propagation const& p, LeanObserver const& l, double z) {
+// Whether the source terms at height z decide what the terms at the reference's
+// own height, within `z_error` m of z, would.  In the table they are the same when
+// no row lies within kBinGuard bins.  Past its ends (out of line: rare) they are
+// linear in z: factor - 1 = (I - I_antenna) / rise with the rise in steps to the
+// antenna's height, so an error e of the rise and one of I move the travel time by
+// (dI + |factor - 1| e) / (|rise| - e) of `path_bins`; that and the index's change
+// over half the segment have to stay below 2^-22 bins, which kBinGuard leaves over.
+__device__ __noinline__ bool terms_decided_past_table(Propagation const& p, double height, double factor,
+                                                      double z_error, double path_bins, double half_bins) {
+  bool const above = height > 0.;
+  double const steps = z_error * p.inv_step, antenna = s_observer.dest_height;
+  double const rise = fabs(above ? height - antenna : antenna - fabs(height));
+  double const rise_error = steps + 0x1p-50 * (fabs(height) + fabs(antenna));
+  double const excess = fabs(factor - 1.) + 0x1p-52;
+  double const integral_error = (above ? fabs(p.slope_i_upper) * z_error : fabs(p.slope_i_lower) * steps) +
+                                0x1p-50 * (fabs(s_observer.dest_integral) + excess * rise);
+  double const index_error = fabs(above ? p.slope_n_upper : p.slope_n_lower) * steps;
+  return ((integral_error + excess * rise_error) * path_bins <
+          (0x1p-22 - 4. * index_error * half_bins) * (rise - rise_error)) & (rise > rise_error);
+}
+__device__ __forceinline__ bool terms_decided(Propagation const& p, LeanObserver const& l, double factor, double z,
+                                              double z_error, double path_bins, double half_bins) {
   if (p.homogeneous > 0.) return true;
   double const height = (z - p.min_height) * p.inv_step, guard = l.bin_guard_m * p.inv_step;
   int row;
-  return (fabs(lean_nearest(height + 0.5, row)) > guard) & (fabs(height) > guard);
+  if (!((fabs(lean_nearest(height + 0.5, row)) > guard) & (fabs(height) > guard))) return false;
+  if ((height > 0.) & (height + 0.5 < static_cast<double>(p.table_size - 1))) return true;
+  return terms_decided_past_table(p, height, factor, z_error, path_bins, half_bins);
 }
 __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks, uint64_t begin, unsigned const* list,
                                               unsigned count, Propagation const& p, unsigned long long* win,
@@ -2086,7 +2108,9 @@ __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks,
                                      fma(duration, at, ct.x), cd.x, cd.y, ce.x, st.factor, st.n_src);
       StagedSegment<float> seg;
       deposited = zhs_lean(m, half_bins, pack_constant(ce.y) * l.scale, cd.x, cd.y, ce.x, l, subdivided, seg) &
-                  lean_terms(st) & table_row_decided(p, l, z) & (m.dist * l.rate_over_c >= 4. * half_bins);
+                  lean_terms(st) & (m.dist * l.rate_over_c >= 4. * half_bins) &
+                  terms_decided(p, l, st.factor, z, 0x1p-46 * (fabs(cb.x) + fabs(cc.y)), m.dist * l.rate_over_c,
+                                half_bins);
       deposited = deposited && account_staged(seg, l, c);
       if (deposited) deposit_differences(seg, l, win, width);
     }

@@ -6,6 +6,8 @@ precision's sample counts per bin and counters equal the oracle's."""
 import numpy as np
 import pytest
 
+import cases
+
 pytestmark = pytest.mark.gpu
 
 COUNTERS = ("coreas_contributions", "zhs_contributions", "zhs_subtracks", "valid_tracks", "fixed_point_overflows")
@@ -96,6 +98,30 @@ def test_detection_time_just_below_the_first_half_bin(pkg, oracle, showers, edge
     observers["sample_rate_hz"] = 1.0
     observers["number_of_bins"] = 8
     wl = dict(observers=observers, homogeneous=1.0, table=None)
+    check(pkg, oracle, showers, wl, showers.to_records(seg))
+
+
+def test_divided_tracks_above_the_table_beside_the_antenna_height(pkg, oracle, showers):
+    """Divided tracks past the table's upper end, a few nanometres above the
+    antenna: the travel time's factor 1 + (I - I_antenna) / height then turns on
+    differences at the rounding of the height itself."""
+    count = 3000
+    rng = np.random.default_rng(8)
+    table = vars(cases.uniform_table(1.0003, 0.0, 2000.0, 1.0))
+    z = 2000.0 + rng.uniform(1e-9, 8e-9, count)
+    start = np.stack([np.zeros(count), np.full(count, -50.0), z], axis=1)
+    end = np.stack([np.zeros(count), np.full(count, 50.0), z + rng.uniform(-1e-9, 1e-9, count)], axis=1)
+    t0 = rng.uniform(0.0, 100e-9, count)
+    observers = np.zeros(1, pkg.abi.OBSERVER)
+    observers["position_m"][0] = (3.0e4, 0.0, 2000.0 - 1e-9)
+    observers["start_time_s"] = 3.0e4 / showers.SPEED_OF_LIGHT
+    observers["duration_s"] = 8191 / 1e10
+    observers["sample_rate_hz"] = 1e10
+    observers["number_of_bins"] = 8192
+    seg = dict(start=start, end=end, t_start=t0, t_end=t0 + 100.0 / (0.99 * showers.SPEED_OF_LIGHT),
+               pid=np.full(count, 11, np.int32), energy_gev=np.full(count, 1e-3),
+               direction=np.tile([0.0, 1.0, 0.0], (count, 1)), weight=np.ones(count))
+    wl = dict(observers=observers, homogeneous=0.0, table=table)
     check(pkg, oracle, showers, wl, showers.to_records(seg))
 
 
