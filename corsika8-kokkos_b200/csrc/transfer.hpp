@@ -60,7 +60,8 @@ class SlotRing {
 
   // Fills the segments in order: issue(segment, offset, bytes, slot) queues on
   // `stream` the work that writes bytes [offset, offset + bytes) of a segment
-  // into `slot`.  Returns once everything has been copied out.
+  // into `slot`.  Returns once everything has been copied out.  The copying
+  // threads work on the calling thread's device.
   template <class Issue>
   cudaError_t run(std::vector<Segment> const& segments, cudaStream_t stream, Issue issue) {
     std::vector<Piece> pieces;
@@ -84,12 +85,20 @@ class SlotRing {
       return cudaSuccess;
     };
     unsigned const cores = std::max(1u, std::thread::hardware_concurrency() / 2);
+    int device = 0;
+    if (cudaError_t const err = cudaGetDevice(&device)) return err;
     Shared shared(n);
     Workers workers(shared);
     if (total >= kThreadedBytes && depth > 1) {
       std::size_t const wanted = std::min<std::size_t>({kWorkers, cores, total / kBytesPerWorker});
       for (std::size_t k = 0; k < wanted; ++k)
-        if (!workers.start([&] { drain(shared, n, empty); })) break;
+        if (!workers.start([&] {
+              if (cudaError_t const err = cudaSetDevice(device))  // a new thread's is device 0
+                shared.error.store(err);
+              else
+                drain(shared, n, empty);
+            }))
+          break;
     }
     for (std::size_t i = 0; i < n; ++i) {
       if (i >= depth) {  // the slot's last piece has to be out
