@@ -714,13 +714,16 @@ class Accumulator {
   };
 
   // Copies after the stream's earlier work and returns when they are done:
-  // page-locked destinations directly, pageable ones through the slots.
+  // page-locked destinations directly, pageable ones through the slots.  Device
+  // memory is refused: the slots are emptied by host threads.
   void copy_out(Transfers const& transfers) {
     Transfers pageable;
     for (std::size_t k = 0; k < transfers.out.size(); ++k) {
       SlotRing::Segment const& d = transfers.out[k];
+      ResultMemory const memory = result_memory(d.destination);
+      if (memory == ResultMemory::kDevice) check(cudaErrorInvalidValue, "trace download to device memory");
       stats_.device_to_host_bytes += d.bytes;
-      if (ring_.usable() && !is_pinned(d.destination))
+      if (ring_.usable() && memory == ResultMemory::kPageable)
         pageable.add(d.destination, transfers.from[k], d.bytes);
       else
         check(cudaMemcpyAsync(d.destination, transfers.from[k], d.bytes, cudaMemcpyDeviceToHost, stream_),

@@ -492,6 +492,8 @@ class Server {
       for (int a = 0; a < 2; ++a) {
         void* const to = a == 0 ? coreas : zhs;
         if (ev.bins[a] == 0 || to == nullptr) continue;
+        if (result_memory(to) == ResultMemory::kDevice)
+          check(cudaErrorInvalidValue, "server fetch to device memory");
         out.push_back({to, 3 * ev.bins[a] * sizeof(double)});
         of.push_back(a);
       }

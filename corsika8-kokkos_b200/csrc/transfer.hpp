@@ -23,6 +23,20 @@
 namespace c8r {
 namespace {
 
+// Where a caller's result buffer lies: ordinary host memory (through the slots),
+// memory that the copy engine writes (page-locked, managed), or device memory,
+// which no result is copied to.
+enum class ResultMemory { kPageable, kDirect, kDevice };
+inline ResultMemory result_memory(void const* p) {
+  cudaPointerAttributes attributes{};
+  if (cudaPointerGetAttributes(&attributes, p) != cudaSuccess) {
+    cudaGetLastError();
+    return ResultMemory::kPageable;
+  }
+  if (attributes.type == cudaMemoryTypeDevice) return ResultMemory::kDevice;
+  return attributes.type == cudaMemoryTypeUnregistered ? ResultMemory::kPageable : ResultMemory::kDirect;
+}
+
 class SlotRing {
  public:
   static constexpr std::size_t kSlotBytes = std::size_t{1} << 19;

@@ -117,10 +117,23 @@ void check_copies(SlotRing& ring) {
   expect(wrong_device == 0, "every call on the owner's device");
 }
 
+// A result buffer's memory decides its route.
+void check_memory() {
+  char pageable, locked, managed, device;
+  kinds[&locked] = cudaMemoryTypeHost;
+  kinds[&managed] = cudaMemoryTypeManaged;
+  kinds[&device] = cudaMemoryTypeDevice;
+  expect(c8r::result_memory(&pageable) == c8r::ResultMemory::kPageable, "ordinary memory through the slots");
+  expect(c8r::result_memory(&locked) == c8r::ResultMemory::kDirect, "page-locked memory directly");
+  expect(c8r::result_memory(&managed) == c8r::ResultMemory::kDirect, "managed memory directly");
+  expect(c8r::result_memory(&device) == c8r::ResultMemory::kDevice, "device memory refused");
+}
+
 }  // namespace
 
 int main() {
   cudaSetDevice(kOwner);
+  check_memory();
   std::vector<unsigned char> slots(4 * SlotRing::kSlotBytes);
   {
     SlotRing ring;

@@ -50,3 +50,42 @@ def test_device_output_step_matches_host(pkg, showers, deterministic):
     else:  # FP64 atomics: the two projections sum in different orders
         for g, w in zip(got, want):
             assert np.abs(g - w).max() <= 1e-12 * np.abs(w).max()
+
+
+def test_results_to_device_memory_are_refused(pkg, showers):
+    """A device pointer in place of a host buffer is an error, not a crash: from the
+    accumulator (which is sealed by the attempt, as by any failed fixed download)
+    and from the server (whose event stays fetchable)."""
+    import ctypes
+
+    import torch
+
+    wl, gen, _ = showers.workload_config("plain_c0", bins=512)
+    records = showers.shower_records(700, seed=3, **gen)
+    raw = torch.from_numpy(records.view(np.uint8).reshape(-1)).cuda()
+    config = showers.make_config(wl)
+    values = 3 * 512 * len(wl["observers"])
+    out = torch.zeros(values, dtype=torch.int64, device="cuda")
+    host = np.zeros(values, np.int64)
+    for coreas, zhs in ((out.data_ptr(), host.ctypes.data), (host.ctypes.data, out.data_ptr())):
+        acc = pkg.RadioAccumulator(config)
+        acc.accumulate_lepton_tracks(raw.data_ptr(), records.size)
+        status = acc._lib.c8r_download_fixed(acc._h, coreas, zhs, None)
+        assert status == pkg.abi.C8R_CUDA_ERROR
+        acc.close()
+        acc = pkg.RadioAccumulator(config)
+        acc.accumulate_lepton_tracks(raw.data_ptr(), records.size)
+        want = acc.download_fixed()
+        acc.close()
+    server = pkg.RadioServer(budget_bytes=1 << 30)
+    event = server.open(config)
+    server.add_device(event, raw.data_ptr(), records.size)
+    server.close_event(event)
+    counters, info = pkg.abi.Counters(), pkg.abi.ServerEventInfo()
+    for fetch in (server._lib.c8r_server_fetch, server._lib.c8r_server_fetch_fixed):
+        status = fetch(server._h, event, host.ctypes.data, out.data_ptr(), ctypes.byref(counters), ctypes.byref(info))
+        assert status == pkg.abi.C8R_CUDA_ERROR
+    got = server.fetch_fixed(event)
+    server.close()
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert not out.any()
