@@ -301,6 +301,7 @@ class Accumulator {
     }
     if (count >= host_batch_ && staged_ == 0)  // room for the batches projected together, in one go
       ensure_capacity(std::max(host_batch_, std::min(host_count_ + count, kProjectRecords)));
+    bool ingested = false;
     while (count != 0) {
       if (host_count_ == 0) check(cudaEventSynchronize(host_ready_[host_index_]), "staging wait");
       std::size_t const copied = std::min(count, host_batch_ - host_count_);
@@ -311,9 +312,11 @@ class Accumulator {
       count -= copied;
       if (host_count_ != host_batch_) break;
       ingest_host_batch();
+      ingested = true;
       if (staged_ > kProjectRecords - std::min(kProjectRecords, host_batch_)) project_staged(true);
     }
-    project_staged(true);
+    // a call that fills no batch leaves tracks staged by stage_device to their projection
+    if (ingested) project_staged(true);
   }
 
   static bool is_pinned(void const* p) {

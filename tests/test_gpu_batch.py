@@ -124,3 +124,27 @@ def test_tuning_cache_round_trip(pkg, tmp_path, torch_cuda):
     path.write_text(text.replace("team_size=512", "team_size=5x"))
     with pytest.raises(pkg.RadioError, match="not a count"):
         pkg.tuning_cache_load(path, "batched 64 events")
+
+
+def test_part_filled_host_calls_leave_staged_tracks_staged(pkg, oracle, showers, torch_cuda):
+    """A host call that fills no batch, and one of no records, do not project tracks
+    that stage_lepton_tracks left for a batched projection."""
+    torch = torch_cuda
+    wl, gen, _ = showers.workload_config("plain_c0", bins=1024)
+    records = showers.shower_records(901, seed=23, **gen)
+    config = showers.make_config(wl)
+    want = oracle.restatement().project(config, records, threads=8)
+    raw = torch.from_numpy(records.view(np.uint8).reshape(-1)).cuda()
+    stream = torch.cuda.Stream()
+    acc = pkg.RadioAccumulator(config, stream=stream.cuda_stream)
+    batch = pkg.RadioBatch(stream=stream.cuda_stream)
+    acc.stage_lepton_tracks(raw.data_ptr(), 800)
+    acc.enqueue_host_lepton_tracks(records[800:])
+    acc.enqueue_host_lepton_tracks(None)
+    assert acc.statistics().track_observer_pairs == 0
+    batch.project([acc])
+    assert acc.statistics().track_observer_pairs == 2 * 800 * len(wl["observers"])
+    got = acc.download_fixed()
+    batch.close()
+    acc.close()
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
