@@ -590,7 +590,7 @@ class Accumulator {
     if (host.fixed_point_overflows != 0)
       throw std::runtime_error(
           "radio fixed-point accumulator overflowed; increase fixed_point_field_limit_V_per_m");
-    Transfers transfers;
+    std::vector<ResultCopy> results;
     for (int a = 0; a < 2; ++a) {
       double* out = a == 0 ? coreas : zhs;
       std::size_t const values = 3 * bins_[a];
@@ -601,12 +601,12 @@ class Accumulator {
                             static_cast<uint32_t>(observers_host_[a].size()), max_observer_bins_[a],
                             stream_),
               "decode launch");
-        transfers.add(out, decoded_[a].ptr, values * sizeof(double));
+        results.push_back({out, decoded_[a].ptr, values * sizeof(double)});
       } else {
-        transfers.add(out, float_traces_[a].ptr, values * sizeof(double));
+        results.push_back({out, float_traces_[a].ptr, values * sizeof(double)});
       }
     }
-    copy_out(transfers);
+    copy_out(results);
     check(cudaStreamSynchronize(stream_), "download fence");
     if (counters) std::memcpy(counters, &host, sizeof(host));
     downloaded_ = true;
@@ -652,14 +652,14 @@ class Accumulator {
     sealed_ = true;
     DeviceCounters host{};
     fetch_counters(host);
-    Transfers transfers;
+    std::vector<ResultCopy> results;
     for (int a = 0; a < 2; ++a) {
       long long* out = a == 0 ? coreas : zhs;
       std::size_t const values = 3 * bins_[a];
       if (values == 0 || out == nullptr) continue;
-      transfers.add(out, fixed_traces_[a].ptr, values * sizeof(long long));
+      results.push_back({out, fixed_traces_[a].ptr, values * sizeof(long long)});
     }
-    copy_out(transfers);
+    copy_out(results);
     check(cudaStreamSynchronize(stream_), "download fence");
     if (counters) std::memcpy(counters, &host, sizeof(host));
     downloaded_ = true;
@@ -686,17 +686,17 @@ class Accumulator {
     sealed_ = true;
     DeviceCounters host{};
     fetch_counters(host);
-    Transfers transfers;
+    std::vector<ResultCopy> results;
     for (int a = 0; a < 2; ++a) {
       long long* out = a == 0 ? coreas : zhs;
       std::size_t const values = 3 * config_bins_[a];
       if (values == 0) continue;
       if (fixed_traces_[a].ptr && bins_[a] == config_bins_[a])
-        transfers.add(out, fixed_traces_[a].ptr, values * sizeof(long long));
+        results.push_back({out, fixed_traces_[a].ptr, values * sizeof(long long)});
       else
         std::memset(out, 0, values * sizeof(long long));  // algorithm disabled
     }
-    copy_out(transfers);
+    copy_out(results);
     check(cudaStreamSynchronize(stream_), "download fence");
     if (counters) std::memcpy(counters, &host, sizeof(host));
     if (host.fixed_point_overflows != 0)
@@ -706,40 +706,12 @@ class Accumulator {
 
   std::size_t config_bins(int a) const { return config_bins_[a]; }
 
-  // Device buffers and the host memory that takes them.
-  struct Transfers {
-    std::vector<SlotRing::Segment> out;
-    std::vector<unsigned char const*> from;
-    void add(void* destination, void const* source, std::size_t bytes) {
-      out.push_back({destination, bytes});
-      from.push_back(static_cast<unsigned char const*>(source));
-    }
-  };
-
-  // Copies after the stream's earlier work and returns when they are done:
-  // page-locked destinations directly, pageable ones through the slots.  Device
-  // memory is refused: the slots are emptied by host threads.
-  void copy_out(Transfers const& transfers) {
-    Transfers pageable;
-    for (std::size_t k = 0; k < transfers.out.size(); ++k) {
-      SlotRing::Segment const& d = transfers.out[k];
-      ResultMemory const memory = result_memory(d.destination);
-      if (memory == ResultMemory::kDevice) check(cudaErrorInvalidValue, "trace download to device memory");
-      stats_.device_to_host_bytes += d.bytes;
-      if (ring_.usable() && memory == ResultMemory::kPageable)
-        pageable.add(d.destination, transfers.from[k], d.bytes);
-      else
-        check(cudaMemcpyAsync(d.destination, transfers.from[k], d.bytes, cudaMemcpyDeviceToHost, stream_),
-              "trace download");
-    }
-    if (pageable.out.empty()) return;
+  // Copies results to the caller after the stream's earlier work.
+  void copy_out(std::vector<ResultCopy> const& results) {
+    for (ResultCopy const& r : results) stats_.device_to_host_bytes += r.bytes;
     // the slots are the host staging halves: no batch is filling (flushed), none is being uploaded
     for (auto& e : host_ready_) check(cudaEventSynchronize(e), "staging wait");
-    check(ring_.run(pageable.out, stream_,
-                    [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
-                      return cudaMemcpyAsync(slot, pageable.from[k] + offset, bytes, cudaMemcpyDeviceToHost, stream_);
-                    }),
-          "trace download");
+    check(copy_results(ring_, results, stream_), "trace download");
   }
 
   void statistics(c8r_statistics& out) {

@@ -486,7 +486,8 @@ class Server {
     try {
       std::lock_guard<std::mutex> copy_lock(fetch_mu_);
       check(cudaMemcpyAsync(&host, ev.counters, sizeof host, cudaMemcpyDeviceToHost, fetch_), "server fetch");
-      // through the pinned slots: copied, or decoded by a kernel straight into them
+      bool const decoded = ev.fixed && !fixed_out;
+      std::vector<ResultCopy> raw;
       std::vector<SlotRing::Segment> out;
       std::vector<int> of;
       for (int a = 0; a < 2; ++a) {
@@ -494,20 +495,23 @@ class Server {
         if (ev.bins[a] == 0 || to == nullptr) continue;
         if (result_memory(to) == ResultMemory::kDevice)
           check(cudaErrorInvalidValue, "server fetch to device memory");
-        out.push_back({to, 3 * ev.bins[a] * sizeof(double)});
-        of.push_back(a);
+        std::size_t const bytes = 3 * ev.bins[a] * sizeof(double);
+        if (decoded) {
+          out.push_back({to, bytes});
+          of.push_back(a);
+        } else {
+          raw.push_back({to, ev.fixed ? static_cast<void const*>(ev.fixed_traces[a]) : ev.float_traces[a], bytes});
+        }
       }
+      check(copy_results(ring_, raw, fetch_), "server fetch");
+      // decoded by a kernel straight into the slots
       check(ring_.run(out, fetch_,
                       [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
                         int const a = of[k];
-                        std::size_t const first = offset / sizeof(double), n = bytes / sizeof(double);
-                        if (ev.fixed && !fixed_out)
-                          return launch_decode_run(reinterpret_cast<long long const*>(ev.fixed_traces[a]),
-                                                   static_cast<double*>(slot), ev.bins[a], first, n, ev.caches[a],
-                                                   ev.observers[a], ev.limit, a, fetch_);
-                        void const* src = ev.fixed ? static_cast<void const*>(ev.fixed_traces[a] + first)
-                                                   : static_cast<void const*>(ev.float_traces[a] + first);
-                        return cudaMemcpyAsync(slot, src, bytes, cudaMemcpyDeviceToHost, fetch_);
+                        return launch_decode_run(reinterpret_cast<long long const*>(ev.fixed_traces[a]),
+                                                 static_cast<double*>(slot), ev.bins[a], offset / sizeof(double),
+                                                 bytes / sizeof(double), ev.caches[a], ev.observers[a], ev.limit, a,
+                                                 fetch_);
                       }),
             "server fetch");
       check(cudaStreamSynchronize(fetch_), "server fetch");

@@ -202,5 +202,33 @@ class SlotRing {
   std::vector<cudaEvent_t> filled_;
 };
 
+// One result: device memory and where it goes.
+struct ResultCopy {
+  void* to;
+  void const* from;
+  std::size_t bytes;
+};
+// Copies results after the stream's earlier work: page-locked and managed
+// destinations each by one copy (in flight on return), pageable ones through the
+// slots.  Device memory is refused: the slots are emptied by host threads.
+inline cudaError_t copy_results(SlotRing& ring, std::vector<ResultCopy> const& results, cudaStream_t stream) {
+  std::vector<SlotRing::Segment> pageable;
+  std::vector<unsigned char const*> from;
+  for (ResultCopy const& r : results) {
+    ResultMemory const memory = result_memory(r.to);
+    if (memory == ResultMemory::kDevice) return cudaErrorInvalidValue;
+    if (memory == ResultMemory::kPageable && ring.usable()) {
+      pageable.push_back({r.to, r.bytes});
+      from.push_back(static_cast<unsigned char const*>(r.from));
+    } else if (cudaError_t const err = cudaMemcpyAsync(r.to, r.from, r.bytes, cudaMemcpyDeviceToHost, stream)) {
+      return err;
+    }
+  }
+  if (pageable.empty()) return cudaSuccess;
+  return ring.run(pageable, stream, [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
+    return cudaMemcpyAsync(slot, from[k] + offset, bytes, cudaMemcpyDeviceToHost, stream);
+  });
+}
+
 }  // namespace
 }  // namespace c8r

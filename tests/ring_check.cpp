@@ -117,6 +117,30 @@ void check_copies(SlotRing& ring) {
   expect(wrong_device == 0, "every call on the owner's device");
 }
 
+// Page-locked results take one copy each, straight to them; pageable ones go
+// through the slots; a device pointer among them is an error.
+void check_routes(SlotRing& ring) {
+  std::size_t const bytes = 3 * SlotRing::kSlotBytes + 5;
+  std::vector<unsigned char> const a = pattern(bytes, 3), b = pattern(bytes, 4);
+  std::vector<unsigned char> x(bytes), y(bytes);
+  kinds[x.data()] = cudaMemoryTypeHost;
+  runtime_copies = 0;
+  expect(c8r::copy_results(ring, {{x.data(), a.data(), bytes}}, nullptr) == cudaSuccess, "page-locked result");
+  expect(runtime_copies == 1, "page-locked: one copy");
+  finish_queued();
+  expect(x == a, "page-locked result arrives");
+  runtime_copies = 0;
+  expect(c8r::copy_results(ring, {{x.data(), b.data(), bytes}, {y.data(), a.data(), bytes}}, nullptr) == cudaSuccess,
+         "results of both kinds");
+  expect(runtime_copies == 1 + 4, "one copy and four slots");
+  finish_queued();
+  expect(x == b && y == a, "results of both kinds arrive");
+  kinds[x.data()] = cudaMemoryTypeDevice;
+  expect(c8r::copy_results(ring, {{x.data(), a.data(), bytes}}, nullptr) == cudaErrorInvalidValue, "device memory");
+  expect(x == b, "device memory untouched");
+  kinds.clear();
+}
+
 // A result buffer's memory decides its route.
 void check_memory() {
   char pageable, locked, managed, device;
@@ -139,6 +163,7 @@ int main() {
     SlotRing ring;
     expect(ring.use(slots.data(), slots.size()) == cudaSuccess, "slots");
     check_copies(ring);
+    check_routes(ring);
   }
   if (failures) return 1;
   std::printf("ok\n");

@@ -164,3 +164,39 @@ def test_decoded_fetch_equals_download(pkg, showers, torch_cuda):
     acc.close()
     assert np.array_equal(waveforms.coreas, want.coreas) and np.array_equal(waveforms.zhs, want.zhs)
     assert info["rounds"] >= 1
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("deterministic", [True, False])
+def test_fetches_into_page_locked_and_pageable_memory(pkg, showers, torch_cuda, pinned, deterministic):
+    """Raw and decoded fetches of traces longer than the copy slots hold at a time
+    equal the accumulator's results, into either kind of memory."""
+    wl, gen, _ = showers.workload_config("tiled_c1", bins=2049)
+    records = showers.shower_records(1_200, seed=77, **gen)
+    raw = torch_cuda.from_numpy(records.view(np.uint8).reshape(-1)).cuda()
+    config = showers.make_config(wl, deterministic=deterministic)
+    values = 3 * 2049 * len(wl["observers"])
+    server = pkg.RadioServer(budget_bytes=2 << 30)
+
+    def alone(fixed):
+        acc = pkg.RadioAccumulator(config)
+        acc.accumulate_lepton_tracks(raw.data_ptr(), records.size)
+        got = acc.download_fixed() if fixed else acc.download()
+        acc.close()
+        return (got[0], got[1]) if fixed else (got.coreas, got.zhs)
+
+    for fixed in ((True, False) if deterministic else (False,)):
+        kind = torch_cuda.int64 if fixed else torch_cuda.float64
+        out = [torch_cuda.zeros(values, dtype=kind, pin_memory=pinned) for _ in range(2)]
+        event = server.open(config)
+        server.add_device(event, raw.data_ptr(), records.size)
+        server.close_event(event)
+        fetch = server._lib.c8r_server_fetch_fixed if fixed else server._lib.c8r_server_fetch
+        assert fetch(server._h, event, out[0].data_ptr(), out[1].data_ptr(), None, None) == 0
+        for got, want in zip(out, alone(fixed)):
+            want = want.reshape(-1)
+            if deterministic:
+                assert np.array_equal(got.numpy(), want)
+            else:
+                assert np.abs(got.numpy() - want).max() <= 2e-12 * np.abs(want).max()
+    server.close()
