@@ -2638,29 +2638,6 @@ __global__ void decode_kernel(const long long* __restrict__ fixed, double* __res
   }
 }
 
-// A run of decoded values, [begin, begin + count) of a trace buffer's rows
-// [X | Y | Z], into `out` (page-locked host memory): value times the decode
-// factor of its observer (downloadSet, RadioAccumulator.inl:865-867), found by
-// its waveform offset.
-__global__ void decode_run_kernel(const long long* __restrict__ fixed, double* __restrict__ out, uint64_t total_bins,
-                                  uint64_t begin, uint64_t count, const ObserverCache* __restrict__ observers,
-                                  uint32_t observer_count, double limit, int differentiated) {
-  for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count;
-       i += static_cast<uint64_t>(gridDim.x) * blockDim.x) {
-    uint64_t const bin = (begin + i) % total_bins;
-    uint32_t lo = 0, hi = observer_count;  // last observer whose offset is at most bin
-    while (hi - lo > 1) {
-      uint32_t const mid = (lo + hi) >> 1;
-      if (observers[mid].offset <= bin)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    double const scale = differentiated ? observers[lo].sample_rate : 1.;
-    out[i] = static_cast<double>(fixed[begin + i]) * (limit / (kHeadroom * scale));
-  }
-}
-
 // The output step on the device: CoREAS fields added as they are, ZHS
 // potentials differentiated into fields E_i = -(A_{i+1} - A_i) fs at the bin
 // midpoints (RadioProcess.inl:213-223; one sample fewer per observer), both
@@ -2935,16 +2912,6 @@ cudaError_t launch_output(const long long* fixed, const double* floating, double
   dim3 const grid(static_cast<unsigned>(bx), observer_count);
   output_kernel<<<grid, 256, 0, stream>>>(fixed, floating, out, total_bins, observers, factors,
                                           observer_count, differentiate ? 1 : 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_decode_run(const long long* fixed, double* out, uint64_t total_bins, uint64_t begin,
-                              uint64_t count, const ObserverCache* observers, uint32_t observer_count, double limit,
-                              int algorithm, cudaStream_t stream) {
-  if (count == 0) return cudaSuccess;
-  uint64_t const blocks = (count + 255) / 256;
-  decode_run_kernel<<<static_cast<unsigned>(blocks < 1024 ? blocks : 1024), 256, 0, stream>>>(
-      fixed, out, total_bins, begin, count, observers, observer_count, limit, algorithm == 1 ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -314,11 +314,6 @@ cudaError_t launch_output(const long long* fixed, const double* floating, double
                           const ObserverCache* observers, const double* factors, uint32_t observer_count,
                           uint64_t max_bins, bool differentiate, cudaStream_t stream);
 
-// Decodes values [begin, begin + count) of a trace buffer into `out`.
-cudaError_t launch_decode_run(const long long* fixed, double* out, uint64_t total_bins, uint64_t begin,
-                              uint64_t count, const ObserverCache* observers, uint32_t observer_count, double limit,
-                              int algorithm, cudaStream_t stream);
-
 // Fixed-point decode on the device: out[r*bins + i] = in[r*bins + i] * factor(observer).
 cudaError_t launch_decode(const long long* fixed, double* out, uint64_t total_bins,
                           const uint64_t* observer_offsets, const double* factors,

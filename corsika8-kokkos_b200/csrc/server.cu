@@ -60,6 +60,39 @@ constexpr std::size_t kGranule = 256;
 constexpr std::size_t kFetchBytes = 4 * SlotRing::kSlotBytes;
 std::size_t round_up(std::size_t bytes) { return (bytes + kGranule - 1) / kGranule * kGranule; }
 
+// downloadSet's decode (RadioAccumulator.inl:849-898), value x factor per observer,
+// for runs of an algorithm's values (rows [X | Y | Z] of all its bins).
+class TraceDecoder {
+ public:
+  TraceDecoder(std::vector<c8r_observer_snapshot> const& observers, int algorithm, double limit) {
+    std::size_t end = 0;
+    for (auto const& s : observers) {
+      end += static_cast<std::size_t>(s.number_of_bins);
+      ends_.push_back(end);
+      factors_.push_back(decode_factor(s, algorithm, limit));
+    }
+  }
+  // Values [first, first + count) of the traces, `in` and `out` their first ones.
+  void decode(long long const* in, double* out, std::size_t first, std::size_t count) const {
+    std::size_t const total = ends_.back();
+    while (count != 0) {
+      std::size_t const bin = first % total;
+      std::size_t const o = static_cast<std::size_t>(std::upper_bound(ends_.begin(), ends_.end(), bin) - ends_.begin());
+      std::size_t const n = std::min(count, ends_[o] - bin);
+      double const factor = factors_[o];
+      for (std::size_t i = 0; i < n; ++i) out[i] = static_cast<double>(in[i]) * factor;
+      in += n;
+      out += n;
+      first += n;
+      count -= n;
+    }
+  }
+
+ private:
+  std::vector<std::size_t> ends_;  // of each observer's bins
+  std::vector<double> factors_;
+};
+
 // First-fit sub-allocator over one device reservation, coalescing on release.
 class Arena {
  public:
@@ -504,15 +537,23 @@ class Server {
         }
       }
       check(copy_results(ring_, raw, fetch_), "server fetch");
-      // decoded by a kernel straight into the slots
-      check(ring_.run(out, fetch_,
-                      [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
-                        int const a = of[k];
-                        return launch_decode_run(reinterpret_cast<long long const*>(ev.fixed_traces[a]),
-                                                 static_cast<double*>(slot), ev.bins[a], offset / sizeof(double),
-                                                 bytes / sizeof(double), ev.caches[a], ev.observers[a], ev.limit, a,
-                                                 fetch_);
-                      }),
+      // The copy engine fills the slots and the copying threads decode: a kernel
+      // would wait for an SM behind every projection launch of the other events,
+      // whose CTAs take a whole SM each (63 MB decoded while another event's
+      // launches of 100 ms ran: 150 to 280 ms with a decode kernel a slot).
+      std::vector<TraceDecoder> decoders;
+      for (int const a : of) decoders.emplace_back(ev.snapshots[a], a, ev.limit);
+      check(ring_.run(
+                out, fetch_,
+                [&](std::size_t k, std::size_t offset, std::size_t bytes, void* slot) {
+                  auto const* from = reinterpret_cast<unsigned char const*>(ev.fixed_traces[of[k]]);
+                  return cudaMemcpyAsync(slot, from + offset, bytes, cudaMemcpyDeviceToHost, fetch_);
+                },
+                [&](std::size_t k, std::size_t offset, std::size_t bytes, void const* slot) {
+                  std::size_t const first = offset / sizeof(double);
+                  decoders[k].decode(static_cast<long long const*>(slot), static_cast<double*>(out[k].destination) + first,
+                                     first, bytes / sizeof(double));
+                }),
             "server fetch");
       check(cudaStreamSynchronize(fetch_), "server fetch");
     } catch (...) {

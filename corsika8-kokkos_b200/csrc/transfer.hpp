@@ -74,10 +74,11 @@ class SlotRing {
 
   // Fills the segments in order: issue(segment, offset, bytes, slot) queues on
   // `stream` the work that writes bytes [offset, offset + bytes) of a segment
-  // into `slot`.  Returns once everything has been copied out.  The copying
+  // into `slot`, emit(segment, offset, bytes, slot) moves them on to the segment's
+  // destination.  Returns once everything has been copied out.  The copying
   // threads work on the calling thread's device.
-  template <class Issue>
-  cudaError_t run(std::vector<Segment> const& segments, cudaStream_t stream, Issue issue) {
+  template <class Issue, class Emit>
+  cudaError_t run(std::vector<Segment> const& segments, cudaStream_t stream, Issue issue, Emit emit) {
     std::vector<Piece> pieces;
     std::size_t total = 0;
     for (std::size_t s = 0; s < segments.size(); ++s)
@@ -95,7 +96,7 @@ class SlotRing {
       cudaError_t const err = cudaEventSynchronize(filled_[i % depth]);
       if (err != cudaSuccess) return err;
       Piece const& p = pieces[i];
-      std::memcpy(static_cast<unsigned char*>(segments[p.segment].destination) + p.offset, slots_[i % depth], p.bytes);
+      emit(p.segment, p.offset, p.bytes, static_cast<void const*>(slots_[i % depth]));
       return cudaSuccess;
     };
     unsigned const cores = std::max(1u, std::thread::hardware_concurrency() / 2);
@@ -138,6 +139,13 @@ class SlotRing {
     }
     workers.join();
     return static_cast<cudaError_t>(shared.error.load());
+  }
+  // The same, the bytes copied as they are.
+  template <class Issue>
+  cudaError_t run(std::vector<Segment> const& segments, cudaStream_t stream, Issue issue) {
+    return run(segments, stream, issue, [&](std::size_t k, std::size_t offset, std::size_t bytes, void const* slot) {
+      std::memcpy(static_cast<unsigned char*>(segments[k].destination) + offset, slot, bytes);
+    });
   }
 
  private:

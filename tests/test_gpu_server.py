@@ -200,3 +200,39 @@ def test_fetches_into_page_locked_and_pageable_memory(pkg, showers, torch_cuda, 
             else:
                 assert np.abs(got.numpy() - want).max() <= 2e-12 * np.abs(want).max()
     server.close()
+
+
+def test_decoded_fetch_does_not_wait_for_another_event(pkg, showers, torch_cuda):
+    """A finished event's decoded traces are fetched while a long event keeps every
+    SM busy: the fetch needs no SM, so it ends within a fraction of the long
+    event's time (it took half of it and more when each slot was decoded by a
+    kernel, which waits for the end of a projection launch)."""
+    import time
+
+    torch = torch_cuda
+    wl, gen, _ = showers.workload_config("tiled_c1")  # 160 antennas x 8192 bins: 63 MB of traces
+    records = showers.shower_records(65_536, seed=21, **gen)
+    raw = device(torch, records)
+    light = showers.make_config(wl, precision=1)
+    heavy = showers.make_config(wl, precision=1, zhs_subtrack_refinement=64)
+    server = pkg.RadioServer(budget_bytes=6 << 30)
+    shares = []
+    for _ in range(3):  # the first trial warms up
+        done = server.open(light)
+        server.add_device(done, raw.data_ptr(), 2000)
+        server.close_event(done)
+        server.wait(done)
+        running = server.open(heavy)
+        for _ in range(12):
+            server.add_device(running, raw.data_ptr(), records.size)
+        begin = time.perf_counter()
+        server.close_event(running)
+        time.sleep(0.02)
+        at = time.perf_counter()
+        server.fetch(done)
+        fetched = time.perf_counter() - at
+        server.wait(running)
+        shares.append(fetched / (time.perf_counter() - begin))
+        server.fetch_fixed(running)
+    server.close()
+    assert min(shares[1:]) < 0.25, shares
