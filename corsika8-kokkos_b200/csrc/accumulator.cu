@@ -520,7 +520,7 @@ class Accumulator {
   cudaStream_t stream() const { return stream_; }
   bool sealed() const { return sealed_; }
   void note_batch_projection(std::size_t count, uint64_t items) {
-    EventPlan const ev = make_event(count);
+    EventPlan const ev = make_event(count, 0);
     uint64_t const pairs_c = count * ev.observer_count[0], pairs_z = count * ev.observer_count[1];
     stats_.track_observer_pairs += pairs_c + pairs_z;
     if (fuse_) stats_.fused_track_observer_pairs += pairs_c;
@@ -769,7 +769,13 @@ class Accumulator {
   }
 
   // Work-plan access for the batched launcher.
-  EventPlan event_plan(std::size_t count) const { return make_event(count); }
+  EventPlan event_plan(std::size_t count, uint64_t ctas) const { return make_event(count, ctas); }
+  uint64_t observers() const {
+    return std::max(coreas_enabled_ ? observers_host_[0].size() : 0, zhs_enabled_ ? observers_host_[1].size() : 0);
+  }
+  double item() const {
+    return item_cost(static_cast<uint32_t>(window_bins_), precision_ == Precision::kFP64, propagation_.refinement);
+  }
   bool fixed() const { return fixed_; }
   Precision precision() const { return precision_; }
   bool study() const { return study_; }
@@ -941,7 +947,8 @@ class Accumulator {
 
   std::size_t chunk_hint() const { return tuning_.track_tile_size; }
 
-  EventPlan make_event(std::size_t count) const {
+  // `ctas`: the CTAs its work items are cut for (0: a launch without work items).
+  EventPlan make_event(std::size_t count, uint64_t ctas) const {
     EventPlan ev;
     std::memset(&ev, 0, sizeof ev);
     ev.tracks = tracks_.ptr;
@@ -959,8 +966,7 @@ class Accumulator {
     ev.counters = counters_.ptr;
     ev.window = static_cast<uint32_t>(window_bins_);
     std::size_t chunk = tuning_.track_tile_size;
-    if (chunk == 0)
-      chunk = auto_chunk(count, std::max(ev.observer_count[0], ev.observer_count[1]), static_cast<uint64_t>(sms_));
+    if (chunk == 0) chunk = auto_chunk(count, observers(), ctas, item());
     chunk = std::min<std::size_t>(chunk, kMaxChunkTracks);
     ev.chunk_size = static_cast<uint32_t>(chunk);
     ev.chunks = static_cast<uint32_t>((count + chunk - 1) / chunk);
@@ -988,7 +994,7 @@ class Accumulator {
   }
 
   void project_direct(std::size_t count) {
-    EventPlan const ev = make_event(count);
+    EventPlan const ev = make_event(count, 0);
     bool const c = ev.observer_count[0] != 0, z = ev.observer_count[1] != 0;
     if (fuse_) {
       check(launch_direct(ev, count, true, true, fixed_, precision_, stream_), "direct launch");
@@ -1006,7 +1012,7 @@ class Accumulator {
   // The reference's tile shape (RadioAccumulator.inl:699-847): fused when the
   // observer grids match, else one launch per algorithm.
   void project_tiled(std::size_t count) {
-    EventPlan const ev = make_event(count);
+    EventPlan const ev = make_event(count, 0);
     bool const c = ev.observer_count[0] != 0, z = ev.observer_count[1] != 0;
     if (fuse_) {
       check(launch_tiled(ev, count, true, true, fixed_, precision_, stream_), "tiled launch");
@@ -1023,7 +1029,7 @@ class Accumulator {
 
   // The precision study's generic kernel, both algorithms in one launch.
   void project_study(std::size_t count) {
-    EventPlan const ev = make_event(count);
+    EventPlan const ev = make_event(count, 0);
     bool const c = ev.observer_count[0] != 0, z = ev.observer_count[1] != 0;
     check(launch_study(ev, count, c, z, fixed_, arithmetic_, stream_), "study launch");
     stats_.track_observer_pairs += count * (ev.observer_count[0] + ev.observer_count[1]);
@@ -1039,7 +1045,7 @@ class Accumulator {
   // With kernel timing on, both run on stream_, so that each launch's events
   // bracket that launch alone.
   void project_windowed(std::size_t count) {
-    EventPlan const ev = make_event(count);
+    EventPlan const ev = make_event(count, static_cast<uint64_t>(sms_));
     int per_sm = windowed_ctas_per_sm(static_cast<int>(ev.window), threads_, fixed_, precision_);
     if (per_sm <= 0) throw cuda_error("windowed radio kernel does not fit on this device");
     bool const both = !timing_ && ev.observer_count[0] != 0 && ev.observer_count[1] != 0;
@@ -1061,8 +1067,7 @@ class Accumulator {
       plan.reruns = reruns_.ptr;
       plan.handbacks = reruns_.ptr + 1;
       uint64_t ctas = static_cast<uint64_t>(per_sm) * sms_;
-      // a launch of few rounds is planned to end evenly; a tail would add a round
-      append_work(plan, ev, ctas, static_cast<uint64_t>(ev.chunks) * ev.observer_count[algorithm] > 4 * ctas);
+      append_work(plan, ev, ctas, tail_pays(ev.chunks, ev.chunk_size, ev.observer_count[algorithm], ctas, item()));
       if (ctas > plan.total_items) ctas = plan.total_items;
       plan.deferred_stride = deferred_list_stride(plan);
       attach_deferred(plan, deferred_lists(algorithm, deferred_words(plan, ctas, fixed_)), ctas, fixed_);
@@ -1316,7 +1321,6 @@ class Batch {
       if (e->sealed()) throw std::logic_error("radio endpoint already committed; reset before new tracks");
       if (e->stream() != stream_) throw std::invalid_argument("batched accumulators must share the batch stream");
       if (e->study()) throw std::invalid_argument("precision-study accumulators cannot be batched");
-      EventPlan ev = e->event_plan(e->staged());
       if (active.empty()) {
         fixed = e->fixed();
         precision = e->precision();
@@ -1324,6 +1328,7 @@ class Batch {
       } else if (e->fixed() != fixed || e->precision() != precision) {
         throw std::invalid_argument("batched accumulators must share precision and trace mode");
       }
+      EventPlan const ev = e->event_plan(e->staged(), static_cast<uint64_t>(e->sms()));
       window = std::max(window, ev.window);
       active.push_back({i, ev});
     }

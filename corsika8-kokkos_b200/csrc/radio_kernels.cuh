@@ -182,27 +182,37 @@ inline void attach_deferred(WorkPlan& plan, unsigned* words, uint64_t ctas, bool
   plan.drain_next_item = reinterpret_cast<unsigned*>(plan.item_state + plan.total_items);
 }
 
+// How append_work divides `chunks` long chunks of `big` tracks when it ends the
+// list on short items: the first `head` stay long, the rest of the tracks go in
+// chunks of `small`, a quarter as long (at least 8192 tracks), about two items for
+// each of the `ctas` persistent CTAs.
+struct TailSplit {
+  uint64_t head, small;
+};
+inline TailSplit split_tail(uint64_t chunks, uint64_t big, uint64_t per, uint64_t ctas) {
+  constexpr uint64_t kSplit = 4, kMinTailChunk = 8192;
+  uint64_t const quarter = (big + kSplit - 1) / kSplit;
+  // whole track tiles, so that short items start on a tile as long ones do
+  uint64_t const small = track_capacity(quarter > kMinTailChunk ? quarter : kMinTailChunk);
+  if (small >= big) return {chunks, small};
+  uint64_t const short_items = (2 * ctas + per - 1) / per;
+  uint64_t const replaced = (short_items * small + big - 1) / big;  // long chunks they cover
+  return {replaced >= chunks ? 0 : chunks - replaced, small};
+}
+
 // Appends the (chunk, observer) work items of `ev` for plan.algorithm to
 // `plan` (first_item, event_count and total_items follow).  With `fine_tail`
-// and a free event slot, the last chunks go in as a second entry of chunks a
-// quarter as long (at least 8192 tracks), about two items for each of the
-// `ctas` persistent CTAs: the launch then ends on short items instead of one
-// CTA finishing a long item while the others wait.  Every track stays in
-// exactly one item.  Returns the number of items appended.
+// and a free event slot, the last chunks go in as a second entry of short chunks
+// (split_tail): the launch then ends on short items instead of one CTA finishing a
+// long item while the others wait.  Every track stays in exactly one item.
+// Returns the number of items appended.
 inline uint64_t append_work(WorkPlan& plan, EventPlan ev, uint64_t ctas, bool fine_tail) {
-  constexpr uint64_t kSplit = 4, kMinTailChunk = 8192;
   uint64_t const per = ev.observer_count[plan.algorithm];
   if (per == 0 || ev.chunks == 0 || plan.event_count >= kPlanEntries) return 0;
   uint64_t const big = ev.chunk_size;
-  // whole track tiles, so that short items start on a tile as long ones do
-  uint64_t const small = track_capacity((big + kSplit - 1) / kSplit > kMinTailChunk ? (big + kSplit - 1) / kSplit
-                                                                                    : kMinTailChunk);
-  uint64_t head = ev.chunks;
-  if (fine_tail && plan.event_count + 2 <= kPlanEntries && small < big) {
-    uint64_t const short_items = (2 * ctas + per - 1) / per;
-    uint64_t const replaced = (short_items * small + big - 1) / big;  // long chunks they cover
-    head = replaced >= ev.chunks ? 0 : ev.chunks - replaced;
-  }
+  TailSplit split{ev.chunks, 0};
+  if (fine_tail && plan.event_count + 2 <= kPlanEntries) split = split_tail(ev.chunks, big, per, ctas);
+  uint64_t const head = split.head, small = split.small;
   uint64_t const before = plan.total_items;
   if (head > 0) {
     EventPlan e = ev;
@@ -225,37 +235,77 @@ inline uint64_t append_work(WorkPlan& plan, EventPlan ev, uint64_t ctas, bool fi
   return plan.total_items - before;
 }
 
-// Tracks per work item for `count` tracks at `observers` observers of one
-// algorithm's launch on `ctas` persistent CTAs.  An item
-// costs a pass over its antenna's window (zeroed, summed and flushed: as long as
-// about 4400 tracks take) beside its tracks, and the launch lasts as many rounds
-// as the busiest CTA has items.  Up to 262144 tracks a CTA the number of chunks
-// is the one with the least rounds x (4400 + tracks); above that, items of about
-// a sixteenth of a CTA's share (at least an eighth of the launch up to 262144
-// tracks) and a tail of short ones even out what the antennas' different loads
-// leave (append_work).
-inline uint64_t auto_chunk(uint64_t count, uint64_t observers, uint64_t ctas) {
-  constexpr uint64_t kItemCost = 4400, kFewTracks = 262144, kMostChunks = 64;
-  if (count == 0 || observers == 0 || ctas == 0) return kTrackTile;
-  uint64_t chunk = 0;
-  if (count <= kFewTracks * ctas / observers) {
-    uint64_t least = ~0ull;
-    for (uint64_t chunks = 1; chunks <= kMostChunks; ++chunks) {
-      uint64_t const tracks = track_capacity((count + chunks - 1) / chunks);
-      uint64_t const items = (count + tracks - 1) / tracks * observers;
-      uint64_t const cost = (items + ctas - 1) / ctas * (kItemCost + tracks);
-      if (cost < least) {
+// What an item costs beside its tracks, in tracks: the window zeroed, summed and
+// flushed, a part of it whatever the window's size; relative to the tracks' own
+// time, which is 2.2 times as long in FP64 and grows with the subtrack refinement.
+// Fitted, with the two margins of plan_cost, to 2044 timed launches (1 to 300
+// antennas, 1500 to 9.5e6 tracks, windows of 900 to 8192 bins, 1 to 296 chunks with
+// and without a short tail): the plan of least cost is within 0.6% of the fastest
+// timed one in the mean, 6.8% at worst.
+inline double item_cost(uint32_t window, bool fp64, uint32_t refinement) {
+  return (2000. + 1.5 * window) * (fp64 ? 0.4 : 1.) / (refinement > 1 ? refinement : 1u);
+}
+
+// Length of a launch over `count` tracks at `per` observers in chunks of `chunk`
+// tracks, in tracks: without a tail as many rounds as the busiest CTA has items,
+// and a fifth more, since the antennas' loads differ; with a short tail, which
+// evens that out, the mean load and half a short item.  (A list of short items
+// alone is one without a tail.)
+inline double plan_cost(uint64_t count, uint64_t per, uint64_t ctas, uint64_t chunk, bool tail, double item) {
+  uint64_t const chunks = (count + chunk - 1) / chunk;
+  TailSplit const split = tail ? split_tail(chunks, chunk, per, ctas) : TailSplit{chunks, 0};
+  uint64_t const left = count - (split.head * chunk < count ? split.head * chunk : count);
+  uint64_t const short_chunks = split.head < chunks && left > 0 ? (left + split.small - 1) / split.small : 0;
+  double const longest = static_cast<double>(chunk < count ? chunk : count);
+  double const rounds = static_cast<double>((split.head * per + ctas - 1) / ctas) * (item + longest);
+  if (short_chunks == 0) return 1.2 * rounds;
+  double const shortest = static_cast<double>(split.small < count ? split.small : count);
+  if (split.head == 0)
+    return 1.2 * static_cast<double>((short_chunks * per + ctas - 1) / ctas) * (item + shortest);
+  double const mean = (static_cast<double>((split.head + short_chunks) * per) * item +
+                       static_cast<double>(count) * static_cast<double>(per)) / static_cast<double>(ctas);
+  double const even = mean + 0.5 * (item + shortest);
+  return 1.1 * (rounds > even ? rounds : even);
+}
+
+// Whether a launch of `chunks` chunks ends sooner on short items.
+inline bool tail_pays(uint64_t chunks, uint64_t chunk, uint64_t per, uint64_t ctas, double item) {
+  if (chunks == 0 || per == 0 || ctas == 0) return false;
+  uint64_t const count = chunks * chunk;
+  return plan_cost(count, per, ctas, chunk, true, item) < plan_cost(count, per, ctas, chunk, false, item);
+}
+
+// Tracks per work item for `count` tracks at `per` observers of one algorithm's
+// launch on `ctas` persistent CTAs: of the plans that fill 1, 2, .. rounds, with or
+// without a tail, the one of least cost.  Long launches keep at least 16 items a
+// CTA, or items of 262144 tracks: the per-CTA deferred lists hold an item each.
+// (The former rule took at most 64 chunks and no tail below four rounds: 9.5e6
+// tracks at 1 / 5 antennas, 6e6 at 8, CoREAS and ZHS together, FP64 1800 / 5545 / 5415
+// -> 922 / 3624 / 3479 us, mixed 828 / 2513 / 2461 -> 516 / 1706 / 1617.)
+inline uint64_t auto_chunk(uint64_t count, uint64_t per, uint64_t ctas, double item) {
+  constexpr uint64_t kLongest = 262144, kRounds = 32;
+  if (count == 0 || per == 0 || ctas == 0) return kTrackTile;
+  uint64_t const share = (count * per + 16 * ctas - 1) / (16 * ctas);
+  uint64_t const longest = share > kLongest ? share : kLongest;
+  uint64_t const fewest = (count + longest - 1) / longest;
+  uint64_t best = 0;
+  double least = 0.;
+  auto consider = [&](uint64_t chunks) {
+    if (chunks < fewest) return;
+    uint64_t const chunk = track_capacity((count + chunks - 1) / chunks);
+    if (chunk == best) return;
+    for (bool tail : {false, true}) {
+      double const cost = plan_cost(count, per, ctas, chunk, tail, item);
+      if (best == 0 || cost < least) {
         least = cost;
-        chunk = tracks;
+        best = chunk;
       }
     }
-    return chunk;
-  }
-  uint64_t const target = (16 * ctas + observers - 1) / observers;
-  chunk = (count + target - 1) / target;
-  chunk = chunk > 8192 ? chunk : 8192;
-  uint64_t const eighth = (count + 7) / 8 < kFewTracks ? (count + 7) / 8 : kFewTracks;
-  return track_capacity(chunk > eighth ? chunk : eighth);
+  };
+  consider(fewest);
+  uint64_t const first = (fewest * per + ctas - 1) / ctas;
+  for (uint64_t round = first; round < first + kRounds; ++round) consider(round * ctas / per);
+  return best;
 }
 
 enum class Precision : int { kFP64 = 0, kMixed = 1 };

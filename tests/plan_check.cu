@@ -3,9 +3,11 @@
 // attach_deferred, the arithmetic that keeps every kernel access of a launch
 // inside its buffers.  Prints "ok" or the first failed check; exit status 1
 // on a failure.
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <vector>
 
 #include "radio_kernels.cuh"
@@ -96,9 +98,84 @@ void check_storage(WorkPlan plan, uint64_t ctas, bool fixed) {
   expect(first + (ctas - 1) * plan.deferred_stride + plan.deferred_stride - 1 < first + lists, "second-pass index");
 }
 
+// Length of a launch, in tracks, on CTAs that take items in order as they come
+// free: groups of equal items, one group after the other.
+struct Items {
+  uint64_t count;
+  double length;
+};
+double launch_length(std::vector<Items> const& groups, uint64_t ctas) {
+  std::vector<double> busy(ctas, 0.);
+  bool first = true;
+  for (Items const& g : groups) {
+    uint64_t n = g.count;
+    if (first) {
+      for (double& b : busy) b = static_cast<double>(n / ctas) * g.length;
+      n %= ctas;
+      std::make_heap(busy.begin(), busy.end(), std::greater<double>());
+    }
+    first = false;
+    for (uint64_t i = 0; i < n; ++i) {
+      std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+      busy.back() += g.length;
+      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+    }
+  }
+  return *std::max_element(busy.begin(), busy.end());
+}
+
+// Chunks of `chunk` tracks over `count`, the last one perhaps shorter.
+void append_chunks(std::vector<Items>& groups, uint64_t count, uint64_t chunk, uint64_t per, double item) {
+  if (count == 0) return;
+  groups.push_back({count / chunk * per, item + static_cast<double>(chunk)});
+  if (count % chunk) groups.push_back({per, item + static_cast<double>(count % chunk)});
+}
+
+double planned_length(uint64_t count, uint64_t per, uint64_t ctas, uint64_t chunk, bool tail, double item) {
+  uint64_t const chunks = (count + chunk - 1) / chunk;
+  TailSplit const split = tail ? split_tail(chunks, chunk, per, ctas) : TailSplit{chunks, 0};
+  uint64_t const head = split.head < chunks ? split.head * chunk : count;
+  std::vector<Items> groups;
+  append_chunks(groups, head, chunk, per, item);
+  append_chunks(groups, count - head, split.small, per, item);
+  return launch_length(groups, ctas);
+}
+
+// The automatic chunks of 1 to 300 antennas and 1e3 to 4e7 tracks: the launch is
+// within 15% and one item's window of the shortest one over every number of chunks
+// that the deferred lists allow, and its lists hold no more than 16 items a CTA
+// would or 262144 tracks.
+void check_auto_chunk(uint64_t ctas) {
+  for (uint64_t per : {1, 2, 3, 5, 8, 16, 30, 48, 64, 100, 147, 148, 149, 160, 240, 300})
+    for (uint64_t count : {1000, 4097, 20000, 100003, 300000, 1000000, 2000000, 4000000, 6000000, 9500000, 40000000})
+      for (double item : {item_cost(900, true, 1), item_cost(8192, false, 1), item_cost(4096, true, 4)}) {
+        uint64_t const chunk = auto_chunk(count, per, ctas, item);
+        uint64_t const share = (count * per + 16 * ctas - 1) / (16 * ctas);
+        uint64_t const longest = share > 262144 ? share : 262144;
+        expect(chunk >= kTrackTile && chunk % kTrackTile == 0, "whole track tiles", chunk, count);
+        expect(chunk <= track_capacity(longest), "a chunk the deferred lists allow", chunk, longest);
+        uint64_t const chunks = (count + chunk - 1) / chunk;
+        double const length =
+            planned_length(count, per, ctas, chunk, tail_pays(chunks, chunk, per, ctas, item), item);
+        double shortest = 1e300;
+        for (uint64_t c = (count + longest - 1) / longest; c <= 600; c += c < 200 ? 1 : 10) {
+          uint64_t const other = track_capacity((count + c - 1) / c);
+          if (other < 256) break;
+          for (bool tail : {false, true}) {
+            double const l = planned_length(count, per, ctas, other, tail, item);
+            if (l < shortest) shortest = l;
+          }
+        }
+        if (shortest == 1e300) continue;
+        expect(length <= 1.15 * shortest + item, "launch length within 15% and a window of the shortest",
+               count * 1000 + per, chunk);
+      }
+}
+
 }  // namespace
 
 int main() {
+  check_auto_chunk(148);
   // the 1e7 x 160 workload's ZHS launch, a served round, a batched launch of
   // several events, small launches, and one past the two-pass cap
   struct Case {
