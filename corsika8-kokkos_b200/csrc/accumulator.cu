@@ -520,7 +520,7 @@ class Accumulator {
   cudaStream_t stream() const { return stream_; }
   bool sealed() const { return sealed_; }
   void note_batch_projection(std::size_t count, uint64_t items) {
-    EventPlan const ev = make_event(count, 0);
+    EventPlan const ev = make_event(count, false);
     uint64_t const pairs_c = count * ev.observer_count[0], pairs_z = count * ev.observer_count[1];
     stats_.track_observer_pairs += pairs_c + pairs_z;
     if (fuse_) stats_.fused_track_observer_pairs += pairs_c;
@@ -769,7 +769,7 @@ class Accumulator {
   }
 
   // Work-plan access for the batched launcher.
-  EventPlan event_plan(std::size_t count, uint64_t ctas) const { return make_event(count, ctas); }
+  EventPlan event_plan(std::size_t count, double batch_work) const { return make_event(count, true, batch_work); }
   uint64_t observers() const {
     return std::max(coreas_enabled_ ? observers_host_[0].size() : 0, zhs_enabled_ ? observers_host_[1].size() : 0);
   }
@@ -947,8 +947,9 @@ class Accumulator {
 
   std::size_t chunk_hint() const { return tuning_.track_tile_size; }
 
-  // `ctas`: the CTAs its work items are cut for (0: a launch without work items).
-  EventPlan make_event(std::size_t count, uint64_t ctas) const {
+  // `items`: its launch has work items, cut for the whole GPU or, in a batched launch
+  // of `batch_work` (batch_chunk), for the event's share of it.
+  EventPlan make_event(std::size_t count, bool items, double batch_work = 0.) const {
     EventPlan ev;
     std::memset(&ev, 0, sizeof ev);
     ev.tracks = tracks_.ptr;
@@ -966,7 +967,11 @@ class Accumulator {
     ev.counters = counters_.ptr;
     ev.window = static_cast<uint32_t>(window_bins_);
     std::size_t chunk = tuning_.track_tile_size;
-    if (chunk == 0) chunk = auto_chunk(count, observers(), ctas, item());
+    uint64_t const ctas = static_cast<uint64_t>(sms_);
+    if (chunk == 0 && items)
+      chunk = batch_work > 0. ? batch_chunk(count, observers(), ctas, item(), batch_work)
+                              : auto_chunk(count, observers(), ctas, item());
+    chunk = std::max<std::size_t>(chunk, 1);
     chunk = std::min<std::size_t>(chunk, kMaxChunkTracks);
     ev.chunk_size = static_cast<uint32_t>(chunk);
     ev.chunks = static_cast<uint32_t>((count + chunk - 1) / chunk);
@@ -994,7 +999,7 @@ class Accumulator {
   }
 
   void project_direct(std::size_t count) {
-    EventPlan const ev = make_event(count, 0);
+    EventPlan const ev = make_event(count, false);
     bool const c = ev.observer_count[0] != 0, z = ev.observer_count[1] != 0;
     if (fuse_) {
       check(launch_direct(ev, count, true, true, fixed_, precision_, stream_), "direct launch");
@@ -1012,7 +1017,7 @@ class Accumulator {
   // The reference's tile shape (RadioAccumulator.inl:699-847): fused when the
   // observer grids match, else one launch per algorithm.
   void project_tiled(std::size_t count) {
-    EventPlan const ev = make_event(count, 0);
+    EventPlan const ev = make_event(count, false);
     bool const c = ev.observer_count[0] != 0, z = ev.observer_count[1] != 0;
     if (fuse_) {
       check(launch_tiled(ev, count, true, true, fixed_, precision_, stream_), "tiled launch");
@@ -1029,7 +1034,7 @@ class Accumulator {
 
   // The precision study's generic kernel, both algorithms in one launch.
   void project_study(std::size_t count) {
-    EventPlan const ev = make_event(count, 0);
+    EventPlan const ev = make_event(count, false);
     bool const c = ev.observer_count[0] != 0, z = ev.observer_count[1] != 0;
     check(launch_study(ev, count, c, z, fixed_, arithmetic_, stream_), "study launch");
     stats_.track_observer_pairs += count * (ev.observer_count[0] + ev.observer_count[1]);
@@ -1045,7 +1050,7 @@ class Accumulator {
   // With kernel timing on, both run on stream_, so that each launch's events
   // bracket that launch alone.
   void project_windowed(std::size_t count) {
-    EventPlan const ev = make_event(count, static_cast<uint64_t>(sms_));
+    EventPlan const ev = make_event(count, true);
     int per_sm = windowed_ctas_per_sm(static_cast<int>(ev.window), threads_, fixed_, precision_);
     if (per_sm <= 0) throw cuda_error("windowed radio kernel does not fit on this device");
     bool const both = !timing_ && ev.observer_count[0] != 0 && ev.observer_count[1] != 0;
@@ -1067,7 +1072,7 @@ class Accumulator {
       plan.reruns = reruns_.ptr;
       plan.handbacks = reruns_.ptr + 1;
       uint64_t ctas = static_cast<uint64_t>(per_sm) * sms_;
-      append_work(plan, ev, ctas, tail_pays(ev.chunks, ev.chunk_size, ev.observer_count[algorithm], ctas, item()));
+      append_work(plan, ev, ctas, tail_pays(ev, algorithm, ctas, item()));
       if (ctas > plan.total_items) ctas = plan.total_items;
       plan.deferred_stride = deferred_list_stride(plan);
       attach_deferred(plan, deferred_lists(algorithm, deferred_words(plan, ctas, fixed_)), ctas, fixed_);
@@ -1314,6 +1319,7 @@ class Batch {
     Precision precision = Precision::kFP64;
     int threads = 0;
     uint32_t window = 1;
+    double work = 0.;
     for (std::size_t i = 0; i < n; ++i) {
       Accumulator* e = events[i];
       if (e == nullptr) throw std::invalid_argument("null radio accumulator in batch");
@@ -1328,9 +1334,16 @@ class Batch {
       } else if (e->fixed() != fixed || e->precision() != precision) {
         throw std::invalid_argument("batched accumulators must share precision and trace mode");
       }
-      EventPlan const ev = e->event_plan(e->staged(), static_cast<uint64_t>(e->sms()));
-      window = std::max(window, ev.window);
-      active.push_back({i, ev});
+      window = std::max(window, e->window_bins());
+      work += static_cast<double>(e->observers()) * (static_cast<double>(e->staged()) + e->item());
+      active.push_back({i, EventPlan{}});
+    }
+    // of the events that share a launch, when they are more than one launch takes
+    if (active.size() > static_cast<std::size_t>(kMaxEventsPerLaunch))
+      work *= static_cast<double>(kMaxEventsPerLaunch) / static_cast<double>(active.size());
+    for (auto& a : active) {
+      Accumulator const& e = *events[a.first];
+      a.second = e.event_plan(e.staged(), active.size() > 1 ? work : 0.);
     }
     if (active.empty()) return out;
     out.fixed = fixed;
@@ -1358,7 +1371,10 @@ class Batch {
         if (members.empty()) continue;
         for (std::size_t m = 0; m < members.size(); ++m)
           out.items[active[members[m]].first] +=
-              append_work(l.plan, active[members[m]].second, ctas, m + 1 == members.size());
+              append_work(l.plan, active[members[m]].second, ctas,
+                          m + 1 == members.size() &&
+                              (m > 0 || tail_pays(active[members[m]].second, algorithm, ctas,
+                                                  events[active[members[m]].first]->item())));
         uint64_t const items = l.plan.total_items;
         if (ctas > items) ctas = items;
         l.plan.deferred_stride = deferred_list_stride(l.plan);

@@ -268,26 +268,32 @@ inline double plan_cost(uint64_t count, uint64_t per, uint64_t ctas, uint64_t ch
   return 1.1 * (rounds > even ? rounds : even);
 }
 
-// Whether a launch of `chunks` chunks ends sooner on short items.
-inline bool tail_pays(uint64_t chunks, uint64_t chunk, uint64_t per, uint64_t ctas, double item) {
-  if (chunks == 0 || per == 0 || ctas == 0) return false;
-  uint64_t const count = chunks * chunk;
-  return plan_cost(count, per, ctas, chunk, true, item) < plan_cost(count, per, ctas, chunk, false, item);
+// Whether a launch of one algorithm's items of `ev` alone ends sooner on short items.
+inline bool tail_pays(EventPlan const& ev, int algorithm, uint64_t ctas, double item) {
+  uint64_t const per = ev.observer_count[algorithm], count = static_cast<uint64_t>(ev.chunks) * ev.chunk_size;
+  if (count == 0 || per == 0 || ctas == 0) return false;
+  return plan_cost(count, per, ctas, ev.chunk_size, true, item) < plan_cost(count, per, ctas, ev.chunk_size, false, item);
+}
+
+// The least number of chunks whose deferred lists, an item for each CTA, stay small:
+// at least 16 items a CTA, or items of 262144 tracks.
+inline uint64_t fewest_chunks(uint64_t count, uint64_t per, uint64_t ctas) {
+  constexpr uint64_t kLongest = 262144;
+  uint64_t const share = (count * per + 16 * ctas - 1) / (16 * ctas);
+  uint64_t const longest = share > kLongest ? share : kLongest;
+  return (count + longest - 1) / longest;
 }
 
 // Tracks per work item for `count` tracks at `per` observers of one algorithm's
 // launch on `ctas` persistent CTAs: of the plans that fill 1, 2, .. rounds, with or
-// without a tail, the one of least cost.  Long launches keep at least 16 items a
-// CTA, or items of 262144 tracks: the per-CTA deferred lists hold an item each.
+// without a tail, the one of least cost.
 // (The former rule took at most 64 chunks and no tail below four rounds: 9.5e6
 // tracks at 1 / 5 antennas, 6e6 at 8, CoREAS and ZHS together, FP64 1800 / 5545 / 5415
 // -> 922 / 3624 / 3479 us, mixed 828 / 2513 / 2461 -> 516 / 1706 / 1617.)
 inline uint64_t auto_chunk(uint64_t count, uint64_t per, uint64_t ctas, double item) {
-  constexpr uint64_t kLongest = 262144, kRounds = 32;
+  constexpr uint64_t kRounds = 32;
   if (count == 0 || per == 0 || ctas == 0) return kTrackTile;
-  uint64_t const share = (count * per + 16 * ctas - 1) / (16 * ctas);
-  uint64_t const longest = share > kLongest ? share : kLongest;
-  uint64_t const fewest = (count + longest - 1) / longest;
+  uint64_t const fewest = fewest_chunks(count, per, ctas);
   uint64_t best = 0;
   double least = 0.;
   auto consider = [&](uint64_t chunks) {
@@ -306,6 +312,26 @@ inline uint64_t auto_chunk(uint64_t count, uint64_t per, uint64_t ctas, double i
   uint64_t const first = (fewest * per + ctas - 1) / ctas;
   for (uint64_t round = first; round < first + kRounds; ++round) consider(round * ctas / per);
   return best;
+}
+
+// The same for an event of a batched launch, whose items fill the GPU together: the
+// more chunks, the more windows its `share` of the CTAs passes over (the event's
+// part of the launch's work, `total`), the fewer, the longer the launch waits for
+// its last items (half an item; a whole one or two cost up to 27%: 3 events of 20000
+// tracks at 100 antennas); the number with the least of both.  Cut for the whole GPU each, 64
+// events of 1500 tracks at 16 antennas took 1738 us in FP64, 604 in chunks of 8192
+// tracks at least, 437 so.
+inline uint64_t batch_chunk(uint64_t count, uint64_t per, uint64_t ctas, double item, double total) {
+  if (count == 0 || per == 0 || ctas == 0) return kTrackTile;
+  double const work = static_cast<double>(per) * (static_cast<double>(count) + item);
+  double const window = static_cast<double>(per) * item / (static_cast<double>(ctas) * (work / total));
+  uint64_t chunks = fewest_chunks(count, per, ctas);
+  auto cost = [&](uint64_t c) {
+    return static_cast<double>(c) * window + 0.5 * static_cast<double>(count) / static_cast<double>(c);
+  };
+  uint64_t const most = (count + kTrackTile - 1) / kTrackTile;
+  while (chunks < most && cost(chunks + 1) < cost(chunks)) ++chunks;
+  return track_capacity((count + chunks - 1) / chunks);
 }
 
 enum class Precision : int { kFP64 = 0, kMixed = 1 };

@@ -8,6 +8,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <functional>
+#include <utility>
 #include <vector>
 
 #include "radio_kernels.cuh"
@@ -156,7 +157,9 @@ void check_auto_chunk(uint64_t ctas) {
         expect(chunk <= track_capacity(longest), "a chunk the deferred lists allow", chunk, longest);
         uint64_t const chunks = (count + chunk - 1) / chunk;
         double const length =
-            planned_length(count, per, ctas, chunk, tail_pays(chunks, chunk, per, ctas, item), item);
+            planned_length(count, per, ctas, chunk,
+                                             tail_pays(event(static_cast<uint32_t>(chunk), static_cast<uint32_t>(chunks),
+                                                             static_cast<uint32_t>(per)), 0, ctas, item), item);
         double shortest = 1e300;
         for (uint64_t c = (count + longest - 1) / longest; c <= 600; c += c < 200 ? 1 : 10) {
           uint64_t const other = track_capacity((count + c - 1) / c);
@@ -172,9 +175,35 @@ void check_auto_chunk(uint64_t ctas) {
       }
 }
 
+// Events of a batched launch, cut for their share of the GPU: the items' windows add
+// at most a third to the work that one item an antenna would be, or an item's
+// length a CTA in all where few events share the launch, and no chunk passes what
+// the whole launch's lists are sized for.
+void check_batch(std::vector<std::pair<uint64_t, uint64_t>> const& events, double item, uint64_t ctas) {
+  double work = 0., planned = 0.;
+  for (auto const& e : events) work += static_cast<double>(e.second) * (static_cast<double>(e.first) + item);
+  for (auto const& e : events) {
+    uint64_t const chunk = batch_chunk(e.first, e.second, ctas, item, work);
+    uint64_t const share = (e.first * e.second + 16 * ctas - 1) / (16 * ctas);
+    expect(chunk <= track_capacity(share > 262144 ? share : 262144), "a batched chunk the lists allow", chunk);
+    planned += static_cast<double>((e.first + chunk - 1) / chunk * e.second) * item +
+               static_cast<double>(e.first * e.second);
+  }
+  expect(planned <= 4. / 3. * work + static_cast<double>(8 * ctas) * item, "windows of a batched launch",
+         static_cast<uint64_t>(planned), static_cast<uint64_t>(work));
+}
+
 }  // namespace
 
 int main() {
+  for (double item : {item_cost(900, true, 1), item_cost(8192, false, 1)}) {
+    check_batch(std::vector<std::pair<uint64_t, uint64_t>>(64, {1500, 16}), item, 148);
+    check_batch(std::vector<std::pair<uint64_t, uint64_t>>(64, {300, 16}), item, 148);
+    check_batch(std::vector<std::pair<uint64_t, uint64_t>>(32, {5000, 40}), item, 148);
+    check_batch(std::vector<std::pair<uint64_t, uint64_t>>(16, {1000000, 160}), item, 148);
+    check_batch({{5000000, 160}, {1000, 16}, {20000, 300}, {300, 5}}, item, 148);
+    check_batch({{100000, 16}}, item, 148);
+  }
   check_auto_chunk(148);
   // the 1e7 x 160 workload's ZHS launch, a served round, a batched launch of
   // several events, small launches, and one past the two-pass cap
