@@ -294,8 +294,12 @@ __host__ __device__ __forceinline__ void divide3(double& x, double& y, double& z
 // point: the reference's (1 + (I_src - I_dst) / height) * dist / c with the
 // parenthesised factor taken from `st` (the same IEEE value), or n dist / c.
 // kTime = false skips the refractive index and travel time (the Fraunhofer
-// midpoint uses only k and distance).
-template <bool kTime>
+// midpoint uses only k and distance).  kDivide takes the four quotients by
+// divisions: the plain shapes, which wait for their atomics and not for the FP64
+// pipe, lose more to the written-out form's range checks and registers than they
+// save (3e5 x 160, direct shape, written-out / divisions: FP64 25.6 / 23.8 ms, mixed
+// 24.8 / 23.2, floating 16.6 / 15.7; the windowed FP64 CoREAS kernel 4.6 / 5.0 at 1e6).
+template <bool kTime, bool kDivide = false>
 __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCache const& o,
                                                double sx, double sy, double sz) {
   Path r;
@@ -304,10 +308,16 @@ __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCa
   r.kx = dx;
   r.ky = dy;
   r.kz = dz;
-  divide3(r.kx, r.ky, r.kz, dist);
+  if (kDivide) {
+    r.kx = dx / dist;
+    r.ky = dy / dist;
+    r.kz = dz / dist;
+  } else {
+    divide3(r.kx, r.ky, r.kz, dist);
+  }
   r.dist = dist;
   if (!kTime) return r;
-  r.time = over_light_speed(st.factor * dist);
+  r.time = kDivide ? st.factor * dist / kSpeedOfLight : over_light_speed(st.factor * dist);
   r.n_src = st.n_src;
   r.n_dst = st.n_dst;
   return r;
@@ -315,11 +325,11 @@ __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCa
 
 // propagate, RadioProjection.inl:170-238: the source terms looked up in the
 // table for this observer, then the path.
-template <bool kTime>
+template <bool kTime, bool kDivide = false>
 __device__ __forceinline__ Path propagate(Propagation const& p, ObserverCache const& o,
                                           double sx, double sy, double sz) {
   SourceTerms const st = kTime ? source_terms(p, destination_of(o), sz) : SourceTerms{0., 0., 0.};
-  return propagate_with<kTime>(st, o, sx, sy, sz);
+  return propagate_with<kTime, kDivide>(st, o, sx, sy, sz);
 }
 
 // ---------------------------------------------------------------- filtered paths

@@ -317,7 +317,7 @@ __device__ __forceinline__ void deposit_bin(Sink& sink, uint64_t bin, Deposit<Am
 // midpoint field over the Doppler-compressed duration.  Kept out of line: it
 // is taken by a minority of pairs, and its third propagation would otherwise
 // grow the hot loop's instruction footprint.  Returns the counts it adds.
-template <bool kFixed, class Amp, bool kPre, class Sink>
+template <bool kFixed, class Amp, bool kPre, bool kDivide = false, class Sink>
 __device__ __noinline__ Counts coreas_near_cone(Track const t, Propagation const& p,
                                                 ObserverCache const& o, Sink sink,
                                                 bool start_before_end, SourceTerms const pre_mid) {
@@ -326,7 +326,8 @@ __device__ __noinline__ Counts coreas_near_cone(Track const t, Propagation const
   double const cf = t.constant * o.sample_rate;
   double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
   double const mt = (t.ts + t.te) * 0.5;
-  Path const pm = kPre ? propagate_with<true>(pre_mid, o, mx, my, mz) : propagate<true>(p, o, mx, my, mz);
+  Path const pm =
+      kPre ? propagate_with<true, kDivide>(pre_mid, o, mx, my, mz) : propagate<true, kDivide>(p, o, mx, my, mz);
   double const mr = mt + pm.time;
   double const md = doppler(pm.n_src, t.bx, t.by, t.bz, pm.kx, pm.ky, pm.kz);
   Vec3<Amp> const k{static_cast<Amp>(pm.kx), static_cast<Amp>(pm.ky), static_cast<Amp>(pm.kz)};
@@ -362,12 +363,15 @@ __device__ __noinline__ Counts coreas_near_cone(Track const t, Propagation const
 // path) every amplitude evaluated exactly as the reference.
 // kPre: the start, end and midpoint source terms are `terms` (precomputed at
 // ingest for the event's shared destination row), else looked up.
-template <bool kFixed, class Amp, class Sink, bool kPre = false>
+// kDivide: see propagate_with (the plain shapes).
+template <bool kFixed, class Amp, class Sink, bool kPre = false, bool kDivide = false>
 __device__ __forceinline__ void coreas_pair(Track const& t, Propagation const& p,
                                             ObserverCache const& o, Sink& sink, Counts& c,
                                             SourceTerms const* terms = nullptr) {
-  Path const ps = kPre ? propagate_with<true>(terms[0], o, t.sx, t.sy, t.sz) : propagate<true>(p, o, t.sx, t.sy, t.sz);
-  Path const pe = kPre ? propagate_with<true>(terms[1], o, t.ex, t.ey, t.ez) : propagate<true>(p, o, t.ex, t.ey, t.ez);
+  Path const ps = kPre ? propagate_with<true, kDivide>(terms[0], o, t.sx, t.sy, t.sz)
+                       : propagate<true, kDivide>(p, o, t.sx, t.sy, t.sz);
+  Path const pe = kPre ? propagate_with<true, kDivide>(terms[1], o, t.ex, t.ey, t.ez)
+                       : propagate<true, kDivide>(p, o, t.ex, t.ey, t.ez);
   double const pre = doppler(ps.n_src, t.bx, t.by, t.bz, ps.kx, ps.ky, ps.kz);
   double const post = doppler(pe.n_src, t.bx, t.by, t.bz, pe.kx, pe.ky, pe.kz);
   double sr = t.ts + ps.time;
@@ -376,7 +380,7 @@ __device__ __forceinline__ void coreas_pair(Track const& t, Propagation const& p
   Vec3<Amp> const beta{static_cast<Amp>(t.bx), static_cast<Amp>(t.by), static_cast<Amp>(t.bz)};
 
   if (ps.n_dst > 1. && (fabs(pre) < kCoreasThreshold || fabs(post) < kCoreasThreshold)) {
-    Counts const d = coreas_near_cone<kFixed, Amp, kPre>(t, p, o, sink, sr < er, kPre ? terms[2] : SourceTerms{});
+    Counts const d = coreas_near_cone<kFixed, Amp, kPre, kDivide>(t, p, o, sink, sr < er, kPre ? terms[2] : SourceTerms{});
     c.coreas += d.coreas;
     c.overflows += d.overflows;
     c.mag += d.mag;
@@ -738,14 +742,14 @@ __device__ __noinline__ Counts zhs_multi_tail(ObserverCache const& o, Sink sink,
 // (the reference-shaped direct kernel), each index is binned by the
 // reference's own expression.
 //
-template <bool kFixed, bool kRuns, class Amp, class Sink>
+template <bool kFixed, bool kRuns, class Amp, bool kDivide = false, class Sink>
 __device__ __forceinline__ void zhs_segment(double p1x, double p1y, double p1z, double p2x,
                                             double p2y, double p2z, double t1, double t2,
                                             Track const& t, Propagation const& p,
                                             ObserverCache const& o, Sink& sink, Counts& c,
                                             bool subdivided) {
   double const mx = (p1x + p2x) * 0.5, my = (p1y + p2y) * 0.5, mz = (p1z + p2z) * 0.5;
-  Path const path = propagate<true>(p, o, mx, my, mz);
+  Path const path = propagate<true, kDivide>(p, o, mx, my, mz);
   double const bk = t.bx * path.kx + t.by * path.ky + t.bz * path.kz;
   double const nbk = path.n_src * bk;
   double const mt = (t1 + t2) * 0.5;
@@ -1341,10 +1345,11 @@ struct Subdivision {
   double divisor;
   int subtracks;
 };
+template <bool kDivide = false>
 __device__ __forceinline__ Subdivision subdivide(Track t, Propagation const& p, ObserverCache const& o) {
   derive_track(t);
   double const mx = (t.sx + t.ex) * 0.5, my = (t.sy + t.ey) * 0.5, mz = (t.sz + t.ez) * 0.5;
-  Path const pm = propagate<false>(p, o, mx, my, mz);
+  Path const pm = propagate<false, kDivide>(p, o, mx, my, mz);
   double const uk = (t.bx * pm.kx + t.by * pm.ky + t.bz * pm.kz) / t.beta_module;
   double const s2 = 1. - uk * uk;
   double const fraunhofer = s2 * t.length * t.length / pm.dist / o.wavelength * 2. * kPi;
@@ -1370,14 +1375,15 @@ __device__ __forceinline__ bool surely_one_segment(Track const& t, ObserverCache
          (fma(-w, w, square) * factor < 1. - 0x1p-20);
 }
 
-// accumulate_zhs, RadioProjection.inl:483-529, every decision exact.
-template <bool kFixed, bool kRuns, class Amp, class Sink>
+// accumulate_zhs, RadioProjection.inl:483-529, every decision exact (the plain
+// shapes: kDivide, see propagate_with).
+template <bool kFixed, class Amp, class Sink>
 __device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
                                          ObserverCache const& o, Sink& sink, Counts& c) {
   double divisor = 1.;
   int subtracks = 1;
   if (!surely_one_segment(t, o)) {
-    Subdivision const d = subdivide(t, p, o);
+    Subdivision const d = subdivide<true>(t, p, o);
     divisor = d.divisor;
     subtracks = d.subtracks;
   }
@@ -1405,8 +1411,7 @@ __device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
 #pragma unroll 1
   for (long long index = 0; index < segments; ++index) {
     double const p2x = p1x + rx, p2y = p1y + ry, p2z = p1z + rz, t2 = t1 + rt;
-    zhs_segment<kFixed, kRuns, Amp>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, sink, c,
-                                           subdivided);
+    zhs_segment<kFixed, false, Amp, true>(p1x, p1y, p1z, p2x, p2y, p2z, t1, t2, t, p, o, sink, c, subdivided);
     p1x = p2x;
     p1y = p2y;
     p1z = p2z;
@@ -1789,7 +1794,7 @@ __global__ void __launch_bounds__(256) direct_kernel(const __grid_constant__ Eve
         sink.row[r] = kFixed ? ev.fixed[0] + r * ev.total_bins[0] + o.offset : nullptr;
         sink.frow[r] = kFixed ? nullptr : ev.floating[0] + r * ev.total_bins[0] + o.offset;
       }
-      coreas_pair<kFixed, Amp>(t, ev.propagation, o, sink, c);
+      coreas_pair<kFixed, Amp, GlobalSink, false, true>(t, ev.propagation, o, sink, c);
     }
     if (kZhs && oi < ev.observer_count[1]) {
       ObserverCache const& o = ev.observers[1][oi];
@@ -1798,7 +1803,7 @@ __global__ void __launch_bounds__(256) direct_kernel(const __grid_constant__ Eve
         sink.row[r] = kFixed ? ev.fixed[1] + r * ev.total_bins[1] + o.offset : nullptr;
         sink.frow[r] = kFixed ? nullptr : ev.floating[1] + r * ev.total_bins[1] + o.offset;
       }
-      zhs_pair<kFixed, false, Amp>(t, ev.propagation, o, sink, c);
+      zhs_pair<kFixed, Amp>(t, ev.propagation, o, sink, c);
     }
   }
   flush_counts(c, ev.counters);
@@ -1865,7 +1870,7 @@ __global__ void __launch_bounds__(kTileThreads) tiled_kernel(const __grid_consta
           sink.row[r] = kFixed ? ev.fixed[0] + r * ev.total_bins[0] + o.offset : nullptr;
           sink.frow[r] = kFixed ? nullptr : ev.floating[0] + r * ev.total_bins[0] + o.offset;
         }
-        coreas_pair<kFixed, Amp>(t, ev.propagation, o, sink, c);
+        coreas_pair<kFixed, Amp, GlobalSink, false, true>(t, ev.propagation, o, sink, c);
       }
       if (kZhs && oi < ev.observer_count[1]) {
         ObserverCache const& o = observers[1][observer_lane];
@@ -1874,7 +1879,7 @@ __global__ void __launch_bounds__(kTileThreads) tiled_kernel(const __grid_consta
           sink.row[r] = kFixed ? ev.fixed[1] + r * ev.total_bins[1] + o.offset : nullptr;
           sink.frow[r] = kFixed ? nullptr : ev.floating[1] + r * ev.total_bins[1] + o.offset;
         }
-        zhs_pair<kFixed, false, Amp>(t, ev.propagation, o, sink, c);
+        zhs_pair<kFixed, Amp>(t, ev.propagation, o, sink, c);
       }
     }
   }
