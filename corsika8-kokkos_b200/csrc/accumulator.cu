@@ -886,14 +886,14 @@ class Accumulator {
     choose_window();
   }
 
-  // Shared-memory window: the longest trace, capped by the tuning's
-  // observer_tile_size and by what the device's shared memory holds.
+  // Shared-memory window: the longest trace, or the part of it that the tuning's
+  // observer_tile_size asks for, as far as the device's shared memory holds it.
   void choose_window() {
-    int const device_window = windowed_max_bins(device_);
-    std::size_t window = largest_bins_;
-    if (tuning_.observer_tile_size != 0) window = std::min<std::size_t>(window, tuning_.observer_tile_size);
-    window_bins_ = std::min<std::size_t>(window, static_cast<std::size_t>(device_window));
-    if (window_bins_ == 0) window_bins_ = 1;
+    int const most = windowed_max_bins(device_);
+    window_bins_ = window_for(largest_bins_, most);
+    if (tuning_.observer_tile_size != 0)
+      window_bins_ = window_for(std::min<std::size_t>({largest_bins_, static_cast<std::size_t>(most > 0 ? most : 1),
+                                                        static_cast<std::size_t>(tuning_.observer_tile_size)}), most);
   }
 
   // Source terms precomputed at ingest when every observer of both enabled

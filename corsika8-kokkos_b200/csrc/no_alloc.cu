@@ -273,8 +273,7 @@ void accumulate_no_alloc(c8r_config const& config, c8r_lepton_transport_record c
   bool const fixed = config.deterministic != 0;
   c8r::Precision const precision =
       config.precision == C8R_PRECISION_MIXED ? c8r::Precision::kMixed : c8r::Precision::kFP64;
-  uint32_t const window =
-      static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(largest, dev.max_window)));
+  uint32_t const window = c8r::window_for(largest, dev.max_window);
   int const threads = c8r::kWindowThreads;
   int const per_sm = c8r::windowed_ctas_per_sm(static_cast<int>(window), threads, fixed, precision);
   if (per_sm <= 0) throw std::runtime_error("windowed radio kernel does not fit on this device");

@@ -314,7 +314,7 @@ class Server {
       ev->bins[a] = offset;
       ev->observers[a] = static_cast<uint32_t>(caches[a].size());
     }
-    ev->window = static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(largest, max_window_)));
+    ev->window = window_for(largest, max_window_);
     std::vector<double2> table;
     if (!homogeneous) {
       table.resize(p.table_size);

@@ -193,9 +193,24 @@ void check_batch(std::vector<std::pair<uint64_t, uint64_t>> const& events, doubl
          static_cast<uint64_t>(planned), static_cast<uint64_t>(work));
 }
 
+// The window is the whole trace while it fits; of a longer one the part that leaves
+// the kernel inside the shared memory that does not cut into the L1 cache.
+void check_windows() {
+  for (int most : {1, 4096, 8277, 8362, 9000})
+    for (uint64_t longest : {1, 2, 4096, 8192, 8277, 8278, 8362, 8363, 24000, 1 << 20}) {
+      uint32_t const window = window_for(longest, most);
+      expect(window >= 1 && window <= static_cast<uint64_t>(most) && window <= longest, "window fits", window, most);
+      if (longest <= static_cast<uint64_t>(most))
+        expect(window == longest, "the whole trace", window, longest);
+      else
+        expect(24ull * window + 2048 <= 196 * 1024, "a part beside the full L1", window, longest);
+    }
+}
+
 }  // namespace
 
 int main() {
+  check_windows();
   for (double item : {item_cost(900, true, 1), item_cost(8192, false, 1)}) {
     check_batch(std::vector<std::pair<uint64_t, uint64_t>>(64, {1500, 16}), item, 148);
     check_batch(std::vector<std::pair<uint64_t, uint64_t>>(64, {300, 16}), item, 148);
