@@ -837,7 +837,7 @@ struct StagedSegment<double> {
 // counts the bins between (x just below 1/2, where x + 1/2 rounds to 1): the
 // last sample then would not be in the bin after the run, as
 // deposit_differences takes it.  The caller discards whatever `out` holds.
-template <bool kFixed, class Amp, bool kPre = false>
+template <class Amp, bool kPre = false>
 __device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, double t1, double t2, double mt,
                                           Track const& t, Propagation const& p,
                                           ObserverCache const& o, bool subdivided,
@@ -877,9 +877,7 @@ __device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, doubl
   double const frac_last = single ? (tiny ? (t2 - t1) * fs : fabs(d2 * fs - d1 * fs))
                                   : fabs(x2 + 0.5 - eb);
   double const den_last = single && tiny ? path.dist : dd;
-  // FP32 values are staged in fixed-point units
-  Amp const unit = kFixed && sizeof(Amp) == sizeof(float) ? static_cast<Amp>(o.fixed_scale_f) : static_cast<Amp>(1);
-  out.last = amp_div(static_cast<Amp>(sc * frac_last), static_cast<Amp>(den_last)) * unit;
+  out.last = amp_div(static_cast<Amp>(sc * frac_last), static_cast<Amp>(den_last));
   out.flags = 0u;
   out.start = 0u;
   out.count = 0u;
@@ -893,9 +891,9 @@ __device__ __forceinline__ bool zhs_stage(double mx, double my, double mz, doubl
   }
   if (single) return true;
   double const frac_first = fabs(sb + 0.5 - x1);
-  out.first = amp_div(static_cast<Amp>(sc * frac_first), static_cast<Amp>(dd)) * unit;
+  out.first = amp_div(static_cast<Amp>(sc * frac_first), static_cast<Amp>(dd));
   double const mc = (subdivided ? 1. : sign) * t.constant;
-  out.mid = amp_div(static_cast<Amp>(mc), static_cast<Amp>(dd)) * unit;
+  out.mid = amp_div(static_cast<Amp>(mc), static_cast<Amp>(dd));
   // first sample, add_sample(detection_time1): bin nearest(x1)
   double const bv1 = nearest_bin(x1);
   if (bv1 != sb) return false;
@@ -941,10 +939,11 @@ __device__ __forceinline__ bool surely_undivided(LeanPoint const& m, LeanObserve
 // duration in bins, `constant` the charge constant in the observer's units.
 // Its detection times are m.x -+ |half_bins (1 - n w)|, in time order, and the
 // potential's sign times 1 / (1 - n w) is 1 / |1 - n w|.  False when a guard
-// cannot decide (the caller evaluates the segment exactly).
+// cannot decide (the caller evaluates the segment exactly).  `cut`: an end of the
+// trace cuts the segment.
 __device__ __forceinline__ bool zhs_lean(LeanPoint const& m, double half_bins, float constant, double bx, double by,
                                          double bz, LeanObserver const& l, bool subdivided,
-                                         StagedSegment<float>& out) {
+                                         StagedSegment<float>& out, bool& cut) {
   double const reach = fabs(half_bins * m.factor);
   double const x1 = m.x - reach, x2 = m.x + reach;
   out.flags = 0u;
@@ -955,7 +954,9 @@ __device__ __forceinline__ bool zhs_lean(LeanPoint const& m, double half_bins, f
   double const r1 = lean_nearest(x1, b1), r2 = lean_nearest(x2, b2);
   bool const decided = (fabs(r1) < 0.5 - kBinGuard) & (fabs(r2) < 0.5 - kBinGuard) & (reach > kBinGuard) &
                        (fabs(m.factor) >= 1.e-6);
+  cut = false;
   if ((x2 < -1.) | (x1 > l.past)) return m.ok;  // off the trace
+  cut = (static_cast<unsigned>(b1) >= l.bins) | (static_cast<unsigned>(b2) >= l.bins);
   // from here |x1|, |x2| < 2^27: reach is below 2^25 and one of them is near the trace
   float const amplitude = __fdividef(constant, static_cast<float>(fabs(m.factor) * m.dist));
   out.perp = Vec3<float>{static_cast<float>(fma(-m.dx, m.along, bx)), static_cast<float>(fma(-m.dy, m.along, by)),
@@ -1473,7 +1474,10 @@ __device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propag
   ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
   bool staged = z.one;
   if constexpr (sizeof(Amp) == sizeof(float)) {
-    staged = zhs_lean(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, false, seg) & staged;
+    // a cut segment is the drain's, as in zhs_lean_differences: a sample's FP32 value
+    // is then the same bits whether its item runs with checked adds or without
+    bool cut;
+    staged = zhs_lean(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, false, seg, cut) & staged & !cut;
   } else if (staged) {
     double2 const cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T), ct = __ldg(r + 3 * T);
     Track t;
@@ -1481,7 +1485,7 @@ __device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propag
     t.by = z.by;
     t.bz = z.bz;
     t.constant = __ldg(r + kConst / 2 * T).y;
-    staged = zhs_stage<kFixed, Amp, true>(cm.x, cm.y, cn.x, ct.x, ct.x + (ct.y - ct.x), cn.y, t, p,
+    staged = zhs_stage<Amp, true>(cm.x, cm.y, cn.x, ct.x, ct.x + (ct.y - ct.x), cn.y, t, p,
                                           copy_words(s_observer), false, seg, z.terms);
   }
   if (!staged) {
@@ -1954,11 +1958,6 @@ __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t
   return lo;
 }
 
-__device__ __noinline__ Subdivision subdivide_row(const double* __restrict__ tracks, uint64_t row,
-                                                  Propagation const& p, ObserverCache const& o) {
-  return subdivide(load_track(tracks, row), p, o);
-}
-
 // The step of a divided track's sequential additions (RadioProjection.inl:505-512).
 struct Steps {
   double x, y, z, t;
@@ -1981,11 +1980,12 @@ __device__ __forceinline__ Steps subtrack_steps(Track const& t, double divisor, 
   return r;
 }
 
-// Segments [from, to) of a divided track evaluated exactly, sample by sample, by
-// one lane: what the filtered drain leaves undecided.
+// Segments from, from + stride, .. of a divided track (`from` alone for a stride of 0)
+// evaluated exactly and deposited sample by sample, as zhs_drain does: what the
+// filtered drain leaves undecided.
 template <class Amp>
-__device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tracks, uint64_t row, long long from,
-                                                  long long to, Propagation const& p, ObserverCache const& o,
+__device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tracks, uint64_t row, unsigned from,
+                                                  unsigned stride, Propagation const& p, ObserverCache const& o,
                                                   DifferenceSink sink) {
   Counts c;
   Track const t = load_track(tracks, row);
@@ -1994,10 +1994,16 @@ __device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tra
   Steps const r = subtrack_steps(t, d.divisor, refinement);
   bool const subdivided = d.subtracks > 1 || refinement > 1;
   double x = t.sx, y = t.sy, z = t.sz, time = t.ts;
+  long long const segments = static_cast<long long>(d.subtracks) * refinement;
+  long long const stop = stride != 0u || segments <= from ? segments : static_cast<long long>(from) + 1;
+  long long due = from;
 #pragma unroll 1
-  for (long long s = 0; s < to; ++s) {
+  for (long long s = 0; s < stop; ++s) {
     double const nx = x + r.x, ny = y + r.y, nz = z + r.z, next = time + r.t;
-    if (s >= from) zhs_segment<true, true, Amp>(x, y, z, nx, ny, nz, time, next, t, p, o, sink, c, subdivided);
+    if (s == due) {
+      due += stride;
+      zhs_segment<true, true, Amp>(x, y, z, nx, ny, nz, time, next, t, p, o, sink, c, subdivided);
+    }
     x = nx;
     y = ny;
     z = nz;
@@ -2006,20 +2012,18 @@ __device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tra
   return c;
 }
 
-// Deferred ZHS pairs in mixed precision and fixed point, the whole trace in the
-// window: the warp's pairs (a lane each, below `count`) are divided exactly,
-// then their segments are dealt out to the lanes in turn -- lane j of a step
-// takes segment base + j of the flattened list, its owner found by shuffles --
-// and each lane evaluates and deposits its segment on its own by the filtered
-// arithmetic, at start + (index + 1/2) (end - start) / divisor.  That is within
-// s 2u of the coordinates' and times' magnitudes of the reference's s sequential
-// additions: with those below 2^24 bins (regular_track) and s <= 64, below 2^-20
-// bins, inside kBinGuard.  Longer divisions, irregular tracks and segments that
-// a guard cannot decide are evaluated exactly.  Little is held per lane (a row,
-// an index, one FP64 number), so the function fits the registers of the track
-// loop's kernel: the pair-per-lane drain it replaces there spilled 1700 words a
-// pair at 64 registers.
-constexpr long long kLeanSegments = 64;
+// Whether a track's `segments` may be evaluated by lean_segment below, which takes a
+// segment's middle at start + (index + 1/2) (end - start) / divisor where the
+// reference adds up s segments.  With u = 2^-53, the two differ by less than (s + 4) u
+// of the largest coordinate and of the largest time, so the detection time by (s + 4) u
+// (4 sqrt(3) |coordinate| fs / c + |time| fs), which has to stay below 2^-20 bins, a part
+// of kBinGuard (s up to 60 at the filtered paths' limits, 300 in a shower of 100 km).
+__device__ __forceinline__ bool lean_divisible(Track const& t, double pack, long long segments, LeanObserver const& l) {
+  double const furthest = fmax(fmax(fmax(fabs(t.sx), fabs(t.sy)), fmax(fabs(t.sz), fabs(t.ex))),
+                               fmax(fabs(t.ey), fabs(t.ez)));
+  double const bins = 7. * furthest * l.rate_over_c + fmax(fabs(t.ts), fabs(t.te)) * l.rate;
+  return (static_cast<double>(segments + 4) * bins <= 0x1p33) & ((pack_flags(pack) & kTrackRegular & l.usable) != 0u);
+}
 // Whether the source terms at height z decide what the terms at the reference's
 // own height, within `z_error` m of z, would.  In the table they are the same when
 // no row lies within kBinGuard bins.  Past its ends (out of line: rare) they are
@@ -2049,6 +2053,56 @@ __device__ __forceinline__ bool terms_decided(Propagation const& p, LeanObserver
   if ((height > 0.) & (height + 0.5 < static_cast<double>(p.table_size - 1))) return true;
   return terms_decided_past_table(p, height, factor, z_error, path_bins, half_bins);
 }
+// A deferred track's division seen from the item's observer, out of line.  Refined
+// tracks are all deferred, most of them undivided but for that: their Fraunhofer
+// number is surely below 1.
+struct Division {
+  double divisor;
+  int subtracks;
+  bool lean;  // lean_divisible
+};
+__device__ __noinline__ Division divide_row(const double* __restrict__ tracks, uint64_t row, Propagation const& p) {
+  int const refinement = static_cast<int>(p.refinement);
+  Track const t = load_track(tracks, row);
+  Subdivision d{1., 1};
+  if (refinement == 1 || !surely_one_segment(t, s_observer)) d = subdivide(t, p, s_observer);
+  double const pack = __ldg(track_ref(tracks, row) + kPack / 2 * kTrackTile).y;
+  return {d.divisor, d.subtracks, lean_divisible(t, pack, static_cast<long long>(d.subtracks) * refinement, s_lean)};
+}
+
+// Segment `index` of a divided track (lean_divisible) by the filtered arithmetic,
+// staged.  Both drains evaluate a segment by this function first.  False when a
+// guard cannot decide.
+__device__ __forceinline__ bool lean_segment(double2 const* __restrict__ r, unsigned index, bool subdivided,
+                                             double fraction, Propagation const& p, LeanObserver const& l,
+                                             StagedSegment<float>& seg) {
+  constexpr unsigned T = kTrackTile;
+  double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T);
+  double2 const cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
+  double const at = (static_cast<double>(index) + 0.5) * fraction;
+  double const z = fma(cc.y - cb.x, at, cb.x), duration = ct.y - ct.x;
+  double const half_bins = duration * fraction * l.half_rate;
+  SourceTerms const st = source_terms(p, destination_of(s_observer), z);
+  LeanPoint const m = lean_point(l, fma(cb.y - ca.x, at, ca.x), fma(cc.x - ca.y, at, ca.y), z,
+                                 fma(duration, at, ct.x), cd.x, cd.y, ce.x, st.factor, st.n_src);
+  bool cut;
+  return zhs_lean(m, half_bins, pack_constant(ce.y) * l.scale, cd.x, cd.y, ce.x, l, subdivided, seg, cut) &
+         lean_terms(st) & (m.dist * l.rate_over_c >= 4. * half_bins) &
+         terms_decided(p, l, st.factor, z, 0x1p-46 * (fabs(cb.x) + fabs(cc.y)), m.dist * l.rate_over_c, half_bins);
+}
+
+// Deferred ZHS pairs in mixed precision and fixed point, the whole trace in the
+// window: the warp's pairs (a lane each, below `count`) are divided exactly,
+// then their segments are dealt out to the lanes in turn -- lane j of a step
+// takes segment base + j of the flattened list, its owner found by shuffles --
+// and each lane evaluates and deposits its segment on its own by lean_segment.
+// Longer divisions, irregular tracks and segments that a guard cannot decide are
+// evaluated exactly, the tracks by the whole warp, every 32nd segment a lane (each lane adds up the
+// points in between: 128 additions where a segment is 900 operations; by its own lane
+// alone 262144 tracks x 24 antennas refined 64 fold took 41.6 ms in 8192 bins).
+// Little is held per lane (a row, an index, one FP64 number), so the function fits
+// the registers of the track loop's kernel: the pair-per-lane drain it replaces there
+// spilled 1700 words a pair at 64 registers.
 __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks, uint64_t begin, unsigned const* list,
                                               unsigned count, Propagation const& p, unsigned long long* win,
                                               uint32_t width) {
@@ -2058,25 +2112,18 @@ __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks,
   uint64_t row = 0;
   double fraction = 1.;
   unsigned mine = 0;
+  bool exact = false;
   if (lane < count) {
     row = begin + list[lane];
     int const refinement = static_cast<int>(p.refinement);
-    // refined tracks all come here, most of them undivided but for that: their
-    // Fraunhofer number is surely below 1
-    Subdivision d{1., 1};
-    if (refinement == 1 || !zhs_point<false, false>(track_ref(tracks, row), p, copy_words(s_lean)).one)
-      d = subdivide_row(tracks, row, p, s_observer);
+    Division const d = divide_row(tracks, row, p);
     // both products as the reference forms them (RadioProjection.inl:503, :527)
     rare.subtracks = static_cast<unsigned long long>(static_cast<long long>(d.subtracks));
     if (refinement > 1)
       rare.subtracks += static_cast<unsigned long long>(static_cast<long long>(d.subtracks * (refinement - 1)));
-    long long const segments = static_cast<long long>(d.subtracks) * refinement;
     fraction = 1. / (d.divisor * static_cast<double>(refinement));
-    unsigned const flags = pack_flags(__ldg(track_ref(tracks, row) + kPack / 2 * kTrackTile).y);
-    if (segments > kLeanSegments || !(flags & kTrackRegular & s_lean.usable))
-      add_counts(rare, zhs_exact_segments<float>(tracks, row, 0, segments, p, s_observer, DifferenceSink{win, width}));
-    else if (segments > 0)
-      mine = static_cast<unsigned>(segments);
+    exact = !d.lean;
+    if (d.lean && d.subtracks > 0) mine = static_cast<unsigned>(d.subtracks * refinement);
   }
   unsigned incl = mine;
 #pragma unroll
@@ -2101,28 +2148,18 @@ __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks,
     bool deposited = true;
     if (j < total) {
       LeanObserver const l = copy_words(s_lean);
-      double2 const* r = track_ref(tracks, its_row);
-      constexpr unsigned T = kTrackTile;
-      double2 const ca = __ldg(r), cb = __ldg(r + T), cc = __ldg(r + 2 * T), ct = __ldg(r + 3 * T);
-      double2 const cd = __ldg(r + 4 * T), ce = __ldg(r + 5 * T);
-      double const at = (static_cast<double>(index) + 0.5) * its_fraction;
-      double const z = fma(cc.y - cb.x, at, cb.x), duration = ct.y - ct.x;
-      double const half_bins = duration * its_fraction * l.half_rate;
-      SourceTerms const st = source_terms(p, destination_of(s_observer), z);
-      LeanPoint const m = lean_point(l, fma(cb.y - ca.x, at, ca.x), fma(cc.x - ca.y, at, ca.y), z,
-                                     fma(duration, at, ct.x), cd.x, cd.y, ce.x, st.factor, st.n_src);
       StagedSegment<float> seg;
-      deposited = zhs_lean(m, half_bins, pack_constant(ce.y) * l.scale, cd.x, cd.y, ce.x, l, subdivided, seg) &
-                  lean_terms(st) & (m.dist * l.rate_over_c >= 4. * half_bins) &
-                  terms_decided(p, l, st.factor, z, 0x1p-46 * (fabs(cb.x) + fabs(cc.y)), m.dist * l.rate_over_c,
-                                half_bins);
-      deposited = deposited && account_staged(seg, l, c);
+      deposited = lean_segment(track_ref(tracks, its_row), index, subdivided, its_fraction, p, l, seg) &&
+                  account_staged(seg, l, c);
       if (deposited) deposit_differences(seg, l, win, width);
     }
     if (__any_sync(0xffffffffu, !deposited) && !deposited)
-      add_counts(rare, zhs_exact_segments<float>(tracks, its_row, index, static_cast<long long>(index) + 1, p,
-                                                 s_observer, DifferenceSink{win, width}));
+      add_counts(rare, zhs_exact_segments<float>(tracks, its_row, index, 0u, p, s_observer,
+                                                 DifferenceSink{win, width}));
   }
+  for (unsigned left = __ballot_sync(0xffffffffu, exact); left != 0u; left &= left - 1u)
+    add_counts(rare, zhs_exact_segments<float>(tracks, __shfl_sync(0xffffffffu, row, __ffs(static_cast<int>(left)) - 1),
+                                               lane, 32u, p, s_observer, DifferenceSink{win, width}));
   add_counts(rare, counts_of(c));
   return rare;
 }
@@ -2132,10 +2169,11 @@ __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks,
 // one deferred pair each and evaluate its Fraunhofer number and subdivision
 // exactly; the warp then steps through segment index s = 0, 1, ...: every lane
 // whose pair has a segment s forms its endpoints by the reference's
-// sequential additions, stages it (mixed precision: by the filtered arithmetic
-// first, exactly where a guard cannot decide), and the warp deposits the staged
-// samples together.  A segment that needs the per-index binning deposits on
-// its own lane.  Every lane of the warp calls it.
+// sequential additions, stages it (FP64: exactly; mixed precision: by lean_segment),
+// and the warp deposits the staged samples together.  A segment that cannot be
+// staged is evaluated exactly and deposited on its own lane: in mixed precision the
+// same steps as zhs_drain_lean's, so that a pair's FP32 values are the same bits
+// whether its item runs with checked adds or without.  Every lane of the warp calls it.
 template <bool kFixed, bool kDifferences, class Amp, class Sink>
 __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint64_t begin,
                                          unsigned const* list, unsigned count,
@@ -2147,6 +2185,8 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
   long long segments = 0;
   bool subdivided = false;
   double p1x = 0., p1y = 0., p1z = 0., t1 = 0., rx = 0., ry = 0., rz = 0., rt = 0.;
+  double fraction = 1.;  // mixed precision: of the track, a segment
+  bool lean = false;     // and whether lean_segment may evaluate it
   if (lane < count) {
     row = begin + list[lane];
     Track const t = load_track(tracks, row);
@@ -2162,6 +2202,10 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
     rz = step.z;
     rt = step.t;
     segments = static_cast<long long>(d.subtracks) * refinement;
+    if constexpr (sizeof(Amp) == sizeof(float)) {
+      fraction = 1. / (d.divisor * static_cast<double>(refinement));
+      lean = lean_divisible(t, __ldg(track_ref(tracks, row) + kPack / 2 * kTrackTile).y, segments, l);
+    }
     p1x = t.sx;
     p1y = t.sy;
     p1z = t.sz;
@@ -2179,22 +2223,17 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
       asm volatile("" : "+l"(r));
       double2 const e = __ldg(r + 4 * kTrackTile), f = __ldg(r + 5 * kTrackTile);
       double const p2x = p1x + rx, p2y = p1y + ry, p2z = p1z + rz, t2 = t1 + rt;
-      double const mx = (p1x + p2x) * 0.5, my = (p1y + p2y) * 0.5, mz = (p1z + p2z) * 0.5, mt = (t1 + t2) * 0.5;
-      bool staged = false;
-      if constexpr (sizeof(Amp) == sizeof(float)) {
-        SourceTerms const st = source_terms(p, destination_of(o), mz);
-        LeanPoint const m = lean_point(l, mx, my, mz, mt, e.x, e.y, f.x, st.factor, st.n_src);
-        staged = zhs_lean(m, (t2 - t1) * l.half_rate, pack_constant(f.y) * l.scale, e.x, e.y, f.x, l, subdivided, seg) &
-                 ((pack_flags(f.y) & kTrackRegular & l.usable) != 0u) & lean_terms(st);
-      }
       Track t;
       t.bx = e.x;
       t.by = e.y;
       t.bz = f.x;
-      if (!staged) {
-        t.constant = __ldg(r + kConst / 2 * kTrackTile).y;
-        staged = zhs_stage<kFixed, Amp>(mx, my, mz, t1, t2, mt, t, p, o, subdivided, seg);
-      }
+      t.constant = __ldg(r + kConst / 2 * kTrackTile).y;
+      bool staged;
+      if constexpr (sizeof(Amp) == sizeof(float))
+        staged = lean && lean_segment(r, static_cast<unsigned>(s), subdivided, fraction, p, l, seg);
+      else
+        staged = zhs_stage<Amp>((p1x + p2x) * 0.5, (p1y + p2y) * 0.5, (p1z + p2z) * 0.5, t1, t2,
+                                        (t1 + t2) * 0.5, t, p, o, subdivided, seg);
       if (!staged) {
         seg.count = 0u;
         seg.flags = 0u;

@@ -125,6 +125,37 @@ def test_divided_tracks_above_the_table_beside_the_antenna_height(pkg, oracle, s
     check(pkg, oracle, showers, wl, showers.to_records(seg))
 
 
+@pytest.mark.parametrize("name,refinement,shift", [("ice_c2", 1, 0.0), ("ice_c2", 3, 0.0), ("plain_c0", 1, 52e-9), ("plain_c0", 2, 0.0)])
+@pytest.mark.parametrize("precision", [0, 1])
+def test_items_run_again_give_the_same_bits(pkg, oracle, showers, name, refinement, shift, precision):
+    """A sample's fixed-point value does not depend on the way its item went: one
+    item an antenna near the fixed-point limit, run again with checked adds,
+    against items so small that none is (which items are depends on the order that
+    the ingest's atomics leave the tracks in, so else the traces would too)."""
+    import torch
+
+    wl, gen, _ = showers.workload_config(name, bins=1001)
+    records = (showers.ice_records if gen.get("ice") else showers.shower_records)(6_000, seed=3, **gen)
+    wl["observers"] = wl["observers"][::5].copy()
+    wl["observers"]["start_time_s"] += shift  # into the pulse: the trace's start cuts segments
+    extra = dict(zhs_subtrack_refinement=refinement)
+    floating = showers.make_config(wl, deterministic=False, **extra)
+    coreas, zhs, _ = oracle.restatement().project(floating, records, threads=16)
+    peak = max(np.abs(coreas).max(), 1e10 * np.abs(zhs).max())
+    config = showers.make_config(wl, precision=precision, kernel=2, **extra)
+    config.fixed_point_field_limit_v_per_m = 1.5 * peak
+    raw = torch.from_numpy(records.view(np.uint8).reshape(-1)).cuda()
+    got = []
+    for tracks in (8192, 32):
+        acc = pkg.RadioAccumulator(config, pkg.TuningParameters(track_tile_size=tracks))
+        acc.accumulate_lepton_tracks(raw.data_ptr(), records.size)
+        got.append(acc.download_fixed() + (acc.statistics().window_reruns,))
+        acc.close()
+    assert got[0][3] > 0
+    for k in range(2):
+        assert np.array_equal(got[0][k], got[1][k]), (k, np.count_nonzero(got[0][k] != got[1][k]))
+
+
 @pytest.mark.parametrize("scale", [1e-6, 1e3, 1e6])
 def test_times_outside_the_guards_reach(pkg, oracle, showers, scale):
     """Track times shifted until the filtered paths' bounds no longer cover them
