@@ -2428,10 +2428,10 @@ __device__ __forceinline__ bool tally_fits(uint64_t count, uint32_t width) {
   return (count / blockDim.x + 1u) * width < 0xffffffffull;
 }
 
-// Notes an item for the third pass; one thread of the CTA writes it.
+// Notes an item for the second pass (kPass 3); one thread of the CTA writes it.
 __device__ __forceinline__ void hand_back(WorkPlan const& plan, uint64_t item) {
   if (threadIdx.x != 0) return;
-  plan.item_state[atomicAdd(plan.drain_next_item, 1u)].item = item;
+  plan.item_state[atomicAdd(plan.drain_next_item, 1u)] = {item};
   if (plan.handbacks) atomicAdd(plan.handbacks, 1ull);
 }
 
@@ -2507,19 +2507,17 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
     s_deferred_list = (kPass == 3 ? plan.drain_deferred : plan.deferred) +
                       static_cast<size_t>(blockIdx.x) * plan.deferred_stride;
   Counts c;
-  for (uint64_t turn = blockIdx.x;; turn += gridDim.x) {
-    uint64_t item;
-    if constexpr (kPass == 3) {  // the handed-back items, every gridDim.x-th
-      if (turn >= *plan.drain_next_item) break;
-      item = plan.item_state[turn].item;
-      __syncthreads();
-    } else {
-      __syncthreads();
-      if (threadIdx.x == 0) item_shared = atomicAdd(plan.next_item, 1u);
-      __syncthreads();
-      item = item_shared;
-      if (item >= plan.total_items) break;
-    }
+  for (;;) {
+    // the next item: of the plan, or of those that the first pass handed back (most
+    // launches have none: the last pass then ends without a turn taken)
+    unsigned const handed = kPass == 3 ? plan.drain_next_item[0] : 0u;
+    if (kPass == 3 && handed == 0u) break;
+    __syncthreads();
+    if (threadIdx.x == 0) item_shared = atomicAdd(kPass == 3 ? plan.drain_next_item + 1 : plan.next_item, 1u);
+    __syncthreads();
+    uint64_t item = item_shared;
+    if (item >= (kPass == 3 ? handed : plan.total_items)) break;
+    if constexpr (kPass == 3) item = plan.item_state[item].item;
     EventPlan const& ev = plan.events[find_event(plan.events, plan.event_count, item)];
     constexpr int algorithm = kAlgorithm;
     uint64_t const local = item - ev.first_item;
@@ -2787,10 +2785,10 @@ cudaError_t windowed_launch(WorkPlan const& plan, int ctas, int threads, cudaStr
 }
 
 // The passes of a two-pass fixed-point ZHS launch, one after the other on
-// the stream; drain_next_item counts the items the first hands back.
+// the stream; drain_next_item counts the items handed back and those taken up.
 template <class Amp, bool kPre>
 cudaError_t windowed_two_pass(WorkPlan const& plan, int ctas, int threads, cudaStream_t stream) {
-  cudaError_t err = cudaMemsetAsync(plan.drain_next_item, 0, sizeof(unsigned), stream);
+  cudaError_t err = cudaMemsetAsync(plan.drain_next_item, 0, 2 * sizeof(unsigned), stream);
   if (err != cudaSuccess) return err;
   err = windowed_launch<true, Amp, 1, kPre, 1>(plan, ctas, threads, stream);
   if (err != cudaSuccess) return err;
@@ -2805,9 +2803,7 @@ cudaError_t windowed_dispatch_algorithm(WorkPlan const& plan, int ctas, int thre
   bool const pre = plan_precomputed(plan);
   if (plan.item_state != nullptr) {
     if constexpr (kFixed && kAlgorithm == 1) {
-      if (plan.drain_deferred == nullptr || plan.drain_next_item == nullptr ||
-          plan.deferred_capacity < plan.deferred_stride)
-        return cudaErrorInvalidValue;
+      if (plan.drain_deferred == nullptr || plan.drain_next_item == nullptr) return cudaErrorInvalidValue;
       return pre ? windowed_two_pass<Amp, true>(plan, ctas, threads, stream)
                  : windowed_two_pass<Amp, false>(plan, ctas, threads, stream);
     } else {

@@ -100,7 +100,6 @@ constexpr int kWindowThreads = 640;  // upper bound (and default) of the windowe
 // A work item that the first pass of a two-pass ZHS launch handed back.
 struct ItemState {
   uint64_t item;
-  uint64_t pad_;
 };
 
 struct WorkPlan {
@@ -122,13 +121,12 @@ struct WorkPlan {
   unsigned long long* handbacks;
   // Two-pass ZHS (fixed point), when item_state is set: the first pass projects
   // the items it can with unchecked window adds and appends the others to
-  // item_state, counted by drain_next_item; the second projects those in full,
-  // with its own lists (`drain_deferred`, deferred_stride entries a CTA).
-  // attach_deferred sets these; deferred_capacity is the stride of `deferred`.
+  // item_state, counted by drain_next_item[0]; the second takes those in turn,
+  // counted by drain_next_item[1], and projects them in full, with its own lists
+  // (`drain_deferred`, deferred_stride entries a CTA).  attach_deferred sets these.
   ItemState* item_state;
   unsigned int* drain_deferred;
   unsigned int* drain_next_item;
-  uint32_t deferred_capacity;
 };
 
 // A work item spans at most kMaxChunkTracks tracks: a deferred-list entry is
@@ -151,7 +149,7 @@ constexpr uint64_t kTwoPassMaxWords = 1ull << 30;
 
 inline uint64_t two_pass_words(WorkPlan const& plan, uint64_t ctas) {
   return 2 * ctas * plan.deferred_stride +
-         plan.total_items * (sizeof(ItemState) / sizeof(unsigned)) + 1;
+         plan.total_items * (sizeof(ItemState) / sizeof(unsigned)) + 2;
 }
 
 // ZHS launches in fixed point run in two passes when their storage fits.
@@ -161,8 +159,7 @@ inline bool two_pass(WorkPlan const& plan, uint64_t ctas, bool fixed) {
 
 // 32-bit words of deferred-list storage a launch of `plan` (deferred_stride
 // and total_items set) over `ctas` CTAs needs: its CTAs' lists, and for two
-// passes the first pass's longer lists, the second pass's lists, the items'
-// states and its work counter.
+// passes the second pass's lists, the handed-back items and their two counters.
 inline uint64_t deferred_words(WorkPlan const& plan, uint64_t ctas, bool fixed) {
   if (!two_pass(plan, ctas, fixed)) return ctas * plan.deferred_stride;
   return two_pass_words(plan, ctas);
@@ -174,7 +171,6 @@ inline void attach_deferred(WorkPlan& plan, unsigned* words, uint64_t ctas, bool
   plan.item_state = nullptr;
   plan.drain_deferred = nullptr;
   plan.drain_next_item = nullptr;
-  plan.deferred_capacity = plan.deferred_stride;
   if (!two_pass(plan, ctas, fixed)) return;
   uint64_t const first = ctas * plan.deferred_stride;
   plan.drain_deferred = words + first;

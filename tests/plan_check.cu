@@ -82,20 +82,19 @@ void check_storage(WorkPlan plan, uint64_t ctas, bool fixed) {
     expect(words == lists, "one pass: the CTAs' lists", words, lists);
     return;
   }
-  uint64_t const first = static_cast<uint64_t>(plan.deferred_capacity) * ctas;
-  expect(plan.deferred_capacity >= plan.deferred_stride, "first-pass list holds an item",
-         plan.deferred_capacity, plan.deferred_stride);
+  uint64_t const first = lists;
   expect(plan.drain_deferred == base + first, "second-pass lists follow the first pass's");
   unsigned* const states = reinterpret_cast<unsigned*>(plan.item_state);
   expect(states == base + first + lists, "item states follow the lists");
   expect(plan.drain_next_item == states + plan.total_items * (sizeof(ItemState) / sizeof(unsigned)),
-         "counter follows the states");
-  expect(static_cast<uint64_t>(plan.drain_next_item - base) + 1 == words, "storage ends at the counter",
-         static_cast<uint64_t>(plan.drain_next_item - base) + 1, words);
+         "counters follow the states");
+  expect(static_cast<uint64_t>(plan.drain_next_item - base) + 2 == words, "storage ends at the counters",
+         static_cast<uint64_t>(plan.drain_next_item - base) + 2, words);
+  expect(reinterpret_cast<uintptr_t>(plan.item_state) % alignof(ItemState) == 0, "item states aligned");
   expect(words <= kTwoPassMaxWords, "two passes within the cap", words, kTwoPassMaxWords);
   // the kernels' last indices: first-pass list of the last CTA, its last
   // entry; second-pass list likewise; the last item's state
-  expect((ctas - 1) * plan.deferred_capacity + plan.deferred_capacity - 1 < first, "first-pass index");
+  expect((ctas - 1) * plan.deferred_stride + plan.deferred_stride - 1 < first, "first-pass index");
   expect(first + (ctas - 1) * plan.deferred_stride + plan.deferred_stride - 1 < first + lists, "second-pass index");
 }
 
