@@ -233,13 +233,14 @@ inline uint64_t append_work(WorkPlan& plan, EventPlan ev, uint64_t ctas, bool fi
 
 // What an item costs beside its tracks, in tracks: the window zeroed, summed and
 // flushed, a part of it whatever the window's size; relative to the tracks' own
-// time, which is 2.2 times as long in FP64 and grows with the subtrack refinement.
+// time, which is 2.2 times as long in FP64 and grows with the subtrack refinement (of
+// ZHS, half of the tracks' time).
 // Fitted, with the two margins of plan_cost, to 2044 timed launches (1 to 300
 // antennas, 1500 to 9.5e6 tracks, windows of 900 to 8192 bins, 1 to 296 chunks with
 // and without a short tail): the plan of least cost is within 0.6% of the fastest
 // timed one in the mean, 6.8% at worst.
 inline double item_cost(uint32_t window, bool fp64, uint32_t refinement) {
-  return (2000. + 1.5 * window) * (fp64 ? 0.4 : 1.) / (refinement > 1 ? refinement : 1u);
+  return (2000. + 1.5 * window) * (fp64 ? 0.4 : 1.) * 2. / (1. + (refinement > 1 ? refinement : 1u));
 }
 
 // Length of a launch over `count` tracks at `per` observers in chunks of `chunk`
