@@ -1425,7 +1425,7 @@ __device__ __forceinline__ void zhs_pair(Track const& t, Propagation const& p,
 
 // The segment of an undivided track seen from the item's observer, from the
 // track's columns `r`, by the filtered arithmetic.  `one`: the track is surely
-// one segment (the Fraunhofer number surely below 1, no refinement) and inside
+// one segment but for refinement (the Fraunhofer number surely below 1) and inside
 // the filtered paths' bounds.
 struct ZhsPoint {
   LeanPoint m;
@@ -1434,7 +1434,7 @@ struct ZhsPoint {
   SourceTerms terms;
   bool one;
 };
-template <bool kPre, bool kMayRefine>
+template <bool kPre>
 __device__ __forceinline__ ZhsPoint zhs_point(double2 const* __restrict__ r, Propagation const& p,
                                               LeanObserver const& l) {
   constexpr unsigned T = kTrackTile;
@@ -1454,7 +1454,7 @@ __device__ __forceinline__ ZhsPoint zhs_point(double2 const* __restrict__ r, Pro
   z.m = lean_point(l, cm.x, cm.y, cn.x, cn.y, cd.x, cd.y, ce.x, z.terms.factor, z.terms.n_src);
   z.half_bins = half * l.rate;
   z.constant = pack_constant(ce.y) * l.scale;
-  z.one = ((flags & kTrackRegular & l.usable) != 0u) & (!kMayRefine || p.refinement == 1u) & z.m.ok &
+  z.one = ((flags & kTrackRegular & l.usable) != 0u) & z.m.ok &
           surely_undivided(z.m, l, z.half_bins, cd.x, cd.y, ce.x);
   if (!kPre) z.one = z.one & lean_terms(z.terms);
   return z;
@@ -1467,11 +1467,11 @@ __device__ __forceinline__ ZhsPoint zhs_point(double2 const* __restrict__ r, Pro
 // arithmetic, FP64 exactly; both decide "one segment" from the filtered
 // midpoint, which spares FP64 the exact Fraunhofer number (a square root and
 // seven divisions).
-template <bool kFixed, bool kPre, bool kMayRefine, class Amp>
+template <bool kFixed, bool kPre, class Amp>
 __device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propagation const& p,
                                            LeanObserver const& l, StagedSegment<Amp>& seg) {
   constexpr unsigned T = kTrackTile;
-  ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
+  ZhsPoint const z = zhs_point<kPre>(r, p, l);
   bool staged = z.one;
   if constexpr (sizeof(Amp) == sizeof(float)) {
     // a cut segment is the drain's, as in zhs_lean_differences: a sample's FP32 value
@@ -2169,11 +2169,12 @@ __device__ __noinline__ Counts zhs_drain_lean(const double* __restrict__ tracks,
 // one deferred pair each and evaluate its Fraunhofer number and subdivision
 // exactly; the warp then steps through segment index s = 0, 1, ...: every lane
 // whose pair has a segment s forms its endpoints by the reference's
-// sequential additions, stages it (FP64: exactly; mixed precision: by lean_segment),
-// and the warp deposits the staged samples together.  A segment that cannot be
-// staged is evaluated exactly and deposited on its own lane: in mixed precision the
-// same steps as zhs_drain_lean's, so that a pair's FP32 values are the same bits
-// whether its item runs with checked adds or without.  Every lane of the warp calls it.
+// sequential additions, stages it (FP64: exactly; mixed precision: by the filtered
+// arithmetic), and the warp deposits the staged samples together.  A segment that
+// cannot be staged is evaluated exactly and deposited on its own lane.  In mixed
+// precision and fixed point these are zhs_drain_lean's steps (lean_segment, else
+// zhs_segment), so that a pair's FP32 values are the same bits whether its item runs
+// with checked adds or without.  Every lane of the warp calls it.
 template <bool kFixed, bool kDifferences, class Amp, class Sink>
 __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint64_t begin,
                                          unsigned const* list, unsigned count,
@@ -2185,7 +2186,7 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
   long long segments = 0;
   bool subdivided = false;
   double p1x = 0., p1y = 0., p1z = 0., t1 = 0., rx = 0., ry = 0., rz = 0., rt = 0.;
-  double fraction = 1.;  // mixed precision: of the track, a segment
+  double fraction = 1.;  // mixed precision, fixed point: of the track, a segment
   bool lean = false;     // and whether lean_segment may evaluate it
   if (lane < count) {
     row = begin + list[lane];
@@ -2202,7 +2203,7 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
     rz = step.z;
     rt = step.t;
     segments = static_cast<long long>(d.subtracks) * refinement;
-    if constexpr (sizeof(Amp) == sizeof(float)) {
+    if constexpr (kFixed && sizeof(Amp) == sizeof(float)) {
       fraction = 1. / (d.divisor * static_cast<double>(refinement));
       lean = lean_divisible(t, __ldg(track_ref(tracks, row) + kPack / 2 * kTrackTile).y, segments, l);
     }
@@ -2228,12 +2229,22 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
       t.by = e.y;
       t.bz = f.x;
       t.constant = __ldg(r + kConst / 2 * kTrackTile).y;
-      bool staged;
-      if constexpr (sizeof(Amp) == sizeof(float))
-        staged = lean && lean_segment(r, static_cast<unsigned>(s), subdivided, fraction, p, l, seg);
-      else
-        staged = zhs_stage<Amp>((p1x + p2x) * 0.5, (p1y + p2y) * 0.5, (p1z + p2z) * 0.5, t1, t2,
-                                        (t1 + t2) * 0.5, t, p, o, subdivided, seg);
+      double const mx = (p1x + p2x) * 0.5, my = (p1y + p2y) * 0.5, mz = (p1z + p2z) * 0.5, mt = (t1 + t2) * 0.5;
+      bool staged = false;
+      if constexpr (sizeof(Amp) == sizeof(float)) {
+        if constexpr (kFixed) {
+          staged = lean && lean_segment(r, static_cast<unsigned>(s), subdivided, fraction, p, l, seg);
+        } else {  // the sums' order decides the last bits anyway: at the sequential points
+          SourceTerms const st = source_terms(p, destination_of(o), mz);
+          LeanPoint const m = lean_point(l, mx, my, mz, mt, e.x, e.y, f.x, st.factor, st.n_src);
+          bool cut;
+          staged = zhs_lean(m, (t2 - t1) * l.half_rate, pack_constant(f.y) * l.scale, e.x, e.y, f.x, l, subdivided, seg,
+                            cut) &
+                   ((pack_flags(f.y) & kTrackRegular & l.usable) != 0u) & lean_terms(st);
+        }
+      }
+      if (!staged && !(kFixed && sizeof(Amp) == sizeof(float)))
+        staged = zhs_stage<Amp>(mx, my, mz, t1, t2, mt, t, p, o, subdivided, seg);
       if (!staged) {
         seg.count = 0u;
         seg.flags = 0u;
@@ -2378,15 +2389,15 @@ __device__ __noinline__ Counts zhs_difference_loop(const double* __restrict__ tr
   uint32_t const step = blockDim.x / kTrackTile * (kTrackTile * kTrackColumns);
   for (uint32_t base = 0; base < count; base += blockDim.x, r += step) {
     uint32_t const k = base + threadIdx.x;
-    bool deferred = false;
+    bool deferred = kMayRefine && k < count && p.refinement != 1u;  // refined: the drain divides it
     LeanObserver const l = copy_words(s_lean);
     if constexpr (sizeof(Amp) == sizeof(float)) {
-      if (k < count) {
-        ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
+      if (k < count && !deferred) {
+        ZhsPoint const z = zhs_point<kPre>(r, p, l);
         deferred = !(z.one && zhs_lean_differences(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, win, c));
       }
-    } else if (k < count) {
-      ZhsPoint const z = zhs_point<kPre, kMayRefine>(r, p, l);
+    } else if (k < count && !deferred) {
+      ZhsPoint const z = zhs_point<kPre>(r, p, l);
       deferred = !z.one;
       if (z.one) {
         constexpr unsigned T = kTrackTile;
@@ -2416,7 +2427,7 @@ __device__ __noinline__ Counts zhs_staged_loop(const double* __restrict__ tracks
     StagedSegment<Amp> seg;
     seg.count = 0u;
     seg.flags = 0u;
-    if (k < count) deferred = !zhs_common<kFixed, kPre, true, Amp>(r, p, s_lean, seg);
+    if (k < count) deferred = p.refinement != 1u || !zhs_common<kFixed, kPre, Amp>(r, p, s_lean, seg);
     deposit_staged<kFixed>(staging, seg, s_observer, sink, c);
     push_deferred(deferred, k);
   }
