@@ -1891,17 +1891,19 @@ __global__ void __launch_bounds__(kTileThreads) tiled_kernel(const __grid_consta
 }
 
 // ---------------------------------------------------------------- windowed
-// Threads of a CTA of the one-pass ZHS kernel (floating traces, the
-// no-allocation entry point, launches past the two-pass storage cap, and the
-// third pass of two-pass launches).  Its drain's live state needs more
-// registers than its track loop (168 against 112 in FP32, 135 in FP64), so a
-// CTA sized for the drain runs 12 warps an SM.  Measured on the 1e7 x 160
-// workload in one pass (ms per ZHS launch), FP32: 384 threads 96.8, 512
-// 100.9, 576 97.3, 640 88.3, 768 79.9, 832 82.7, 864 80.6 -- the track loop
-// gains more from the warps than the drain loses to its spills; FP64: 384
-// 117.0, 480 128.5.
+// Threads of a CTA of the ZHS kernels that stage: of one pass (floating traces, the
+// no-allocation entry point, launches past the two-pass storage cap) and of the last
+// of two (items handed back: refined tracks, long traces, items near the fixed-point
+// limit).  Their drain's live state needs more registers than their track loop, which
+// gains from the warps.  us, FP64 at 384 / 480 threads: 262144 x 24 floating 519 / 484,
+// refined twice 1453 / 1242, fixed in 24000 bins 927 / 781; mixed at 768 / 640 / 512:
+// floating 329 / 339 / 343, fixed in 24000 bins 788 / 731 / 696, 60000 x 160 refined
+// twice 3804 / 3416 / 3165.  480 threads' FP64 staging leaves room for 8202 bins; a
+// longer window takes 384.
 constexpr int kZhsThreadsFloat = 768;
-constexpr int kZhsThreadsDouble = 384;
+constexpr int kZhsHandedThreadsFloat = 512;
+constexpr int kZhsThreadsDouble = 480;
+constexpr int kZhsThreadsDoubleLong = 384;
 // Two passes (fixed point): the first, whose track loop is a function of its own,
 // runs larger CTAs.  FP32 1024 threads (1e7 x 160 workload: 23.0 ms, 24.0 at 896),
 // FP64 640.
@@ -1912,15 +1914,28 @@ constexpr int kZhsLoopThreadsDouble = 640;
 template <class Amp, int kPass = 0>
 constexpr int zhs_threads_max() {
   return kPass == 1 ? (sizeof(Amp) == sizeof(float) ? kZhsLoopThreadsFloat : kZhsLoopThreadsDouble)
-                    : (sizeof(Amp) == sizeof(float) ? kZhsThreadsFloat : kZhsThreadsDouble);
+         : sizeof(Amp) == sizeof(double) ? kZhsThreadsDouble
+         : kPass == 3                    ? kZhsHandedThreadsFloat
+                                         : kZhsThreadsFloat;
 }
-// The ZHS block for a team of `threads`: the team when it is smaller than the
-// default team, else the largest block of the amplitude type and pass.
+// Dynamic shared memory of a CTA (227 KB less the static part and a kilobyte's room).
+constexpr size_t kSharedBytes = 227u * 1024u - 1024u;
+// Dynamic shared memory of a launch: the window and, for a ZHS kernel that stages, 32
+// staging slots a warp of its `block` threads.
+template <class Amp>
+constexpr size_t windowed_smem_bytes(uint32_t window, int algorithm, int pass, int block) {
+  return static_cast<size_t>(window) * 3 * sizeof(unsigned long long) +
+         (algorithm == 1 && pass != 1 ? static_cast<size_t>(block) * sizeof(StagedSegment<Amp>) : 0);
+}
+// The ZHS block for a team of `threads` and a window: the team when it is smaller than
+// the default team, else the largest block of the amplitude type and pass whose
+// staging fits beside the window.
 template <class Amp, int kPass = 0>
-constexpr int zhs_block(int threads) {
-  return threads < kWindowThreads
-             ? (threads < zhs_threads_max<Amp, kPass>() ? threads : zhs_threads_max<Amp, kPass>())
-             : zhs_threads_max<Amp, kPass>();
+constexpr int zhs_block(int threads, uint32_t window) {
+  int most = zhs_threads_max<Amp, kPass>();
+  if (windowed_smem_bytes<Amp>(window, 1, kPass, most) > kSharedBytes && most == kZhsThreadsDouble)
+    most = kZhsThreadsDoubleLong;
+  return threads < kWindowThreads && threads < most ? threads : most;
 }
 // CoREAS in mixed precision and fixed point: ms of the 1e7 x 160 workload at 640 /
 // 768 / 896 / 1024 threads 26.4 / 24.3 / 23.9 / 22.5, in ice (5e6 x 64) 5.1 / 4.4 /
@@ -1937,14 +1952,14 @@ template <bool kFixed, class Amp, bool kPre>
 constexpr int coreas_block(int threads) {
   return threads < kWindowThreads ? threads : coreas_threads_max<kFixed, Amp, kPre>();
 }
-// staging slots of the ZHS kernel: 32 per warp of its largest CTA that stages
-// (pass 1 does not)
-template <class Amp>
-constexpr size_t staging_bytes() {
-  return static_cast<size_t>(zhs_threads_max<Amp, 0>()) * sizeof(StagedSegment<Amp>);
-}
-constexpr size_t kStagingBytes =
-    staging_bytes<float>() > staging_bytes<double>() ? staging_bytes<float>() : staging_bytes<double>();
+static_assert(windowed_smem_bytes<double>(kPartialWindowBins, 1, 3, kZhsThreadsDouble) <= kSharedBytes &&
+                  windowed_smem_bytes<float>(kPartialWindowBins, 0, 0, 0) + 2048 <= 196u * 1024u,
+              "the window of longer traces");
+// The staging that every window leaves room for.
+constexpr size_t kStagingBytes = kZhsThreadsFloat * sizeof(StagedSegment<float>) >
+                                         kZhsThreadsDoubleLong * sizeof(StagedSegment<double>)
+                                     ? kZhsThreadsFloat * sizeof(StagedSegment<float>)
+                                     : kZhsThreadsDoubleLong * sizeof(StagedSegment<double>);
 
 __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t n, uint64_t item) {
   uint32_t lo = 0, hi = n;  // last event with first_item <= item
@@ -2768,13 +2783,6 @@ cudaError_t tiled_dispatch(EventPlan const& ev, uint64_t bound, bool coreas, boo
   return cudaGetLastError();
 }
 
-// window | (ZHS, but for pass 1) per-warp staging slots
-template <class Amp>
-size_t windowed_smem_bytes(uint32_t window, int algorithm, int pass) {
-  return static_cast<size_t>(window) * 3 * sizeof(unsigned long long) +
-         (algorithm == 1 && pass != 1 ? staging_bytes<Amp>() : 0);
-}
-
 // Every event of the plan carries precomputed source terms.
 bool plan_precomputed(WorkPlan const& plan) {
   if (plan.event_count == 0) return false;
@@ -2785,12 +2793,13 @@ bool plan_precomputed(WorkPlan const& plan) {
 
 template <bool kFixed, class Amp, int kAlgorithm, bool kPre, int kPass = 0>
 cudaError_t windowed_launch(WorkPlan const& plan, int ctas, int threads, cudaStream_t stream) {
-  size_t const bytes = windowed_smem_bytes<Amp>(plan.window, kAlgorithm, kPass);
+  int const block =
+      kAlgorithm == 1 ? zhs_block<Amp, kPass>(threads, plan.window) : coreas_block<kFixed, Amp, kPre>(threads);
+  size_t const bytes = windowed_smem_bytes<Amp>(plan.window, kAlgorithm, kPass, block);
   cudaError_t err = cudaFuncSetAttribute(windowed_kernel<kFixed, Amp, kAlgorithm, kPre, kPass>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(bytes));
   if (err != cudaSuccess) return err;
-  int const block = kAlgorithm == 1 ? zhs_block<Amp, kPass>(threads) : coreas_block<kFixed, Amp, kPre>(threads);
   windowed_kernel<kFixed, Amp, kAlgorithm, kPre, kPass><<<ctas, block, bytes, stream>>>(plan);
   return cudaGetLastError();
 }
@@ -2835,8 +2844,9 @@ cudaError_t windowed_dispatch(WorkPlan const& plan, int ctas, int threads, cudaS
 template <bool kFixed, class Amp>
 int ctas_per_sm(int window, int threads) {
   int worst = 1 << 30;
+  uint32_t const bins = static_cast<uint32_t>(window);
   auto probe = [&](auto kernel, int block, int algorithm, int pass = 0) {
-    size_t const bytes = windowed_smem_bytes<Amp>(static_cast<uint32_t>(window), algorithm, pass);
+    size_t const bytes = windowed_smem_bytes<Amp>(static_cast<uint32_t>(window), algorithm, pass, block);
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     int blocks = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, bytes) != cudaSuccess)
@@ -2845,13 +2855,13 @@ int ctas_per_sm(int window, int threads) {
   };
   probe(windowed_kernel<kFixed, Amp, 0, false>, coreas_block<kFixed, Amp, false>(threads), 0);
   probe(windowed_kernel<kFixed, Amp, 0, true>, coreas_block<kFixed, Amp, true>(threads), 0);
-  probe(windowed_kernel<kFixed, Amp, 1, false>, zhs_block<Amp>(threads), 1);
-  probe(windowed_kernel<kFixed, Amp, 1, true>, zhs_block<Amp>(threads), 1);
+  probe(windowed_kernel<kFixed, Amp, 1, false>, zhs_block<Amp>(threads, bins), 1);
+  probe(windowed_kernel<kFixed, Amp, 1, true>, zhs_block<Amp>(threads, bins), 1);
   if constexpr (kFixed) {  // the two passes
-    probe(windowed_kernel<true, Amp, 1, false, 1>, zhs_block<Amp, 1>(threads), 1, 1);
-    probe(windowed_kernel<true, Amp, 1, true, 1>, zhs_block<Amp, 1>(threads), 1, 1);
-    probe(windowed_kernel<true, Amp, 1, false, 3>, zhs_block<Amp, 3>(threads), 1, 3);
-    probe(windowed_kernel<true, Amp, 1, true, 3>, zhs_block<Amp, 3>(threads), 1, 3);
+    probe(windowed_kernel<true, Amp, 1, false, 1>, zhs_block<Amp, 1>(threads, bins), 1, 1);
+    probe(windowed_kernel<true, Amp, 1, true, 1>, zhs_block<Amp, 1>(threads, bins), 1, 1);
+    probe(windowed_kernel<true, Amp, 1, false, 3>, zhs_block<Amp, 3>(threads, bins), 1, 3);
+    probe(windowed_kernel<true, Amp, 1, true, 3>, zhs_block<Amp, 3>(threads, bins), 1, 3);
   }
   return worst;
 }

@@ -372,13 +372,13 @@ cudaError_t launch_windowed(WorkPlan const& plan, bool fixed, Precision precisio
 // Largest window (bins) that fits the opt-in shared memory of this device.
 int windowed_max_bins(int device);
 // The window of a launch whose longest trace has `longest` bins, `max_bins` the
-// largest that fits: the whole trace, or a part of it that leaves the kernel inside
-// 196 KB of shared memory (a kilobyte reserved, one for the static part).  The next
-// configuration, 228 KB, halves the L1 cache that the tracks, the table and the
+// largest that fits: the whole trace, or a part of it that leaves the CoREAS kernel
+// inside 196 KB of shared memory and the last ZHS pass room for its FP64 staging.  The
+// next configuration, 228 KB, halves the L1 cache that the tracks, the table and the
 // bins past the window go through: CoREAS of 262144 tracks x 24 antennas x 24000
 // bins ran 617 us with 8362 bins and 372 with 8202 in FP64, 609 and 322 in mixed
 // precision, also where every sample lies past both.
-constexpr uint64_t kPartialWindowBins = (196u * 1024u - 2048u) / (3 * sizeof(unsigned long long));
+constexpr uint64_t kPartialWindowBins = 8192;
 inline uint32_t window_for(uint64_t longest, int max_bins) {
   uint64_t const most = max_bins > 0 ? static_cast<uint64_t>(max_bins) : 0;
   if (longest <= most) return static_cast<uint32_t>(longest > 0 ? longest : 1);
