@@ -29,13 +29,6 @@ namespace c8r {
 namespace {
 
 constexpr std::size_t kDefaultHostBatch = 4096;   // RadioAccumulator.hpp:49
-// Fewer tracks than this run the direct kernel (the reference's threshold is
-// 16384, RadioAccumulator.hpp:101).  The windowed launches cost 45 to 55 us
-// whatever their size, the direct kernel's time is its serial chain of atomics:
-// direct / windowed us at 1, 64, 512, 4096, 16000 FP64 tracks x 16 antennas: 20/55,
-// 33/55, 98/57, 170/67, 242/91, x 160: 20/51, 32/57, 185/82, 339/137, 1029/292;
-// floating traces x 16: 17/24, 25/26, 57/39, 97/59, 147/107.
-constexpr std::size_t kDirectThreshold = 256;
 // Full batches of one pageable host call are ingested as they fill and
 // projected together, at most so many records at a time: a projection costs
 // its launches and a pass over every antenna's window whatever its size.
@@ -490,8 +483,10 @@ class Accumulator {
       begin = timing_event();
       check(cudaEventRecord(begin, stream_), "event");
     }
-    bool const direct = kernel_ == C8R_KERNEL_DIRECT ||
-                        (kernel_ == C8R_KERNEL_AUTO && count < kDirectThreshold);
+    bool const direct =
+        kernel_ == C8R_KERNEL_DIRECT ||
+        (kernel_ == C8R_KERNEL_AUTO && direct_pays(count, observers(), zhs_enabled_, propagation_.refinement, fixed_,
+                                                   precision_ == Precision::kFP64, window_bins_ >= largest_bins_));
     if (study_)
       project_study(count);
     else if (kernel_ == C8R_KERNEL_TILED)

@@ -1895,15 +1895,15 @@ __global__ void __launch_bounds__(kTileThreads) tiled_kernel(const __grid_consta
 // no-allocation entry point, launches past the two-pass storage cap) and of the last
 // of two (items handed back: refined tracks, long traces, items near the fixed-point
 // limit).  Their drain's live state needs more registers than their track loop, which
-// gains from the warps.  us, FP64 at 384 / 480 threads: 262144 x 24 floating 519 / 484,
-// refined twice 1453 / 1242, fixed in 24000 bins 927 / 781; mixed at 768 / 640 / 512:
-// floating 329 / 339 / 343, fixed in 24000 bins 788 / 731 / 696, 60000 x 160 refined
-// twice 3804 / 3416 / 3165.  480 threads' FP64 staging leaves room for 8202 bins; a
-// longer window takes 384.
+// gains from the warps.  us, FP64 at 384 / 480 threads: 262144 x 24 floating 519 / 478,
+// refined twice 1453 / 1259, handed back in 24000 bins 927 / 776 but 60000 x 16 refined
+// fourfold 586 / 745 (CoREAS included); mixed at 768 / 640 / 512: floating 329 / 339 /
+// 343, handed back in 24000 bins 788 / 731 / 696, 60000 x 160 refined twice 3804 / 3416 /
+// 3165.  480 threads' FP64 staging leaves room for 8202 bins; a longer window takes 384.
 constexpr int kZhsThreadsFloat = 768;
 constexpr int kZhsHandedThreadsFloat = 512;
 constexpr int kZhsThreadsDouble = 480;
-constexpr int kZhsThreadsDoubleLong = 384;
+constexpr int kZhsHandedThreadsDouble = 384;
 // Two passes (fixed point): the first, whose track loop is a function of its own,
 // runs larger CTAs.  FP32 1024 threads (1e7 x 160 workload: 23.0 ms, 24.0 at 896),
 // FP64 640.
@@ -1914,9 +1914,8 @@ constexpr int kZhsLoopThreadsDouble = 640;
 template <class Amp, int kPass = 0>
 constexpr int zhs_threads_max() {
   return kPass == 1 ? (sizeof(Amp) == sizeof(float) ? kZhsLoopThreadsFloat : kZhsLoopThreadsDouble)
-         : sizeof(Amp) == sizeof(double) ? kZhsThreadsDouble
-         : kPass == 3                    ? kZhsHandedThreadsFloat
-                                         : kZhsThreadsFloat;
+         : kPass == 3 ? (sizeof(Amp) == sizeof(float) ? kZhsHandedThreadsFloat : kZhsHandedThreadsDouble)
+                      : (sizeof(Amp) == sizeof(float) ? kZhsThreadsFloat : kZhsThreadsDouble);
 }
 // Dynamic shared memory of a CTA (227 KB less the static part and a kilobyte's room).
 constexpr size_t kSharedBytes = 227u * 1024u - 1024u;
@@ -1934,7 +1933,7 @@ template <class Amp, int kPass = 0>
 constexpr int zhs_block(int threads, uint32_t window) {
   int most = zhs_threads_max<Amp, kPass>();
   if (windowed_smem_bytes<Amp>(window, 1, kPass, most) > kSharedBytes && most == kZhsThreadsDouble)
-    most = kZhsThreadsDoubleLong;
+    most = kZhsHandedThreadsDouble;
   return threads < kWindowThreads && threads < most ? threads : most;
 }
 // CoREAS in mixed precision and fixed point: ms of the 1e7 x 160 workload at 640 /
@@ -1952,14 +1951,14 @@ template <bool kFixed, class Amp, bool kPre>
 constexpr int coreas_block(int threads) {
   return threads < kWindowThreads ? threads : coreas_threads_max<kFixed, Amp, kPre>();
 }
-static_assert(windowed_smem_bytes<double>(kPartialWindowBins, 1, 3, kZhsThreadsDouble) <= kSharedBytes &&
+static_assert(windowed_smem_bytes<double>(kPartialWindowBins, 1, 0, kZhsThreadsDouble) <= kSharedBytes &&
                   windowed_smem_bytes<float>(kPartialWindowBins, 0, 0, 0) + 2048 <= 196u * 1024u,
               "the window of longer traces");
 // The staging that every window leaves room for.
 constexpr size_t kStagingBytes = kZhsThreadsFloat * sizeof(StagedSegment<float>) >
-                                         kZhsThreadsDoubleLong * sizeof(StagedSegment<double>)
+                                         kZhsHandedThreadsDouble * sizeof(StagedSegment<double>)
                                      ? kZhsThreadsFloat * sizeof(StagedSegment<float>)
-                                     : kZhsThreadsDoubleLong * sizeof(StagedSegment<double>);
+                                     : kZhsHandedThreadsDouble * sizeof(StagedSegment<double>);
 
 __device__ __forceinline__ uint32_t find_event(EventPlan const* events, uint32_t n, uint64_t item) {
   uint32_t lo = 0, hi = n;  // last event with first_item <= item

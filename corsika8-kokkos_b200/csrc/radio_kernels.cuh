@@ -331,6 +331,31 @@ inline uint64_t batch_chunk(uint64_t count, uint64_t per, uint64_t ctas, double 
   return track_capacity((count + chunks - 1) / chunks);
 }
 
+// Whether `count` tracks at `observers` antennas go to the direct kernel where the
+// choice is automatic; `whole`: the longest trace fits a window.  The windowed launches
+// cost 25 us an algorithm whatever their size, the direct kernel waits for its serial
+// chain of atomics (longest for ZHS's many samples at few antennas).  Timed on 7560
+// launches of 64 to 16000 tracks at 1 to 300 antennas; of the two kernels the rule
+// takes the slower one by 0.2 to 3% in the mean of each class below.  us, direct /
+// windowed, 8192 bins x 160 antennas unless given:
+//   below 256 tracks       direct; 128 tracks FP64 210 / 67, but 33 / 57 where few samples meet the trace
+//   both algorithms        windowed; FP64 256 tracks 202 / 89, 4096 393 / 153
+//   CoREAS alone           FP64 512 tracks 30 / 47, 16000 219 / 155; floating 600 bins 4096 tracks 44 / 55
+//   refined (not mixed in fixed point in one window: there the drain is windowed's
+//                          fastest)   FP64 fourfold 16 antennas 4096 tracks 241 / 149,
+//                          160 antennas 4096 tracks 470 / 719
+// From 16384 tracks (the reference's threshold, RadioAccumulator.hpp:101) windowed.
+inline bool direct_pays(uint64_t count, uint64_t observers, bool zhs, uint32_t refinement, bool fixed, bool fp64,
+                        bool whole) {
+  constexpr uint64_t kFewest = 256, kMost = 16384;
+  if (count < kFewest || count >= kMost) return count < kFewest;
+  double const n = static_cast<double>(count), antennas = static_cast<double>(observers);
+  if (!zhs) return !fixed || n * n * antennas < 26000. * 26000.;
+  if (refinement <= 1 || (fixed && !fp64 && whole)) return false;
+  double const refined = antennas * refinement * refinement;
+  return n * refined * refined >= 40000. * 40000.;
+}
+
 enum class Precision : int { kFP64 = 0, kMixed = 1 };
 
 // Record ingest: LeptonTransportRecord AoS -> compacted SoA kinematics
@@ -373,7 +398,7 @@ cudaError_t launch_windowed(WorkPlan const& plan, bool fixed, Precision precisio
 int windowed_max_bins(int device);
 // The window of a launch whose longest trace has `longest` bins, `max_bins` the
 // largest that fits: the whole trace, or a part of it that leaves the CoREAS kernel
-// inside 196 KB of shared memory and the last ZHS pass room for its FP64 staging.  The
+// inside 196 KB of shared memory and the ZHS kernels room for their FP64 staging.  The
 // next configuration, 228 KB, halves the L1 cache that the tracks, the table and the
 // bins past the window go through: CoREAS of 262144 tracks x 24 antennas x 24000
 // bins ran 617 us with 8362 bins and 372 with 8202 in FP64, 609 and 322 in mixed

@@ -192,6 +192,45 @@ void check_batch(std::vector<std::pair<uint64_t, uint64_t>> const& events, doubl
          static_cast<uint64_t>(planned), static_cast<uint64_t>(work));
 }
 
+// The automatic kernel at measured points (us of the direct and of the windowed kernel):
+// the choice is within a quarter of the faster one, and never changes from 16384 tracks on.
+void check_kernel_choice() {
+  struct Point {
+    uint64_t tracks, antennas;
+    bool zhs;
+    uint32_t refinement;
+    bool fixed, fp64, whole;
+    double direct, windowed;
+  };
+  Point const points[] = {
+      {4096, 16, true, 1, true, true, true, 175., 78.},
+      {256, 160, true, 1, true, true, true, 221., 88.},
+      {1024, 300, true, 1, true, false, true, 105., 71.},
+      {512, 48, true, 1, false, true, true, 98., 57.},
+      {512, 160, false, 1, true, true, true, 29., 45.},
+      {16000, 160, false, 1, true, true, true, 227., 156.},
+      {4096, 48, false, 1, false, false, true, 34., 36.},
+      {4096, 16, true, 4, true, true, true, 259., 161.},
+      {4096, 160, true, 4, true, true, true, 472., 781.},
+      {16000, 300, true, 16, true, true, true, 3594., 6497.},
+      {8192, 160, true, 16, true, false, true, 1753., 1706.},
+      {8192, 160, true, 16, true, false, false, 1854., 4120.},
+      {4096, 160, true, 3, false, true, true, 228., 412.},
+      {2048, 16, true, 2, false, false, true, 75., 60.},
+      {16000, 5, true, 3, true, true, false, 278., 156.},
+  };
+  for (Point const& p : points) {
+    double const chosen =
+        direct_pays(p.tracks, p.antennas, p.zhs, p.refinement, p.fixed, p.fp64, p.whole) ? p.direct : p.windowed;
+    expect(chosen <= 1.25 * (p.direct < p.windowed ? p.direct : p.windowed), "the faster kernel", p.tracks, p.antennas);
+  }
+  for (uint64_t tracks : {16384, 100000, 10000000})
+    for (uint32_t refinement : {1, 4, 64})
+      for (int flags = 0; flags < 16; ++flags)
+        expect(!direct_pays(tracks, 300, flags & 1, refinement, flags & 2, flags & 4, flags & 8), "windowed", tracks);
+  expect(direct_pays(1, 1, true, 1, true, true, true) && direct_pays(255, 300, false, 1, false, false, false), "direct");
+}
+
 // The window is the whole trace while it fits; of a longer one the part that leaves
 // the kernel inside the shared memory that does not cut into the L1 cache.
 void check_windows() {
@@ -209,6 +248,7 @@ void check_windows() {
 }  // namespace
 
 int main() {
+  check_kernel_choice();
   check_windows();
   for (double item : {item_cost(900, true, 1), item_cost(8192, false, 1)}) {
     check_batch(std::vector<std::pair<uint64_t, uint64_t>>(64, {1500, 16}), item, 148);
