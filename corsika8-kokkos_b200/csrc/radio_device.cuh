@@ -294,11 +294,13 @@ __host__ __device__ __forceinline__ void divide3(double& x, double& y, double& z
 // point: the reference's (1 + (I_src - I_dst) / height) * dist / c with the
 // parenthesised factor taken from `st` (the same IEEE value), or n dist / c.
 // kTime = false skips the refractive index and travel time (the Fraunhofer
-// midpoint uses only k and distance).  kDivide takes the four quotients by
-// divisions: the plain shapes, which wait for their atomics and not for the FP64
-// pipe, lose more to the written-out form's range checks and registers than they
-// save (3e5 x 160, direct shape, written-out / divisions: FP64 25.6 / 23.8 ms, mixed
-// 24.8 / 23.2, floating 16.6 / 15.7; the windowed FP64 CoREAS kernel 4.6 / 5.0 at 1e6).
+// midpoint uses only k and distance).  kDivide takes the three quotients by the
+// distance as divisions: the plain shapes, which wait for their atomics and not for
+// the FP64 pipe, lose more to the written-out form's range checks and registers than
+// they save (3e5 x 160, direct shape, written-out / divisions: FP64 25.6 / 24.6 ms,
+// mixed 24.8 / 23.2, floating 16.7 / 15.6; the travel time divided too, 200 mixed
+// tracks x 16 antennas refined fourfold take 152 us for 131; the windowed FP64 CoREAS
+// kernel 4.6 written out, 5.0 divided, at 1e6 x 160).
 template <bool kTime, bool kDivide = false>
 __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCache const& o,
                                                double sx, double sy, double sz) {
@@ -317,7 +319,7 @@ __device__ __forceinline__ Path propagate_with(SourceTerms const& st, ObserverCa
   }
   r.dist = dist;
   if (!kTime) return r;
-  r.time = kDivide ? st.factor * dist / kSpeedOfLight : over_light_speed(st.factor * dist);
+  r.time = over_light_speed(st.factor * dist);
   r.n_src = st.n_src;
   r.n_dst = st.n_dst;
   return r;
