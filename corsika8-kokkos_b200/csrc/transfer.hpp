@@ -75,8 +75,9 @@ class SlotRing {
   // Fills the segments in order: issue(segment, offset, bytes, slot) queues on
   // `stream` the work that writes bytes [offset, offset + bytes) of a segment
   // into `slot`, emit(segment, offset, bytes, slot) moves them on to the segment's
-  // destination.  Returns once everything has been copied out.  The copying
-  // threads work on the calling thread's device.
+  // destination.  Returns once everything has been copied out.  Only the calling
+  // thread calls the CUDA runtime: a new thread's device is 0, whatever the owner's,
+  // and its first call costs as much as the copy of a megabyte.
   template <class Issue, class Emit>
   cudaError_t run(std::vector<Segment> const& segments, cudaStream_t stream, Issue issue, Emit emit) {
     std::vector<Piece> pieces;
@@ -93,52 +94,35 @@ class SlotRing {
       return err != cudaSuccess ? err : cudaEventRecord(filled_[i % depth], stream);
     };
     auto empty = [&](std::size_t i) {
-      cudaError_t const err = cudaEventSynchronize(filled_[i % depth]);
-      if (err != cudaSuccess) return err;
       Piece const& p = pieces[i];
       emit(p.segment, p.offset, p.bytes, static_cast<void const*>(slots_[i % depth]));
-      return cudaSuccess;
     };
     unsigned const cores = std::max(1u, std::thread::hardware_concurrency() / 2);
-    int device = 0;
-    if (cudaError_t const err = cudaGetDevice(&device)) return err;
     Shared shared(n);
     Workers workers(shared);
     if (total >= kThreadedBytes && depth > 1) {
       std::size_t const wanted = std::min<std::size_t>({kWorkers, cores, total / kBytesPerWorker});
       for (std::size_t k = 0; k < wanted; ++k)
-        if (!workers.start([&] {
-              if (cudaError_t const err = cudaSetDevice(device))  // a new thread's is device 0
-                shared.error.store(err);
-              else
-                drain(shared, n, empty);
-            }))
-          break;
+        if (!workers.start([&] { drain(shared, n, empty); })) break;
     }
-    for (std::size_t i = 0; i < n; ++i) {
-      if (i >= depth) {  // the slot's last piece has to be out
+    for (std::size_t issued = 0, filled = 0; filled < n;) {
+      // a slot takes its next piece when its last one is out
+      if (issued < n && (issued < depth || shared.done[issued - depth].load(std::memory_order_acquire))) {
+        if (cudaError_t const err = fill(issued)) return err;
+        ++issued;
+      } else if (filled < issued) {
+        if (cudaError_t const err = cudaEventSynchronize(filled_[filled % depth])) return err;
         if (workers.none()) {
-          if (cudaError_t const err = empty(i - depth)) return err;
-        } else {
-          while (!shared.done[i - depth].load(std::memory_order_acquire)) {
-            if (int const err = shared.error.load()) return static_cast<cudaError_t>(err);
-            std::this_thread::yield();
-          }
+          empty(filled);
+          shared.done[filled].store(true, std::memory_order_relaxed);
         }
+        shared.filled.store(++filled, std::memory_order_release);
+      } else {
+        std::this_thread::yield();
       }
-      if (cudaError_t const err = fill(i)) {
-        shared.error.store(err);
-        return err;
-      }
-      shared.issued.store(i + 1, std::memory_order_release);
-    }
-    if (workers.none()) {
-      for (std::size_t i = n > depth ? n - depth : 0; i < n; ++i)
-        if (cudaError_t const err = empty(i)) return err;
-      return cudaSuccess;
     }
     workers.join();
-    return static_cast<cudaError_t>(shared.error.load());
+    return cudaSuccess;
   }
   // The same, the bytes copied as they are.
   template <class Issue>
@@ -156,18 +140,16 @@ class SlotRing {
     explicit Shared(std::size_t n) : done(new std::atomic<bool>[n ? n : 1]) {
       for (std::size_t i = 0; i < n; ++i) done[i].store(false);
     }
-    std::atomic<std::size_t> issued{0}, next{0};
-    std::atomic<int> error{0};
+    std::atomic<std::size_t> filled{0}, next{0};
+    std::atomic<bool> stop{false};
     std::unique_ptr<std::atomic<bool>[]> done;
   };
-  // Joins its threads on every way out; what has not been issued by then never is.
+  // Joins its threads on every way out; what has not been filled by then never is.
   class Workers {
    public:
     explicit Workers(Shared& shared) : shared_(shared) {}
     ~Workers() {
-      if (threads_.empty()) return;
-      int none = 0;
-      shared_.error.compare_exchange_strong(none, static_cast<int>(cudaErrorUnknown));
+      shared_.stop.store(true);
       join();
     }
     template <class F>
@@ -194,14 +176,11 @@ class SlotRing {
     for (;;) {
       std::size_t const i = shared.next.fetch_add(1);
       if (i >= n) return;
-      while (shared.issued.load(std::memory_order_acquire) <= i) {
-        if (shared.error.load()) return;
+      while (shared.filled.load(std::memory_order_acquire) <= i) {
+        if (shared.stop.load()) return;
         std::this_thread::yield();
       }
-      if (cudaError_t const err = empty(i)) {
-        shared.error.store(err);
-        return;
-      }
+      empty(i);
       shared.done[i].store(true, std::memory_order_release);
     }
   }

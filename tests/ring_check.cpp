@@ -17,7 +17,7 @@ namespace {
 
 constexpr int kOwner = 3;  // the device of the accumulator or server
 thread_local int t_device = 0;
-std::atomic<int> wrong_device{0}, worker_waits{0}, runtime_copies{0};
+std::atomic<int> wrong_device{0}, event_waits{0}, runtime_copies{0};
 std::mutex mu;
 struct Copy {
   void* to;
@@ -60,7 +60,7 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) {
 }
 cudaError_t cudaEventSynchronize(cudaEvent_t) {
   note_device();
-  ++worker_waits;
+  ++event_waits;
   finish_queued();
   return cudaSuccess;
 }
@@ -99,8 +99,9 @@ std::vector<unsigned char> pattern(std::size_t n, unsigned seed) {
   return out;
 }
 
-// Copies of several sizes reach their destinations whole, and every runtime call,
-// the copying threads' among them, is made on the owner's device.
+// Copies of several sizes reach their destinations whole, and every runtime call is
+// made on the owner's device (the copying threads, whose device is 0, make none).
+// A copy that fails on its way ends the call with its error.
 void check_copies(SlotRing& ring) {
   for (std::size_t bytes : {std::size_t{1}, SlotRing::kSlotBytes, SlotRing::kSlotBytes + 1, std::size_t{23} << 20}) {
     std::vector<unsigned char> const a = pattern(bytes, 1), b = pattern(bytes / 2 + 1, 2);
@@ -113,7 +114,19 @@ void check_copies(SlotRing& ring) {
     expect(err == cudaSuccess, "copy returns success");
     expect(x == a && y == b, "copies arrive whole");
   }
-  expect(worker_waits > 0, "the copies waited for their slots");
+  for (std::size_t bad : {0, 3, 20, 45}) {
+    std::vector<unsigned char> const a = pattern(std::size_t{23} << 20, 5);
+    std::vector<unsigned char> x(a.size());
+    std::size_t pieces = 0;
+    cudaError_t const err = ring.run({{x.data(), x.size()}}, nullptr,
+                                     [&](std::size_t, std::size_t at, std::size_t n, void* slot) {
+                                       if (pieces++ == bad) return cudaErrorUnknown;
+                                       return cudaMemcpyAsync(slot, a.data() + at, n, cudaMemcpyDeviceToHost, nullptr);
+                                     });
+    expect(err == cudaErrorUnknown, "a failed copy ends the call");
+    finish_queued();
+  }
+  expect(event_waits > 0, "the copies waited for their slots");
   expect(wrong_device == 0, "every call on the owner's device");
 }
 
