@@ -60,6 +60,14 @@ constexpr std::size_t kGranule = 256;
 constexpr std::size_t kFetchBytes = 4 * SlotRing::kSlotBytes;
 std::size_t round_up(std::size_t bytes) { return (bytes + kGranule - 1) / kGranule * kGranule; }
 
+// Integers to fields: value x factor.  By AVX-512 where the host has it (8 conversions
+// an instruction for 1): the threads that empty the copy slots then run at the speed
+// of the copy.  Both round each conversion and product to nearest.
+__attribute__((target_clones("arch=skylake-avx512", "default"))) void decode_values(long long const* in, double* out,
+                                                                                  std::size_t n, double factor) {
+  for (std::size_t i = 0; i < n; ++i) out[i] = static_cast<double>(in[i]) * factor;
+}
+
 // downloadSet's decode (RadioAccumulator.inl:849-898), value x factor per observer,
 // for runs of an algorithm's values (rows [X | Y | Z] of all its bins).
 class TraceDecoder {
@@ -79,8 +87,7 @@ class TraceDecoder {
       std::size_t const bin = first % total;
       std::size_t const o = static_cast<std::size_t>(std::upper_bound(ends_.begin(), ends_.end(), bin) - ends_.begin());
       std::size_t const n = std::min(count, ends_[o] - bin);
-      double const factor = factors_[o];
-      for (std::size_t i = 0; i < n; ++i) out[i] = static_cast<double>(in[i]) * factor;
+      decode_values(in, out, n, factors_[o]);
       in += n;
       out += n;
       first += n;
