@@ -2,7 +2,8 @@
 their bins sit on an edge: traces of one, two and odd numbers of bins, cut
 through the pulse at either end, samples at whole and half bins, and antennas
 inside a track's reach.  FP64 traces equal the oracle's bit for bit; mixed
-precision's sample counts per bin and counters equal the oracle's."""
+precision's sample counts per bin and counters equal the oracle's, and its
+amplitudes are the oracle's to FP32."""
 import numpy as np
 import pytest
 
@@ -24,14 +25,31 @@ def project(pkg, config, records, tuning=None):
     return got
 
 
-def check(pkg, oracle, showers, workload, records, tuning=None, **extra):
-    for precision, counting in ((0, False), (0, True), (1, True)):
+# Mixed against FP64 traces, relative to a trace's 2-norm and to its peak: a sample's
+# amplitude takes a dozen FP32 roundings (2^-24 each: 7e-7 in all) and, where the Doppler
+# factor is as small as the filtered paths take it (1e-6), 2^-43 of that factor, 1.2e-7;
+# samples of opposite sign cancel in a bin.  Measured up to 1.1e-6 and 1.7e-6.  Not
+# where a track's two CoREAS samples share their bin and all but cancel
+# (amplitudes=False): what is left of 1e11 units is then their rounding.
+MIXED_BOUND = 5e-6
+
+
+def check(pkg, oracle, showers, workload, records, tuning=None, amplitudes=True, **extra):
+    for precision, counting in ((0, False), (0, True), (1, True)) + (((1, False),) if amplitudes else ()):
         config = showers.make_config(workload, precision=precision, kernel=2, count_samples=counting, **extra)
         got = project(pkg, config, records, tuning)
         want = oracle.restatement().project(showers.make_config(workload, count_samples=counting, **extra), records,
                                             threads=16)
         for k in range(2):
-            assert np.array_equal(got[k], want[k]), (precision, counting, k, np.count_nonzero(got[k] != want[k]))
+            if precision == 0 or counting:
+                assert np.array_equal(got[k], want[k]), (precision, counting, k, np.count_nonzero(got[k] != want[k]))
+                continue
+            ends = np.cumsum(workload["observers"]["number_of_bins"].astype(int))
+            for g, w in zip(np.split(got[k], ends[:-1], axis=1), np.split(want[k], ends[:-1], axis=1)):
+                error, w = g.astype(np.float64) - w, w.astype(np.float64)
+                units = len(records)  # a sample's conversion rounds by half a unit
+                assert np.linalg.norm(error) <= MIXED_BOUND * np.linalg.norm(w) + units, k
+                assert np.abs(error).max() <= MIXED_BOUND * np.abs(w).max() + units, k
         for key in COUNTERS:
             assert got[2][key] == want[2][key], (precision, counting, key)
 
@@ -98,7 +116,7 @@ def test_detection_time_just_below_the_first_half_bin(pkg, oracle, showers, edge
     observers["sample_rate_hz"] = 1.0
     observers["number_of_bins"] = 8
     wl = dict(observers=observers, homogeneous=1.0, table=None)
-    check(pkg, oracle, showers, wl, showers.to_records(seg))
+    check(pkg, oracle, showers, wl, showers.to_records(seg), amplitudes=False)
 
 
 def test_divided_tracks_above_the_table_beside_the_antenna_height(pkg, oracle, showers):
@@ -122,7 +140,7 @@ def test_divided_tracks_above_the_table_beside_the_antenna_height(pkg, oracle, s
                pid=np.full(count, 11, np.int32), energy_gev=np.full(count, 1e-3),
                direction=np.tile([0.0, 1.0, 0.0], (count, 1)), weight=np.ones(count))
     wl = dict(observers=observers, homogeneous=0.0, table=table)
-    check(pkg, oracle, showers, wl, showers.to_records(seg))
+    check(pkg, oracle, showers, wl, showers.to_records(seg), amplitudes=False)
 
 
 @pytest.mark.parametrize("name,refinement,shift", [("ice_c2", 1, 0.0), ("ice_c2", 3, 0.0), ("plain_c0", 1, 52e-9), ("plain_c0", 2, 0.0)])
@@ -154,6 +172,16 @@ def test_items_run_again_give_the_same_bits(pkg, oracle, showers, name, refineme
     assert got[0][3] > 0
     for k in range(2):
         assert np.array_equal(got[0][k], got[1][k]), (k, np.count_nonzero(got[0][k] != got[1][k]))
+
+
+@pytest.mark.parametrize("refinement", [1, 3, 64])
+def test_divided_tracks_inside_the_cone(pkg, oracle, showers, refinement):
+    """Tracks in ice seen from inside and outside the Cherenkov cone (Doppler factors
+    of both signs), divided for the antennas, then refined as well."""
+    wl, gen, _ = showers.workload_config("ice_c2", bins=1000)
+    records = showers.ice_records(4_001, seed=5, **gen)
+    wl["observers"] = wl["observers"][::5].copy()
+    check(pkg, oracle, showers, wl, records, zhs_subtrack_refinement=refinement)
 
 
 @pytest.mark.parametrize("scale", [1e-6, 1e3, 1e6])
