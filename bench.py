@@ -318,7 +318,7 @@ def run_ours(args):
     if not args.no_variants and world == 1 and precision != 0:
         accuracy = trace_accuracy(pkg, showers, wl, device_records, n, precision, kernel, stream)
 
-    # roofline of the dominant kernel (the windowed ZHS launch, two thirds of a
+    # roofline of the dominant kernel (the windowed ZHS launch, half of a
     # step) and of the CoREAS launch, from events on their launch stream
     per = {k: counters[k] / args.steps for k in ("zhs_subtracks", "coreas_contributions",
                                                   "zhs_contributions")}
@@ -358,7 +358,7 @@ def run_ours(args):
 
     roofline = roof(zhs_flops, zhs_ms, "zhs")
     roofline.update({
-        "kernel": "windowed_kernel<fixed,float,ZHS> (dominant, 62% of the step)",
+        "kernel": "windowed_kernel<fixed,float,ZHS> (dominant, half of the step)",
         "peak_source": "FP64 FMA stream measured in this run on this GPU (c8r_probe_peaks); "
                        "of measured",
         "traffic_source": ("DRAM bytes read + written per track from an ncu capture of the same "

@@ -222,7 +222,7 @@ class Accumulator {
     counters_.allocate(1);
     slot_.allocate(1);
     next_item_.allocate(2);  // one work counter per algorithm
-    reruns_.allocate(2);  // items re-run with checked adds, items handed to a drain pass
+    reruns_.allocate(2);  // items re-run with checked adds, items handed back
     staging_.allocate(checked_mul(host_batch_, sizeof(c8r_lepton_transport_record)));
     for (auto& h : host_) {
       h.allocate(std::max(checked_mul(host_batch_, kUsedBytes), kHostHalfBytes));
@@ -1460,7 +1460,7 @@ extern "C" {
 
 // Part of the tuning cache's key: raised whenever the kernels' launch shapes
 // change, so that a tile tuned for earlier kernels is not applied to these.
-const char* c8r_version(void) { return "c8radio-b200 1.2 (sm_100a)"; }
+const char* c8r_version(void) { return "c8radio-b200 1.3 (sm_100a)"; }
 
 const char* c8r_last_error(const c8r_accumulator* handle) {
   if (handle == nullptr) return g_last_error.c_str();

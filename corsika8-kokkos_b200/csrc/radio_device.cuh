@@ -358,8 +358,8 @@ __device__ __forceinline__ Path propagate(Propagation const& p, ObserverCache co
 //   32u (|t| + |t0| + time) fs of the reference's (t + time - t0) fs; where x
 //   falls on the trace (fewer than 2^26 bins) that is below 32u 2^27 = 2^-21,
 //   and the ZHS term n w (t - t_mid) adds at most 2^-43 2^20; kBinGuard =
-//   2^-19 covers both, and the 2^-20 of a divided track's segments
-//   (zhs_drain_lean).  Where |x| is larger the error grows like 2^-46 |x|, so
+//   2^-19 covers both, the 2^-20 of a divided track's segments
+//   (lean_divisible) and the 2^-22 of their source terms (terms_decided).  Where |x| is larger the error grows like 2^-46 |x|, so
 //   such an x is off the trace in the reference as well.
 constexpr double kDopplerGuard = 0x1p-43;
 constexpr double kBinGuard = 0x1p-19;
@@ -386,7 +386,8 @@ __device__ __forceinline__ bool regular_track(Track const& t, double duration, T
 }
 
 // 1/sqrt(s2) from the hardware's approximate reciprocal square root (about 20
-// bits) and one third-order step: with r = 1 - s2 y0^2 and |r| <= 2^-17
+// bits) and one third-order step (the binomial series of (1 - r)^(-1/2), Householder's
+// iteration of order 2): with r = 1 - s2 y0^2 and |r| <= 2^-17
 // (checked, so the seed's accuracy is not relied on), y0 (1 + r/2 + 3 r^2/8)
 // is within (5/16) 2^-51 + 3u < 4u of it.  False when s2 lies outside
 // [2^-100, 2^100] or is not a number.

@@ -14,6 +14,7 @@
 //                    trace as an int64 window in shared memory, deposits with
 //                    shared atomics and flushes non-zero bins with checked
 //                    global atomics
+//   tiled_kernel     the reference's large-batch tile shape
 //   decode_kernel    int64 fixed point -> V/m (V s/m) (RadioAccumulator.inl:849-898)
 #include "radio_kernels.cuh"
 
@@ -529,7 +530,7 @@ __device__ __forceinline__ void lean_add(WindowSink& sink, LeanObserver const& l
   long long const x = __float2ll_rn(fmaf(vx, a, l.bias)), y = __float2ll_rn(fmaf(vy, a, l.bias)),
                   z = __float2ll_rn(fmaf(vz, a, l.bias));
   if (kUnchecked) {
-    // through a generic pointer (see deposit_unchecked)
+    // through a generic pointer (see deposit_differences)
     unsigned long long* w = sink.win + 3u * static_cast<unsigned>(bin);
     asm volatile("" : "+l"(w));
     atomicAdd(w, static_cast<unsigned long long>(x));
@@ -2290,7 +2291,7 @@ __device__ __noinline__ Counts zhs_drain(const double* __restrict__ tracks, uint
 template <bool kFixed, class Amp, bool kPre, class Sink>
 __device__ __noinline__ Counts coreas_drain_pair(const double* __restrict__ tracks, uint64_t row,
                                                  unsigned hint, Propagation const& p,
-                                                 ObserverCache const& o, LeanObserver const& l, Sink sink) {
+                                                 ObserverCache const& o, Sink sink) {
   Counts c;
   double2 const* r = track_ref(tracks, row);
   if constexpr (kFixed && sizeof(Amp) == sizeof(float)) {
@@ -2652,7 +2653,7 @@ __global__ void __launch_bounds__(kAlgorithm == 1 ? zhs_threads_max<Amp, kPass>(
         } else if (lane < left) {
           unsigned const entry = s_deferred_list[from + lane];
           d = coreas_drain_pair<kFixed, Amp, kPre>(ev.tracks, begin + (entry & kDeferredOffsetMask),
-                                                   entry >> kDeferredHintShift, p, s_observer, s_lean,
+                                                   entry >> kDeferredHintShift, p, s_observer,
                                                    make_sink(unchecked));
         }
         add_counts(c, d);

@@ -65,7 +65,7 @@ struct EventPlan {
 
 // Source terms written at ingest: when every observer of an event shares one
 // destination row (always in a homogeneous medium), each track record gets
-// the propagation terms of its start, end and two midpoints for that row,
+// the propagation terms of its start, end and midpoint for that row,
 // and the windowed kernels read them instead of looking them up per pair.
 struct IngestTerms {
   int32_t enabled;
