@@ -1475,10 +1475,11 @@ __device__ __forceinline__ bool zhs_common(double2 const* __restrict__ r, Propag
   ZhsPoint const z = zhs_point<kPre>(r, p, l);
   bool staged = z.one;
   if constexpr (sizeof(Amp) == sizeof(float)) {
-    // a cut segment is the drain's, as in zhs_lean_differences: a sample's FP32 value
-    // is then the same bits whether its item runs with checked adds or without
+    // in fixed point a cut segment is the drain's, as in zhs_lean_differences: a sample's
+    // FP32 value is then the same bits whether its item runs with checked adds or without
     bool cut;
-    staged = zhs_lean(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, false, seg, cut) & staged & !cut;
+    staged = zhs_lean(z.m, z.half_bins, z.constant, z.bx, z.by, z.bz, l, false, seg, cut) & staged &
+             !(kFixed && cut);
   } else if (staged) {
     double2 const cm = __ldg(r + 9 * T), cn = __ldg(r + 10 * T), ct = __ldg(r + 3 * T);
     Track t;
@@ -2032,12 +2033,16 @@ __device__ __noinline__ Counts zhs_exact_segments(const double* __restrict__ tra
 // reference adds up s segments.  With u = 2^-53, the two differ by less than (s + 4) u
 // of the largest coordinate and of the largest time, so the detection time by (s + 4) u
 // (4 sqrt(3) |coordinate| fs / c + |time| fs), which has to stay below 2^-20 bins, a part
-// of kBinGuard (s up to 60 at the filtered paths' limits, 300 in a shower of 100 km).
+// of kBinGuard (s up to 60 at the filtered paths' limits, 300 in a shower of 100 km);
+// at most kLeanSegments whatever the magnitudes, so that a warp's segments count in 32
+// bits.
+constexpr long long kLeanSegments = 4096;
 __device__ __forceinline__ bool lean_divisible(Track const& t, double pack, long long segments, LeanObserver const& l) {
   double const furthest = fmax(fmax(fmax(fabs(t.sx), fabs(t.sy)), fmax(fabs(t.sz), fabs(t.ex))),
                                fmax(fabs(t.ey), fabs(t.ez)));
   double const bins = 7. * furthest * l.rate_over_c + fmax(fabs(t.ts), fabs(t.te)) * l.rate;
-  return (static_cast<double>(segments + 4) * bins <= 0x1p33) & ((pack_flags(pack) & kTrackRegular & l.usable) != 0u);
+  return (segments <= kLeanSegments) & (static_cast<double>(segments + 4) * bins <= 0x1p33) &
+         ((pack_flags(pack) & kTrackRegular & l.usable) != 0u);
 }
 // Whether the source terms at height z decide what the terms at the reference's
 // own height, within `z_error` m of z, would.  In the table they are the same when
