@@ -418,12 +418,10 @@ def test_window_cap_on_adds_per_thread(pkg, oracle, showers, torch_cuda):
 
 @pytest.mark.parametrize("precision", [0, 1])
 def test_two_pass_handback_when_the_lists_fill(pkg, oracle, showers, torch_cuda, precision):
-    """Fixed-point ZHS runs the track loop and the drain as two passes.  With
-    subtrack refinement 2 every ZHS pair is deferred, and with 256-track work
-    items each CTA's first-pass list (one item's length here) is full after
-    its first item: every later item is handed back unflushed and projected
-    in full by the second pass.  The traces equal the oracle's (FP64: bit for
-    bit; mixed: counters equal, traces within 1e-4), so no pair is lost or
+    """Fixed-point ZHS runs in two passes.  With subtrack refinement 2 every pair goes
+    to the drain and every 256-track work item is handed back unflushed by the first
+    pass and projected in full by the second.  The traces equal the oracle's (FP64:
+    bit for bit; mixed: counters equal, traces within 1e-4), so no pair is lost or
     deposited twice."""
     wl, records = _workload_records(showers, "plain_c0", 20_000, seed=41)
     config = showers.make_config(wl, precision=precision, kernel=2)

@@ -2,9 +2,11 @@
 from append_work cover every track once in items no longer than the deferred
 entries' offset field, and the deferred-list storage of one- and two-pass
 launches (deferred_words / attach_deferred) keeps the first pass's lists, the
-second pass's lists, the item states and the counter disjoint and inside the
+second pass's lists, the item states and their counters disjoint and inside the
 allocation, with two passes only for fixed-point ZHS launches within the
-storage cap.  tests/plan_check.cu, compiled for the host with nvcc."""
+storage cap; the automatic chunks are near the shortest plan, batched events are cut
+for their share, windows and the automatic kernel follow their rules.
+tests/plan_check.cu, compiled for the host with nvcc."""
 import subprocess
 from pathlib import Path
 
