@@ -578,8 +578,8 @@ __device__ __forceinline__ bool lean_samples(WindowSink& sink, LeanObserver cons
 // FP32 cross product the pair takes 344 instead of 621 warp instructions:
 // 1e7 x 160 x 8192 CoREAS 41.6 -> 22.5 ms, 5e6 x 64 in ice 9.0 -> 3.9 ms, and the
 // traces' relative error falls from 6e-7 to 1.1e-7.  What bounds it now is the
-// shared-memory pipe (74% busy, mostly the six 64-bit atomics) beside 58% of the
-// issue slots.
+// L1 data pipe (79% busy: track columns, observer constants and, two fifths of it, the
+// six 64-bit shared atomics) beside 61% of the issue slots.
 template <bool kPre, bool kUnchecked>
 __device__ __forceinline__ int coreas_lean(double2 const* __restrict__ r, Propagation const& p,
                                            LeanObserver const& l, WindowSink& sink, Tally& c) {
